@@ -368,7 +368,8 @@ __device__ inline int refined_rank(const DevTree& T, int level, uint64_t cell) {
 // cells two neighbouring cubes share meet in L2).
 template <int NK>
 __global__ void __launch_bounds__(INC_T, 2) k_incoming_cube(DevTree T, const int* __restrict__ cubes, int ncubes,
-                                                             int slots, double* part) {
+                                                             int slots, double* part,
+                                                             const int* __restrict__ touched) {
   constexpr int D = 2 * NK + 1, H = (NK + 1) * D * D;
   extern __shared__ double2 w[];                             // [INC_CELLS][INC_KT]
   int* s_row = reinterpret_cast<int*>(w + INC_CELLS * INC_KT);  // outgoing row of each cell, -1: absent or empty
@@ -382,6 +383,9 @@ __global__ void __launch_bounds__(INC_T, 2) k_incoming_cube(DevTree T, const int
   const uint64_t gp = T.node_prefix[G];
   const int O[3] = {4 * int(compact3(gp)), 4 * int(compact3(gp >> 1)), 4 * int(compact3(gp >> 2))};
   const int base = T.pw_base;
+  __shared__ int s_any;
+  if (threadIdx.x == 0) s_any = 0;
+  __syncthreads();
   if (threadIdx.x < INC_CELLS) {
     const int t = threadIdx.x;
     const int c[3] = {t % 6 - 1, (t / 6) % 6 - 1, t / 36 - 1};
@@ -403,8 +407,16 @@ __global__ void __launch_bounds__(INC_T, 2) k_incoming_cube(DevTree T, const int
     s_wrap[t] = static_cast<unsigned char>(wrap);
     if (c[0] >= 0 && c[0] < 4 && c[1] >= 0 && c[1] < 4 && c[2] >= 0 && c[2] < 4)
       s_recv[c[0] + 4 * c[1] + 16 * c[2]] = (node >= 0 && T.node_child0[node] >= 0) ? node - base : -1;
+    if (touched && node >= 0 && touched[node - base] != 0) s_any = 1;
   }
   __syncthreads();
+  // after a sequence of moves: nothing to do when no outgoing row of the cube changed
+  if (touched && !s_any) return;
+  if (touched && threadIdx.x < 32 && slot == 0) {
+    int n = (s_recv[threadIdx.x] >= 0) + (s_recv[threadIdx.x + 32] >= 0);
+    for (int o = 16; o > 0; o >>= 1) n += __shfl_down_sync(0xffffffffu, n, o);
+    if (threadIdx.x == 0) atomicAdd(&T.work[1], 32ull * H * (unsigned long long)n);
+  }
   const int two_l = (l & 1) ? 2 : 1;
   const int kk = threadIdx.x % INC_KT;
   const int line = threadIdx.x / INC_KT, ry = line & 3, rz = line >> 2;
@@ -489,22 +501,24 @@ __global__ void __launch_bounds__(INC_T, 2) k_incoming_cube(DevTree T, const int
 }
 
 template <int NK>
-void launch_incoming_nk(const DevTree& D, const int* cubes, int ncubes, int slots, double* part, cudaStream_t st) {
+void launch_incoming_nk(const DevTree& D, const int* cubes, int ncubes, int slots, double* part, const int* touched,
+                        cudaStream_t st) {
   raise_smem_limit(reinterpret_cast<const void*>(k_incoming_cube<NK>), INC_SMEM);
-  k_incoming_cube<NK><<<unsigned(slots * ncubes), INC_T, INC_SMEM, st>>>(D, cubes, ncubes, slots, part);
+  k_incoming_cube<NK><<<unsigned(slots * ncubes), INC_T, INC_SMEM, st>>>(D, cubes, ncubes, slots, part, touched);
   PDMK_LAUNCH_CHECK();
 }
 
-void launch_incoming(const DevTree& D, const int* cubes, int ncubes, int slots, double* part, cudaStream_t st) {
+void launch_incoming(const DevTree& D, const int* cubes, int ncubes, int slots, double* part, const int* touched,
+                     cudaStream_t st) {
   switch (D.n_diff) {
-    case 4: launch_incoming_nk<4>(D, cubes, ncubes, slots, part, st); break;
-    case 6: launch_incoming_nk<6>(D, cubes, ncubes, slots, part, st); break;
-    case 8: launch_incoming_nk<8>(D, cubes, ncubes, slots, part, st); break;
-    case 12: launch_incoming_nk<12>(D, cubes, ncubes, slots, part, st); break;
-    case 13: launch_incoming_nk<13>(D, cubes, ncubes, slots, part, st); break;
-    case 17: launch_incoming_nk<17>(D, cubes, ncubes, slots, part, st); break;
-    case 19: launch_incoming_nk<19>(D, cubes, ncubes, slots, part, st); break;
-    case 26: launch_incoming_nk<26>(D, cubes, ncubes, slots, part, st); break;
+    case 4: launch_incoming_nk<4>(D, cubes, ncubes, slots, part, touched, st); break;
+    case 6: launch_incoming_nk<6>(D, cubes, ncubes, slots, part, touched, st); break;
+    case 8: launch_incoming_nk<8>(D, cubes, ncubes, slots, part, touched, st); break;
+    case 12: launch_incoming_nk<12>(D, cubes, ncubes, slots, part, touched, st); break;
+    case 13: launch_incoming_nk<13>(D, cubes, ncubes, slots, part, touched, st); break;
+    case 17: launch_incoming_nk<17>(D, cubes, ncubes, slots, part, touched, st); break;
+    case 19: launch_incoming_nk<19>(D, cubes, ncubes, slots, part, touched, st); break;
+    case 26: launch_incoming_nk<26>(D, cubes, ncubes, slots, part, touched, st); break;
     default: throw std::invalid_argument("incoming pass: unsupported mode count");
   }
 }
@@ -1313,10 +1327,8 @@ void DmkTree::run_incoming(bool write_inc) {
   if (write_inc) {
     // about inc_waves resident waves of blocks (two per SM), each walking a
     // strided set of tiles
-    const int kt = (D.H + INC_KT - 1) / INC_KT;
-    const int nc = std::max(n_cubes_, 1);
-    const int slots = std::max(1, std::min(kt, (tune_.inc_waves * 2 * 148 + nc - 1) / nc));
-    if (n_cubes_ > 0) launch_incoming(D, d_cubes_, n_cubes_, slots, part, st_);
+    const int slots = inc_slots();
+    if (n_cubes_ > 0) launch_incoming(D, d_cubes_, n_cubes_, slots, part, nullptr, st_);
     k_diff_finish_cube<<<1, 1024, 0, st_>>>(D, d_cubes_, n_cubes_, slots, part, d_nonleaf_, n_nonleaf_, q2, d_Cl_,
                                             d_Sl_, d_scalars_ + 1);
     PDMK_LAUNCH_CHECK();
@@ -1328,9 +1340,22 @@ void DmkTree::run_incoming(bool write_inc) {
   }
 }
 
+int DmkTree::inc_slots() const {
+  const int kt = (dev_.H + INC_KT - 1) / INC_KT;
+  const int nc = std::max(n_cubes_, 1);
+  return std::max(1, std::min(kt, (tune_.inc_waves * 2 * 148 + nc - 1) / nc));
+}
+
+// The incoming rows next to outgoing rows that changed (touched[expansion
+// node] != 0), after a sequence of moves. The partial energies go unused.
+void DmkTree::launch_incoming_touched(const int* touched) {
+  if (n_cubes_ > 0) launch_incoming(dev_, d_cubes_, n_cubes_, inc_slots(), dev_.partials, touched, st_);
+}
+
 void DmkTree::form_incoming_pw() {
   run_incoming(true);
   diff_cached_ = true;
+  inc_formed_ = true;
 }
 
 void DmkTree::launch_window_energy() {

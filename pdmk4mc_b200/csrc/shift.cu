@@ -81,6 +81,7 @@ struct Header {
   int depth_o, depth_t;
   int path_o[MAXLV], path_t[MAXLV];
   int Xo[MAXLV][3], Xt[MAXLV][3];  // integer box coordinates along each path
+  double d2;                       // k_mc_long: squared length of the displacement
 };
 
 // Tables of one point on its path for levels 2..lmax, one entry per thread
@@ -478,6 +479,338 @@ __device__ int build_receivers(const DevTree& T, const Header& h, Receiver* out)
   const int total = wsum[31];
   __syncthreads();
   return total;
+}
+
+// ---------------------------------------------------------------------------
+// Deferred expansion updates of a Metropolis sequence. An accepted move would
+// read and write about 40 expansion rows (own outgoing and incoming rows and
+// the colleagues' incoming rows of every path level: 39 MB at N = 1e5, 9
+// digits, 10 us from L2). A long sequence keeps its accepted moves in a list
+// instead and leaves the rows as they were at its start; the incoming row of a
+// box B of level l then lacks, for each listed point a (weight w_a = +q at the
+// target, -q at the origin) whose level-l box is B or one of its colleagues,
+//   w_a conj(exp(-i k.(x_a - s_a L)))       (s_a: the image of a next to B),
+// and the difference sum of a candidate point x of charge q in B lacks
+//   c_l q w_a sum_k D(k) cos(k.d),  d = x - x_a + s_a L.
+// D depends on |k| only, so the sum over the stored half grid folds onto the
+// octant m = |k| / dk >= 0 per axis:
+//   sum_{mz,my,mx >= 0} Dw[mz][my][mx] cos(mz tz) cos(my ty) cos(mx tx),  t = dk_l d,
+// with Dw the table times the number of (kx, ky) signs: (n + 1)^3 multiply-adds
+// for a pair of points, where an update row takes (n + 1) (2 n + 1)^2 complex
+// read-modify-writes. When the sequence ends the rows are brought up to date
+// once for all its moves (k_flush_outgoing, then the incoming pass).
+template <int NP>
+struct ModesOf {  // modes per half axis of the digits setting whose residual polynomial has NP terms
+  static constexpr int ND = NP == 7 ? 6 : NP == 13 ? 12 : NP == 19 ? 19 : 26;
+  static constexpr int NW = NP == 7 ? 4 : NP == 13 ? 8 : NP == 19 ? 13 : 17;
+  static constexpr int ROWS = (ND + 1) * (ND + 1);  // (mz, my) rows of the folded table
+  static constexpr int MT = (ROWS + 7) / 8;         // row tiles of the FP64 tensor product
+  static constexpr int KS = (ND + 1 + 3) / 4;       // its steps of four mx
+  // doubles from one mx to the next: a multiple of 8 rows, 4 modulo 16, so that
+  // the eight rows and four mx of an operand load fall on different banks
+  static constexpr int STR = 8 * MT + (20 - 8 * MT % 16) % 16;
+  static constexpr int OCT = 4 * KS * STR;          // the folded table, zero past its rows and modes
+  static constexpr int CT = 3 * 4 * KS * 4;         // cosines of one unit
+};
+
+// an accepted move: point 0 its target (+), point 1 its origin (-); X the box
+// coordinates at level u, the deepest expansion level on the point's path
+struct Pending {
+  double x[2][3];
+  double q;
+  int X[2][3];
+  int u[2];
+};
+
+__device__ inline void fill_pending(const DevTree& T, const Header& h, Pending& e) {
+  const int ut = min(h.depth_t - 1, T.pw_hi), uo = min(h.depth_o - 1, T.pw_hi);
+  e.q = h.q;
+  e.u[0] = ut;
+  e.u[1] = uo;
+  for (int a = 0; a < 3; ++a) {
+    e.x[0][a] = h.xt[a];
+    e.x[1][a] = h.xo[a];
+    e.X[0][a] = ut >= 0 ? h.Xt[ut][a] : 0;
+    e.X[1][a] = uo >= 0 ? h.Xo[uo][a] : 0;
+  }
+}
+
+// the box offset c - a of two box coordinates at a level of `side` boxes, and
+// the image s in {-1, 0, 1} the offset was wrapped by; |offset| > 1: no neighbours
+__device__ inline int box_offset(int c, int a, int side, int& s) {
+  const int d = c - a;
+  s = d == side - 1 ? 1 : (d == 1 - side ? -1 : 0);
+  return d - s * side;
+}
+
+// the folded difference table: element (mx, my, mz) at mx STR + mz (n + 1) + my
+__global__ void k_fold_d2(DevTree T, int stride, int total, double* out) {
+  const int n = T.n_diff, n1 = n + 1, d = 2 * n + 1;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= total) return;
+  const int mx = i / stride, r = i % stride, mz = r / n1, my = r % n1;
+  double v = 0.0;
+  if (mx < n1 && mz < n1) v = T.D2[((n - mz) * d + n + my) * d + n + mx] * (mx ? 2.0 : 1.0) * (my ? 2.0 : 1.0);  // kz < 0 entries carry the factor 2
+  out[i] = v;
+}
+
+// is a listed move's target or origin a neighbour (or the box itself) of the
+// candidate's target (pc = 0) or origin (pc = 1) box at level l?
+__device__ inline bool pair_near(const Header& h, const Pending& e, int l, int pc, int pp) {
+  const int top = (pc == 0 ? h.depth_t : h.depth_o) - 2;
+  if (l > top || l > e.u[pp]) return false;
+  const int* Xc = pc == 0 ? h.Xt[l] : h.Xo[l];
+  bool ok = true;
+  for (int a = 0; a < 3; ++a) {
+    int s;
+    ok = ok && abs(box_offset(Xc[a], e.X[pp][a] >> (e.u[pp] - l), 1 << l, s)) <= 1;
+  }
+  return ok;
+}
+
+// Which (listed move, level) units interact with the candidate, compacted in
+// order by the calling warp into act[] as 256 entry + 16 flags + level (flags:
+// bit 2 pc + pp for a pair of neighbouring points), the number returned to all
+// its lanes.
+__device__ __noinline__ int near_units(const Header& h, const Pending* list, int n_list, int* act) {
+  const int lane = threadIdx.x & 31;
+  const int top = max(h.depth_t, h.depth_o) - 2, nlev = top - 1;  // levels 2 .. top
+  int n = 0;
+  if (nlev > 0)
+    for (int b = 0; b < n_list * nlev; b += 32) {
+      const int i = b + lane;
+      int flags = 0;
+      const int en = i / nlev, l = 2 + i % nlev;
+      if (i < n_list * nlev) {
+        const Pending& e = list[en];
+#pragma unroll
+        for (int p = 0; p < 4; ++p) flags |= int(pair_near(h, e, l, p >> 1, p & 1)) << p;
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, flags != 0);
+      if (flags) act[n + __popc(m & ((1u << lane) - 1u))] = 256 * en + 16 * flags + l;
+      n += __popc(m);
+    }
+  return n;
+}
+
+// Cosines of one unit by one warp, ct[axis][m][pair] = cos(m t): pair 2 pc + pp
+// is the candidate's target (pc = 0) or origin against the listed move's target
+// (pp = 0) or origin; the z axis carries the pair's sign, zero for a pair that
+// does not interact. Lanes 0..23 take (pair, axis, parity of m): exp(i t), then
+// steps of exp(2 i t).
+template <int ND>
+__device__ __noinline__ void unit_cosines(double L, double dk, const Header& h, const Pending& e, int unit, double* ct) {
+  constexpr int N1 = ND + 1, KP = 4 * ((N1 + 3) / 4);
+  const int lane = threadIdx.x & 31, l = unit & 15;
+  if (lane < 4 * (KP - N1)) ct[N1 * 4 + lane] = 0.0;  // the x axis past its last mode
+  if (lane < 24) {
+    const int pair = lane / 6, axis = (lane >> 1) % 3, odd = lane & 1;
+    const int pc = pair >> 1, pp = pair & 1;
+    const bool near = (unit >> (4 + pair)) & 1;
+    double sgn = 1.0, th = 0.0;
+    if (axis == 2) sgn = near ? (pc == pp ? 1.0 : -1.0) : 0.0;
+    if (near) {
+      const int* Xc = pc == 0 ? h.Xt[l] : h.Xo[l];
+      int s;
+      box_offset(Xc[axis], e.X[pp][axis] >> (e.u[pp] - l), 1 << l, s);
+      th = dk * ((pc == 0 ? h.xt[axis] : h.xo[axis]) - e.x[pp][axis] - s * L);
+    }
+    double sn, cs;
+    sincos(th, &sn, &cs);
+    const double2 z1 = make_double2(cs, sn), st = cmul(z1, z1);
+    double2 v = odd ? make_double2(cs * sgn, sn * sgn) : make_double2(sgn, 0.0);
+    double* dst = ct + axis * KP * 4 + pair;
+    for (int m = odd; m < N1; m += 2) {
+      dst[m * 4] = v.x;
+      v = cmul(v, st);
+    }
+  }
+}
+
+// This lane's part of the pair sums of two units (their cosines side by side at
+// ct; `two` false: the second is absent), the units' factors w0 and w1 applied.
+// The inner sum over mx is a product of the folded table (rows (mz, my)) with
+// eight columns of cosines, done on the FP64 tensor pipe (mma m8n8k4): the FMA
+// pipe runs at the same rate, but there each table value and each cosine had
+// to reach every lane's registers (4 wavefronts for a 16-byte broadcast), and
+// shared memory held a unit at 2 290 cycles of an SM; its floor is 500. The
+// calling warp takes row tiles t0, t0 + step, ...
+template <int ND>
+__device__ __forceinline__ double unit_pair_rows(const double* __restrict__ oct, const double* __restrict__ ct, bool two,
+                                                 double w0, double w1, int t0, int step) {
+  using MO = ModesOf<ND == 6 ? 7 : ND == 12 ? 13 : ND == 19 ? 19 : 25>;
+  constexpr int N1 = ND + 1, KP = 4 * MO::KS;
+  const int lane = threadIdx.x & 31, q4 = lane & 3, q8 = lane >> 2;
+  double b[MO::KS];
+#pragma unroll
+  for (int k = 0; k < MO::KS; ++k) b[k] = (q8 < 4 || two) ? ct[(q8 >> 2) * MO::CT + (4 * k + q4) * 4 + (q8 & 3)] : 0.0;
+  const int u = q4 >> 1;  // the unit of this lane's two result columns
+  const double* cy = ct + u * MO::CT + KP * 4 + 2 * (q4 & 1);
+  const double* cz = cy + KP * 4;
+  const bool act = u == 0 || two;
+  double out = 0.0;
+#pragma unroll 2
+  for (int t = t0; t < MO::MT; t += step) {
+    const double* ap = oct + q4 * MO::STR + 8 * t + q8;
+    double c0 = 0.0, c1 = 0.0;
+#pragma unroll
+    for (int k = 0; k < MO::KS; ++k)
+      asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+          : "+d"(c0), "+d"(c1)
+          : "d"(ap[4 * k * MO::STR]), "d"(b[k]));
+    const int r = 8 * t + q8;
+    if (act && r < MO::ROWS) {
+      const int mz = r / N1, my = r % N1;
+      const double2 y = *reinterpret_cast<const double2*>(cy + my * 4), z = *reinterpret_cast<const double2*>(cz + mz * 4);
+      out = fma(c0 * y.x, z.x, out);
+      out = fma(c1 * y.y, z.y, out);
+    }
+  }
+  return out * (u ? w1 : w0);
+}
+
+// This thread's part of the difference sums of both paths (energy_shift.cpp:
+// 92-140), modes threadIdx.x, threadIdx.x + T, ... of every level. What bounds it
+// is the rows' way from L2: a box that both paths share is read once (most
+// trial moves stay in their box), and ILP modes are loaded before the first is
+// used.
+template <int ND, int T, int ILP>
+__device__ double diff_sum(const DevTree& tr, const Header& h, const Tables& oo, const Tables& to, int lo_max, int lt_max,
+                           const double* c_level) {
+  constexpr int D = 2 * ND + 1, H = (ND + 1) * D * D;
+  double e = 0;
+  for (int l = 2; l <= max(lo_max, lt_max); ++l) {
+    const bool has_o = l <= lo_max, has_t = l <= lt_max;
+    const bool same = has_o && has_t && h.path_o[l] == h.path_t[l];
+    const double2* ro = has_o ? tr.inc + size_t(h.path_o[l] - tr.pw_base) * H : nullptr;
+    const double2* rt = has_t && !same ? tr.inc + size_t(h.path_t[l] - tr.pw_base) * H : nullptr;
+    double s = 0;
+    for (int k0 = threadIdx.x; k0 < H; k0 += T * ILP) {
+      double2 co[ILP], cn[ILP];
+      double dv[ILP];
+#pragma unroll
+      for (int j = 0; j < ILP; ++j) {
+        const int k = k0 + j * T;
+        dv[j] = k < H ? tr.D2[k] : 0.0;
+        if (k < H && ro) co[j] = ro[k];
+        if (k < H && rt) cn[j] = rt[k];
+      }
+#pragma unroll
+      for (int j = 0; j < ILP; ++j) {
+        const int k = k0 + j * T;
+        if (k >= H) break;
+        const int ix = k % D, iy = (k / D) % D, iz = k / (D * D);
+        double v = 0;
+        if (has_o) {
+          const double2 o = cmul(oo.lev[l][2][iz], cmul(oo.lev[l][1][iy], oo.lev[l][0][ix]));
+          v -= o.x * co[j].x - o.y * co[j].y - (o.x * o.x + o.y * o.y);
+        }
+        if (has_t) {
+          const double2 c = same ? co[j] : cn[j];
+          const double2 t = cmul(to.lev[l][2][iz], cmul(to.lev[l][1][iy], to.lev[l][0][ix]));
+          v += t.x * c.x - t.y * c.y;
+        }
+        s += v * dv[j];
+      }
+    }
+    e += s * c_level[l];
+  }
+  return e;
+}
+
+// Outgoing rows at the end of a sequence: out_B += sum of the listed points
+// whose path passes through B. Blocks (node, part of the row); a node no move
+// touched returns at once. Points are taken 8 at a time in list order: their
+// phase tables go to shared memory (one sincos per entry, as build_tables),
+// then each thread adds them to its modes. FP64-bound: 10 operations per point
+// and mode.
+constexpr int FO_T = 256, FO_PTS = 8;
+
+template <int ND>
+__global__ void __launch_bounds__(FO_T) k_flush_outgoing(DevTree T, const Pending* __restrict__ list,
+                                                         const int* __restrict__ n_list, const int* __restrict__ touched,
+                                                         int parts2) {
+  constexpr int D = 2 * ND + 1, H = (ND + 1) * D * D, TAB = 3 * D;
+  __shared__ double2 tab[FO_PTS][TAB];
+  __shared__ int sel[FO_PTS];
+  __shared__ int s_n, s_next;
+  // level-2 nodes in parts2 parts, the others whole
+  const int n2 = T.level_start[3] - T.level_start[2];
+  int node = T.pw_base, part = 0, parts = 1;
+  if (int(blockIdx.x) < n2 * parts2) {
+    node += blockIdx.x / parts2;
+    part = blockIdx.x % parts2;
+    parts = parts2;
+  } else {
+    node += n2 + int(blockIdx.x) - n2 * parts2;
+  }
+  if (touched[node - T.pw_base] == 0) return;
+  const int l = T.node_level[node];
+  const uint64_t pf = T.node_prefix[node];
+  const int X[3] = {int(compact3(pf)), int(compact3(pf >> 1)), int(compact3(pf >> 2))};
+  const int n = *n_list;
+  const int k0 = int(long(H) * part / parts), k1 = int(long(H) * (part + 1) / parts);
+  double2* row = T.out + size_t(node - T.pw_base) * H;
+  if (threadIdx.x == 0 && part == 0) atomicAdd(&T.work[1], 32ull * H);
+  int at = 0;  // points are 2 n: (move, target / origin)
+  while (at < 2 * n) {
+    // warp 0 collects the next points of this node, in list order
+    if (threadIdx.x < 32) {
+      int cnt = 0;
+      int b = at;
+      for (; b < 2 * n && cnt < FO_PTS; b += 32) {
+        const int i = b + threadIdx.x;
+        bool in = false;
+        if (i < 2 * n) {
+          const Pending& e = list[i >> 1];
+          const int p = i & 1, u = e.u[p];
+          in = u >= l && (e.X[p][0] >> (u - l)) == X[0] && (e.X[p][1] >> (u - l)) == X[1] &&
+               (e.X[p][2] >> (u - l)) == X[2];
+        }
+        unsigned m = __ballot_sync(0xffffffffu, in);
+        const int room = FO_PTS - cnt;
+        const int rank = __popc(m & ((1u << threadIdx.x) - 1u));
+        if (in && rank < room) sel[cnt + rank] = i;
+        if (__popc(m) > room) {  // full: the scan goes on after the last point taken
+          int last = 0;
+          for (int k = 0; k < room; ++k) {
+            last = __ffs(m) - 1;
+            m &= m - 1;
+          }
+          cnt = FO_PTS;
+          b = b + last + 1 - 32;
+        } else {
+          cnt += __popc(m);
+        }
+      }
+      if (threadIdx.x == 0) {
+        s_n = cnt;
+        s_next = b;
+      }
+    }
+    __syncthreads();
+    const int cnt = s_n;
+    at = s_next;
+    for (int t = threadIdx.x; t < cnt * TAB; t += FO_T) {
+      const int c = t / TAB, r = t % TAB, axis = r / D, m = r % D - ND;
+      const Pending& e = list[sel[c] >> 1];
+      const int p = sel[c] & 1;
+      const double th = level_dk(T, l) * (e.x[p][axis] - center_of(T.L, l, X[axis]));
+      double sn, cs;
+      sincos(-double(m) * th, &sn, &cs);
+      const double sc = axis == 2 ? (p == 0 ? e.q : -e.q) : 1.0;
+      tab[c][r] = cmul(make_double2(cs * sc, sn * sc), root6(-(2 * X[axis] + 1) * m));
+    }
+    __syncthreads();
+    if (cnt > 0)
+      for (int k = k0 + threadIdx.x; k < k1; k += FO_T) {
+        const int ix = k % D, iy = (k / D) % D, iz = k / (D * D);
+        double2 v = row[k];
+        for (int c = 0; c < cnt; ++c) v = cadd(v, cmul(tab[c][2 * D + iz], cmul(tab[c][D + iy], tab[c][ix])));
+        row[k] = v;
+      }
+    __syncthreads();
+  }
 }
 
 struct ShiftArgs {
@@ -1291,27 +1624,744 @@ __global__ void __launch_bounds__(MC_T, 1) k_mc(DevTree T, McArgs a) {
 }
 
 // ---------------------------------------------------------------------------
+// Long Metropolis sequences. As k_mc, one cooperative launch with the whole
+// move on every SM, and with the row updates deferred (see Pending), which
+// leaves the chain of one move as the cost: k_mc spent 4.3 us in the resolve,
+// 1.0-1.7 in the tables, 1.0 in the source lists, 2.1 in the decision and up
+// to 2.6 waiting for the previous commit (N = 1e5, clock stamps). Here
+//   - the warps of a block work side by side: difference modes, window modes,
+//     near field, and a helper that resolves the next move (each block has a
+//     fixed share of the modes, so a thread keeps its root coefficients and
+//     table values in registers);
+//   - a move's header, phase tables and source lists are made during the move
+//     before it, the tables and lists while the block waits for the others'
+//     sums; positions come from pos4, an array by particle that a move's commit
+//     updates, so no slot is read and a particle swapped to another slot does
+//     not matter. Only a particle moved twice in a row is resolved again;
+//   - the blocks exchange one double each in a 16-byte packet {sum, epoch,
+//     pool fill} that every block polls: arrival and data in one round trip;
+//   - a commit writes the slots of two leaves, so the next move waits for it
+//     only if one of them is among its sources (the exchange orders it for
+//     every later move).
+constexpr int MCL_T = 512, MCL_W = MCL_T / 32;
+constexpr int MCL_UNITS = 16;   // pair units whose cosines are held at a time
+constexpr int MCL_LEVB = 3;     // levels whose rows one thread loads together
+constexpr int MCL_POLL = 5;     // packets a lane polls together
+
+struct SrcList {
+  int beg[36], end[36], leaf[36], lvl[36], cnt[36], pre[37];  // leaf: the node id of a leaf source, else -1; lvl -1: absent
+  unsigned long long pfx[36];
+  double off[36][3];
+};
+
+struct McLongArgs {
+  const int* idx;
+  const double* disp;
+  const double* u;
+  double beta;
+  int n_moves;
+  double* dE_out;
+  int* acc_out;
+  double c_window;
+  unsigned long long* packets;  // [2][G][2], double-buffered by move parity, epochs cleared at launch
+  unsigned int* committed;      // epoch of the last committed move
+  double4* pos4;                // position and charge by particle, for the particles of this launch
+  long long spin_limit;
+  Pending* list;
+  int* n_list;
+  int* touched;
+  const double* oct;
+  int per_block;
+};
+
+template <int NP>
+constexpr size_t mcl_bytes(int per_block) {
+  using M = ModesOf<NP>;
+  // the folded table in shared memory where it leaves room for deep trees' phase tables (n = 26: read through L1)
+  return (M::ND <= 19 ? size_t(M::OCT) * 8 : 0) + size_t(MCL_UNITS) * M::CT * 8 + sizeof(Pending) * per_block +
+         sizeof(int) * (MAXLV * per_block + 8);
+}
+
+__device__ inline void packet_store(unsigned long long* p, double v, unsigned epoch, unsigned extra) {
+  const unsigned long long lo = (unsigned long long)__double_as_longlong(v);
+  const unsigned long long hi = (unsigned long long)epoch | ((unsigned long long)extra << 32);
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}\n" ::"l"(p),
+               "l"(lo), "l"(hi)
+               : "memory");
+}
+__device__ inline void packet_load(const unsigned long long* p, double& v, unsigned& epoch, unsigned& extra) {
+  unsigned long long lo, hi;
+  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}\n"
+               : "=l"(lo), "=l"(hi)
+               : "l"(p)
+               : "memory");
+  v = __longlong_as_double((long long)lo);
+  epoch = unsigned(hi);
+  extra = unsigned(hi >> 32);
+}
+
+// positions and charges of the particles a launch will move
+__global__ void k_gather_moves(DevTree T, const int* __restrict__ idx, int n, double4* pos4) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= n) return;
+  const int i = idx[m], s = T.orig_slot[i], p = s - T.n_slots;
+  pos4[i] = p < 0 ? make_double4(T.sx[s], T.sy[s], T.sz[s], T.sq[s]) : make_double4(T.px[p], T.py[p], T.pz[p], T.pq[p]);
+}
+
+// resolve() for one warp from a known position, the three bitmap words of a
+// lane's level loaded together (bm, wp: the levels' bitmap and prefix pointers
+// in shared memory)
+__device__ __noinline__ void resolve_warp(const DevTree& T, int i, double4 at, double d0, double d1, double d2, Header& h,
+                                          const uint32_t* const* bm, const int* const* wp) {
+  const int lane = threadIdx.x & 31;
+  const double L = T.L;
+  const double xo[3] = {at.x, at.y, at.z};
+  const double xt[3] = {wrap_mod(xo[0] + d0, L), wrap_mod(xo[1] + d1, L), wrap_mod(xo[2] + d2, L)};
+  const int half = lane >> 4, l = lane & 15;
+  const double* p = half == 0 ? xt : xo;
+  const uint32_t g[3] = {grid_coord(p[0], L), grid_coord(p[1], L), grid_coord(p[2], L)};
+  const uint64_t key = morton3(g[0], g[1], g[2]);
+  const bool lv = l < T.max_depth;
+  const uint64_t cell = l == 0 || !lv ? 0 : key >> (3 * (KEY_BITS - l));
+  uint32_t w0 = 0, w1 = 0;
+  int pr = 0;
+  if (lv && l >= 2) {
+    w0 = bm[l - 1][cell >> 8];
+    pr = wp[l - 1][cell >> 8];
+  }
+  if (lv && l <= T.maxref) w1 = bm[l][cell >> 5];
+  int node = -1;
+  bool is_leaf = false;
+  const unsigned c5 = unsigned(cell >> 3) & 31u;
+  if (lv && (l <= 1 || ((w0 >> c5) & 1u))) {
+    node = l == 0 ? 0 : (l == 1 ? 1 + int(cell) : T.level_start_d[l] + 8 * (pr + __popc(w0 & ((1u << c5) - 1u))) + int(cell & 7));
+    is_leaf = !(l <= T.maxref && ((w1 >> (cell & 31)) & 1u));
+  }
+  const unsigned leaves = (__ballot_sync(0xffffffffu, is_leaf) >> (16 * half)) & 0xffffu;
+  const int leaf_level = __ffs(leaves) - 1;
+  if (l <= leaf_level) {
+    int* path = half == 0 ? h.path_t : h.path_o;
+    int(*X)[3] = half == 0 ? h.Xt : h.Xo;
+    path[l] = node;
+    for (int a = 0; a < 3; ++a) X[l][a] = int(g[a] >> (KEY_BITS - l));
+  }
+  if (lane == 0) {
+    h.i_orig = i;
+    h.q = at.w;
+    for (int a = 0; a < 3; ++a) {
+      h.xo[a] = xo[a];
+      h.xt[a] = xt[a];
+    }
+    h.d2 = d0 * d0 + d1 * d1 + d2 * d2;
+    h.depth_t = leaf_level + 1;
+  }
+  if (lane == 16) h.depth_o = leaf_level + 1;
+  __syncwarp();
+}
+
+// res_meta without the leaf's current count
+__device__ __noinline__ void source_static(const DevTree& T, int leaf, int l, const int* Xl, int src, SrcList& M) {
+  const double b = level_box(T, l);
+  int j = -1;
+  if (src == 0) j = leaf;
+  else if (src <= 27) j = (src - 1 == 13) ? -1 : T.col27[size_t(leaf) * 27 + (src - 1)];
+  else j = T.coarse8[size_t(leaf) * 8 + (src - 28)];
+  int beg = 0, end = 0, lj = -1, lf = -1;
+  unsigned long long pj = 0;
+  double off[3] = {0, 0, 0};
+  if (j >= 0) {
+    lj = T.node_level[j];
+    pj = T.node_prefix[j];
+    const int ch = T.node_child0[j];
+    beg = T.node_begin[j];
+    end = T.node_end[j];
+    if (ch < 0) lf = j;
+    const double bj = level_box(T, lj);
+    const int Xj[3] = {int(compact3(pj)), int(compact3(pj >> 1)), int(compact3(pj >> 2))};
+    for (int d = 0; d < 3; ++d)
+      off[d] = -periodic_shift_d(center_of(T.L, l, Xl[d]), center_of(T.L, lj, Xj[d]), T.L, b, bj) * T.L;
+  }
+  M.beg[src] = beg;
+  M.end[src] = end;
+  M.leaf[src] = lf;
+  M.lvl[src] = lj;
+  M.pfx[src] = pj;
+  for (int d = 0; d < 3; ++d) M.off[src][d] = off[d];
+}
+
+// build_tables with the mode counts known and the root box's spacing given
+template <int NP>
+__device__ __noinline__ void build_tables_of(const DevTree& T, const Header& h, int p, double2* tab, int t0, int nthr) {
+  using MO = ModesOf<NP>;
+  constexpr int nw = MO::NW, nd = MO::ND;
+  constexpr int DW = 2 * nw + 1, D = 2 * nd + 1;
+  constexpr int root_n = 2 * DW + nw + 1, lev_n = 2 * D + nd + 1;
+  const double* x = p == 0 ? h.xo : h.xt;
+  const int(*X)[3] = p == 0 ? h.Xo : h.Xt;
+  const int lmax = (p == 0 ? h.depth_o : h.depth_t) - 2;
+  const int total = root_n + (lmax >= 2 ? lmax - 1 : 0) * lev_n;
+  for (int e = t0; e < total; e += nthr) {
+    const bool root = e < root_n;
+    const int l = root ? 0 : 2 + (e - root_n) / lev_n;
+    const int rem = root ? e : (e - root_n) % lev_n;
+    const int w = root ? DW : D;
+    const int axis = rem < w ? 0 : (rem < 2 * w ? 1 : 2);
+    const int t = rem - axis * w, m = t - (root ? nw : nd);
+    const int Xa = root ? 0 : X[l][axis];
+    const double xr = root ? x[axis] - 0.5 * T.L : x[axis] - center_of(T.L, l, Xa);
+    const double th = (root ? T.delta_k[0] : level_dk(T, l)) * xr;
+    const int dec = root ? 3 : 2 * Xa + 1;
+    double2* dst = tab + (root ? axis * DW : 3 * DW + (l - 2) * 3 * D + axis * D);
+    double sn, cs;
+    sincos(-double(m) * th, &sn, &cs);
+    const double sc = axis == 2 ? h.q : 1.0;
+    dst[t] = cmul(make_double2(cs * sc, sn * sc), root6(-dec * m));
+  }
+}
+
+__device__ inline void group_sync(int id, int n) { asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(n) : "memory"); }
+
+template <int NP>
+__global__ void __launch_bounds__(MCL_T, 1) k_mc_long(const __grid_constant__ DevTree T, McLongArgs a) {
+  using MO = ModesOf<NP>;
+  static_assert(MO::STR % 16 == 4 && MO::STR >= 8 * MO::MT, "bank layout");
+  constexpr int D = 2 * MO::ND + 1, H = (MO::ND + 1) * D * D;
+  constexpr int DW = 2 * MO::NW + 1, HW = (MO::NW + 1) * DW * DW;
+  extern __shared__ double2 sm2[];
+  // The chain of one move runs once through a lot of code: functions used in
+  // several places are not inlined (they read the tree's description from
+  // shared memory), so that the loop stays in the instruction caches.
+  __shared__ __align__(16) unsigned char ts_raw[sizeof(DevTree)];
+  __shared__ Header hb[3];
+  __shared__ SrcList src[2][2];
+  __shared__ double c_level[MAXLV + 2];
+  __shared__ double red[MCL_W];
+  __shared__ const uint32_t* s_bm[MAXLV];
+  __shared__ const int* s_wp[MAXLV];
+  __shared__ Proposal P;
+  __shared__ double s_box[MAXLV], s_ibox[MAXLV];
+  __shared__ int s_acc, s_ok, s_units, s_wait, s_pn, s_pool;
+  const ResidualPoly<NP> poly(T);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const DevTree& Ts = *reinterpret_cast<const DevTree*>(ts_raw);
+  for (int i = tid; i < int(sizeof(DevTree) / 4); i += MCL_T)
+    reinterpret_cast<unsigned*>(ts_raw)[i] = reinterpret_cast<const unsigned*>(&T)[i];
+  const int G = gridDim.x, B = blockIdx.x;
+  // roles: warps [0, wd) difference modes, [wd, wd + ww) window modes, the
+  // last the helper, the rest the near field. At most two modes a thread.
+  const int hb0 = int(long(H) * B / G), hb1 = int(long(H) * (B + 1) / G);
+  const int wb0 = int(long(HW) * B / G), wb1 = int(long(HW) * (B + 1) / G);
+  const int wd = min(9, (H / G + 1 + 31) / 32), ww = min(3, (HW / G + 1 + 31) / 32);
+  const int w_near = wd + ww;
+  const bool commits = B == G / 2;  // the block that moves the particles, by its last near-field warp
+  const int n_near = 32 * (MCL_W - 1 - w_near - (commits ? 1 : 0));
+  const int dt = tid, wt = tid - 32 * wd, nt_ = tid - 32 * w_near;
+  // phase tables of this move and the next, then the deferred-update part
+  const int per = 3 * DW + max(T.max_depth - 1, 0) * 3 * D;
+  double* dyn = reinterpret_cast<double*>(sm2 + 4 * per);
+  const double* oct = a.oct;
+  if (MO::ND <= 19) {
+    for (int i = tid; i < MO::OCT; i += MCL_T) dyn[i] = a.oct[i];
+    oct = dyn;
+    dyn += MO::OCT;
+  }
+  double* ct = dyn;
+  dyn += MCL_UNITS * MO::CT;
+  Pending* mine = reinterpret_cast<Pending*>(dyn);
+  int* act = reinterpret_cast<int*>(mine + a.per_block);
+  int n_mine = 0, n_acc = 0;  // listed moves: this block's, all blocks'
+  if (tid >= 2 && tid < MAXLV + 2) {
+    const double dk = level_dk(T, tid);
+    c_level[tid] = dk * dk * dk / (8.0 * 3.14159265358979323846 * 3.14159265358979323846 * 3.14159265358979323846) *
+                   level_dscale(tid);
+  }
+  if (tid < MAXLV) {
+    s_box[tid] = level_box(T, tid);
+    s_ibox[tid] = 1.0 / s_box[tid];
+  }
+  if (tid < MAXLV && tid < T.max_depth) {
+    s_bm[tid] = T.bm_d[tid];
+    s_wp[tid] = T.wprefix_d[tid];
+  }
+  // this thread's modes: D2 and W values, root coefficients
+  double tab_v[2] = {0.0, 0.0};
+  double2 root_g[2] = {make_double2(0, 0), make_double2(0, 0)}, root_d[2];
+  if (warp < wd) {
+    for (int j = 0; j < 2; ++j)
+      if (hb0 + dt + j * 32 * wd < hb1) tab_v[j] = T.D2[hb0 + dt + j * 32 * wd];
+  } else if (warp < w_near) {
+    for (int j = 0; j < 2; ++j)
+      if (wb0 + wt + j * 32 * ww < wb1) {
+        tab_v[j] = T.W[wb0 + wt + j * 32 * ww];
+        root_g[j] = T.out_root[wb0 + wt + j * 32 * ww];
+      }
+  }
+  unsigned long long work_de = 0;
+  bool prev_acc = false;
+  auto load_at = [&](int i) {
+    const double* p = &a.pos4[i].x;
+    return make_double4(__ldcg(p), __ldcg(p + 1), __ldcg(p + 2), __ldcg(p + 3));
+  };
+  // the helper's next move and the index after it
+  int nx_i = 0, nn_i = 0, prev_i = -1;
+  double nx_d[3] = {0, 0, 0};
+  double4 nx_at = make_double4(0, 0, 0, 0);
+  auto tables_of = [&](int m, int p, Tables& tb) { alloc_tables(sm2 + ((m & 1) * 2 + p) * per, T, tb); };
+  auto build_next = [&](int m, const Header& h, int t0, int nthr) {  // both paths' tables of move m
+#pragma unroll 1
+    for (int p = 0; p < 2; ++p) build_tables_of<NP>(Ts, h, p, sm2 + ((m & 1) * 2 + p) * per, t0, nthr);
+  };
+  // a leaf source's current count; a commit that changes it later makes the
+  // near field count again
+  auto count_source = [&](SrcList& M, int j) {
+    M.cnt[j] = M.lvl[j] < 0 ? 0 : (M.leaf[j] >= 0 ? __ldcg(T.leaf_count + M.leaf[j]) : M.end[j] - M.beg[j]);
+  };
+  auto lists_next = [&](int m, const Header& h, int t) {  // source t of 72
+    const int p = t / 36;
+    const int lv = (p == 0 ? h.depth_t : h.depth_o) - 1;
+    source_static(Ts, p == 0 ? h.path_t[lv] : h.path_o[lv], lv, p == 0 ? h.Xt[lv] : h.Xo[lv], t % 36, src[m & 1][p]);
+    count_source(src[m & 1][p], t % 36);
+  };
+  // the rows of this block's modes go to L2 ahead of their use
+  auto prefetch_rows = [&](const Header& h) {
+    for (int p = 0; p < 2; ++p) {
+      const int top = (p == 0 ? h.depth_t : h.depth_o) - 2;
+      for (int l = 2; l <= top; ++l) {
+        const double2* row = T.inc + size_t((p == 0 ? h.path_t[l] : h.path_o[l]) - T.pw_base) * H;
+        for (int k = hb0 + 8 * lane; k < hb1; k += 256) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + k));
+      }
+    }
+  };
+  if (tid == 0) s_pool = s_pn = __ldcg(T.pool_n);
+  __syncthreads();
+  if (warp == MCL_W - 1) {
+    const int i = a.idx[0];
+    resolve_warp(Ts, i, load_at(i), a.disp[0], a.disp[1], a.disp[2], hb[0], s_bm, s_wp);
+    if (a.n_moves > 1) {
+      nx_i = a.idx[1];
+      nx_at = load_at(nx_i);
+      for (int c = 0; c < 3; ++c) nx_d[c] = a.disp[3 + c];
+    }
+    if (a.n_moves > 2) nn_i = a.idx[2];
+  }
+  __syncthreads();
+  build_next(0, hb[0], tid, MCL_T);
+  if (tid < 72) lists_next(0, hb[0], tid);
+  if (tid == 0) s_units = s_wait = 0;
+  __syncthreads();
+
+  for (int m = 0; m < a.n_moves; ++m) {
+    const Header& h = hb[m % 3];
+    Header& hn = hb[(m + 1) % 3];
+    const bool more = m + 1 < a.n_moves;
+    const unsigned epoch = unsigned(m) + 1u;
+    Tables to, oo;
+    tables_of(m, 0, oo);
+    tables_of(m, 1, to);
+    SrcList* S = src[m & 1];
+    const int lo_max = h.depth_o - 2, lt_max = h.depth_t - 2;
+    const double u_m = tid == 0 ? a.u[m] : 0.0;
+    double v = 0.0;  // this thread's share of dE
+    if (warp < wd) {
+      // difference (src/energy_shift.cpp:92-140); the rows of MCL_LEVB levels
+      // are loaded together, once where both paths share the box
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int k = hb0 + dt + j * 32 * wd;
+        if (k < hb1) {
+          const int ix = k % D, iy = (k / D) % D, iz = k / (D * D);
+          const int top = max(lo_max, lt_max);
+          double s = 0;
+          for (int l0 = 2; l0 <= top; l0 += MCL_LEVB) {
+            double2 co[MCL_LEVB], cn[MCL_LEVB];
+#pragma unroll
+            for (int q = 0; q < MCL_LEVB; ++q) {
+              const int l = l0 + q;
+              if (l <= lo_max) co[q] = __ldcg(T.inc + size_t(h.path_o[l] - T.pw_base) * H + k);
+              if (l <= lt_max && !(l <= lo_max && h.path_o[l] == h.path_t[l]))
+                cn[q] = __ldcg(T.inc + size_t(h.path_t[l] - T.pw_base) * H + k);
+            }
+#pragma unroll
+            for (int q = 0; q < MCL_LEVB; ++q) {
+              const int l = l0 + q;
+              if (l <= lo_max) {
+                const double2 o = cmul(oo.lev[l][2][iz], cmul(oo.lev[l][1][iy], oo.lev[l][0][ix]));
+                s -= (o.x * co[q].x - o.y * co[q].y - (o.x * o.x + o.y * o.y)) * c_level[l];
+              }
+              if (l <= lt_max) {
+                if (l <= lo_max && h.path_o[l] == h.path_t[l]) cn[q] = co[q];
+                const double2 t = cmul(to.lev[l][2][iz], cmul(to.lev[l][1][iy], to.lev[l][0][ix]));
+                s += (t.x * cn[q].x - t.y * cn[q].y) * c_level[l];
+              }
+            }
+          }
+          v += s * tab_v[j];
+        }
+      }
+    } else if (warp < w_near) {
+      // window (src/energy_shift.cpp:72-90)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int k = wb0 + wt + j * 32 * ww;
+        if (k < wb1) {
+          const double2 t = phase_at(to.root, k, DW), o = phase_at(oo.root, k, DW);
+          const double2 g = root_g[j];
+          root_d[j] = make_double2(t.x - o.x, t.y - o.y);
+          v += (root_d[j].x * (g.x - o.x) + root_d[j].y * (g.y - o.y)) * tab_v[j];
+        }
+      }
+      v *= a.c_window;
+    } else if (nt_ < n_near) {
+      // near field of the target and the origin (src/energy_shift.cpp:
+      // 233-302): the pairs of both paths split evenly over the blocks
+      if (s_wait) {  // the epoch of a commit that writes a leaf among the sources
+        if (nt_ == 0) {
+          int ok = 0;
+          for (long long it = 0; it < a.spin_limit; ++it)
+            if (ld_acquire(a.committed) >= unsigned(s_wait)) {
+              ok = 1;
+              break;
+            }
+          if (ok) s_pn = __ldcg(T.pool_n);
+          else atomicOr(T.err, 2);
+        }
+        group_sync(1, n_near);
+        for (int t = nt_; t < 72; t += n_near) count_source(S[t / 36], t % 36);
+        group_sync(1, n_near);
+      }
+      if (nt_ < 64) {  // exclusive prefix of a path's 36 counts, one warp each
+        SrcList& M = S[nt_ >> 5];
+        int c0 = M.cnt[lane], c1 = lane < 4 ? M.cnt[32 + lane] : 0;
+        int x = c0;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, x, o);
+          if (lane >= o) x += y;
+        }
+        const int tot = __shfl_sync(0xffffffffu, x, 31);
+        int y1 = c1;
+        for (int o = 1; o < 4; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, y1, o);
+          if (lane >= o) y1 += y;
+        }
+        M.pre[lane] = x - c0;
+        if (lane < 4) M.pre[32 + lane] = tot + y1 - c1;
+        if (lane == 3) M.pre[36] = tot + y1;
+      }
+      group_sync(1, n_near);
+      const int nt = S[0].pre[36], np = nt + S[1].pre[36];
+      const int e0 = int((long(B) * np) / G), e1 = int((long(B + 1) * np) / G);
+      const double eps = 2.220446049250313e-16;
+      for (int e = e0 + nt_; e < e1; e += n_near) {
+        const int p = e < nt ? 0 : 1;
+        const SrcList& M = S[p];
+        const int ee = p == 0 ? e : e - nt;
+        int lo = 0, hi = 36;  // largest source with pre[] <= ee
+        while (hi - lo > 1) {
+          const int mid = (lo + hi) >> 1;
+          if (M.pre[mid] <= ee) lo = mid;
+          else hi = mid;
+        }
+        const int sl = M.beg[lo] + (ee - M.pre[lo]);
+        const double4 w = make_double4(__ldcg(T.sx + sl), __ldcg(T.sy + sl), __ldcg(T.sz + sl), __ldcg(T.sq + sl));
+        const int lv = (p == 0 ? h.depth_t : h.depth_o) - 1;
+        const double b = s_box[lv];
+        const double* x = p == 0 ? h.xt : h.xo;
+        const double dx = x[0] - (w.x + M.off[lo][0]), dy = x[1] - (w.y + M.off[lo][1]), dz = x[2] - (w.z + M.off[lo][2]);
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        if (r2 > eps && r2 < b * b) {
+          const double r = w.w * poly.from_r2(r2, s_ibox[lv]);
+          v += p == 0 ? r : -r;
+        }
+      }
+      // arrivals parked in the overflow pool that belong to a source's subtree
+      const int pn = s_pn;
+      if (pn > 0)
+        for (int e2 = B * n_near + nt_; e2 < 2 * 36 * pn; e2 += G * n_near) {
+          const int p = e2 / (36 * pn), sj = (e2 / pn) % 36, qi = e2 % pn;
+          const SrcList& M = S[p];
+          if (M.lvl[sj] < 0 || __ldcg(T.p_orig + qi) < 0) continue;
+          const int pl = __ldcg(T.p_leaf + qi);
+          const int ll = T.node_level[pl], lj = M.lvl[sj];
+          if (ll < lj || (T.node_prefix[pl] >> (3 * (ll - lj))) != M.pfx[sj]) continue;
+          const double b = level_box(T, (p == 0 ? h.depth_t : h.depth_o) - 1);
+          const double* x = p == 0 ? h.xt : h.xo;
+          const double dx = x[0] - (__ldcg(T.px + qi) + M.off[sj][0]), dy = x[1] - (__ldcg(T.py + qi) + M.off[sj][1]),
+                       dz = x[2] - (__ldcg(T.pz + qi) + M.off[sj][2]);
+          const double r2 = dx * dx + dy * dy + dz * dz;
+          if (r2 > eps && r2 < b * b) {
+            const double r = __ldcg(T.pq + qi) * poly(sqrt(r2), b);
+            v += p == 0 ? r : -r;
+          }
+        }
+      v *= h.q;
+    } else if (warp == MCL_W - 1 && more) {
+      // helper: resolve the next move from what it loaded a move ago, and load
+      // for the move after it. Of the commits that may have been running then,
+      // the last move's position is in its header and the one before is in
+      // pos4 by now
+      const Header& hp = hb[(m + 2) % 3];  // move m - 1
+      double4 at = nx_at;
+      if (m > 1 && prev_i == nx_i) at = load_at(nx_i);
+      if (m > 0 && hp.i_orig == nx_i && prev_acc) at = make_double4(hp.xt[0], hp.xt[1], hp.xt[2], hp.q);
+      const int i = nx_i;
+      const double d0 = nx_d[0], d1 = nx_d[1], d2 = nx_d[2];
+      if (m > 0) prev_i = hp.i_orig;
+      if (m + 2 < a.n_moves) {
+        nx_i = nn_i;
+        nx_at = load_at(nn_i);
+        for (int c = 0; c < 3; ++c) nx_d[c] = a.disp[3 * size_t(m + 2) + c];
+        if (m + 3 < a.n_moves) nn_i = a.idx[m + 3];
+      }
+      resolve_warp(Ts, i, at, d0, d1, d2, hn, s_bm, s_wp);
+      prefetch_rows(hn);
+    }
+    // what the listed moves changed in the rows the difference sums read: the
+    // mode warps, which are done before the near field
+    if (warp < w_near) {
+      const int nu = s_units;
+      for (int u0 = 0; u0 < nu; u0 += MCL_UNITS) {
+        const int n = min(MCL_UNITS, nu - u0);
+        for (int w = warp; w < n; w += w_near) {
+          const int unit = act[u0 + w];
+          unit_cosines<MO::ND>(T.L, level_dk(T, unit & 15), h, mine[unit >> 8], unit, ct + w * MO::CT);
+        }
+        group_sync(2, 32 * w_near);
+        for (int w = 0; w < n; w += 2) {
+          const int ua = act[u0 + w], ub = act[u0 + min(w + 1, n - 1)];
+          v += unit_pair_rows<MO::ND>(oct, ct + w * MO::CT, w + 1 < n, c_level[ua & 15] * h.q * mine[ua >> 8].q,
+                                      c_level[ub & 15] * h.q * mine[ub >> 8].q, (warp + w) % w_near, w_near);
+        }
+        if (u0 + MCL_UNITS < nu) group_sync(2, 32 * w_near);
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) red[warp] = v;
+    __syncthreads();
+    unsigned long long* pk = a.packets + size_t(m & 1) * 2 * G;
+    if (warp == 0) {
+      // publish this block's sum, then gather everybody's in a fixed order
+      double x = lane < MCL_W ? red[lane] : 0.0;
+#pragma unroll
+      for (int o = MCL_W / 2; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      if (lane == 0) {
+        if (commits && prev_acc) asm volatile("fence.acq_rel.gpu;" ::: "memory");  // releases the commit since the last packet
+        packet_store(pk + 2 * B, x, epoch, commits ? unsigned(s_pool) : 0u);
+      }
+      // the self term (src/energy_shift.cpp:30-41, one image per lane) while
+      // the others' packets are on their way
+      double dr2 = h.d2;
+      if (lane < 27) {
+        const int mx = lane % 3 - 1, my = (lane / 3) % 3 - 1, mz = lane / 9 - 1;
+        const double ax = h.xt[0] - (h.xo[0] + mx * T.L), ay = h.xt[1] - (h.xo[1] + my * T.L),
+                     az = h.xt[2] - (h.xo[2] + mz * T.L);
+        dr2 = fmin(dr2, ax * ax + ay * ay + az * az);
+      }
+      for (int o = 16; o > 0; o >>= 1) dr2 = fmin(dr2, __shfl_xor_sync(0xffffffffu, dr2, o));
+      const double self = poly.from_r2(dr2, s_ibox[2]) * h.q * h.q;
+      double tot = 0.0;
+      bool ok = true;
+      for (int b0 = 0; b0 < G; b0 += 32 * MCL_POLL) {
+        double pv[MCL_POLL];
+        unsigned px[MCL_POLL];
+        for (long long it = 0;; ++it) {
+          bool all = true;
+#pragma unroll
+          for (int j = 0; j < MCL_POLL; ++j) {
+            const int b = b0 + lane + 32 * j;
+            unsigned pe = epoch;
+            pv[j] = 0.0;
+            if (b < G) packet_load(pk + 2 * b, pv[j], pe, px[j]);
+            all = all && pe == epoch;
+          }
+          if (all) break;
+          if (it >= a.spin_limit || ((it & 1023) == 1023 && (ldm<true>(T.err) & 2))) {
+            ok = false;
+            break;
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < MCL_POLL; ++j) {
+          tot += pv[j];
+          if (b0 + lane + 32 * j == G / 2) {
+            s_pn = int(px[j]);
+            ld_acquire(a.committed);  // the commits before that packet are visible from here on
+          }
+        }
+      }
+      if (!ok) atomicOr(T.err, 2);
+      ok = __all_sync(0xffffffffu, ok);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) tot += __shfl_down_sync(0xffffffffu, tot, o);
+      if (lane == 0) {
+        const double dE = tot - self;
+        const int accd = u_m < exp(-a.beta * dE) ? 1 : 0;
+        s_acc = accd;
+        s_ok = ok;
+        s_wait = 0;
+        if (B == 0) {
+          if (a.dE_out) a.dE_out[m] = dE;
+          if (a.acc_out) a.acc_out[m] = accd;
+          const int nlev = max(lo_max - 1, 0) + max(lt_max - 1, 0);
+          work_de += 24ull * HW + 16ull * nlev * H + 8ull * H + 32ull * (unsigned long long)(S[0].pre[36] + S[1].pre[36]);
+        }
+      }
+    } else if (more) {
+      if (warp >= MCL_W - 3) {
+        const int t = tid - 32 * (MCL_W - 3);
+        if (t < 72) lists_next(m + 1, hn, t);
+      } else {
+        build_next(m + 1, hn, tid - 32, MCL_T - 128);
+      }
+    }
+    __syncthreads();
+    if (!s_ok) return;
+    const bool accd = s_acc != 0;
+    const bool again = accd && more && hn.i_orig == h.i_orig;  // resolved from the old position
+    if (accd) {
+      if (warp >= wd && warp < w_near) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int k = wb0 + wt + j * 32 * ww;
+          if (k < wb1) {
+            root_g[j] = cadd(root_g[j], root_d[j]);
+            T.out_root[k] = root_g[j];
+          }
+        }
+      }
+      if (warp == 1 && n_acc % G == B) {
+        // this block keeps the move, lists it for the end of the launch and
+        // marks the outgoing rows it changes
+        if (lane == 0) {
+          fill_pending(T, h, mine[n_mine]);
+          a.list[n_acc] = mine[n_mine];
+        }
+        for (int l = T.pw_lo + lane; l <= T.pw_hi; l += 32) {
+          if (l <= h.depth_t - 1) atomicAdd(a.touched + (h.path_t[l] - T.pw_base), 1);
+          if (l <= h.depth_o - 1) atomicAdd(a.touched + (h.path_o[l] - T.pw_base), 1);
+        }
+      }
+      if (n_acc % G == B) ++n_mine;
+      ++n_acc;
+    }
+    // Does this move's commit, or the last one's (the counts may be older),
+    // write a leaf the next move reads? A source box on the move's target or
+    // origin path holds that leaf.
+    if (more && (accd || prev_acc) && warp >= 2 && warp < 5 && tid - 64 < 72) {
+      const SrcList& M = src[(m + 1) & 1][(tid - 64) / 36];
+      const int j = (tid - 64) % 36;
+      const int l = M.lvl[j];
+      auto holds = [&](const Header& g) {
+        return (l < g.depth_t && morton3(g.Xt[l][0], g.Xt[l][1], g.Xt[l][2]) == M.pfx[j]) ||
+               (l < g.depth_o && morton3(g.Xo[l][0], g.Xo[l][1], g.Xo[l][2]) == M.pfx[j]);
+      };
+      if (l >= 0 && ((accd && holds(h)) || (prev_acc && holds(hb[(m + 2) % 3])))) s_wait = accd ? int(epoch) : int(epoch) - 1;
+    }
+    if (again) {  // the particle just moved moves again: resolve it from where it is now
+      __syncthreads();
+      if (warp == MCL_W - 1) {
+        const double4 at = make_double4(h.xt[0], h.xt[1], h.xt[2], h.q);
+        double dn[3];
+        for (int c = 0; c < 3; ++c) dn[c] = a.disp[3 * size_t(m + 1) + c];
+        resolve_warp(Ts, h.i_orig, at, dn[0], dn[1], dn[2], hn, s_bm, s_wp);
+      }
+      __syncthreads();
+      if (tid < 72) lists_next(m + 1, hn, tid);
+      else build_next(m + 1, hn, tid - 72, MCL_T - 72);
+      if (tid == 0) s_wait = int(epoch);
+      __syncthreads();
+    }
+    if (more && warp == 1) {
+      __syncwarp();
+      const int nu = near_units(hn, mine, n_mine, act);
+      if (lane == 0) s_units = nu;
+    }
+    prev_acc = accd;
+    if (accd && commits && warp == MCL_W - 2 && lane == 0) {
+      P.i_orig = h.i_orig;
+      P.q = h.q;
+      for (int c = 0; c < 3; ++c) {
+        P.xo[c] = h.xo[c];
+        P.xt[c] = h.xt[c];
+      }
+      P.depth_o = h.depth_o;
+      P.depth_t = h.depth_t;
+      for (int l = 0; l < MAXLV; ++l) {
+        P.path_o[l] = l < h.depth_o ? h.path_o[l] : -1;
+        P.path_t[l] = l < h.depth_t ? h.path_t[l] : -1;
+      }
+      P.accepted = 1;
+      P.valid = 1;
+      P.n_recv = 0;
+    }
+    __syncthreads();
+    // the commit runs beside the next move's sums
+    if (accd && commits && warp == MCL_W - 2 && lane == 0) {
+      a.pos4[P.i_orig] = make_double4(P.xt[0], P.xt[1], P.xt[2], P.q);
+      P.slot = __ldcg(T.orig_slot + P.i_orig);
+      atomicAdd(&T.work[0], 1ull);
+      atomicAdd(&T.work[1], 32ull * (unsigned long long)HW);
+      commit_move(T, P);
+      s_pool = int(*(volatile int*)T.pool_n);
+      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(a.committed), "r"(epoch) : "memory");
+    }
+  }
+  if (B == 0 && tid == 0) {
+    *a.n_list = n_acc;
+    atomicAdd(&T.work[2], work_de);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Replica sets: the Metropolis sequences of many independent trees in one
 // launch, one thread block per tree (the block resolves, sums, decides,
 // updates and commits its tree's moves with block barriers only). Small
 // replicas do not need a whole GPU per move, so running them side by side
 // fills the SMs with independent work.
+// Expansion updates are deferred as in k_mc_long: a block that updated its
+// tree's rows move by move moved about 30 MB per accepted move through one SM
+// (1.7 ms a move with 256 replicas; the whole set ran at 4.3 TB/s of DRAM).
 constexpr int REP_T = 256;
+constexpr int REP_CHUNK = 128;  // most moves between two updates of the rows
+constexpr int REP_ILP = 4;      // modes a thread loads before it uses the first
+constexpr int REP_UNITS = 8;    // pair units whose cosines are held at a time
 
 template <int NP>
-__global__ void __launch_bounds__(REP_T, 2) k_mc_rep(const DevTree* __restrict__ trees, int m, const int* __restrict__ idx,
-                                                  const double* __restrict__ disp, const double* __restrict__ u,
-                                                  double beta, double* __restrict__ dE_out, int* __restrict__ acc_out) {
+constexpr size_t rep_lazy_bytes() {
+  using M = ModesOf<NP>;
+  return (M::ND <= 19 ? size_t(M::OCT) * 8 : 0) + size_t(REP_UNITS) * M::CT * 8 +
+         sizeof(int) * MAXLV * REP_CHUNK;
+}
+
+struct RepArgs {
+  const DevTree* trees;
+  int m, m0, cnt;       // moves per tree; this launch runs [m0, m0 + cnt)
+  const int* idx;
+  const double* disp;
+  const double* u;
+  double beta;
+  double* dE_out;
+  int* acc_out;
+  Pending* const* list; // per tree
+  int* const* n_list;
+  int* const* touched;
+  const double* const* oct;
+};
+
+template <int NP>
+__global__ void __launch_bounds__(REP_T, 2) k_mc_rep(RepArgs a) {
+  using MO = ModesOf<NP>;
+  constexpr int D = 2 * MO::ND + 1, H = (MO::ND + 1) * D * D;
+  constexpr int DW = 2 * MO::NW + 1, HW = (MO::NW + 1) * DW * DW;
   extern __shared__ double2 sm2[];
   __shared__ __align__(16) unsigned char ts_raw[sizeof(DevTree)];
   __shared__ Header h;
   __shared__ double red[4][32];
   __shared__ double c_level[MAXLV + 2];
-  __shared__ Receiver rs[MAX_RECV];
   __shared__ Proposal P;
-  __shared__ int s_acc;
+  __shared__ int s_acc, s_units;
   {
-    const unsigned* src = reinterpret_cast<const unsigned*>(trees + blockIdx.x);
+    const unsigned* src = reinterpret_cast<const unsigned*>(a.trees + blockIdx.x);
     unsigned* dst = reinterpret_cast<unsigned*>(ts_raw);
     for (int i = threadIdx.x; i < int(sizeof(DevTree) / 4); i += blockDim.x) dst[i] = src[i];
   }
@@ -1325,9 +2375,21 @@ __global__ void __launch_bounds__(REP_T, 2) k_mc_rep(const DevTree* __restrict__
   }
   const double dk0 = T.delta_k[0];
   const double c_window = dk0 * dk0 * dk0 / (8.0 * pi * pi * pi);
-  for (int mv = 0; mv < m; ++mv) {
-    const size_t c = size_t(blockIdx.x) * m + mv;
-    resolve(T, idx[c], disp + 3 * c, h);
+  Pending* list = a.list[blockIdx.x];
+  int* touched = a.touched[blockIdx.x];
+  const double* oct = a.oct[blockIdx.x];
+  double* dyn = reinterpret_cast<double*>(sm2 + 2 * (3 * DW + max(T.max_depth - 1, 0) * 3 * D));
+  if (MO::ND <= 19) {
+    for (int i = threadIdx.x; i < MO::OCT; i += blockDim.x) dyn[i] = oct[i];
+    oct = dyn;
+    dyn += MO::OCT;
+  }
+  double* ct = dyn;
+  int* act = reinterpret_cast<int*>(dyn + REP_UNITS * MO::CT);
+  int n_acc = 0;
+  for (int mv = a.m0; mv < a.m0 + a.cnt; ++mv) {
+    const size_t c = size_t(blockIdx.x) * a.m + mv;
+    resolve(T, a.idx[c], a.disp + 3 * c, h);
     const int lo_max = h.depth_o - 2, lt_max = h.depth_t - 2;
     const int uo = min(h.depth_o - 1, T.pw_hi), ut = min(h.depth_t - 1, T.pw_hi);
     const int per = 3 * (2 * T.n_window + 1) + max(max(uo, ut) - 1, 0) * 3 * (2 * T.n_diff + 1);
@@ -1337,28 +2399,33 @@ __global__ void __launch_bounds__(REP_T, 2) k_mc_rep(const DevTree* __restrict__
     build_tables(T, h.xo, h.q, h.Xo, uo, oo, threadIdx.x, blockDim.x);
     build_tables(T, h.xt, h.q, h.Xt, ut, to, threadIdx.x, blockDim.x);
     __syncthreads();
+    if (threadIdx.x < 32) {
+      const int nu = near_units(h, list, n_acc, act);
+      if (threadIdx.x == 0) s_units = nu;
+    }
     double acc[4] = {0, 0, 0, 0};
-    for (int k = threadIdx.x; k < T.Hw; k += blockDim.x) {
-      const double2 t = phase_at(to.root, k, T.dw), o = phase_at(oo.root, k, T.dw);
+    for (int k = threadIdx.x; k < HW; k += REP_T) {
+      const double2 t = phase_at(to.root, k, DW), o = phase_at(oo.root, k, DW);
       const double2 g = T.out_root[k];
       const double ar = t.x - o.x, ai = t.y - o.y, br = g.x - o.x, bi = g.y - o.y;
       acc[0] += (ar * br + ai * bi) * T.W[k];
     }
-    const int base = T.pw_base, d = T.dd, n = T.n_diff;
-    for (int k = threadIdx.x; k < T.H; k += blockDim.x) {
-      const int ix = k % d, iy = (k / d) % d, iz = k / (d * d);
-      double sd = 0;
-      for (int l = 2; l <= lo_max; ++l) {
-        const double2 o = cmul(oo.lev[l][2][iz], cmul(oo.lev[l][1][iy], oo.lev[l][0][ix]));
-        const double2 cc = T.inc[size_t(h.path_o[l] - base) * T.H + k];
-        sd -= (o.x * cc.x - o.y * cc.y - (o.x * o.x + o.y * o.y)) * c_level[l];
+    acc[1] = diff_sum<MO::ND, REP_T, REP_ILP>(T, h, oo, to, lo_max, lt_max, c_level);
+    __syncthreads();
+    // what the listed moves changed in the rows just read
+    for (int u0 = 0; u0 < s_units; u0 += REP_UNITS) {
+      const int n = min(REP_UNITS, s_units - u0), warp = threadIdx.x >> 5;
+      if (warp < n) {
+        const int unit = act[u0 + warp];
+        unit_cosines<MO::ND>(T.L, level_dk(T, unit & 15), h, list[unit >> 8], unit, ct + warp * MO::CT);
       }
-      for (int l = 2; l <= lt_max; ++l) {
-        const double2 t = cmul(to.lev[l][2][iz], cmul(to.lev[l][1][iy], to.lev[l][0][ix]));
-        const double2 cc = T.inc[size_t(h.path_t[l] - base) * T.H + k];
-        sd += (t.x * cc.x - t.y * cc.y) * c_level[l];
+      __syncthreads();
+      for (int w = 0; w < n; w += 2) {
+        const int ua = act[u0 + w], ub = act[u0 + min(w + 1, n - 1)];
+        acc[1] += unit_pair_rows<MO::ND>(oct, ct + w * MO::CT, w + 1 < n, c_level[ua & 15] * h.q * list[ua >> 8].q,
+                                         c_level[ub & 15] * h.q * list[ub >> 8].q, warp, REP_T / 32);
       }
-      acc[1] += sd * T.D2[k];
+      __syncthreads();
     }
     const int lt = h.depth_t - 1, lo = h.depth_o - 1;
     acc[2] = residual_sum(T, poly, h.path_t[lt], lt, h.Xt[lt], h.xt);
@@ -1369,22 +2436,27 @@ __global__ void __launch_bounds__(REP_T, 2) k_mc_rep(const DevTree* __restrict__
       double self = 0;
       if (h.dr != 0) self = poly(h.dr, level_box(T, 2)) * h.q * h.q;
       const double dE = acc[0] * c_window + acc[1] + (acc[2] - acc[3]) * h.q - self;
-      const int accd = u[c] < exp(-beta * dE) ? 1 : 0;
+      const int accd = a.u[c] < exp(-a.beta * dE) ? 1 : 0;
       s_acc = accd;
-      if (dE_out) dE_out[c] = dE;
-      if (acc_out) acc_out[c] = accd;
+      if (a.dE_out) a.dE_out[c] = dE;
+      if (a.acc_out) a.acc_out[c] = accd;
     }
     __syncthreads();
     if (!s_acc) continue;
-    // accept-and-update (src/tree.cpp:447-597) by this block
-    const int nr = build_receivers(T, h, rs);
+    // accept-and-update (src/tree.cpp:447-597) by this block: the root row,
+    // the membership, and the move's turn in the list
     if (threadIdx.x == 0) {
+      Pending e;
+      fill_pending(T, h, e);
+      list[n_acc] = e;
+      for (int l = T.pw_lo; l <= e.u[0]; ++l) ++touched[h.path_t[l] - T.pw_base];
+      for (int l = T.pw_lo; l <= e.u[1]; ++l) ++touched[h.path_o[l] - T.pw_base];
       P.i_orig = h.i_orig;
       P.slot = h.slot;
       P.q = h.q;
-      for (int a = 0; a < 3; ++a) {
-        P.xo[a] = h.xo[a];
-        P.xt[a] = h.xt[a];
+      for (int x = 0; x < 3; ++x) {
+        P.xo[x] = h.xo[x];
+        P.xt[x] = h.xt[x];
       }
       P.depth_o = h.depth_o;
       P.depth_t = h.depth_t;
@@ -1394,62 +2466,22 @@ __global__ void __launch_bounds__(REP_T, 2) k_mc_rep(const DevTree* __restrict__
       }
       P.accepted = 1;
       P.valid = 1;
-      P.n_recv = nr;
+      P.n_recv = 0;
       atomicAdd(&T.work[0], 1ull);
-      atomicAdd(&T.work[1], 32ull * ((unsigned long long)T.Hw + (unsigned long long)nr * T.H));
+      atomicAdd(&T.work[1], 32ull * (unsigned long long)T.Hw);
       commit_move(T, P);
     }
-    for (int k = threadIdx.x; k < T.Hw; k += blockDim.x) {
-      const double2 t = phase_at(to.root, k, T.dw), o = phase_at(oo.root, k, T.dw);
+    ++n_acc;
+    for (int k = threadIdx.x; k < HW; k += REP_T) {
+      const double2 t = phase_at(to.root, k, DW), o = phase_at(oo.root, k, DW);
       T.out_root[k] = csub(cadd(T.out_root[k], t), o);
-    }
-    for (int k = threadIdx.x; k < T.H; k += blockDim.x) {
-      const int ix = k % d, iy = (k / d) % d, iz = k / (d * d);
-      const int a0 = ((ix - n) % 3 + 3) % 3, a1 = ((iy - n) % 3 + 3) % 3, a2 = ((iz - n) % 3 + 3) % 3;
-      int r = 0;
-      while (r < nr) {
-        const int l = rs[r].level;
-        int re = r + 1;
-        while (re < nr && rs[re].level == l) ++re;
-        const double2 pt0 = cmul(to.lev[l][2][iz], cmul(to.lev[l][1][iy], to.lev[l][0][ix]));
-        const double2 po0 = cmul(oo.lev[l][2][iz], cmul(oo.lev[l][1][iy], oo.lev[l][0][ix]));
-        const double2 pt1 = cmul(pt0, root6(-2)), pt2 = cmul(pt0, root6(-4));
-        const double2 po1 = cmul(po0, root6(-2)), po2 = cmul(po0, root6(-4));
-        const int two_l = (l & 1) ? 2 : 1;
-        for (; r < re; r += UPD_UNROLL) {
-          double2 v[UPD_UNROLL];
-          size_t off[UPD_UNROLL];
-#pragma unroll
-          for (int q = 0; q < UPD_UNROLL; ++q) {
-            if (r + q < re) {
-              const Receiver& R = rs[r + q];
-              off[q] = size_t(R.off) * T.H + k;
-              v[q] = R.is_out ? T.out[off[q]] : T.inc[off[q]];
-            }
-          }
-#pragma unroll
-          for (int q = 0; q < UPD_UNROLL; ++q) {
-            if (r + q < re) {
-              const Receiver& R = rs[r + q];
-              // the exponent sum lies in [-12, 12]
-              const int et = ((a0 * R.ft[0] + a1 * R.ft[1] + a2 * R.ft[2]) * two_l + 12) % 3;
-              const int eo = ((a0 * R.fo[0] + a1 * R.fo[1] + a2 * R.fo[2]) * two_l + 12) % 3;
-              double2 del = make_double2(0.0, 0.0);
-              if (R.has_t) del = et == 0 ? pt0 : (et == 1 ? pt1 : pt2);
-              if (R.has_o) del = csub(del, eo == 0 ? po0 : (eo == 1 ? po1 : po2));
-              if (R.is_out) T.out[off[q]] = cadd(v[q], del);
-              else T.inc[off[q]] = make_double2(v[q].x + del.x, v[q].y - del.y);
-            }
-          }
-        }
-        r = re;
-      }
     }
     __syncthreads();
   }
+  if (threadIdx.x == 0) *a.n_list[blockIdx.x] = n_acc;
 }
 
-using McRepKernel = void (*)(const DevTree*, int, const int*, const double*, const double*, double, double*, int*);
+using McRepKernel = void (*)(RepArgs);
 McRepKernel mc_rep_kernel(int np) {
   switch (np) {
     case 7: return k_mc_rep<7>;
@@ -1469,6 +2501,50 @@ McKernel mc_kernel(int np) {
     case 25: return k_mc<25>;
     default: throw std::invalid_argument("unsupported residual polynomial");
   }
+}
+
+using McLongKernel = void (*)(DevTree, McLongArgs);
+McLongKernel mc_long_kernel(int np) {
+  switch (np) {
+    case 7: return k_mc_long<7>;
+    case 13: return k_mc_long<13>;
+    case 19: return k_mc_long<19>;
+    case 25: return k_mc_long<25>;
+    default: throw std::invalid_argument("unsupported residual polynomial");
+  }
+}
+
+size_t mc_long_smem(int np, int per_block) {
+  switch (np) {
+    case 7: return mcl_bytes<7>(per_block);
+    case 13: return mcl_bytes<13>(per_block);
+    case 19: return mcl_bytes<19>(per_block);
+    default: return mcl_bytes<25>(per_block);
+  }
+}
+
+size_t rep_lazy_smem(int np) {
+  switch (np) {
+    case 7: return rep_lazy_bytes<7>();
+    case 13: return rep_lazy_bytes<13>();
+    case 19: return rep_lazy_bytes<19>();
+    default: return rep_lazy_bytes<25>();
+  }
+}
+
+// outgoing rows of the nodes the listed moves touched
+void launch_flush_outgoing(const DevTree& D, const Pending* list, const int* n_list, const int* touched, cudaStream_t st) {
+  const int n_pw = D.level_start[D.pw_hi + 1] - D.pw_base;
+  const int n2 = D.level_start[3] - D.level_start[2], parts2 = 8;
+  const unsigned grid = unsigned(n2 * parts2 + n_pw - n2);
+  switch (D.n_diff) {
+    case 6: k_flush_outgoing<6><<<grid, FO_T, 0, st>>>(D, list, n_list, touched, parts2); break;
+    case 12: k_flush_outgoing<12><<<grid, FO_T, 0, st>>>(D, list, n_list, touched, parts2); break;
+    case 19: k_flush_outgoing<19><<<grid, FO_T, 0, st>>>(D, list, n_list, touched, parts2); break;
+    case 26: k_flush_outgoing<26><<<grid, FO_T, 0, st>>>(D, list, n_list, touched, parts2); break;
+    default: throw std::invalid_argument("unsupported mode count");
+  }
+  PDMK_LAUNCH_CHECK();
 }
 
 // ---------------------------------------------------------------------------
@@ -1941,6 +3017,44 @@ void DmkTree::update_shift(long i, double dx, double dy, double dz) {
   moved_ = true;
 }
 
+// The deferred-update list of a tree, its marks and the folded difference
+// table, kept with the tree for its later sequences.
+void DmkTree::ensure_pending(int cap) {
+  DevTree& D = dev_;
+  if (!d_oct_) {
+    int stride = 0, n_oct = 0;
+    switch (D.n_poly) {
+      case 7: stride = ModesOf<7>::STR, n_oct = ModesOf<7>::OCT; break;
+      case 13: stride = ModesOf<13>::STR, n_oct = ModesOf<13>::OCT; break;
+      case 19: stride = ModesOf<19>::STR, n_oct = ModesOf<19>::OCT; break;
+      case 25: stride = ModesOf<25>::STR, n_oct = ModesOf<25>::OCT; break;
+      default: throw std::invalid_argument("unsupported residual polynomial");
+    }
+    const int n_pw = D.level_start[D.pw_hi + 1] - D.pw_base;
+    d_oct_ = static_cast<double*>(alloc(sizeof(double) * size_t(n_oct)));
+    k_fold_d2<<<unsigned((n_oct + 255) / 256), 256, 0, st_>>>(D, stride, n_oct, d_oct_);
+    PDMK_LAUNCH_CHECK();
+    d_touched_ = static_cast<int*>(alloc(sizeof(int) * (size_t(n_pw) + 1)));
+    d_n_list_ = d_touched_ + n_pw;
+  }
+  if (cap > pending_cap_) {
+    d_pending_ = alloc(sizeof(Pending) * size_t(cap));
+    pending_cap_ = cap;
+  }
+}
+
+// Empties the list, before a sequence that fills it.
+void DmkTree::clear_pending() {
+  const int n_pw = dev_.level_start[dev_.pw_hi + 1] - dev_.pw_base;
+  PDMK_CUDA(cudaMemsetAsync(d_touched_, 0, sizeof(int) * (size_t(n_pw) + 1), st_));
+}
+
+// Brings the expansion rows up to date with the listed moves.
+void DmkTree::flush_pending() {
+  launch_flush_outgoing(dev_, static_cast<const Pending*>(d_pending_), d_n_list_, d_touched_, st_);
+  launch_incoming_touched(d_touched_);
+}
+
 // One cooperative launch per kMcChunk moves on every SM (k_mc). The grid is
 // the SM count, which the occupancy query confirms can be co-resident; the
 // cooperative launch refuses to start otherwise, so the grid barriers inside
@@ -1948,6 +3062,7 @@ void DmkTree::update_shift(long i, double dx, double dy, double dz) {
 void DmkTree::mc_run_persistent(int n_moves, const int* d_idx, const double* d_disp, const double* d_u, double beta,
                                 double* d_dE, int* d_acc) {
   DevTree& D = dev_;
+  if (mc_run_long(n_moves, d_idx, d_disp, d_u, beta, d_dE, d_acc)) return;
   const size_t smem = tables_smem(D, D.max_depth, 2);
   const McKernel kern = mc_kernel(D.n_poly);
   if (mc_grid_ == 0) {
@@ -1987,6 +3102,69 @@ void DmkTree::mc_run_persistent(int n_moves, const int* d_idx, const double* d_d
     PDMK_LAUNCH_CHECK();
     time_end(2);
   }
+}
+
+// The same for a sequence long enough to defer its row updates (k_mc_long);
+// false when it is not. The passes that bring the rows up to date cost with the
+// number of rows, an update move by move with the number of moves.
+bool DmkTree::mc_run_long(int n_moves, const int* d_idx, const double* d_disp, const double* d_u, double beta, double* d_dE,
+                          int* d_acc) {
+  DevTree& D = dev_;
+  const int n_pw = D.pw_hi >= D.pw_lo ? D.level_start[D.pw_hi + 1] - D.pw_base : 0;
+  if (!inc_formed_ || n_pw == 0 || n_moves < std::max(16, n_pw / 32)) return false;
+  const McLongKernel kern = mc_long_kernel(D.n_poly);
+  const size_t smem = tables_smem(D, D.max_depth, 4) + mc_long_smem(D.n_poly, kPendPerBlock);
+  if (mcl_grid_ == 0) {
+    int dev = 0, sms = 0, coop = 0, per_sm = 0;
+    PDMK_CUDA(cudaGetDevice(&dev));
+    PDMK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    PDMK_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    if (!coop) throw CudaError("device does not support cooperative launches");
+    raise_smem_limit(reinterpret_cast<const void*>(kern), smem);
+    PDMK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, MCL_T, smem));
+    // a thread holds at most two of its block's modes
+    if (per_sm < 1 || sms < 144) return false;
+    d_pos4_ = alloc(sizeof(double4) * size_t(N_));
+    d_packets_ = static_cast<unsigned long long*>(alloc(sizeof(unsigned long long) * 4 * size_t(sms) + 64));
+    mcl_grid_ = sms;
+  }
+  prepare_box_lists();
+  const int chunk = std::min(n_pw >= 1024 ? 2048 : 1024, kPendPerBlock * mcl_grid_);
+  ensure_pending(std::min(chunk, n_moves));
+  const double pi = 3.14159265358979323846;
+  for (int m0 = 0; m0 < n_moves; m0 += chunk) {
+    const int cnt = std::min(chunk, n_moves - m0);
+    McLongArgs a{};
+    a.idx = d_idx + m0;
+    a.disp = d_disp + 3 * size_t(m0);
+    a.u = d_u + m0;
+    a.beta = beta;
+    a.n_moves = cnt;
+    a.dE_out = d_dE ? d_dE + m0 : nullptr;
+    a.acc_out = d_acc ? d_acc + m0 : nullptr;
+    a.c_window = std::pow(D.delta_k[0], 3) / std::pow(2 * pi, 3);
+    a.packets = d_packets_;
+    a.committed = reinterpret_cast<unsigned int*>(d_packets_ + 4 * size_t(mcl_grid_));
+    a.pos4 = static_cast<double4*>(d_pos4_);
+    a.spin_limit = 1LL << 21;  // about a second of polling
+    a.list = static_cast<Pending*>(d_pending_);
+    a.n_list = d_n_list_;
+    a.touched = d_touched_;
+    a.oct = d_oct_;
+    a.per_block = kPendPerBlock;
+    clear_pending();
+    PDMK_CUDA(cudaMemsetAsync(d_packets_, 0, sizeof(unsigned long long) * 4 * size_t(mcl_grid_) + 64, st_));
+    k_gather_moves<<<unsigned((cnt + 255) / 256), 256, 0, st_>>>(D, a.idx, cnt, a.pos4);
+    PDMK_LAUNCH_CHECK();
+    void* args[] = {&D, &a};
+    time_begin(2);
+    PDMK_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kern), dim3(unsigned(mcl_grid_)),
+                                          dim3(unsigned(MCL_T)), args, smem, st_));
+    PDMK_LAUNCH_CHECK();
+    flush_pending();
+    time_end(2);
+  }
+  return true;
 }
 
 void DmkTree::mc_run_device(int n_moves, const int* d_idx, const double* d_disp, const double* d_u, double beta,
@@ -2123,30 +3301,70 @@ void DmkTree::replicas_mc_run(const std::vector<DmkTree*>& ts, int m, const int*
   if (ts.empty() || m <= 0) return;
   const int np = ts[0]->dev_.n_poly;
   size_t smem = 0;
-  std::vector<DevTree> hd;
   for (DmkTree* t : ts) {
     if (t->dev_.n_poly != np) throw std::invalid_argument("replicas must share the digits setting");
     t->ensure_packed();
     smem = std::max(smem, tables_smem(t->dev_, t->dev_.max_depth, 2));
-    hd.push_back(t->dev_);
   }
   cudaStream_t st = ts[0]->st_;
-  std::vector<cudaEvent_t> evs(ts.size());
+  // Each tree's list is filled by its block of the launch on the first tree's
+  // stream and its rows are updated on its own stream; the trees' streams and
+  // the first one meet at events around each launch.
+  const size_t nt = ts.size();
+  std::vector<cudaEvent_t> evs(nt);
   for (auto& e : evs) PDMK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  for (size_t i = 1; i < ts.size(); ++i) {
-    PDMK_CUDA(cudaEventRecord(evs[i], ts[i]->st_));
-    PDMK_CUDA(cudaStreamWaitEvent(st, evs[i], 0));
+  const int chunk = std::min(m, REP_CHUNK);
+  std::vector<unsigned char> blob(nt * (sizeof(DevTree) + 4 * sizeof(void*)));
+  DevTree* h_trees = reinterpret_cast<DevTree*>(blob.data());
+  void** h_ptr = reinterpret_cast<void**>(blob.data() + nt * sizeof(DevTree));
+  for (size_t i = 0; i < nt; ++i) {
+    DmkTree* t = ts[i];
+    const bool has_rows = t->dev_.pw_hi >= t->dev_.pw_lo;
+    t->ensure_pending(chunk);
+    if (has_rows) t->prepare_box_lists();
+    h_trees[i] = t->dev_;
+    h_ptr[i] = t->d_pending_;
+    h_ptr[nt + i] = t->d_n_list_;
+    h_ptr[2 * nt + i] = t->d_touched_;
+    h_ptr[3 * nt + i] = t->d_oct_;
   }
-  DevTree* d_trees = nullptr;
-  PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d_trees), sizeof(DevTree) * hd.size(), st));
-  PDMK_CUDA(cudaMemcpyAsync(d_trees, hd.data(), sizeof(DevTree) * hd.size(), cudaMemcpyHostToDevice, st));
+  unsigned char* d_blob = nullptr;
+  PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d_blob), blob.size(), st));
+  PDMK_CUDA(cudaMemcpyAsync(d_blob, blob.data(), blob.size(), cudaMemcpyHostToDevice, st));
+  void** d_ptr = reinterpret_cast<void**>(d_blob + nt * sizeof(DevTree));
   const McRepKernel kern = mc_rep_kernel(np);
+  smem += rep_lazy_smem(np);
   raise_smem_limit(reinterpret_cast<const void*>(kern), smem);
-  kern<<<unsigned(ts.size()), REP_T, smem, st>>>(d_trees, m, d_idx, d_disp, d_u, beta, d_dE, d_acc);
-  PDMK_LAUNCH_CHECK();
-  PDMK_CUDA(cudaFreeAsync(d_trees, st));
-  PDMK_CUDA(cudaEventRecord(evs[0], st));
-  for (size_t i = 1; i < ts.size(); ++i) PDMK_CUDA(cudaStreamWaitEvent(ts[i]->st_, evs[0], 0));
+  RepArgs a{};
+  a.trees = reinterpret_cast<const DevTree*>(d_blob);
+  a.m = m;
+  a.idx = d_idx;
+  a.disp = d_disp;
+  a.u = d_u;
+  a.beta = beta;
+  a.dE_out = d_dE;
+  a.acc_out = d_acc;
+  a.list = reinterpret_cast<Pending* const*>(d_ptr);
+  a.n_list = reinterpret_cast<int* const*>(d_ptr + nt);
+  a.touched = reinterpret_cast<int* const*>(d_ptr + 2 * nt);
+  a.oct = reinterpret_cast<const double* const*>(d_ptr + 3 * nt);
+  for (a.m0 = 0; a.m0 < m; a.m0 += chunk) {
+    a.cnt = std::min(chunk, m - a.m0);
+    for (size_t i = 0; i < nt; ++i) {
+      ts[i]->clear_pending();
+      if (i == 0) continue;
+      PDMK_CUDA(cudaEventRecord(evs[i], ts[i]->st_));
+      PDMK_CUDA(cudaStreamWaitEvent(st, evs[i], 0));
+    }
+    kern<<<unsigned(nt), REP_T, smem, st>>>(a);
+    PDMK_LAUNCH_CHECK();
+    PDMK_CUDA(cudaEventRecord(evs[0], st));
+    for (size_t i = 0; i < nt; ++i) {
+      if (i > 0) PDMK_CUDA(cudaStreamWaitEvent(ts[i]->st_, evs[0], 0));
+      if (ts[i]->dev_.pw_hi >= ts[i]->dev_.pw_lo) ts[i]->flush_pending();
+    }
+  }
+  PDMK_CUDA(cudaFreeAsync(d_blob, st));
   for (auto& e : evs) PDMK_CUDA(cudaEventDestroy(e));  // released once the waits resolve
   for (DmkTree* t : ts) {
     t->last_valid_ = false;

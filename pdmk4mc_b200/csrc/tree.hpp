@@ -280,6 +280,7 @@ class DmkTree {
   void launch_window_energy();  // enqueue the window energy into d_scalars_[0]
   void launch_res_energy();     // enqueue the near-field energy into d_scalars_[2]
   void run_incoming(bool write_inc);
+  int inc_slots() const;
 
   double L_;
   int n_per_leaf_;
@@ -343,6 +344,23 @@ class DmkTree {
   int mc_grid_ = 0;
   double* mc_partials_ = nullptr;
   unsigned int* mc_sync_ = nullptr;
+  // deferred expansion updates of Metropolis sequences (shift.cu)
+  static constexpr int kPendPerBlock = 16;  // listed moves one block of the persistent kernel keeps
+  bool inc_formed_ = false;  // the incoming rows follow from the outgoing ones (a deferred update recomputes them)
+  int mcl_grid_ = 0;
+  void* d_pos4_ = nullptr;   // position and charge by particle, for the particles of a sequence
+  unsigned long long* d_packets_ = nullptr;
+  bool mc_run_long(int n_moves, const int* d_idx, const double* d_disp, const double* d_u, double beta, double* d_dE,
+                   int* d_acc);
+  void* d_pending_ = nullptr;
+  int pending_cap_ = 0;
+  int* d_touched_ = nullptr;
+  int* d_n_list_ = nullptr;
+  double* d_oct_ = nullptr;
+  void ensure_pending(int cap);
+  void clear_pending();
+  void flush_pending();
+  void launch_incoming_touched(const int* touched);
   void mc_run_persistent(int n_moves, const int* d_idx, const double* d_disp, const double* d_u, double beta,
                          double* d_dE, int* d_acc);
   static constexpr int kTimedEvery = 8;
