@@ -7,13 +7,16 @@
 // eval_energy_diff / eval_energy_res (src/energy.cpp:21-173).
 //
 // The outgoing expansion of a box, rho_B(k) = sum_j q_j exp(-i k.x_j) over
-// the half grid kz <= 0, is evaluated as the complex contraction
-//   out[(kz,ky), kx] = sum_j (q_j ez_j[kz] ey_j[ky]) ex_j[kx]
-// with box-centred coordinates: exp(-i k.x) = exp(-i k.c_B) exp(-i k.(x-c_B)),
-// where k.c_B is an exact multiple of pi/3 (k = m dk_l, dk_l bs_l = 2 pi / 3),
-// so the decentring factor is an exact sixth root of unity per axis. A table
-// pass writes each work item's per-particle factors ex, ey, ez to HBM once;
-// the contraction streams them chunk by chunk into shared memory.
+// the half grid kz <= 0, is evaluated with box-centred coordinates:
+// exp(-i k.x) = exp(-i k.c_B) exp(-i k.(x-c_B)), where k.c_B is an exact
+// multiple of pi/3 (k = m dk_l, dk_l bs_l = 2 pi / 3), so the decentring
+// factor is an exact sixth root of unity per axis. The charges are real, so
+// the centred sums follow from real ones: with f_2m = cos(m dk x) and
+// f_2m+1 = sin(m dk x),
+//   T[a][b][c] = sum_j q_j f_a(z_j) f_b(y_j) f_c(x_j)
+// holds every sign combination of (kz, ky, kx) as sums of eight entries, and
+// its (2n+1)^3 entries are half the multiply-adds of the complex products
+// over the half grid's (n+1)(2n+1)^2 modes.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -44,285 +47,223 @@ __device__ inline double block_sum(double v, double* sm) {
 }
 
 // ---------------------------------------------------------------------------
-// NUDFT work item: one row tile of one box over one slot range
+// NUDFT work item: one box (or one split-K chunk of it) over one slot range
 struct NudftWork {
   double cx, cy, cz;  // box centre
   double dk;
   int X, Y, Z;        // integer box coordinates at its level
   int M;              // decentring multiplier: 1 for levels >= 2, 3 for the root
   int s_begin, s_end;
-  int row_tile;
-  int pad_;
   double2* out;       // H complex outputs of this box (or of this split-K chunk)
-  const double2* tab; // factor tables of this item's particle chunks (shared by its row tiles)
 };
 
-// Each thread owns one (kz, ky) row and TC <= 20 of its kx columns: 4 TC FP64
-// accumulators stay in registers (wider tiles spill), and the row factor
-// q ez ey costs one complex multiply per TC multiply-adds.
+// T as an FP64 tensor-core product (mma m8n8k4): rows (a, b), columns c,
+// summed over particles. Rows come in tiles of eight b for one a, the two a
+// (cosine, sine) of one kz together: a warp holds CPW such (kz, b tile) pairs
+// against all column tiles, so an A element (one product fz fy) feeds NT
+// instructions and a column value 2 CPW. What bounds it: the FP64 pipe, which
+// issues tensor instructions at the rate of plain ones (37.1 against 36.6
+// TFLOP/s measured on independent chains); per step of four particles a warp
+// issues 2 CPW NT of them for 2 CPW products and 3 CPW + NT shared loads.
 template <int NK>
 struct NudftShape {
   static constexpr int D = 2 * NK + 1;
-  static constexpr int CG = (D + 19) / 20;            // column groups per row
-  static constexpr int TC = (D + CG - 1) / CG;        // columns per thread
-  static constexpr int DP = TC * CG;                  // padded row stride in smem
-  static constexpr int ROWS = (NK + 1) * D;
-  static constexpr int WORK = ROWS * CG;              // thread tasks per box
-  static constexpr int TMAX = 512;
-  static constexpr int TILES = (WORK + TMAX - 1) / TMAX;
-  static constexpr int THREADS = ((WORK + TILES - 1) / TILES + 31) / 32 * 32;
-  // particles per shared-memory chunk: 32, or 16 when 32 would not fit
-  static constexpr int KC = 2 * 32 * (2 * DP + NK + 1) * 16 > 200 * 1024 ? 16 : 32;
-  static constexpr int SMEM = 2 * KC * (2 * DP + NK + 1) * int(sizeof(double2));  // double-buffered
+  static constexpr int N1 = NK + 1;                  // modes per half axis, zero included
+  static constexpr int NT = (2 * N1 + 7) / 8;        // tiles of eight entries (four modes) per axis
+  static constexpr int PAIRS = N1 * NT;              // (kz, b tile) pairs of a box
+  // pairs per warp: accumulators of 8 CPW NT registers, and a last block that
+  // is nearly full
+  static constexpr int CPW = NT >= 17 ? 1 : NT >= 9 ? 2 : NT >= 7 ? 3 : NT >= 4 ? 5 : NT == 3 ? 7 : NK >= 6 ? 4 : 3;
+  static constexpr int WARPS = 4;
+  static constexpr int THREADS = 32 * WARPS;
+  static constexpr int TILES = (PAIRS + WARPS * CPW - 1) / (WARPS * CPW);  // blocks per item
+  // one particle's factors in shared memory: fx, fy, fz; the stride is 4
+  // modulo 8, so that the 4 particles x 8 entries of an operand load fall on
+  // different banks
+  static constexpr int STR = 24 * NT + 4;
+  static constexpr int KC = 2 * 32 * STR * 8 <= 100 * 1024 ? 32 : 16;  // particles per chunk
+  static constexpr int SMEM = 2 * KC * STR * int(sizeof(double));       // double-buffered
 };
 
-// per-axis factors exp(-i m dk (x - c)) * w6^{-M (2X+1) m}, m = m0 .. m0+cnt-1.
-// The six chains m = m0 + r + 6 i each keep one root of unity, so they step
-// by exp(-6 i dk (x - c)) with the root applied once per chain: a dependency
-// chain of about cnt / 6 complex products instead of 2 cnt.
-__device__ inline void axis_factors(double xr, double dk, int M, int X, int m0, int cnt, double scale, double2* dst) {
-  const double th = dk * xr;
-  double s, c;
-  sincos(-double(m0) * th, &s, &c);
-  const double2 v0 = make_double2(c * scale, s * scale);
-  sincos(-th, &s, &c);
-  const double2 st = make_double2(c, s);
-  const double2 st2 = cmul(st, st), st3 = cmul(st2, st), st6 = cmul(st3, st3);
-  const int dec = M * (2 * X + 1);
-  double2 v[6];
-  v[0] = v0;
-  v[1] = cmul(v0, st);
-  v[2] = cmul(v0, st2);
-  v[3] = cmul(v0, st3);
-  v[4] = cmul(v[1], st3);
-  v[5] = cmul(v[2], st3);
-#pragma unroll
-  for (int r = 0; r < 6; ++r) v[r] = cmul(v[r], root6(-dec * (m0 + r)));
-  for (int t = 0; t < cnt; t += 6) {
-#pragma unroll
-    for (int r = 0; r < 6; ++r) {
-      if (t + r < cnt) {
-        dst[t + r] = v[r];
-        v[r] = cmul(v[r], st6);
-      }
-    }
-  }
-}
-
-// Factor tables of one particle chunk of a work item, in shared memory:
-// ex [KC][DP], ey [KC][DP], ez [KC][NK+1] (charge folded into ez), rows past
-// the item's last particle and the padding columns D .. DP-1 zero. Tasks are
-// (particle, axis, half) so that each recurrence chain covers half an axis.
+// Factors of a chunk's particles into shared memory, one thread per particle
+// and axis: cos and sin of m th, m = 0 .. NK, by two interleaved chains of
+// steps exp(2 i th); the charge is folded into fz. Particles past the end get
+// zeros. (A block spends about 3 % of its time here; a separate pass wrote
+// and read 1.6 KB per particle and level, 2.8 ms at N = 1e6.)
 template <int NK>
-__device__ void nudft_build(const NudftWork& w, int base, double2* buf, const double* __restrict__ sx,
-                            const double* __restrict__ sy, const double* __restrict__ sz,
-                            const double* __restrict__ sq) {
+__device__ __forceinline__ void nudft_factors(const NudftWork& w, int base, double* buf, const double* __restrict__ sx,
+                                              const double* __restrict__ sy, const double* __restrict__ sz,
+                                              const double* __restrict__ sq) {
   using S = NudftShape<NK>;
-  double2* ex = buf;
-  double2* ey = ex + S::KC * S::DP;
-  double2* ez = ey + S::KC * S::DP;
-  const int nk = min(S::KC, w.s_end - base);
-  for (int t = threadIdx.x; t < S::KC * 6; t += blockDim.x) {
-    int j = t / 6, a = (t / 2) % 3, half = t & 1;
-    if (j >= nk) {
-      double2* dst = a == 0 ? ex + j * S::DP : (a == 1 ? ey + j * S::DP : ez + j * (NK + 1));
-      int len = a == 2 ? NK + 1 : S::DP;
-      for (int u = half; u < len; u += 2) dst[u] = make_double2(0.0, 0.0);
+  for (int t = threadIdx.x; t < S::KC * 3; t += S::THREADS) {
+    const int j = t % S::KC, axis = t / S::KC, s = base + j;
+    double* dst = buf + j * S::STR + axis * 8 * S::NT;
+    if (s >= w.s_end) {
+      for (int e = 0; e < 2 * S::N1; ++e) dst[e] = 0.0;
       continue;
     }
-    int s = base + j;
-    if (a == 0) {
-      int h = (S::D + 1) / 2;
-      int m0 = half ? -NK + h : -NK, cnt = half ? S::D - h : h;
-      axis_factors(sx[s] - w.cx, w.dk, w.M, w.X, m0, cnt, 1.0, ex + j * S::DP + (m0 + NK));
-      if (half)
-        for (int u = S::D; u < S::DP; ++u) ex[j * S::DP + u] = make_double2(0.0, 0.0);
-    } else if (a == 1) {
-      int h = (S::D + 1) / 2;
-      int m0 = half ? -NK + h : -NK, cnt = half ? S::D - h : h;
-      axis_factors(sy[s] - w.cy, w.dk, w.M, w.Y, m0, cnt, 1.0, ey + j * S::DP + (m0 + NK));
-    } else {
-      int h = (NK + 2) / 2;
-      int m0 = half ? -NK + h : -NK, cnt = half ? NK + 1 - h : h;
-      axis_factors(sz[s] - w.cz, w.dk, w.M, w.Z, m0, cnt, sq[s], ez + j * (NK + 1) + (m0 + NK));
+    const double x = axis == 0 ? sx[s] - w.cx : (axis == 1 ? sy[s] - w.cy : sz[s] - w.cz);
+    const double sc = axis == 2 ? sq[s] : 1.0;
+    double sn, cs;
+    sincos(w.dk * x, &sn, &cs);
+    const double2 z1 = make_double2(cs, sn), st = cmul(z1, z1);
+    double2 e = make_double2(sc, 0.0), o = make_double2(cs * sc, sn * sc);
+#pragma unroll 2
+    for (int m = 0; m < S::N1; m += 2) {
+      *reinterpret_cast<double2*>(dst + 2 * m) = e;
+      e = cmul(e, st);
+      if (m + 1 < S::N1) *reinterpret_cast<double2*>(dst + 2 * m + 2) = o;
+      o = cmul(o, st);
     }
   }
 }
 
-// Table pass: one block per (item, particle chunk) builds the chunk's tables
-// in shared memory and writes them to the item's table range in HBM with
-// coalesced stores, once for all row tiles of the item.
 template <int NK>
-__global__ void __launch_bounds__(NudftShape<NK>::KC * 6)
-    k_nudft_tables(const NudftWork* __restrict__ work, const int2* __restrict__ chunks, const double* __restrict__ sx,
-                   const double* __restrict__ sy, const double* __restrict__ sz, const double* __restrict__ sq) {
+__global__ void __launch_bounds__(NudftShape<NK>::THREADS, 2)
+    k_nudft(const NudftWork* __restrict__ work, const double* __restrict__ sx, const double* __restrict__ sy,
+            const double* __restrict__ sz, const double* __restrict__ sq) {
   using S = NudftShape<NK>;
-  constexpr int BUF = S::KC * (2 * S::DP + NK + 1);
-  extern __shared__ double2 smem[];
-  const int2 ch = chunks[blockIdx.x];
-  const NudftWork w = work[ch.x];
-  nudft_build<NK>(w, w.s_begin + ch.y * S::KC, smem, sx, sy, sz, sq);
-  __syncthreads();
-  double2* dst = const_cast<double2*>(w.tab) + size_t(ch.y) * BUF;
-  for (int i = threadIdx.x; i < BUF; i += blockDim.x) dst[i] = smem[i];
-}
-
-__device__ inline void cp_async16(void* smem_dst, const void* gmem_src) {
-  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
-  const size_t g = __cvta_generic_to_global(gmem_src);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(g) : "memory");
-}
-__device__ inline void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ inline void cp_async_wait_prior() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
-
-// Contraction pass: one (item, row tile) per block. The chunk tables stream
-// from HBM into two shared-memory buffers by asynchronous copies issued a
-// chunk ahead, so every thread does the same work between two barriers.
-template <int NK>
-__global__ void __launch_bounds__(NudftShape<NK>::THREADS) k_nudft(const NudftWork* __restrict__ work) {
-  using S = NudftShape<NK>;
-  constexpr int BUF = S::KC * (2 * S::DP + NK + 1);  // complex entries per table buffer
-  extern __shared__ double2 smem[];
-  const NudftWork w = work[blockIdx.x];
-  const int g = w.row_tile * S::THREADS + threadIdx.x;
-  const bool active = g < S::WORK;
-  const int row = active ? g / S::CG : 0;
-  const int cg = active ? g % S::CG : 0;
-  const int kz = row / S::D, ky = row % S::D;
-  const int c0 = cg * S::TC;
+  constexpr int NT = S::NT, CPW = S::CPW, STR = S::STR, N1 = S::N1, D = S::D;
+  extern __shared__ double smem_d[];
+  const NudftWork w = work[blockIdx.x / S::TILES];
+  const int tile = blockIdx.x % S::TILES;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int q4 = lane & 3, q8 = lane >> 2;
+  const int g0 = (tile * S::WARPS + warp) * CPW;  // this warp's first pair
+  int oz[CPW], oy[CPW];                            // shared-memory offsets of a pair's fz and fy entries
+#pragma unroll
+  for (int i = 0; i < CPW; ++i) {
+    const int g = min(g0 + i, S::PAIRS - 1);
+    oz[i] = 16 * NT + 2 * (g / NT);
+    oy[i] = 8 * NT + 8 * (g % NT) + q8;
+  }
+  double acc[CPW][2][NT][2];
+#pragma unroll
+  for (int i = 0; i < CPW; ++i)
+#pragma unroll
+    for (int z = 0; z < 2; ++z)
+#pragma unroll
+      for (int t = 0; t < NT; ++t) acc[i][z][t][0] = acc[i][z][t][1] = 0.0;
+  // the entries past the last mode stay zero
+  constexpr int PADN = 8 * NT - 2 * N1;
+  if constexpr (PADN > 0)
+    for (int t = threadIdx.x; t < 2 * S::KC * 3 * PADN; t += S::THREADS)
+      smem_d[(t / (3 * PADN)) * STR + (t / PADN % 3) * 8 * NT + 2 * N1 + t % PADN] = 0.0;
   const int nch = (w.s_end - w.s_begin + S::KC - 1) / S::KC;
-  auto fetch = [&](int c) {
-    const double2* src = w.tab + size_t(c) * BUF;
-    double2* dst = smem + (c & 1) * BUF;
-    for (int i = threadIdx.x; i < BUF; i += blockDim.x) cp_async16(dst + i, src + i);
-  };
-  double2 acc[S::TC];
-#pragma unroll
-  for (int c = 0; c < S::TC; ++c) acc[c] = make_double2(0.0, 0.0);
-  if (nch > 0) fetch(0);
-  cp_async_commit();
+  if (nch > 0) nudft_factors<NK>(w, w.s_begin, smem_d, sx, sy, sz, sq);
+  __syncthreads();
   for (int ci = 0; ci < nch; ++ci) {
-    // the next chunk's copies go out before this chunk is contracted (its
-    // buffer was last read before the previous iteration's closing barrier)
-    if (ci + 1 < nch) fetch(ci + 1);
-    cp_async_commit();
-    cp_async_wait_prior();  // everything but the group just committed has landed
-    __syncthreads();
-    const double2* ex = smem + (ci & 1) * BUF;
-    const double2* ey = ex + S::KC * S::DP;
-    const double2* ez = ey + S::KC * S::DP;
-    const int nk = min(S::KC, w.s_end - (w.s_begin + ci * S::KC));
-    if (active) {
+    // the next chunk's factors (its buffer was last read before the barrier
+    // that closed the previous iteration)
+    if (ci + 1 < nch) nudft_factors<NK>(w, w.s_begin + (ci + 1) * S::KC, smem_d + ((ci + 1) & 1) * S::KC * STR, sx, sy, sz, sq);
+    const double* buf = smem_d + (ci & 1) * S::KC * STR + q4 * STR;
+    if (g0 < S::PAIRS) {
 #pragma unroll 1
-      for (int j = 0; j < nk; ++j) {
-        const double2 a = cmul(ez[j * (NK + 1) + kz], ey[j * S::DP + ky]);
-        const double2* xr = ex + j * S::DP + c0;
-        // one shared-memory load per column feeds its four FMAs; the 2 TC
-        // accumulator chains give enough independent work to hide latency
+      for (int ks = 0; ks < S::KC / 4; ++ks) {
+        const double* row = buf + 4 * ks * STR;
+        double b[NT];
 #pragma unroll
-        for (int c = 0; c < S::TC; ++c) {
-          const double2 b = xr[c];
-          acc[c].x = fma(a.x, b.x, acc[c].x);
-          acc[c].y = fma(a.x, b.y, acc[c].y);
-          acc[c].x = fma(-a.y, b.y, acc[c].x);
-          acc[c].y = fma(a.y, b.x, acc[c].y);
+        for (int t = 0; t < NT; ++t) b[t] = row[8 * t + q8];
+#pragma unroll
+        for (int i = 0; i < CPW; ++i) {
+          const double y = row[oy[i]];
+          const double2 z = *reinterpret_cast<const double2*>(row + oz[i]);
+          const double a0 = z.x * y, a1 = z.y * y;
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+            asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                : "+d"(acc[i][0][t][0]), "+d"(acc[i][0][t][1])
+                : "d"(a0), "d"(b[t]));
+            asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                : "+d"(acc[i][1][t][0]), "+d"(acc[i][1][t][1])
+                : "d"(a1), "d"(b[t]));
+          }
         }
       }
     }
     __syncthreads();
   }
-  if (active) {
-    double2* o = w.out + size_t(row) * S::D + c0;
+  // Epilogue: the four modes (-p, +-q, +-r) of p = |kz|, q = |ky|, r = |kx|. A
+  // lane holds the cosine or the sine row of q (lane bit 2), its partner the
+  // other; the first takes ky = +q, the second ky = -q.
+  const int odd = q8 & 1;
+  const double sg = odd ? -1.0 : 1.0;
+  const int dx = w.M * (2 * w.X + 1), dy = w.M * (2 * w.Y + 1), dz = w.M * (2 * w.Z + 1);
 #pragma unroll
-    for (int c = 0; c < S::TC; ++c)
-      if (c0 + c < S::D) o[c] = acc[c];
+  for (int i = 0; i < CPW; ++i) {
+    const int g = g0 + i, p = g / NT, q = 4 * (g % NT) + (q8 >> 1);
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      double own[4], oth[4];  // [kz cosine, sine][kx cosine, sine]
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        own[v] = acc[i][v >> 1][t][v & 1];
+        oth[v] = __shfl_xor_sync(0xffffffffu, own[v], 4);
+      }
+      const int r = 4 * t + q4;
+      if (g < S::PAIRS && q < N1 && r < N1 && !(odd && q == 0)) {
+        // y cosine and y sine entries
+        double c[4], sv[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          c[v] = odd ? oth[v] : own[v];
+          sv[v] = odd ? own[v] : oth[v];
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (h == 1 && r == 0) continue;
+          const double ta = h ? -1.0 : 1.0;  // kx = ta r
+          const double st = sg * ta;
+          const double a1 = c[0] - st * sv[1], b1 = sg * sv[0] + ta * c[1];
+          const double a2 = c[2] - st * sv[3], b2 = sg * sv[2] + ta * c[3];
+          const int ky = odd ? -q : q, kx = h ? -r : r;
+          const double2 v = cmul(make_double2(a1 + b2, a2 - b1), root6(-(dx * kx + dy * ky - dz * p)));
+          w.out[(size_t(NK - p) * D + NK + ky) * D + NK + kx] = v;
+        }
+      }
+    }
   }
 }
 
 template <int NK>
-void launch_nudft(const NudftWork* d_work, int nwork, const int2* d_chunks, int nchunks, const DevTree& T,
-                  cudaStream_t st) {
+void launch_nudft(const NudftWork* d_work, int nwork, const DevTree& T, cudaStream_t st) {
   using S = NudftShape<NK>;
-  constexpr int TAB_SMEM = S::KC * (2 * S::DP + NK + 1) * int(sizeof(double2));
   if (nwork == 0) return;
   // per device and thread-safe: replica energies call this from several host threads
   raise_smem_limit(reinterpret_cast<const void*>(k_nudft<NK>), S::SMEM);
-  raise_smem_limit(reinterpret_cast<const void*>(k_nudft_tables<NK>), TAB_SMEM);
-  if (nchunks > 0) {
-    k_nudft_tables<NK><<<unsigned(nchunks), S::KC * 6, TAB_SMEM, st>>>(d_work, d_chunks, T.sx, T.sy, T.sz, T.sq);
-    PDMK_LAUNCH_CHECK();
-  }
-  k_nudft<NK><<<unsigned(nwork), S::THREADS, S::SMEM, st>>>(d_work);
+  k_nudft<NK><<<unsigned(nwork) * S::TILES, S::THREADS, S::SMEM, st>>>(d_work, T.sx, T.sy, T.sz, T.sq);
   PDMK_LAUNCH_CHECK();
 }
 
-struct NudftInfo {
-  int tiles, kc, buf;  // row tiles per item, particles per chunk, complex entries per chunk table
-};
-
-template <int NK>
-NudftInfo nudft_info_of() {
-  using S = NudftShape<NK>;
-  return {S::TILES, S::KC, S::KC * (2 * S::DP + NK + 1)};
-}
-
-NudftInfo nudft_info(int nk) {
+// blocks of an item
+int nudft_tiles(int nk) {
   switch (nk) {
-    case 4: return nudft_info_of<4>();
-    case 6: return nudft_info_of<6>();
-    case 8: return nudft_info_of<8>();
-    case 12: return nudft_info_of<12>();
-    case 13: return nudft_info_of<13>();
-    case 17: return nudft_info_of<17>();
-    case 19: return nudft_info_of<19>();
-    case 26: return nudft_info_of<26>();
-    case 32: return nudft_info_of<32>();  // Ewald structure factor, level 2
-    case 64: return nudft_info_of<64>();  // Ewald structure factor, level 3
+    case 4: return NudftShape<4>::TILES;
+    case 6: return NudftShape<6>::TILES;
+    case 8: return NudftShape<8>::TILES;
+    case 12: return NudftShape<12>::TILES;
+    case 13: return NudftShape<13>::TILES;
+    case 17: return NudftShape<17>::TILES;
+    case 19: return NudftShape<19>::TILES;
+    case 26: return NudftShape<26>::TILES;
+    case 32: return NudftShape<32>::TILES;  // Ewald structure factor, level 2
+    case 64: return NudftShape<64>::TILES;  // Ewald structure factor, level 3
     default: throw std::invalid_argument("unsupported mode count");
   }
 }
 
-int nudft_tiles(int nk) { return nudft_info(nk).tiles; }
-
-// Lays out the factor tables of a work list whose items are runs of `tiles`
-// consecutive entries (row tiles 0 .. tiles-1 of one box or chunk): each item
-// gets ceil(n / KC) chunk tables, allocated here stream-ordered on `st`, and
-// the list of (first entry, chunk) pairs the table pass runs over. The caller
-// frees `tables` stream-ordered after the contraction.
-void plan_nudft_tables(int nk, std::vector<NudftWork>& wl, double2** tables, std::vector<int2>& chunks,
-                       cudaStream_t st) {
-  const NudftInfo in = nudft_info(nk);
-  size_t nchunk = 0;
-  for (size_t e = 0; e < wl.size(); e += in.tiles) {
-    if (wl[e].row_tile != 0) throw std::logic_error("NUDFT work list: items must start at row tile 0");
-    nchunk += size_t((wl[e].s_end - wl[e].s_begin + in.kc - 1) / in.kc);
-  }
-  PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(tables), sizeof(double2) * size_t(in.buf) * std::max<size_t>(nchunk, 1),
-                            st));
-  chunks.clear();
-  chunks.reserve(nchunk);
-  size_t c = 0;
-  for (size_t e = 0; e < wl.size(); e += in.tiles) {
-    const int n = (wl[e].s_end - wl[e].s_begin + in.kc - 1) / in.kc;
-    for (int t = 0; t < in.tiles && e + t < wl.size(); ++t) wl[e + t].tab = *tables + c * size_t(in.buf);
-    for (int k = 0; k < n; ++k) chunks.push_back(make_int2(int(e), k));
-    c += size_t(n);
-  }
-}
-
-void dispatch_nudft(int nk, const NudftWork* d_work, int nwork, const int2* d_chunks, int nchunks, const DevTree& T,
-                    cudaStream_t st) {
+void dispatch_nudft(int nk, const NudftWork* d_work, int nwork, const DevTree& T, cudaStream_t st) {
   switch (nk) {
-    case 4: launch_nudft<4>(d_work, nwork, d_chunks, nchunks, T, st); break;
-    case 6: launch_nudft<6>(d_work, nwork, d_chunks, nchunks, T, st); break;
-    case 8: launch_nudft<8>(d_work, nwork, d_chunks, nchunks, T, st); break;
-    case 12: launch_nudft<12>(d_work, nwork, d_chunks, nchunks, T, st); break;
-    case 13: launch_nudft<13>(d_work, nwork, d_chunks, nchunks, T, st); break;
-    case 17: launch_nudft<17>(d_work, nwork, d_chunks, nchunks, T, st); break;
-    case 19: launch_nudft<19>(d_work, nwork, d_chunks, nchunks, T, st); break;
-    case 26: launch_nudft<26>(d_work, nwork, d_chunks, nchunks, T, st); break;
-    case 32: launch_nudft<32>(d_work, nwork, d_chunks, nchunks, T, st); break;
-    case 64: launch_nudft<64>(d_work, nwork, d_chunks, nchunks, T, st); break;
+    case 4: launch_nudft<4>(d_work, nwork, T, st); break;
+    case 6: launch_nudft<6>(d_work, nwork, T, st); break;
+    case 8: launch_nudft<8>(d_work, nwork, T, st); break;
+    case 12: launch_nudft<12>(d_work, nwork, T, st); break;
+    case 13: launch_nudft<13>(d_work, nwork, T, st); break;
+    case 17: launch_nudft<17>(d_work, nwork, T, st); break;
+    case 19: launch_nudft<19>(d_work, nwork, T, st); break;
+    case 26: launch_nudft<26>(d_work, nwork, T, st); break;
+    case 32: launch_nudft<32>(d_work, nwork, T, st); break;
+    case 64: launch_nudft<64>(d_work, nwork, T, st); break;
     default: throw std::invalid_argument("unsupported mode count");
   }
 }
@@ -998,8 +939,8 @@ void DmkTree::form_outgoing_pw() {
     int first, n;
     double2* out;
   };
-  // the row tiles of one box (or box chunk) over the slots [sb, se)
-  auto make_work = [&](std::vector<NudftWork>& wl, int nk, int l, uint64_t p, double2* out, int sb, int se) {
+  // one box (or box chunk) over the slots [sb, se)
+  auto make_work = [&](std::vector<NudftWork>& wl, int l, uint64_t p, double2* out, int sb, int se) {
     NudftWork w{};
     double scale = std::ldexp(1.0, -l);
     int X = int(compact3(p)), Y = int(compact3(p >> 1)), Z = int(compact3(p >> 2));
@@ -1014,11 +955,7 @@ void DmkTree::form_outgoing_pw() {
     w.s_begin = sb;
     w.s_end = se;
     w.out = out;
-    int tiles = nudft_tiles(nk);
-    for (int t = 0; t < tiles; ++t) {
-      w.row_tile = t;
-      wl.push_back(w);
-    }
+    wl.push_back(w);
   };
   // the mixed pass: one item per (box or box chunk, pair of 128-row M tiles)
   auto make_mix = [&](std::vector<MixItem>& wl, int nk, int l, uint64_t p, double2* out, int sb, int se) {
@@ -1118,7 +1055,17 @@ void DmkTree::form_outgoing_pw() {
   // Root pass first, on the second stream: the root (node 0, all slots) needs
   // no host view of the tree, so it runs while the host lays out the boxes.
   // Its allocations are made on the tree's stream before the fork event.
-  const int KSPLIT = tune_.ksplit, KSPLIT_ROOT = tune_.ksplit_root;
+  // A small system would leave most SMs idle behind a few blocks that each
+  // walk all particles: its items are cut until about two waves of blocks are
+  // there (not below 64 particles, where the partials' sum costs more).
+  auto fill_split = [&](int split, long particles, int tiles, int resident) {
+    const long want = (2L * resident + tiles - 1) / tiles;  // items for two waves
+    return int(std::min<long>(split, std::max<long>(64, (particles + want - 1) / std::max<long>(want, 1))));
+  };
+  const int KSPLIT_ROOT = mixed ? tune_.ksplit_root : fill_split(tune_.ksplit_root, D.n_slots, nudft_tiles(D.n_window), 296);
+  const long pw_levels = std::max(0, D.pw_hi - D.pw_lo + 1);
+  const int KSPLIT = mixed ? tune_.ksplit
+                           : fill_split(tune_.ksplit, pw_levels * D.n_slots, nudft_tiles(D.n_diff), 296);
   const int nch_root = std::max(1, (D.n_slots + KSPLIT_ROOT - 1) / KSPLIT_ROOT);
   std::vector<Chunked> root_split{{0, nch_root, D.out_root}};
   double2* part_r = nullptr;
@@ -1128,9 +1075,8 @@ void DmkTree::form_outgoing_pw() {
   for (int c = 0; c < nch_root; ++c) {
     int sb = c * KSPLIT_ROOT, se = std::min(D.n_slots, sb + KSPLIT_ROOT);
     if (mixed) make_mix(mroot, D.n_window, 0, 0, part_r + size_t(c) * D.Hw, sb, se);
-    else make_work(wroot, D.n_window, 0, 0, part_r + size_t(c) * D.Hw, sb, se);
+    else make_work(wroot, 0, 0, part_r + size_t(c) * D.Hw, sb, se);
   }
-  double2* tab_root = nullptr;
   unsigned char* mtab_root = nullptr;
   std::vector<int2> ch_root;
   size_t rch, rmeta, rout;
@@ -1139,7 +1085,6 @@ void DmkTree::form_outgoing_pw() {
     plan_mix_tables(D.n_window, mroot, &mtab_root, ch_root);
     d_root = upload(mroot, ch_root, root_split, &rch, &rmeta, &rout);
   } else {
-    plan_nudft_tables(D.n_window, wroot, &tab_root, ch_root, st_);
     d_root = upload(wroot, ch_root, root_split, &rch, &rmeta, &rout);
   }
   PDMK_CUDA(cudaEventRecord(ev_fork_, st_));
@@ -1148,8 +1093,7 @@ void DmkTree::form_outgoing_pw() {
     dispatch_mixed(D.n_window, tmap_root, reinterpret_cast<const MixItem*>(d_root), int(mroot.size()),
                    reinterpret_cast<const int2*>(d_root + rch), int(ch_root.size()), d_mix_, d_mix_err, aux_);
   else
-    dispatch_nudft(D.n_window, reinterpret_cast<const NudftWork*>(d_root), int(wroot.size()),
-                   reinterpret_cast<const int2*>(d_root + rch), int(ch_root.size()), D, aux_);
+    dispatch_nudft(D.n_window, reinterpret_cast<const NudftWork*>(d_root), int(wroot.size()), D, aux_);
   reduce(root_split, part_r, D.Hw, d_root, rmeta, rout, aux_);
   PDMK_CUDA(cudaEventRecord(ev_join_, aux_));
 
@@ -1202,7 +1146,7 @@ void DmkTree::form_outgoing_pw() {
     long cur = 0;
     auto add = [&](int l, uint64_t p, double2* out, int sb, int se) {
       if (mixed) make_mix(mbox, D.n_diff, l, p, out, sb, se);
-      else make_work(wbox, D.n_diff, l, p, out, sb, se);
+      else make_work(wbox, l, p, out, sb, se);
     };
     for (int oi : order) {
       const Box& bx = boxes[oi];
@@ -1220,7 +1164,6 @@ void DmkTree::form_outgoing_pw() {
       }
     }
   }
-  double2* tab_box = nullptr;
   unsigned char* mtab_box = nullptr;
   std::vector<int2> ch_box;
   size_t bch, bmeta, bout;
@@ -1229,7 +1172,6 @@ void DmkTree::form_outgoing_pw() {
     plan_mix_tables(D.n_diff, mbox, &mtab_box, ch_box);
     d_box = upload(mbox, ch_box, box_split, &bch, &bmeta, &bout);
   } else {
-    plan_nudft_tables(D.n_diff, wbox, &tab_box, ch_box, st_);
     d_box = upload(wbox, ch_box, box_split, &bch, &bmeta, &bout);
   }
   time_begin(3);
@@ -1237,15 +1179,13 @@ void DmkTree::form_outgoing_pw() {
     dispatch_mixed(D.n_diff, tmap_box, reinterpret_cast<const MixItem*>(d_box), int(mbox.size()),
                    reinterpret_cast<const int2*>(d_box + bch), int(ch_box.size()), d_mix_, d_mix_err, st_);
   else
-    dispatch_nudft(D.n_diff, reinterpret_cast<const NudftWork*>(d_box), int(wbox.size()),
-                   reinterpret_cast<const int2*>(d_box + bch), int(ch_box.size()), D, st_);
+    dispatch_nudft(D.n_diff, reinterpret_cast<const NudftWork*>(d_box), int(wbox.size()), D, st_);
   time_end(3);
   reduce(box_split, part_b, D.H, d_box, bmeta, bout, st_);
   // the root pass's buffers are released after it joins the tree's stream
   PDMK_CUDA(cudaStreamWaitEvent(st_, ev_join_, 0));
-  for (void* p : {static_cast<void*>(d_root), static_cast<void*>(tab_root), static_cast<void*>(mtab_root),
-                  static_cast<void*>(part_r), static_cast<void*>(d_box), static_cast<void*>(tab_box),
-                  static_cast<void*>(mtab_box), static_cast<void*>(part_b)})
+  for (void* p : {static_cast<void*>(d_root), static_cast<void*>(mtab_root), static_cast<void*>(part_r),
+                  static_cast<void*>(d_box), static_cast<void*>(mtab_box), static_cast<void*>(part_b)})
     if (p) PDMK_CUDA(cudaFreeAsync(p, st_));
   diff_cached_ = false;
 }
@@ -1463,7 +1403,6 @@ double DmkTree::ewald_energy(double* parts) {
   const int Hs = (2 * nk + 1) * (2 * nk + 1) * (nk + 1);
   const int kspl = std::max(4096, (D.n_slots + 295) / 296);
   const int nch = std::max(1, (D.n_slots + kspl - 1) / kspl);
-  const int tiles = nudft_tiles(nk);
   std::vector<NudftWork> wl;
   for (int c = 0; c < nch; ++c) {
     NudftWork w{};
@@ -1472,10 +1411,7 @@ double DmkTree::ewald_energy(double* parts) {
     w.M = 3;  // exp(-i k L/2) = (-1)^m: the root's decentring
     w.s_begin = c * kspl;
     w.s_end = std::min(D.n_slots, (c + 1) * kspl);
-    for (int t = 0; t < tiles; ++t) {
-      w.row_tile = t;
-      wl.push_back(w);
-    }
+    wl.push_back(w);
   }
   double2* part = nullptr;
   double2* S = nullptr;
@@ -1485,20 +1421,10 @@ double DmkTree::ewald_energy(double* parts) {
   PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&part), sizeof(double2) * size_t(Hs) * nch, st_));
   PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&S), sizeof(double2) * size_t(Hs), st_));
   PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&sums), sizeof(double) * (nblk_real + nblk_rec + 8), st_));
-  for (size_t i = 0; i < wl.size(); ++i) wl[i].out = part + size_t(i / tiles) * Hs;
-  double2* tab = nullptr;
-  std::vector<int2> chunks;
-  plan_nudft_tables(nk, wl, &tab, chunks, st_);
-  const size_t off_ch = (sizeof(NudftWork) * wl.size() + 15) & ~size_t(15);
-  std::vector<unsigned char> blob(off_ch + sizeof(int2) * chunks.size() + 16, 0);
-  std::memcpy(blob.data(), wl.data(), sizeof(NudftWork) * wl.size());
-  std::memcpy(blob.data() + off_ch, chunks.data(), sizeof(int2) * chunks.size());
-  PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d_work), blob.size(), st_));
-  PDMK_CUDA(cudaMemcpyAsync(d_work, blob.data(), blob.size(), cudaMemcpyHostToDevice, st_));
-  dispatch_nudft(nk, d_work, int(wl.size()),
-                 reinterpret_cast<const int2*>(reinterpret_cast<unsigned char*>(d_work) + off_ch), int(chunks.size()),
-                 D, st_);
-  PDMK_CUDA(cudaFreeAsync(tab, st_));
+  for (size_t i = 0; i < wl.size(); ++i) wl[i].out = part + i * size_t(Hs);
+  PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d_work), sizeof(NudftWork) * wl.size(), st_));
+  PDMK_CUDA(cudaMemcpyAsync(d_work, wl.data(), sizeof(NudftWork) * wl.size(), cudaMemcpyHostToDevice, st_));
+  dispatch_nudft(nk, d_work, int(wl.size()), D, st_);
   {
     int* d_meta;
     double2** d_outs;
