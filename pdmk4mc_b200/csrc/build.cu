@@ -344,7 +344,7 @@ __global__ void k_leaf_dfs_index(int nl, const int* lid, int* dfs_of_node) {
 
 __global__ void k_node_slots(int n_nodes, const int* child0, const int* dfs_of_node, const int* begin, const int* cap,
                              const int* cnt, const int* cnt_prefix, int* node_begin, int* node_end, int* leaf_count,
-                             int* node_count) {
+                             int* node_count, int* node_dense) {
   int id = blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= n_nodes) return;
   int f = id, g = id;
@@ -355,6 +355,33 @@ __global__ void k_node_slots(int n_nodes, const int* child0, const int* dfs_of_n
   node_end[id] = begin[jg] + cap[jg];
   leaf_count[id] = (child0[id] < 0) ? cnt[jf] : 0;
   node_count[id] = cnt_prefix[jg] + cnt[jg] - cnt_prefix[jf];
+  node_dense[id] = cnt_prefix[jf];
+}
+
+// after moves: the leaves' particles, without the free slots between them,
+// and every node's first one (dense: four rows x, y, z, q of `stride`)
+__global__ void k_gather_dense(int nl, const int* lid, const int* node_begin, const int* leaf_count,
+                               const int* dense_begin, const double* sx, const double* sy, const double* sz,
+                               const double* sq, double* dense, long stride) {
+  const int j = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;  // a warp per leaf
+  if (j >= nl) return;
+  const int id = lid[j], b = node_begin[id], c = leaf_count[id];
+  const long d = dense_begin[j];
+  for (int t = threadIdx.x & 31; t < c; t += 32) {
+    dense[d + t] = sx[b + t];
+    dense[stride + d + t] = sy[b + t];
+    dense[2 * stride + d + t] = sz[b + t];
+    dense[3 * stride + d + t] = sq[b + t];
+  }
+}
+
+__global__ void k_node_dense(int n_nodes, const int* child0, const int* dfs_of_node, const int* dense_begin,
+                             int* node_dense) {
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= n_nodes) return;
+  int f = id;
+  while (child0[f] >= 0) f = child0[f];
+  node_dense[id] = dense_begin[dfs_of_node[f]];
 }
 
 // repack: gather live particles leaf by leaf (slots, then pool entries)
@@ -528,11 +555,12 @@ void DmkTree::build(const double* r_in, const double* q_in, bool on_device) {
   k_keys<<<grid_for(n), TPB, 0, st_>>>(r, n, L_, keys, ord);
   PDMK_LAUNCH_CHECK();
   radix_sort_pairs(keys, ord, n, 8, sort_scr, st_);
-  double *dsx, *dsy, *dsz, *dsq;
-  PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&dsx), size_t(4 * n) * sizeof(double) + 64, st_));
-  dsy = dsx + n;
-  dsz = dsy + n;
-  dsq = dsz + n;
+  // the sorted particles, kept for the outgoing pass: four rows x, y, z, q
+  // (read as one 2-D tensor by the mixed pass, so the stride is even)
+  dense_stride_ = (n + 31) & ~31L;
+  dense_ = static_cast<double*>(alloc(size_t(4 * dense_stride_) * sizeof(double)));
+  double *dsx = dense_, *dsy = dsx + dense_stride_, *dsz = dsy + dense_stride_, *dsq = dsz + dense_stride_;
+  dense_ready_ = true;
   k_gather_sorted<<<grid_for(n), TPB, 0, st_>>>(r, q, ord, n, dsx, dsy, dsz, dsq);
   PDMK_LAUNCH_CHECK();
   if (tmp_in) PDMK_CUDA(cudaFreeAsync(tmp_in, st_));
@@ -574,8 +602,7 @@ void DmkTree::build(const double* r_in, const double* q_in, bool on_device) {
     PDMK_CUDA(cudaStreamSynchronize(st_));
     if (cnt[kBadWord] != 0) {
       for (void* p : {static_cast<void*>(d_lvl), static_cast<void*>(keys), static_cast<void*>(ord), sort_scr,
-                      static_cast<void*>(dsx), static_cast<void*>(d_cnt), static_cast<void*>(lists[0]),
-                      static_cast<void*>(lists[1])})
+                      static_cast<void*>(d_cnt), static_cast<void*>(lists[0]), static_cast<void*>(lists[1])})
         PDMK_CUDA(cudaFreeAsync(p, st_));
       throw BadInput("positions must lie in [0, L) and charges be finite");
     }
@@ -720,6 +747,7 @@ void DmkTree::build(const double* r_in, const double* q_in, bool on_device) {
   D.node_end = static_cast<int*>(alloc(sizeof(int) * n_nodes));
   D.leaf_count = static_cast<int*>(alloc(sizeof(int) * n_nodes));
   D.node_count = static_cast<int*>(alloc(sizeof(int) * n_nodes));
+  node_dense_ = static_cast<int*>(alloc(sizeof(int) * n_nodes));
   D.orig_slot = static_cast<int*>(alloc(sizeof(int) * std::max<long>(n, 1)));
   // persistent per-leaf arrays kept for repacking
   leaf_dev_.lid = lid;
@@ -735,7 +763,6 @@ void DmkTree::build(const double* r_in, const double* q_in, bool on_device) {
   PDMK_CUDA(cudaFreeAsync(src_lo, st_));
   PDMK_CUDA(cudaFreeAsync(lkey, st_));
   PDMK_CUDA(cudaFreeAsync(node_lo, st_));
-  PDMK_CUDA(cudaFreeAsync(dsx, st_));
   PDMK_CUDA(cudaFreeAsync(sort_scr, st_));
   PDMK_CUDA(cudaFreeAsync(ord, st_));
   PDMK_CUDA(cudaFreeAsync(keys, st_));
@@ -806,7 +833,7 @@ void DmkTree::layout_slots(const double* dsx, const double* dsy, const double* d
   PDMK_LAUNCH_CHECK();
   k_node_slots<<<grid_for(D.n_nodes), TPB, 0, st_>>>(D.n_nodes, D.node_child0, leaf_dev_.dfs_of_node, begin,
                                                     leaf_dev_.cap, leaf_dev_.cnt, leaf_dev_.cnt_prefix, D.node_begin,
-                                                    D.node_end, D.leaf_count, D.node_count);
+                                                    D.node_end, D.leaf_count, D.node_count, node_dense_);
   PDMK_LAUNCH_CHECK();
 }
 
@@ -836,19 +863,19 @@ void DmkTree::repack(int leaf_slack) {
     PDMK_CUDA(cudaFreeAsync(scr, st_));
   }
   const long n = N_;
-  double* dense;
+  double* dense = dense_;
+  const long ds = dense_stride_;
   int* dorig;
-  PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&dense), sizeof(double) * 4 * size_t(n) + 64, st_));
   PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&dorig), sizeof(int) * size_t(n) + 64, st_));
   k_repack_gather_slots<<<unsigned(std::max(nl, 1)), 128, 0, st_>>>(nl, leaf_dev_.lid, D.node_begin, D.leaf_count,
                                                                    dense_begin, D.sx, D.sy, D.sz, D.sq, D.s_orig,
-                                                                   dense, dense + n, dense + 2 * n, dense + 3 * n, dorig);
+                                                                   dense, dense + ds, dense + 2 * ds, dense + 3 * ds, dorig);
   PDMK_LAUNCH_CHECK();
   if (pool_used > 0) {
     PDMK_CUDA(cudaMemsetAsync(fill, 0, sizeof(int) * nl, st_));
     k_repack_gather_pool<<<1, 1, 0, st_>>>(pool_used, D.p_leaf, D.p_orig, D.px, D.py, D.pz, D.pq,
-                                          leaf_dev_.dfs_of_node, dense_begin, old_cnt, fill, dense, dense + n,
-                                          dense + 2 * n, dense + 3 * n, dorig);
+                                          leaf_dev_.dfs_of_node, dense_begin, old_cnt, fill, dense, dense + ds,
+                                          dense + 2 * ds, dense + 3 * ds, dorig);
     PDMK_LAUNCH_CHECK();
   }
   PDMK_CUDA(cudaMemcpyAsync(leaf_dev_.cnt, cnt2, sizeof(int) * nl, cudaMemcpyDeviceToDevice, st_));
@@ -856,13 +883,34 @@ void DmkTree::repack(int leaf_slack) {
   PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&src_lo), sizeof(long) * size_t(nl) + 16, st_));
   k_caps_from_counts<<<grid_for(nl), TPB, 0, st_>>>(nl, cnt2, leaf_slack, leaf_dev_.cap, src_lo, dense_begin);
   PDMK_LAUNCH_CHECK();
-  layout_slots(dense, dense + n, dense + 2 * n, dense + 3 * n, dorig, src_lo, leaf_slack);
+  layout_slots(dense, dense + ds, dense + 2 * ds, dense + 3 * ds, dorig, src_lo, leaf_slack);
+  dense_ready_ = true;
   PDMK_CUDA(cudaMemsetAsync(D.pool_n, 0, 4, st_));
   PDMK_CUDA(cudaFreeAsync(src_lo, st_));
-  PDMK_CUDA(cudaFreeAsync(dense, st_));
   PDMK_CUDA(cudaFreeAsync(dorig, st_));
   PDMK_CUDA(cudaFreeAsync(old_cnt, st_));
   PDMK_CUDA(cudaStreamSynchronize(st_));
+}
+
+// The particles without the free slots, for the outgoing pass: kept from the
+// build or the last pack, gathered again after moves.
+void DmkTree::ensure_dense() {
+  if (dense_ready_) return;
+  DevTree& D = dev_;
+  const int nl = leaf_dev_.n;
+  int* cnt;
+  PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&cnt), sizeof(int) * 2 * size_t(nl) + scan_scratch_bytes(nl), st_));
+  int* begin = cnt + nl;
+  k_leaf_counts_from_nodes<<<grid_for(nl), TPB, 0, st_>>>(nl, leaf_dev_.lid, D.leaf_count, cnt);
+  PDMK_LAUNCH_CHECK();
+  exclusive_scan(cnt, begin, nl, begin + nl, st_);
+  k_gather_dense<<<unsigned((nl + 7) / 8), 256, 0, st_>>>(nl, leaf_dev_.lid, D.node_begin, D.leaf_count, begin, D.sx, D.sy,
+                                                          D.sz, D.sq, dense_, dense_stride_);
+  PDMK_LAUNCH_CHECK();
+  k_node_dense<<<grid_for(D.n_nodes), TPB, 0, st_>>>(D.n_nodes, D.node_child0, leaf_dev_.dfs_of_node, begin, node_dense_);
+  PDMK_LAUNCH_CHECK();
+  PDMK_CUDA(cudaFreeAsync(cnt, st_));
+  dense_ready_ = true;
 }
 
 // ---------------------------------------------------------------------------

@@ -47,7 +47,9 @@ __device__ inline double block_sum(double v, double* sm) {
 }
 
 // ---------------------------------------------------------------------------
-// NUDFT work item: one box (or one split-K chunk of it) over one slot range
+// NUDFT work item: one box (or one split-K chunk of it) over a range of the
+// particles in leaf order, pos = rows x, y, z, q (without the leaves' free
+// slots, which were 26 % of the slots at N = 1e6)
 struct NudftWork {
   double cx, cy, cz;  // box centre
   double dk;
@@ -86,14 +88,14 @@ struct NudftShape {
 };
 
 // Factors of a chunk's particles into shared memory, one thread per particle
-// and axis: cos and sin of m th, m = 0 .. NK, by two interleaved chains of
-// steps exp(2 i th); the charge is folded into fz. Particles past the end get
-// zeros. (A block spends about 3 % of its time here; a separate pass wrote
-// and read 1.6 KB per particle and level, 2.8 ms at N = 1e6.)
+// and axis: cos and sin of m th, m = 0 .. NK, by four interleaved chains of
+// steps exp(4 i th) (its own sincos: the chains add roundings, not a drift);
+// the charge is folded into fz. Particles past the end get zeros. (A block
+// spends about 3 % of its time here; a separate pass wrote and read 1.6 KB
+// per particle and level, 2.8 ms at N = 1e6.)
 template <int NK>
-__device__ __forceinline__ void nudft_factors(const NudftWork& w, int base, double* buf, const double* __restrict__ sx,
-                                              const double* __restrict__ sy, const double* __restrict__ sz,
-                                              const double* __restrict__ sq) {
+__device__ __forceinline__ void nudft_factors(const NudftWork& w, int base, double* buf, const double* __restrict__ pos,
+                                              long stride) {
   using S = NudftShape<NK>;
   for (int t = threadIdx.x; t < S::KC * 3; t += S::THREADS) {
     const int j = t % S::KC, axis = t / S::KC, s = base + j;
@@ -102,26 +104,33 @@ __device__ __forceinline__ void nudft_factors(const NudftWork& w, int base, doub
       for (int e = 0; e < 2 * S::N1; ++e) dst[e] = 0.0;
       continue;
     }
-    const double x = axis == 0 ? sx[s] - w.cx : (axis == 1 ? sy[s] - w.cy : sz[s] - w.cz);
-    const double sc = axis == 2 ? sq[s] : 1.0;
+    const double x = pos[axis * stride + s] - (axis == 0 ? w.cx : (axis == 1 ? w.cy : w.cz));
+    const double sc = axis == 2 ? pos[3 * stride + s] : 1.0;
+    const double th = w.dk * x;
     double sn, cs;
-    sincos(w.dk * x, &sn, &cs);
-    const double2 z1 = make_double2(cs, sn), st = cmul(z1, z1);
-    double2 e = make_double2(sc, 0.0), o = make_double2(cs * sc, sn * sc);
-#pragma unroll 2
-    for (int m = 0; m < S::N1; m += 2) {
-      *reinterpret_cast<double2*>(dst + 2 * m) = e;
-      e = cmul(e, st);
-      if (m + 1 < S::N1) *reinterpret_cast<double2*>(dst + 2 * m + 2) = o;
-      o = cmul(o, st);
-    }
+    sincos(4.0 * th, &sn, &cs);
+    const double2 st = make_double2(cs, sn);
+    sincos(th, &sn, &cs);
+    const double2 z1 = make_double2(cs, sn);
+    double2 v[4];
+    v[0] = make_double2(sc, 0.0);
+    v[1] = cscale(z1, sc);
+    v[2] = cmul(v[1], z1);
+    v[3] = cmul(v[2], z1);
+#pragma unroll 1
+    for (int m = 0; m < S::N1; m += 4)
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if (m + c < S::N1) {
+          *reinterpret_cast<double2*>(dst + 2 * (m + c)) = v[c];
+          v[c] = cmul(v[c], st);
+        }
   }
 }
 
 template <int NK>
 __global__ void __launch_bounds__(NudftShape<NK>::THREADS, 2)
-    k_nudft(const NudftWork* __restrict__ work, const double* __restrict__ sx, const double* __restrict__ sy,
-            const double* __restrict__ sz, const double* __restrict__ sq) {
+    k_nudft(const NudftWork* __restrict__ work, const double* __restrict__ pos, long stride) {
   using S = NudftShape<NK>;
   constexpr int NT = S::NT, CPW = S::CPW, STR = S::STR, N1 = S::N1, D = S::D;
   extern __shared__ double smem_d[];
@@ -144,22 +153,26 @@ __global__ void __launch_bounds__(NudftShape<NK>::THREADS, 2)
     for (int z = 0; z < 2; ++z)
 #pragma unroll
       for (int t = 0; t < NT; ++t) acc[i][z][t][0] = acc[i][z][t][1] = 0.0;
+  __shared__ double2 roots[6];  // exp(-i pi m / 3)
+  if (threadIdx.x < 6) roots[threadIdx.x] = root6(-int(threadIdx.x));
   // the entries past the last mode stay zero
   constexpr int PADN = 8 * NT - 2 * N1;
   if constexpr (PADN > 0)
     for (int t = threadIdx.x; t < 2 * S::KC * 3 * PADN; t += S::THREADS)
       smem_d[(t / (3 * PADN)) * STR + (t / PADN % 3) * 8 * NT + 2 * N1 + t % PADN] = 0.0;
   const int nch = (w.s_end - w.s_begin + S::KC - 1) / S::KC;
-  if (nch > 0) nudft_factors<NK>(w, w.s_begin, smem_d, sx, sy, sz, sq);
+  if (nch > 0) nudft_factors<NK>(w, w.s_begin, smem_d, pos, stride);
   __syncthreads();
   for (int ci = 0; ci < nch; ++ci) {
     // the next chunk's factors (its buffer was last read before the barrier
     // that closed the previous iteration)
-    if (ci + 1 < nch) nudft_factors<NK>(w, w.s_begin + (ci + 1) * S::KC, smem_d + ((ci + 1) & 1) * S::KC * STR, sx, sy, sz, sq);
+    if (ci + 1 < nch) nudft_factors<NK>(w, w.s_begin + (ci + 1) * S::KC, smem_d + ((ci + 1) & 1) * S::KC * STR, pos, stride);
     const double* buf = smem_d + (ci & 1) * S::KC * STR + q4 * STR;
     if (g0 < S::PAIRS) {
+      // the last chunk of a short box is mostly empty: only its filled steps
+      const int steps = min(S::KC / 4, (w.s_end - w.s_begin - ci * S::KC + 3) / 4);
 #pragma unroll 1
-      for (int ks = 0; ks < S::KC / 4; ++ks) {
+      for (int ks = 0; ks < steps; ++ks) {
         const double* row = buf + 4 * ks * STR;
         double b[NT];
 #pragma unroll
@@ -188,7 +201,7 @@ __global__ void __launch_bounds__(NudftShape<NK>::THREADS, 2)
   // other; the first takes ky = +q, the second ky = -q.
   const int odd = q8 & 1;
   const double sg = odd ? -1.0 : 1.0;
-  const int dx = w.M * (2 * w.X + 1), dy = w.M * (2 * w.Y + 1), dz = w.M * (2 * w.Z + 1);
+  const int dx = w.M * (2 * w.X + 1) % 6, dy = w.M * (2 * w.Y + 1) % 6, dz = w.M * (2 * w.Z + 1) % 6;
 #pragma unroll
   for (int i = 0; i < CPW; ++i) {
     const int g = g0 + i, p = g / NT, q = 4 * (g % NT) + (q8 >> 1);
@@ -217,7 +230,7 @@ __global__ void __launch_bounds__(NudftShape<NK>::THREADS, 2)
           const double a1 = c[0] - st * sv[1], b1 = sg * sv[0] + ta * c[1];
           const double a2 = c[2] - st * sv[3], b2 = sg * sv[2] + ta * c[3];
           const int ky = odd ? -q : q, kx = h ? -r : r;
-          const double2 v = cmul(make_double2(a1 + b2, a2 - b1), root6(-(dx * kx + dy * ky - dz * p)));
+          const double2 v = cmul(make_double2(a1 + b2, a2 - b1), roots[unsigned(dx * kx + dy * ky - dz * p + 30 * NK) % 6u]);
           w.out[(size_t(NK - p) * D + NK + ky) * D + NK + kx] = v;
         }
       }
@@ -226,12 +239,12 @@ __global__ void __launch_bounds__(NudftShape<NK>::THREADS, 2)
 }
 
 template <int NK>
-void launch_nudft(const NudftWork* d_work, int nwork, const DevTree& T, cudaStream_t st) {
+void launch_nudft(const NudftWork* d_work, int nwork, const double* pos, long stride, cudaStream_t st) {
   using S = NudftShape<NK>;
   if (nwork == 0) return;
   // per device and thread-safe: replica energies call this from several host threads
   raise_smem_limit(reinterpret_cast<const void*>(k_nudft<NK>), S::SMEM);
-  k_nudft<NK><<<unsigned(nwork) * S::TILES, S::THREADS, S::SMEM, st>>>(d_work, T.sx, T.sy, T.sz, T.sq);
+  k_nudft<NK><<<unsigned(nwork) * S::TILES, S::THREADS, S::SMEM, st>>>(d_work, pos, stride);
   PDMK_LAUNCH_CHECK();
 }
 
@@ -252,18 +265,18 @@ int nudft_tiles(int nk) {
   }
 }
 
-void dispatch_nudft(int nk, const NudftWork* d_work, int nwork, const DevTree& T, cudaStream_t st) {
+void dispatch_nudft(int nk, const NudftWork* d_work, int nwork, const double* pos, long stride, cudaStream_t st) {
   switch (nk) {
-    case 4: launch_nudft<4>(d_work, nwork, T, st); break;
-    case 6: launch_nudft<6>(d_work, nwork, T, st); break;
-    case 8: launch_nudft<8>(d_work, nwork, T, st); break;
-    case 12: launch_nudft<12>(d_work, nwork, T, st); break;
-    case 13: launch_nudft<13>(d_work, nwork, T, st); break;
-    case 17: launch_nudft<17>(d_work, nwork, T, st); break;
-    case 19: launch_nudft<19>(d_work, nwork, T, st); break;
-    case 26: launch_nudft<26>(d_work, nwork, T, st); break;
-    case 32: launch_nudft<32>(d_work, nwork, T, st); break;
-    case 64: launch_nudft<64>(d_work, nwork, T, st); break;
+    case 4: launch_nudft<4>(d_work, nwork, pos, stride, st); break;
+    case 6: launch_nudft<6>(d_work, nwork, pos, stride, st); break;
+    case 8: launch_nudft<8>(d_work, nwork, pos, stride, st); break;
+    case 12: launch_nudft<12>(d_work, nwork, pos, stride, st); break;
+    case 13: launch_nudft<13>(d_work, nwork, pos, stride, st); break;
+    case 17: launch_nudft<17>(d_work, nwork, pos, stride, st); break;
+    case 19: launch_nudft<19>(d_work, nwork, pos, stride, st); break;
+    case 26: launch_nudft<26>(d_work, nwork, pos, stride, st); break;
+    case 32: launch_nudft<32>(d_work, nwork, pos, stride, st); break;
+    case 64: launch_nudft<64>(d_work, nwork, pos, stride, st); break;
     default: throw std::invalid_argument("unsupported mode count");
   }
 }
@@ -933,7 +946,9 @@ void DmkTree::ensure_packed() {
 
 void DmkTree::form_outgoing_pw() {
   ensure_packed();
+  ensure_dense();
   DevTree& D = dev_;
+  const int n_all = int(N_);
   // split-K bookkeeping: chunks go to a partial buffer, then reduce
   struct Chunked {
     int first, n;
@@ -987,11 +1002,11 @@ void DmkTree::form_outgoing_pw() {
       PDMK_CUDA(cudaMemsetAsync(d_mix_, 0, sizeof(double) * 2, st_));
     }
     if (!qmax_ready_) {
-      launch_absmax(D.sq, D.n_slots, d_mix_, st_);
+      launch_absmax(dense_ + 3 * dense_stride_, n_all, d_mix_, st_);
       qmax_ready_ = true;
     }
-    make_coord_map(&tmap_root, D.sx, slot_capacity_, mixed_chunk(D.n_window));
-    make_coord_map(&tmap_box, D.sx, slot_capacity_, mixed_chunk(D.n_diff));
+    make_coord_map(&tmap_root, dense_, int(dense_stride_), mixed_chunk(D.n_window));
+    make_coord_map(&tmap_box, dense_, int(dense_stride_), mixed_chunk(D.n_diff));
   }
   int* d_mix_err = mixed ? reinterpret_cast<int*>(d_mix_ + 1) : nullptr;
   auto align16 = [](size_t b) { return (b + 15) & ~size_t(15); };
@@ -1062,18 +1077,18 @@ void DmkTree::form_outgoing_pw() {
     const long want = (2L * resident + tiles - 1) / tiles;  // items for two waves
     return int(std::min<long>(split, std::max<long>(64, (particles + want - 1) / std::max<long>(want, 1))));
   };
-  const int KSPLIT_ROOT = mixed ? tune_.ksplit_root : fill_split(tune_.ksplit_root, D.n_slots, nudft_tiles(D.n_window), 296);
+  const int KSPLIT_ROOT = mixed ? tune_.ksplit_root : fill_split(tune_.ksplit_root, n_all, nudft_tiles(D.n_window), 296);
   const long pw_levels = std::max(0, D.pw_hi - D.pw_lo + 1);
   const int KSPLIT = mixed ? tune_.ksplit
-                           : fill_split(tune_.ksplit, pw_levels * D.n_slots, nudft_tiles(D.n_diff), 296);
-  const int nch_root = std::max(1, (D.n_slots + KSPLIT_ROOT - 1) / KSPLIT_ROOT);
+                           : fill_split(tune_.ksplit, pw_levels * n_all, nudft_tiles(D.n_diff), 296);
+  const int nch_root = std::max(1, (n_all + KSPLIT_ROOT - 1) / KSPLIT_ROOT);
   std::vector<Chunked> root_split{{0, nch_root, D.out_root}};
   double2* part_r = nullptr;
   PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&part_r), sizeof(double2) * (size_t(nch_root) * D.Hw + 1), st_));
   std::vector<NudftWork> wroot;
   std::vector<MixItem> mroot;
   for (int c = 0; c < nch_root; ++c) {
-    int sb = c * KSPLIT_ROOT, se = std::min(D.n_slots, sb + KSPLIT_ROOT);
+    int sb = c * KSPLIT_ROOT, se = std::min(n_all, sb + KSPLIT_ROOT);
     if (mixed) make_mix(mroot, D.n_window, 0, 0, part_r + size_t(c) * D.Hw, sb, se);
     else make_work(wroot, 0, 0, part_r + size_t(c) * D.Hw, sb, se);
   }
@@ -1093,17 +1108,17 @@ void DmkTree::form_outgoing_pw() {
     dispatch_mixed(D.n_window, tmap_root, reinterpret_cast<const MixItem*>(d_root), int(mroot.size()),
                    reinterpret_cast<const int2*>(d_root + rch), int(ch_root.size()), d_mix_, d_mix_err, aux_);
   else
-    dispatch_nudft(D.n_window, reinterpret_cast<const NudftWork*>(d_root), int(wroot.size()), D, aux_);
+    dispatch_nudft(D.n_window, reinterpret_cast<const NudftWork*>(d_root), int(wroot.size()), dense_, dense_stride_, aux_);
   reduce(root_split, part_r, D.Hw, d_root, rmeta, rout, aux_);
   PDMK_CUDA(cudaEventRecord(ev_join_, aux_));
 
-  // host view of node slot ranges and coordinates for the box work list
+  // host view of the nodes' particle ranges and coordinates for the box work list
   // (and, on a new tree, of the children for the box lists: one round trip)
   const int nn = D.n_nodes;
   std::vector<int> nb(nn), ne(nn), lv(nn), c0;
   std::vector<uint64_t> pf(nn);
-  PDMK_CUDA(cudaMemcpyAsync(nb.data(), D.node_begin, 4 * nn, cudaMemcpyDeviceToHost, st_));
-  PDMK_CUDA(cudaMemcpyAsync(ne.data(), D.node_end, 4 * nn, cudaMemcpyDeviceToHost, st_));
+  PDMK_CUDA(cudaMemcpyAsync(nb.data(), node_dense_, 4 * nn, cudaMemcpyDeviceToHost, st_));
+  PDMK_CUDA(cudaMemcpyAsync(ne.data(), D.node_count, 4 * nn, cudaMemcpyDeviceToHost, st_));
   PDMK_CUDA(cudaMemcpyAsync(lv.data(), D.node_level, 4 * nn, cudaMemcpyDeviceToHost, st_));
   PDMK_CUDA(cudaMemcpyAsync(pf.data(), D.node_prefix, 8 * nn, cudaMemcpyDeviceToHost, st_));
   if (!box_lists_ready_) {
@@ -1120,7 +1135,7 @@ void DmkTree::form_outgoing_pw() {
   const int base = D.level_start[D.pw_lo];
   if (D.pw_hi >= D.pw_lo)
     for (int id = base; id < D.level_start[D.pw_hi + 1]; ++id)
-      boxes.push_back({id, nb[id], ne[id], lv[id], D.out + size_t(id - base) * D.H});
+      boxes.push_back({id, nb[id], nb[id] + ne[id], lv[id], D.out + size_t(id - base) * D.H});
   // boxes: largest first (longest-processing-time order), split when large
   std::vector<int> order(boxes.size());
   for (size_t i = 0; i < order.size(); ++i) order[i] = int(i);
@@ -1179,7 +1194,7 @@ void DmkTree::form_outgoing_pw() {
     dispatch_mixed(D.n_diff, tmap_box, reinterpret_cast<const MixItem*>(d_box), int(mbox.size()),
                    reinterpret_cast<const int2*>(d_box + bch), int(ch_box.size()), d_mix_, d_mix_err, st_);
   else
-    dispatch_nudft(D.n_diff, reinterpret_cast<const NudftWork*>(d_box), int(wbox.size()), D, st_);
+    dispatch_nudft(D.n_diff, reinterpret_cast<const NudftWork*>(d_box), int(wbox.size()), dense_, dense_stride_, st_);
   time_end(3);
   reduce(box_split, part_b, D.H, d_box, bmeta, bout, st_);
   // the root pass's buffers are released after it joins the tree's stream
@@ -1384,6 +1399,7 @@ EnergyParts DmkTree::eval_energy() {
 // system is large; the k cube then needs 32 or 64 modes per axis half.
 double DmkTree::ewald_energy(double* parts) {
   ensure_packed();
+  ensure_dense();
   DevTree& D = dev_;
   const double s = 5.0, pi = 3.14159265358979323846;
   const bool l3 = D.max_depth > 4 && D.level_start[4] - D.level_start[3] == 512 && D.n_slots > 300000;
@@ -1401,8 +1417,9 @@ double DmkTree::ewald_energy(double* parts) {
   const int ny = (maxc + RES_TCH - 1) / RES_TCH;
   // structure factor by the NUDFT over all slots, split in chunks
   const int Hs = (2 * nk + 1) * (2 * nk + 1) * (nk + 1);
-  const int kspl = std::max(4096, (D.n_slots + 295) / 296);
-  const int nch = std::max(1, (D.n_slots + kspl - 1) / kspl);
+  const int n_all = int(N_);
+  const int kspl = std::max(4096, (n_all + 295) / 296);
+  const int nch = std::max(1, (n_all + kspl - 1) / kspl);
   std::vector<NudftWork> wl;
   for (int c = 0; c < nch; ++c) {
     NudftWork w{};
@@ -1410,7 +1427,7 @@ double DmkTree::ewald_energy(double* parts) {
     w.dk = dk;
     w.M = 3;  // exp(-i k L/2) = (-1)^m: the root's decentring
     w.s_begin = c * kspl;
-    w.s_end = std::min(D.n_slots, (c + 1) * kspl);
+    w.s_end = std::min(n_all, (c + 1) * kspl);
     wl.push_back(w);
   }
   double2* part = nullptr;
@@ -1424,7 +1441,7 @@ double DmkTree::ewald_energy(double* parts) {
   for (size_t i = 0; i < wl.size(); ++i) wl[i].out = part + i * size_t(Hs);
   PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d_work), sizeof(NudftWork) * wl.size(), st_));
   PDMK_CUDA(cudaMemcpyAsync(d_work, wl.data(), sizeof(NudftWork) * wl.size(), cudaMemcpyHostToDevice, st_));
-  dispatch_nudft(nk, d_work, int(wl.size()), D, st_);
+  dispatch_nudft(nk, d_work, int(wl.size()), dense_, dense_stride_, st_);
   {
     int* d_meta;
     double2** d_outs;

@@ -3014,7 +3014,7 @@ void DmkTree::update_shift(long i, double dx, double dy, double dz) {
   PDMK_CUDA(cudaStreamSynchronize(st_));
   last_valid_ = false;
   diff_cached_ = false;
-  moved_ = true;
+  mark_moved();
 }
 
 // The deferred-update list of a tree, its marks and the folded difference
@@ -3173,7 +3173,7 @@ void DmkTree::mc_run_device(int n_moves, const int* d_idx, const double* d_disp,
     if (n_moves > 0) mc_run_persistent(n_moves, d_idx, d_disp, d_u, beta, d_dE, d_acc);
     last_valid_ = false;
     diff_cached_ = false;
-    moved_ = true;
+    mark_moved();
     return;
   }
   ensure_move_resources();
@@ -3206,7 +3206,7 @@ void DmkTree::mc_run_device(int n_moves, const int* d_idx, const double* d_disp,
   }
   last_valid_ = false;
   diff_cached_ = false;
-  moved_ = true;
+  mark_moved();
 }
 
 // All candidates in one launch of k_shift_batch (one block per candidate).
@@ -3369,7 +3369,7 @@ void DmkTree::replicas_mc_run(const std::vector<DmkTree*>& ts, int m, const int*
   for (DmkTree* t : ts) {
     t->last_valid_ = false;
     t->diff_cached_ = false;
-    t->moved_ = true;
+    t->mark_moved();
   }
 }
 

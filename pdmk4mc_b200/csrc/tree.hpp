@@ -304,11 +304,19 @@ class DmkTree {
     int* cnt_prefix = nullptr;   // exclusive prefix of cnt
     int* dfs_of_node = nullptr;  // node id -> j (leaves only)
   } leaf_dev_;
+  // particles in leaf order without free slots (rows x, y, z, q) and every
+  // node's first one in them
+  double* dense_ = nullptr;
+  long dense_stride_ = 0;
+  int* node_dense_ = nullptr;
+  bool dense_ready_ = false;
+  void ensure_dense();
   void* slot_block_ = nullptr;
   int slot_capacity_ = 0;
   size_t partials_cap_ = 0;
   // energy bookkeeping
   bool diff_cached_ = false;
+  void mark_moved() { moved_ = true, dense_ready_ = false; }
   bool moved_ = false;  // moves ran since the last pack: the overflow pool may hold particles
   bool box_lists_ready_ = false;
   int n_nonleaf_ = 0, n_leaves_ = 0;
