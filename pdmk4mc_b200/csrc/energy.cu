@@ -298,17 +298,21 @@ __global__ void k_reduce_chunks(const double2* part, const int* chunk_first, con
 // colleagues C (form_incoming_pw, src/planewave.cpp:99-155), for the
 // 4 x 4 x 4 boxes of level l below one box G of level l - 2 at once: their
 // 27-box neighbourhoods lie in the 6 x 6 x 6 cube of level-l cells around
-// them. A block stages the cube's outgoing rows for one tile of INC_KT modes
-// in shared memory (image phase applied; absent and empty cells are zero),
-// then each thread sums the 3 x 3 (y, z) neighbourhood of six x columns once
-// and slides the 3-wide x window over them for its 4 receivers. A row tile
-// crosses L2 216 / 64 = 3.4 times per receiving box (8 times with the
-// 4 x 4 x 4 cube around one parent). The energy partial of a block sums its
-// non-leaf receivers, which share one level.
+// them. Per tile of INC_KT modes a block sums in two steps: a thread loads the
+// six z cells of a column, all at once, and leaves its four 3-cell z sums in
+// shared memory; then a thread adds 3 y neighbours of them for the six x and
+// slides the 3-wide x window over the result for 4 receivers. (Staging the raw
+// cells and summing 3 x 3 neighbourhoods from them moved twice the
+// shared-memory words, and the loads waited behind them.) Cells next to no
+// receiver are not loaded and columns without a needed cell are left out: in
+// the deep levels of a clustered tree a cube holds one or two receivers. The
+// periodic image phases are cube roots of unity, separable over the axes, so
+// they are applied to the sums at the cube's faces. The energy partial of a
+// block sums its non-leaf receivers, which share one level.
 constexpr int INC_KT = 16;    // modes per tile
-constexpr int INC_T = 256;    // threads: INC_KT modes x 16 (y, z) lines of 4 receivers along x
+constexpr int INC_T = 288;    // threads: INC_KT modes x 18 columns, half of a full cube's
 constexpr int INC_CELLS = 216;
-constexpr size_t INC_SMEM = sizeof(double2) * INC_CELLS * INC_KT + sizeof(int) * (INC_CELLS + 64) + INC_CELLS;
+constexpr size_t INC_SMEM = sizeof(double2) * INC_KT * (4 * 36 + 64);  // z sums, the receivers' own rows
 
 // rank of a refined cell within its level (Morton order)
 __device__ inline int refined_rank(const DevTree& T, int level, uint64_t cell) {
@@ -320,15 +324,24 @@ __device__ inline int refined_rank(const DevTree& T, int level, uint64_t cell) {
 // slot + slots, ... of cube c, so its set-up (the cube's cell lookup) is
 // paid once, and the cubes sharing a slot walk the same tiles together (the
 // cells two neighbouring cubes share meet in L2).
+// v exp(-2 pi i e / 3)
+__device__ __forceinline__ double2 rot3(double2 v, int e) {
+  if (e == 0) return v;
+  const double h = e == 1 ? -0.86602540378443864676 : 0.86602540378443864676;
+  return make_double2(-0.5 * v.x - h * v.y, -0.5 * v.y + h * v.x);
+}
+
 template <int NK>
-__global__ void __launch_bounds__(INC_T, 2) k_incoming_cube(DevTree T, const int* __restrict__ cubes, int ncubes,
+__global__ void __launch_bounds__(INC_T, 3) k_incoming_cube(DevTree T, const int* __restrict__ cubes, int ncubes,
                                                              int slots, double* part,
                                                              const int* __restrict__ touched) {
   constexpr int D = 2 * NK + 1, H = (NK + 1) * D * D;
-  extern __shared__ double2 w[];                             // [INC_CELLS][INC_KT]
-  int* s_row = reinterpret_cast<int*>(w + INC_CELLS * INC_KT);  // outgoing row of each cell, -1: absent or empty
-  int* s_recv = s_row + INC_CELLS;                           // expansion row of each receiver, -1: none
-  unsigned char* s_wrap = reinterpret_cast<unsigned char*>(s_recv + 64);  // image flags, 2 bits per axis
+  extern __shared__ double2 zs[];            // z sums [z][cy][cx][INC_KT]
+  double2* own = zs + 4 * 36 * INC_KT;       // the receivers' own rows [receiver][INC_KT]
+  __shared__ int s_row[INC_CELLS];           // outgoing row of each cell, -1: absent, empty or not needed
+  __shared__ int s_recv[64];                 // expansion row of each receiver, -1: none
+  __shared__ int s_col[36], s_line[16];      // columns (cx + 6 cy) and receiver lines (y + 4 z) with something to do
+  __shared__ int s_ncol, s_nline, s_any;
   __shared__ double sm[32];
   const int slot = blockIdx.x / ncubes, cb = blockIdx.x % ncubes;
   const int G = cubes[cb];
@@ -337,28 +350,22 @@ __global__ void __launch_bounds__(INC_T, 2) k_incoming_cube(DevTree T, const int
   const uint64_t gp = T.node_prefix[G];
   const int O[3] = {4 * int(compact3(gp)), 4 * int(compact3(gp >> 1)), 4 * int(compact3(gp >> 2))};
   const int base = T.pw_base;
-  __shared__ int s_any;
-  if (threadIdx.x == 0) s_any = 0;
+  const int tid = threadIdx.x;
+  if (tid == 0) s_any = 0;
   __syncthreads();
-  if (threadIdx.x < INC_CELLS) {
-    const int t = threadIdx.x;
-    const int c[3] = {t % 6 - 1, (t / 6) % 6 - 1, t / 36 - 1};
+  if (tid < INC_CELLS) {
+    const int c[3] = {tid % 6 - 1, (tid / 6) % 6 - 1, tid / 36 - 1};
     int g[3];
-    unsigned wrap = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      int v = O[a] + c[a];
-      const int f = v < 0 ? 1 : (v >= side ? 2 : 0);  // 1: image below (-1), 2: above (+1)
-      v = f == 1 ? v + side : (f == 2 ? v - side : v);
-      g[a] = v;
-      wrap |= unsigned(f) << (2 * a);
+      const int v = O[a] + c[a];
+      g[a] = v < 0 ? v + side : (v >= side ? v - side : v);
     }
     const uint64_t m = morton3(uint32_t(g[0]), uint32_t(g[1]), uint32_t(g[2]));
     int node = -1;
     if ((T.bm_d[l - 1][m >> 8] >> ((m >> 3) & 31)) & 1u)
       node = T.level_start_d[l] + 8 * refined_rank(T, l - 1, m >> 3) + int(m & 7);
-    s_row[t] = (node >= 0 && T.node_count[node] > 0) ? node - base : -1;
-    s_wrap[t] = static_cast<unsigned char>(wrap);
+    s_row[tid] = (node >= 0 && T.node_count[node] > 0) ? node - base : -1;
     if (c[0] >= 0 && c[0] < 4 && c[1] >= 0 && c[1] < 4 && c[2] >= 0 && c[2] < 4)
       s_recv[c[0] + 4 * c[1] + 16 * c[2]] = (node >= 0 && T.node_child0[node] >= 0) ? node - base : -1;
     if (touched && node >= 0 && touched[node - base] != 0) s_any = 1;
@@ -366,92 +373,123 @@ __global__ void __launch_bounds__(INC_T, 2) k_incoming_cube(DevTree T, const int
   __syncthreads();
   // after a sequence of moves: nothing to do when no outgoing row of the cube changed
   if (touched && !s_any) return;
-  if (touched && threadIdx.x < 32 && slot == 0) {
-    int n = (s_recv[threadIdx.x] >= 0) + (s_recv[threadIdx.x + 32] >= 0);
+  if (touched && tid < 32 && slot == 0) {
+    int n = (s_recv[tid] >= 0) + (s_recv[tid + 32] >= 0);
     for (int o = 16; o > 0; o >>= 1) n += __shfl_down_sync(0xffffffffu, n, o);
-    if (threadIdx.x == 0) atomicAdd(&T.work[1], 32ull * H * (unsigned long long)n);
+    if (tid == 0) atomicAdd(&T.work[1], 32ull * H * (unsigned long long)n);
   }
+  // which cells lie next to a receiver, the columns that hold one, and the
+  // lines with a receiver
+  {
+    bool need = false;
+    if (tid < INC_CELLS) {
+      const int c[3] = {tid % 6 - 1, (tid / 6) % 6 - 1, tid / 36 - 1};
+      for (int z = max(c[2] - 1, 0); z <= min(c[2] + 1, 3); ++z)
+        for (int y = max(c[1] - 1, 0); y <= min(c[1] + 1, 3); ++y)
+          for (int x = max(c[0] - 1, 0); x <= min(c[0] + 1, 3); ++x) need = need || s_recv[x + 4 * y + 16 * z] >= 0;
+    }
+    __syncthreads();
+    if (tid < INC_CELLS && !need) s_row[tid] = -2;
+    __syncthreads();
+    if (tid < 32) {
+      int n = 0;
+      for (int b = 0; b < 36; b += 32) {
+        bool on = false;
+        if (b + tid < 36)
+          for (int z = 0; z < 6; ++z) on = on || s_row[z * 36 + b + tid] != -2;
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        if (on) s_col[n + __popc(m & ((1u << tid) - 1u))] = b + tid;
+        n += __popc(m);
+      }
+      bool on = false;
+      if (tid < 16)
+        for (int x = 0; x < 4; ++x) on = on || s_recv[x + 4 * tid] >= 0;
+      const unsigned m = __ballot_sync(0xffffffffu, on);
+      if (on) s_line[__popc(m & ((1u << tid) - 1u))] = tid;
+      if (tid == 0) {
+        s_ncol = n;
+        s_nline = __popc(m);
+      }
+    }
+    __syncthreads();
+  }
+  const int ncol = s_ncol, nline = s_nline;
   const int two_l = (l & 1) ? 2 : 1;
-  const int kk = threadIdx.x % INC_KT;
-  const int line = threadIdx.x / INC_KT, ry = line & 3, rz = line >> 2;
-  const double2 w3a = make_double2(-0.5, -0.86602540378443864676);  // exp(-2 pi i / 3)
-  const double2 w3b = make_double2(-0.5, 0.86602540378443864676);   // exp(-4 pi i / 3)
+  // the cube's faces that lie on the box's: the cells there are images
+  bool lo_face[3], hi_face[3];
+  for (int a = 0; a < 3; ++a) {
+    lo_face[a] = O[a] == 0;
+    hi_face[a] = O[a] + 4 == side;
+  }
+  const int kk = tid % INC_KT;
   double e = 0;
   constexpr int ktiles = (H + INC_KT - 1) / INC_KT;
   for (int tile = slot; tile < ktiles; tile += slots) {
     const int k = tile * INC_KT + kk;
     const bool kin = k < H;
-    const int ix = k % D, iy = (k / D) % D, iz = k / (D * D);
     // the image phase is exp(-2 pi i e / 3) with e = sum over axes of
-    // f (i - n) 2^l mod 3 (f = -1 below, +1 above): per axis the terms of
-    // an image below and above, two bits each
-    unsigned below = 0, above = 0;
-    {
-      const int ii[3] = {ix, iy, iz};
+    // f (i - n) 2^l mod 3 (f = -1 below, +1 above)
+    const int ix = k % D, iy = (k / D) % D, iz = k / (D * D);
+    const int ex = (((ix - NK) % 3 + 3) * two_l) % 3, ey = (((iy - NK) % 3 + 3) * two_l) % 3,
+              ez = (((iz - NK) % 3 + 3) * two_l) % 3;
+    // two columns a thread, the loads of both before the first is used
+    for (int c0 = tid / INC_KT; c0 < ncol; c0 += 2 * (INC_T / INC_KT)) {
+      double2 v[2][6];
+      int col[2];
 #pragma unroll
-      for (int ax = 0; ax < 3; ++ax) {
-        const int b = (((ii[ax] - NK) % 3 + 3) * two_l) % 3;
-        above |= unsigned(b) << (2 * ax);
-        below |= unsigned((3 - b) % 3) << (2 * ax);
-      }
-    }
-    // stage the cube: mode kk of cells line, line + 16, ...; all loads issued
-    // before the first is used
-    constexpr int NPT = (INC_CELLS + INC_T / INC_KT - 1) / (INC_T / INC_KT);  // cells per thread
-    double2 vv[NPT];
+      for (int j = 0; j < 2; ++j) {
+        const int ci = c0 + j * (INC_T / INC_KT);
+        col[j] = ci < ncol ? s_col[ci] : -1;
 #pragma unroll
-    for (int i = 0; i < NPT; ++i) {
-      const int c = line + i * (INC_T / INC_KT);
-      const int row = c < INC_CELLS ? s_row[c] : -1;
-      vv[i] = (row >= 0 && kin) ? T.out[size_t(row) * H + k] : make_double2(0.0, 0.0);
-    }
-#pragma unroll
-    for (int i = 0; i < NPT; ++i) {
-      const int c = line + i * (INC_T / INC_KT);
-      if (c >= INC_CELLS) break;
-      double2 v = vv[i];
-      const unsigned wr = s_wrap[c];
-      if (wr) {
-        unsigned ep = 0;
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-          const unsigned f = (wr >> (2 * ax)) & 3u;
-          ep += f == 1 ? (below >> (2 * ax)) & 3u : (f == 2 ? (above >> (2 * ax)) & 3u : 0u);
+        for (int z = 0; z < 6; ++z) {
+          const int row = col[j] >= 0 ? s_row[z * 36 + col[j]] : -1;
+          v[j][z] = (row >= 0 && kin) ? T.out[size_t(row) * H + k] : make_double2(0.0, 0.0);
         }
-        ep = ep >= 3 ? ep - 3 : ep;
-        ep = ep >= 3 ? ep - 3 : ep;
-        if (ep) v = cmul(v, ep == 1 ? w3a : w3b);
       }
-      w[c * INC_KT + kk] = v;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if (col[j] < 0) break;
+        const int cx = col[j] % 6, cy = col[j] / 6;
+        if (cx >= 1 && cx <= 4 && cy >= 1 && cy <= 4)
+#pragma unroll
+          for (int z = 0; z < 4; ++z) own[(cx - 1 + 4 * (cy - 1) + 16 * z) * INC_KT + kk] = v[j][z + 1];
+        if (lo_face[2]) v[j][0] = rot3(v[j][0], (3 - ez) % 3);
+        if (hi_face[2]) v[j][5] = rot3(v[j][5], ez);
+#pragma unroll
+        for (int z = 0; z < 4; ++z) zs[(z * 36 + col[j]) * INC_KT + kk] = cadd(cadd(v[j][z], v[j][z + 1]), v[j][z + 2]);
+      }
     }
     __syncthreads();
-    // the 3 x 3 (y, z) sums of the six x columns of this thread's line
-    double2 col[6];
+    for (int li = tid / INC_KT; li < nline; li += INC_T / INC_KT) {
+      const int line = s_line[li], ry = line & 3, rz = line >> 2;
+      double2 c[6];
 #pragma unroll
-    for (int cx = 0; cx < 6; ++cx) {
-      double2 acc = make_double2(0.0, 0.0);
+      for (int cx = 0; cx < 6; ++cx) {
+        const double2* p = zs + (rz * 36 + ry * 6 + cx) * INC_KT + kk;
+        double2 a = p[0], b = p[12 * INC_KT];
+        if (ry == 0 && lo_face[1]) a = rot3(a, (3 - ey) % 3);
+        if (ry == 3 && hi_face[1]) b = rot3(b, ey);
+        c[cx] = cadd(cadd(a, p[6 * INC_KT]), b);
+      }
+      if (lo_face[0]) c[0] = rot3(c[0], (3 - ex) % 3);
+      if (hi_face[0]) c[5] = rot3(c[5], ex);
+      if (kin) {
+        const double d2 = T.D2[k];
 #pragma unroll
-      for (int dz = 0; dz < 3; ++dz)
-#pragma unroll
-        for (int dy = 0; dy < 3; ++dy) acc = cadd(acc, w[((rz + dz) * 36 + (ry + dy) * 6 + cx) * INC_KT + kk]);
-      col[cx] = acc;
-    }
-    if (kin) {
-      const double d2 = T.D2[k];
-#pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        const int rrow = s_recv[x + 4 * ry + 16 * rz];
-        if (rrow < 0) continue;
-        const double2 inc = cconj(cadd(cadd(col[x], col[x + 1]), col[x + 2]));
-        T.inc[size_t(rrow) * H + k] = inc;
-        const double2 o = w[((rz + 1) * 36 + (ry + 1) * 6 + x + 1) * INC_KT + kk];  // the receiver's own row
-        e += (o.x * inc.x - o.y * inc.y) * d2;
+        for (int x = 0; x < 4; ++x) {
+          const int rrow = s_recv[x + 4 * line];
+          if (rrow < 0) continue;
+          const double2 inc = cconj(cadd(cadd(c[x], c[x + 1]), c[x + 2]));
+          T.inc[size_t(rrow) * H + k] = inc;
+          const double2 o = own[(x + 4 * line) * INC_KT + kk];
+          e += (o.x * inc.x - o.y * inc.y) * d2;
+        }
       }
     }
     __syncthreads();
   }
   double s = block_sum(e, sm);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  if (tid == 0) part[blockIdx.x] = s;
 }
 
 template <int NK>
