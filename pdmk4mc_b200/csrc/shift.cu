@@ -20,6 +20,7 @@
 #include <cmath>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -160,9 +161,9 @@ struct Preload {
 };
 
 template <bool CG = false>
-__device__ void resolve(const DevTree& T, int i, const double* disp, Header& h, const Preload* pre = nullptr) {
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
+__device__ inline void resolve_by_warp(const DevTree& T, int i, const double* disp, Header& h, const Preload* pre = nullptr) {
+  {
+    const int lane = threadIdx.x & 31;
     const bool have = pre && pre->s >= 0;
     const int s = have ? pre->s : ldm<CG>(T.orig_slot + i);
     double xo[3], q;
@@ -229,6 +230,11 @@ __device__ void resolve(const DevTree& T, int i, const double* disp, Header& h, 
     }
     if (lane == 16) h.depth_o = leaf_level + 1;
   }
+}
+
+template <bool CG = false>
+__device__ void resolve(const DevTree& T, int i, const double* disp, Header& h, const Preload* pre = nullptr) {
+  if (threadIdx.x < 32) resolve_by_warp<CG>(T, i, disp, h, pre);
   __syncthreads();
 }
 
@@ -2548,255 +2554,665 @@ void launch_flush_outgoing(const DevTree& D, const Pending* list, const int* n_l
 }
 
 // ---------------------------------------------------------------------------
-// Many candidate moves against one state in one launch: one block per
-// candidate evaluates its whole dE (resolve, phase tables, window and
-// difference sums over all modes, both near-field sums, self term) and
-// reduces it inside the block, so no grid-wide partials are needed and the
-// candidates run side by side on all SMs. Candidates whose paths share boxes
-// read the shared incoming rows through L2.
-constexpr int SB_T = 256;
+// Many points against one state in one launch: candidate moves (k_shift_batch)
+// and potentials (k_potential_batch). A block takes a group of GRP particles;
+// with a point x on level-l box B its difference sum is
+//   Re sum_k D(k) inc_B(k) exp(-i k.x)
+//     = Re sum_{iz,iy} ez[iz] ey[iy] s(iz, iy),  s = sum_ix (D inc_B)[iz,iy,ix] ex[ix],
+// so the inner sums are a matrix product of the row, lines (iz, iy) by columns
+// ix, with the ex of all the group's points on B: FP64 tensor instructions
+// (m8n8k4), whose A operand comes straight from global memory (each row is
+// read once for all its points) and whose cost per mode and point is the four
+// multiply-adds of s. The thread-per-mode form took a product of three phases
+// for every mode and point (10 operations, 12 shared-memory wavefronts per 32
+// modes) and every candidate read its rows alone: 4096 candidates at N = 1e6
+// moved 13.6 GB through L2 in 2.35 ms. Groups are formed along the Morton
+// order of the particles (k_order_particles), so most of a group's points
+// share their boxes; the result of a point does not depend on its group.
+constexpr int BG_T = 256, BG_W = BG_T / 32;
 
 template <int NP>
-__global__ void __launch_bounds__(SB_T) k_shift_batch(DevTree T, const int* __restrict__ idx,
-                                                      const double* __restrict__ disp, double c_window,
-                                                      double* __restrict__ dE_out) {
-  extern __shared__ double2 sm2[];
-  __shared__ Header h;
-  __shared__ double red[4][32];
-  __shared__ double c_level[MAXLV + 2];
-  const ResidualPoly<NP> poly(T);
-  if (threadIdx.x >= 2 && threadIdx.x < MAXLV + 2) {
-    const double dk = level_dk(T, threadIdx.x);
-    c_level[threadIdx.x] = dk * dk * dk / (8.0 * 3.14159265358979323846 * 3.14159265358979323846 *
-                                           3.14159265358979323846) * level_dscale(threadIdx.x);
+struct BatchShape {
+  using MO = ModesOf<NP>;
+  static constexpr int N1 = MO::ND + 1, D = 2 * MO::ND + 1, H = N1 * D * D;
+  static constexpr int DW = 2 * MO::NW + 1, HW = (MO::NW + 1) * DW * DW;
+  static constexpr int LINES = N1 * D, MT = (LINES + 7) / 8, KS = (D + 3) / 4;
+  // D over the octant (|kz|, |ky|, |kx|) in shared memory where it fits; the
+  // row stride is 4 or 12 modulo 16, so that 4 lines x 4 kx fall on different banks
+  static constexpr bool TAB = MO::ND <= 19;
+  static constexpr int DS = N1 % 16 <= 4 ? N1 / 16 * 16 + 4 : N1 % 16 <= 12 ? N1 / 16 * 16 + 12 : N1 / 16 * 16 + 20;
+  static constexpr int TAB_DOUBLES = TAB ? N1 * N1 * DS : 0;
+  __host__ __device__ static int per(int max_depth) { return 3 * DW + (max_depth > 3 ? max_depth - 3 : 0) * 3 * D; }  // phases of one point
+  static size_t smem(int max_depth, int points) {
+    return sizeof(double) * TAB_DOUBLES + sizeof(double2) * size_t(per(max_depth)) * points;
   }
-  const int c = blockIdx.x;
-  resolve(T, idx[c], disp + 3 * c, h);
-  const int lo_max = h.depth_o - 2, lt_max = h.depth_t - 2;
-  const int per = 3 * (2 * T.n_window + 1) + max(max(lo_max, lt_max) - 1, 0) * 3 * (2 * T.n_diff + 1);
-  Tables to, oo;
-  alloc_tables(sm2, T, oo);
-  alloc_tables(sm2 + per, T, to);
-  build_tables(T, h.xo, h.q, h.Xo, lo_max, oo, threadIdx.x, blockDim.x);
-  build_tables(T, h.xt, h.q, h.Xt, lt_max, to, threadIdx.x, blockDim.x);
-  __syncthreads();
-  double acc[4] = {0, 0, 0, 0};
-  for (int k = threadIdx.x; k < T.Hw; k += blockDim.x) {
-    const double2 t = phase_at(to.root, k, T.dw), o = phase_at(oo.root, k, T.dw);
-    const double2 g = T.out_root[k];
-    const double ar = t.x - o.x, ai = t.y - o.y, br = g.x - o.x, bi = g.y - o.y;
-    acc[0] += (ar * br + ai * bi) * T.W[k];
-  }
-  const int base = T.pw_base, d = T.dd;
-  for (int k = threadIdx.x; k < T.H; k += blockDim.x) {
-    const int ix = k % d, iy = (k / d) % d, iz = k / (d * d);
-    double sd = 0;
-    for (int l = 2; l <= lo_max; ++l) {
-      const double2 o = cmul(oo.lev[l][2][iz], cmul(oo.lev[l][1][iy], oo.lev[l][0][ix]));
-      const double2 cc = T.inc[size_t(h.path_o[l] - base) * T.H + k];
-      sd -= (o.x * cc.x - o.y * cc.y - (o.x * o.x + o.y * o.y)) * c_level[l];
+};
+
+// The points of a group and, per level, their distinct boxes
+template <int PTS>
+struct BatchRows {
+  int n[MAXLV];                 // distinct boxes of a level
+  int row[MAXLV][PTS];          // their expansion rows
+  unsigned char npt[MAXLV][PTS];
+  unsigned char pt[MAXLV][PTS][PTS];  // the points on each
+};
+
+// one thread: the rows of points 0 .. PTS-1 (node_of(p, l) < 0: the point has no box at level l)
+template <int PTS, class F>
+__device__ void batch_rows(BatchRows<PTS>& R, int top, F node_of) {
+  for (int l = 2; l <= top; ++l) {
+    int n = 0;
+    for (int p = 0; p < PTS; ++p) {
+      const int row = node_of(p, l);
+      if (row < 0) continue;
+      int r = 0;
+      while (r < n && R.row[l][r] != row) ++r;
+      if (r == n) {
+        R.row[l][r] = row;
+        R.npt[l][r] = 0;
+        ++n;
+      }
+      R.pt[l][r][R.npt[l][r]++] = static_cast<unsigned char>(p);
     }
-    for (int l = 2; l <= lt_max; ++l) {
-      const double2 t = cmul(to.lev[l][2][iz], cmul(to.lev[l][1][iy], to.lev[l][0][ix]));
-      const double2 cc = T.inc[size_t(h.path_t[l] - base) * T.H + k];
-      sd += (t.x * cc.x - t.y * cc.y) * c_level[l];
-    }
-    acc[1] += sd * T.D2[k];
-  }
-  const int lt = h.depth_t - 1, lo = h.depth_o - 1;
-  acc[2] = residual_sum(T, poly, h.path_t[lt], lt, h.Xt[lt], h.xt);
-  __syncthreads();  // the second call reuses the source-list arrays of the first
-  acc[3] = residual_sum(T, poly, h.path_o[lo], lo, h.Xo[lo], h.xo);
-  block_sum4(acc, red);
-  if (threadIdx.x == 0) {
-    double self = 0;
-    if (h.dr != 0) self = poly(h.dr, level_box(T, 2)) * h.q * h.q;
-    dE_out[c] = acc[0] * c_window + acc[1] + (acc[2] - acc[3]) * h.q - self;
+    R.n[l] = n;
   }
 }
 
-using ShiftBatchKernel = void (*)(DevTree, const int*, const double*, double, double*);
-ShiftBatchKernel shift_batch_kernel(int np) {
+template <int NP>
+__device__ void load_octant(const DevTree& T, double* tab) {
+  using S = BatchShape<NP>;
+  if constexpr (S::TAB)
+    for (int i = threadIdx.x; i < S::TAB_DOUBLES; i += BG_T) {
+      const int mx = i % S::DS, r = i / S::DS, mz = r / S::N1, my = r % S::N1;
+      tab[i] = mx < S::N1 ? T.D2[((S::N1 - 1 - mz) * S::D + S::N1 - 1 + my) * S::D + S::N1 - 1 + mx] : 0.0;
+    }
+}
+
+// The products of one row with the columns of up to NT tiles. COLS columns per
+// point: 2 (re, im of ex), or 4 (and those of kx ex, in units of dk). consume(tile,
+// line, c0, c1): this lane's two results, the (re, im) of its column pair (lane
+// & 3) on its line.
+template <int NP, int NT, int COLS, class F>
+__device__ __forceinline__ void row_products(const DevTree& T, const double2* __restrict__ row, const double* __restrict__ tab,
+                                             const double2* const (&ex)[NT], F consume) {
+  using S = BatchShape<NP>;
+  constexpr int KS = S::KS, D = S::D, ND = S::N1 - 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q4 = lane & 3, q8 = lane >> 2;
+  // B: this lane's column (lane >> 2) at ix = 4 s + (lane & 3), for the real
+  // and the imaginary part of the row
+  double bre[NT][KS], bim[NT][KS];
+#pragma unroll
+  for (int t = 0; t < NT; ++t)
+#pragma unroll
+    for (int k = 0; k < KS; ++k) {
+      const int ix = 4 * k + q4;
+      double2 v = make_double2(0.0, 0.0);
+      if (ix < D && ex[t]) v = ex[t][ix];
+      if (COLS == 4 && (q8 & 2)) v = cscale(v, double(ix - ND));
+      bre[t][k] = (q8 & 1) ? v.y : v.x;
+      bim[t][k] = (q8 & 1) ? v.x : -v.y;
+    }
+  for (int mt = warp; mt < S::MT; mt += BG_W) {
+    const int line = min(8 * mt + q8, S::LINES - 1);
+    const int iy = line % D, iz = line / D;
+    const double2* src = row + size_t(line) * D + q4;
+    double2 a[KS];
+#pragma unroll
+    for (int k = 0; k < KS; ++k) a[k] = 4 * k + q4 < D ? src[4 * k] : make_double2(0.0, 0.0);
+    double c[NT][2][2];  // [row real, imaginary][column pair]
+#pragma unroll
+    for (int t = 0; t < NT; ++t) c[t][0][0] = c[t][0][1] = c[t][1][0] = c[t][1][1] = 0.0;
+#pragma unroll
+    for (int k = 0; k < KS; ++k) {
+      const int ix = 4 * k + q4;
+      double d = 0.0;
+      if (ix < D) d = S::TAB ? tab[((ND - iz) * S::N1 + abs(iy - ND)) * S::DS + abs(ix - ND)] : T.D2[size_t(line) * D + ix];
+      const double ar = a[k].x * d, ai = a[k].y * d;
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+            : "+d"(c[t][0][0]), "+d"(c[t][0][1])
+            : "d"(ar), "d"(bre[t][k]));
+        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+            : "+d"(c[t][1][0]), "+d"(c[t][1][1])
+            : "d"(ai), "d"(bim[t][k]));
+      }
+    }
+    if (8 * mt + q8 < S::LINES)
+#pragma unroll
+      for (int t = 0; t < NT; ++t) consume(t, iz, iy, make_double2(c[t][0][0] + c[t][1][0], c[t][0][1] + c[t][1][1]));
+  }
+}
+
+// source lists of a group's points (36 per point) with their prefix sums
+template <int PTS>
+struct BatchSources {
+  int beg[PTS][36], pre[PTS][37], lvl[PTS][36];
+  unsigned long long pfx[PTS][36];
+  double off[PTS][36][3];
+};
+
+// block-cooperative; leaf(p), level(p) and X(p) give a point's leaf (level < 0: no point)
+template <int PTS, class F>
+__device__ void batch_sources(const DevTree& T, BatchSources<PTS>& S, F point) {
+  for (int t = threadIdx.x; t < PTS * 36; t += BG_T) {
+    const int p = t / 36, src = t % 36;
+    int leaf, l;
+    const int* Xl;
+    point(p, leaf, l, Xl);
+    int j = -1;
+    if (l >= 0) {
+      if (src == 0) j = leaf;
+      else if (src <= 27) j = (src - 1 == 13) ? -1 : T.col27[size_t(leaf) * 27 + (src - 1)];
+      else j = T.coarse8[size_t(leaf) * 8 + (src - 28)];
+    }
+    int beg = 0, cnt = 0, lj = -1;
+    unsigned long long pj = 0;
+    double off[3] = {0, 0, 0};
+    if (j >= 0) {
+      lj = T.node_level[j];
+      pj = T.node_prefix[j];
+      beg = T.node_begin[j];
+      cnt = T.node_child0[j] < 0 ? T.leaf_count[j] : T.node_end[j] - beg;
+      const double b = level_box(T, l), bj = level_box(T, lj);
+      const int Xj[3] = {int(compact3(pj)), int(compact3(pj >> 1)), int(compact3(pj >> 2))};
+      for (int d = 0; d < 3; ++d)
+        off[d] = -periodic_shift_d(center_of(T.L, l, Xl[d]), center_of(T.L, lj, Xj[d]), T.L, b, bj) * T.L;
+    }
+    S.beg[p][src] = beg;
+    S.pre[p][src] = cnt;
+    S.lvl[p][src] = lj;
+    S.pfx[p][src] = pj;
+    for (int d = 0; d < 3; ++d) S.off[p][src][d] = off[d];
+  }
+  __syncthreads();
+  if (threadIdx.x < PTS) {
+    int s = 0;
+    for (int src = 0; src < 36; ++src) {
+      const int n = S.pre[threadIdx.x][src];
+      S.pre[threadIdx.x][src] = s;
+      s += n;
+    }
+    S.pre[threadIdx.x][36] = s;
+  }
+  __syncthreads();
+}
+
+// this thread's share of a point's near-field pairs: f(q_j, dx, dy, dz, r2) for
+// each within the cut-off, overflow pool included
+template <int PTS, class F>
+__device__ __forceinline__ void batch_near(const DevTree& T, const BatchSources<PTS>& S, int p, const double* x, double b,
+                                           int pool_n, F f) {
+  const double eps = 2.220446049250313e-16, b2 = b * b;
+  int src = 0;
+  const int total = S.pre[p][36];
+  for (int e = threadIdx.x; e < total; e += BG_T) {
+    while (e >= S.pre[p][src + 1]) ++src;
+    const int s = S.beg[p][src] + (e - S.pre[p][src]);
+    const double dx = x[0] - (T.sx[s] + S.off[p][src][0]), dy = x[1] - (T.sy[s] + S.off[p][src][1]),
+                 dz = x[2] - (T.sz[s] + S.off[p][src][2]);
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    if (r2 > eps && r2 < b2) f(T.sq[s], dx, dy, dz, r2);
+  }
+  for (int e = threadIdx.x; e < 36 * pool_n; e += BG_T) {
+    const int sj = e / pool_n, q = e % pool_n;
+    if (S.lvl[p][sj] < 0 || T.p_orig[q] < 0) continue;
+    const int pl = T.p_leaf[q];
+    const int ll = T.node_level[pl], lj = S.lvl[p][sj];
+    if (ll < lj || (T.node_prefix[pl] >> (3 * (ll - lj))) != S.pfx[p][sj]) continue;
+    const double dx = x[0] - (T.px[q] + S.off[p][sj][0]), dy = x[1] - (T.py[q] + S.off[p][sj][1]),
+                 dz = x[2] - (T.pz[q] + S.off[p][sj][2]);
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    if (r2 > eps && r2 < b2) f(T.pq[q], dx, dy, dz, r2);
+  }
+}
+
+// sums of N values over the block, the results in every thread
+template <int N>
+__device__ void batch_block_sum(double (&v)[N], double (*sm)[BG_W]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    for (int o = 16; o > 0; o >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+  __syncthreads();
+  if (lane == 0)
+#pragma unroll
+    for (int i = 0; i < N; ++i) sm[i][warp] = v[i];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    double s = 0;
+    for (int w = 0; w < BG_W; ++w) s += sm[i][w];
+    v[i] = s;
+  }
+}
+
+// GRP = 4 groups along the Morton order where there are enough particles to
+// fill the SMs with groups, else one particle a block.
+constexpr int BG_GROUP = 4;
+constexpr int kGroupMin = 4 * 148 * 2;  // two groups per SM
+
+// order[]: the particles idx[0 .. m) by the level-4 cell of their positions (one
+// block; the order within a cell is free, no result depends on it)
+__global__ void __launch_bounds__(1024) k_order_particles(DevTree T, const int* __restrict__ idx, int m,
+                                                          int* __restrict__ order) {
+  __shared__ int bin[4096];
+  __shared__ int wsum[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto key = [&](int c) {
+    const int s = T.orig_slot[idx[c]], p = s - T.n_slots;
+    const double x = p < 0 ? T.sx[s] : T.px[p], y = p < 0 ? T.sy[s] : T.py[p], z = p < 0 ? T.sz[s] : T.pz[p];
+    return int(morton3(grid_coord(x, T.L), grid_coord(y, T.L), grid_coord(z, T.L)) >> (3 * (KEY_BITS - 4)));
+  };
+  for (int i = threadIdx.x; i < 4096; i += 1024) bin[i] = 0;
+  __syncthreads();
+  for (int c = threadIdx.x; c < m; c += 1024) atomicAdd(&bin[key(c)], 1);
+  __syncthreads();
+  int v[4], sum = 0;
+  for (int k = 0; k < 4; ++k) {
+    v[k] = bin[4 * threadIdx.x + k];
+    sum += v[k];
+  }
+  int x = sum;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) wsum[warp] = x;
+  __syncthreads();
+  if (warp == 0) {
+    int w = wsum[lane];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += y;
+    }
+    wsum[lane] = w;
+  }
+  __syncthreads();
+  int at = (warp > 0 ? wsum[warp - 1] : 0) + x - sum;
+  for (int k = 0; k < 4; ++k) {
+    bin[4 * threadIdx.x + k] = at;
+    at += v[k];
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < m; c += 1024) order[atomicAdd(&bin[key(c)], 1)] = c;
+}
+
+template <int NP, int GRP>
+__global__ void __launch_bounds__(BG_T) k_shift_batch(DevTree T, const int* __restrict__ idx,
+                                                      const double* __restrict__ disp, const int* __restrict__ order, int m,
+                                                      double c_window, double* __restrict__ dE_out) {
+  using S = BatchShape<NP>;
+  constexpr int PTS = 2 * GRP, NT = (PTS + 3) / 4;  // point 2 g: target of candidate g, 2 g + 1: its origin
+  extern __shared__ double sm_b[];
+  __shared__ Header hs[GRP];
+  __shared__ BatchRows<PTS> rows;
+  __shared__ BatchSources<PTS> srcs;
+  __shared__ double red[PTS > 4 ? PTS : 4][BG_W];
+  __shared__ double c_level[MAXLV + 2];
+  const ResidualPoly<NP> poly(T);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, q4 = lane & 3;
+  double* tab = sm_b;
+  double2* phases = reinterpret_cast<double2*>(sm_b + S::TAB_DOUBLES);
+  const int per = S::per(T.max_depth);
+  const int n = min(GRP, m - int(blockIdx.x) * GRP);
+  if (tid >= 2 && tid < MAXLV + 2) {
+    const double dk = level_dk(T, tid);
+    c_level[tid] = dk * dk * dk / (8.0 * 3.14159265358979323846 * 3.14159265358979323846 * 3.14159265358979323846) *
+                   level_dscale(tid);
+  }
+  int cand[GRP];
+#pragma unroll
+  for (int g = 0; g < GRP; ++g) {
+    const int at = blockIdx.x * GRP + min(g, n - 1);
+    cand[g] = order ? order[at] : at;
+  }
+#pragma unroll
+  for (int g = 0; g < GRP; ++g)
+    if (warp == g) resolve_by_warp(T, idx[cand[g]], disp + 3 * size_t(cand[g]), hs[g]);
+  load_octant<NP>(T, tab);
+  __syncthreads();
+  int top = 0;
+  for (int g = 0; g < n; ++g) top = max(top, max(hs[g].depth_o, hs[g].depth_t) - 2);
+  if (tid == 0)
+    batch_rows<PTS>(rows, top, [&](int p, int l) {
+      const Header& h = hs[p >> 1];
+      const int last = ((p & 1) ? h.depth_o : h.depth_t) - 2;
+      if ((p >> 1) >= n || l > last) return -1;
+      return ((p & 1) ? h.path_o[l] : h.path_t[l]) - T.pw_base;
+    });
+  for (int p = 0; p < 2 * n; ++p) {
+    const Header& h = hs[p >> 1];
+    Tables tb;
+    alloc_tables(phases + size_t(p) * per, T, tb);
+    if (p & 1) build_tables(T, h.xo, h.q, h.Xo, h.depth_o - 2, tb, tid, BG_T);
+    else build_tables(T, h.xt, h.q, h.Xt, h.depth_t - 2, tb, tid, BG_T);
+  }
+  batch_sources<PTS>(T, srcs, [&](int p, int& leaf, int& l, const int*& Xl) {
+    const Header& h = hs[p >> 1];
+    l = (p >> 1) < n ? ((p & 1) ? h.depth_o : h.depth_t) - 1 : -1;
+    if (l < 0) return;
+    leaf = (p & 1) ? h.path_o[l] : h.path_t[l];
+    Xl = (p & 1) ? h.Xo[l] : h.Xt[l];
+  });
+  // window (src/energy_shift.cpp:72-90) and the sum of D over the half grid (|o|^2 = q^2)
+  double v[GRP], sum_d[1] = {0.0};
+#pragma unroll
+  for (int g = 0; g < GRP; ++g) v[g] = 0.0;
+  for (int k = tid; k < S::HW; k += BG_T) {
+    const double2 g0 = T.out_root[k];
+    const double w = T.W[k];
+#pragma unroll
+    for (int g = 0; g < GRP; ++g) {
+      if (g < n) {
+        Tables to, oo;
+        alloc_tables(phases + size_t(2 * g) * per, T, to);
+        alloc_tables(phases + size_t(2 * g + 1) * per, T, oo);
+        const double2 t = phase_at(to.root, k, S::DW), o = phase_at(oo.root, k, S::DW);
+        v[g] += ((t.x - o.x) * (g0.x - o.x) + (t.y - o.y) * (g0.y - o.y)) * w;
+      }
+    }
+  }
+#pragma unroll
+  for (int g = 0; g < GRP; ++g) v[g] *= c_window;
+  if (top >= 2)
+    for (int k = tid; k < S::H; k += BG_T) sum_d[0] += T.D2[k];
+  // near field (src/energy_shift.cpp:233-302)
+  const int pool_n = *T.pool_n;
+#pragma unroll
+  for (int g = 0; g < GRP; ++g) {
+    if (g < n) {
+      const Header& h = hs[g];
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const double b = level_box(T, (p ? h.depth_o : h.depth_t) - 1);
+        double a = 0.0;
+        batch_near<PTS>(T, srcs, 2 * g + p, p ? h.xo : h.xt, b, pool_n,
+                        [&](double q, double, double, double, double r2) { a += q * poly(sqrt(r2), b); });
+        v[g] += (p ? -a : a) * h.q;
+      }
+    }
+  }
+  // difference (src/energy_shift.cpp:92-140), row by row; a warp's sums of a
+  // point add up over the levels in its own words
+  double* mine = &red[0][0];  // [point][warp]
+  if (lane < PTS) red[lane][warp] = 0.0;
+  __syncwarp();
+  for (int l = 2; l <= top; ++l)
+    for (int r = 0; r < rows.n[l]; ++r) {
+      const double2* row = T.inc + size_t(rows.row[l][r]) * S::H;
+      const int np = rows.npt[l][r];
+      const unsigned char* pts = rows.pt[l][r];
+      auto run = [&](auto nt) {
+        constexpr int N = decltype(nt)::value;
+        const double2* ex[N];
+        const double2 *ey[N], *ez[N];
+        double acc[N];
+#pragma unroll
+        for (int t = 0; t < N; ++t) {
+          const int jb = 4 * t + (lane >> 3), jc = 4 * t + q4;  // the points of this lane's B column and results
+          auto lev = [&](int j, int ax) {
+            return phases + size_t(pts[min(j, np - 1)]) * per + 3 * S::DW + (l - 2) * 3 * S::D + ax * S::D;
+          };
+          ex[t] = jb < np ? lev(jb, 0) : nullptr;
+          ey[t] = lev(jc, 1);
+          ez[t] = lev(jc, 2);
+          acc[t] = 0.0;
+        }
+        row_products<NP, N, 2>(T, row, tab, ex, [&](int t, int iz, int iy, double2 sv) {
+          const double2 pz = cmul(ez[t][iz], ey[t][iy]);
+          acc[t] += pz.x * sv.x - pz.y * sv.y;
+        });
+#pragma unroll
+        for (int t = 0; t < N; ++t) {
+          for (int o = 4; o < 32; o <<= 1) acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], o);
+          const int j = 4 * t + lane;
+          if (lane < 4 && j < np) red[pts[j]][warp] += ((pts[j] & 1) ? -c_level[l] : c_level[l]) * acc[t];
+        }
+        __syncwarp();
+      };
+      if (NT > 1 && np > 4) run(std::integral_constant<int, NT>{});
+      else run(std::integral_constant<int, 1>{});
+    }
+  (void)mine;
+  // totals: one thread per candidate adds its points' words of all warps
+  __syncthreads();
+  double diff = 0.0;
+  if (tid < n)
+    for (int p = 0; p < 2; ++p)
+      for (int w = 0; w < BG_W; ++w) diff += red[2 * tid + p][w];
+  batch_block_sum<1>(sum_d, red);
+  batch_block_sum<GRP>(v, red);
+  if (tid < n) {
+    const Header& h = hs[tid];
+    double tot = 0.0;
+#pragma unroll
+    for (int g = 0; g < GRP; ++g)
+      if (g == tid) tot = v[g];
+    for (int l = 2; l <= h.depth_o - 2; ++l) diff += c_level[l] * h.q * h.q * sum_d[0];
+    double self = 0;
+    if (h.dr != 0) self = poly(h.dr, level_box(T, 2)) * h.q * h.q;
+    int c = 0;
+#pragma unroll
+    for (int g = 0; g < GRP; ++g)
+      if (g == tid) c = cand[g];
+    dE_out[c] = tot + diff - self;
+  }
+}
+
+using ShiftBatchKernel = void (*)(DevTree, const int*, const double*, const int*, int, double, double*);
+ShiftBatchKernel shift_batch_kernel(int np, int grp) {
   switch (np) {
-    case 7: return k_shift_batch<7>;
-    case 13: return k_shift_batch<13>;
-    case 19: return k_shift_batch<19>;
-    case 25: return k_shift_batch<25>;
+    case 7: return grp > 1 ? k_shift_batch<7, BG_GROUP> : k_shift_batch<7, 1>;
+    case 13: return grp > 1 ? k_shift_batch<13, BG_GROUP> : k_shift_batch<13, 1>;
+    case 19: return grp > 1 ? k_shift_batch<19, BG_GROUP> : k_shift_batch<19, 1>;
+    case 25: return grp > 1 ? k_shift_batch<25, BG_GROUP> : k_shift_batch<25, 1>;
     default: throw std::invalid_argument("unsupported residual polynomial");
   }
 }
 
+// shared memory of a batch kernel with `points` points a block
+size_t batch_smem(int np, int max_depth, int points) {
+  switch (np) {
+    case 7: return BatchShape<7>::smem(max_depth, points);
+    case 13: return BatchShape<13>::smem(max_depth, points);
+    case 19: return BatchShape<19>::smem(max_depth, points);
+    default: return BatchShape<25>::smem(max_depth, points);
+  }
+}
+
 // ---------------------------------------------------------------------------
-// Potential and field at particles (one block per particle): the same terms
-// as an energy shift, for the particle's own position only. With unit-charge
-// phases u(k) = exp(-i k.x) and the particle's charge q, the interaction with
-// all other particles is
+// Potential and field at particles: the same terms as an energy shift, for the
+// particles' own positions only. With unit-charge phases u(k) = exp(-i k.x) and
+// the particle's charge q, the interaction with all other particles is
 //   c_w sum_{k != 0} W Re(u conj(g - q u)) + sum_l c_l sum_k D (Re(u inc_l) - q |u|^2)
 //       + sum_{j != i} q_j res(r_ij),
 // and the returned potential adds 2 q C, C the particle's self terms of the
 // energy (window: c_w/2 sum W - psi0(0)/(2 bs_2 C0); each difference level on
 // its path: c_l/2 sum D_l - S_l), so that E = 1/2 sum_i q_i phi_i and
 // phi_i = dE/dq_i. The field is -grad phi, each plane wave differentiating to
-// -i k u.
-template <int NP>
-__global__ void __launch_bounds__(SB_T) k_potential_batch(DevTree T, const int* __restrict__ idx, double c_window,
+// -i k u: the row products carry two more columns per point, kx ex, and the y
+// and z derivatives take their factors at the lines.
+template <int NP, int GRP>
+__global__ void __launch_bounds__(BG_T) k_potential_batch(DevTree T, const int* __restrict__ idx,
+                                                          const int* __restrict__ order, int m, double c_window,
                                                           double self_w, const double* __restrict__ Sl,
                                                           double* __restrict__ phi_out, double* __restrict__ field_out) {
-  extern __shared__ double2 sm2[];
-  __shared__ Header h;
-  __shared__ double red[4][32];
+  using S = BatchShape<NP>;
+  constexpr int ND = S::N1 - 1, NW = (S::DW - 1) / 2, NT = (GRP + 1) / 2;
+  extern __shared__ double sm_b[];
+  __shared__ Header hs[GRP];
+  __shared__ BatchRows<GRP> rows;
+  __shared__ BatchSources<GRP> srcs;
+  __shared__ double red[4][BG_W];
+  __shared__ double dsum[GRP][4][BG_W];  // difference part: phi, gradient
   __shared__ double c_level[MAXLV + 2];
   const ResidualPoly<NP> poly(T);
-  if (threadIdx.x >= 2 && threadIdx.x < MAXLV + 2) {
-    const double dk = level_dk(T, threadIdx.x);
-    c_level[threadIdx.x] = dk * dk * dk / (8.0 * 3.14159265358979323846 * 3.14159265358979323846 *
-                                           3.14159265358979323846) * level_dscale(threadIdx.x);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, q4 = lane & 3;
+  double* tab = sm_b;
+  double2* phases = reinterpret_cast<double2*>(sm_b + S::TAB_DOUBLES);
+  const int per = S::per(T.max_depth);
+  const int n = min(GRP, m - int(blockIdx.x) * GRP);
+  if (tid >= 2 && tid < MAXLV + 2) {
+    const double dk = level_dk(T, tid);
+    c_level[tid] = dk * dk * dk / (8.0 * 3.14159265358979323846 * 3.14159265358979323846 * 3.14159265358979323846) *
+                   level_dscale(tid);
   }
-  const int c = blockIdx.x;
+  int cand[GRP];
+#pragma unroll
+  for (int g = 0; g < GRP; ++g) {
+    const int at = blockIdx.x * GRP + min(g, n - 1);
+    cand[g] = order ? order[at] : at;
+  }
   const double zero3[3] = {0.0, 0.0, 0.0};
-  resolve(T, idx[c], zero3, h);
-  const int lo_max = h.depth_o - 2;
-  Tables uu;
-  alloc_tables(sm2, T, uu);
-  build_tables(T, h.xo, 1.0, h.Xo, lo_max, uu, threadIdx.x, blockDim.x);
+#pragma unroll
+  for (int g = 0; g < GRP; ++g)
+    if (warp == g) resolve_by_warp(T, idx[cand[g]], zero3, hs[g]);
+  load_octant<NP>(T, tab);
   __syncthreads();
-  const double q = h.q;
-  double v[4] = {0, 0, 0, 0};   // window, difference, residual
-  double gw[4] = {0, 0, 0, 0};  // gradient of the window term
-  double gd[4] = {0, 0, 0, 0};  // gradient of the difference terms
+  int top = 0;
+  for (int g = 0; g < n; ++g) top = max(top, hs[g].depth_o - 2);
+  if (tid == 0)
+    batch_rows<GRP>(rows, top, [&](int p, int l) {
+      return p < n && l <= hs[p].depth_o - 2 ? hs[p].path_o[l] - T.pw_base : -1;
+    });
+  for (int p = 0; p < n; ++p) {
+    Tables tb;
+    alloc_tables(phases + size_t(p) * per, T, tb);
+    build_tables(T, hs[p].xo, 1.0, hs[p].Xo, hs[p].depth_o - 2, tb, tid, BG_T);
+  }
+  batch_sources<GRP>(T, srcs, [&](int p, int& leaf, int& l, const int*& Xl) {
+    l = p < n ? hs[p].depth_o - 1 : -1;
+    if (l < 0) return;
+    leaf = hs[p].path_o[l];
+    Xl = hs[p].Xo[l];
+  });
+  for (int i = tid; i < GRP * 4 * BG_W; i += BG_T) (&dsum[0][0][0])[i] = 0.0;
+  __syncthreads();
+  for (int l = 2; l <= top; ++l)
+    for (int r = 0; r < rows.n[l]; ++r) {
+      const double2* row = T.inc + size_t(rows.row[l][r]) * S::H;
+      const int np = rows.npt[l][r];
+      const unsigned char* pts = rows.pt[l][r];
+      auto run = [&](auto nt) {
+        constexpr int N = decltype(nt)::value;
+        const double2* ex[N];
+        const double2 *ey[N], *ez[N];
+        double acc[N][3];
+#pragma unroll
+        for (int t = 0; t < N; ++t) {
+          const int jb = 2 * t + (lane >> 4), jc = 2 * t + (q4 >> 1);
+          auto lev = [&](int j, int ax) {
+            return phases + size_t(pts[min(j, np - 1)]) * per + 3 * S::DW + (l - 2) * 3 * S::D + ax * S::D;
+          };
+          ex[t] = jb < np ? lev(jb, 0) : nullptr;
+          ey[t] = lev(jc, 1);
+          ez[t] = lev(jc, 2);
+          acc[t][0] = acc[t][1] = acc[t][2] = 0.0;
+        }
+        row_products<NP, N, 4>(T, row, tab, ex, [&](int t, int iz, int iy, double2 sv) {
+          const double2 u = cmul(cmul(ez[t][iz], ey[t][iy]), sv);
+          if (q4 & 1) {
+            acc[t][0] += u.y;  // x derivative
+          } else {
+            acc[t][0] += u.x;
+            acc[t][1] += u.y * double(iy - ND);
+            acc[t][2] += u.y * double(iz - ND);
+          }
+        });
+#pragma unroll
+        for (int t = 0; t < N; ++t) {
+#pragma unroll
+          for (int k = 0; k < 3; ++k)
+            for (int o = 4; o < 32; o <<= 1) acc[t][k] += __shfl_xor_sync(0xffffffffu, acc[t][k], o);
+          const int j = 2 * t + (lane >> 1);
+          if (lane < 4 && j < np) {
+            const int p = pts[j];
+            const double c = c_level[l], dk = c * level_dk(T, l);
+            if (lane & 1) {
+              dsum[p][1][warp] += dk * acc[t][0];
+            } else {
+              dsum[p][0][warp] += c * acc[t][0];
+              dsum[p][2][warp] += dk * acc[t][1];
+              dsum[p][3][warp] += dk * acc[t][2];
+            }
+          }
+        }
+        __syncwarp();
+      };
+      if (NT > 1 && np > 2) run(std::integral_constant<int, NT>{});
+      else run(std::integral_constant<int, 1>{});
+    }
   double sums[4] = {0, 0, 0, 0};  // sum_{k != 0} W, sum D_2
-  {
-    const int dw = T.dw, nw = T.n_window;
-    const double dk0 = T.delta_k[0];
-    // the k = 0 mode is left out, as in Ewald summation: a neutral system has
-    // g(0) = 0, but all particles but one carry the net charge -q, whose
-    // k = 0 term is the uniform neutralising background's business
-    const int k_zero = (nw * dw + nw) * dw + nw;
-    for (int k = threadIdx.x; k < T.Hw; k += blockDim.x) {
+  // the k = 0 mode is left out, as in Ewald summation: a neutral system has
+  // g(0) = 0, but all particles but one carry the net charge -q, whose
+  // k = 0 term is the uniform neutralising background's business
+  const int k_zero = (NW * S::DW + NW) * S::DW + NW;
+  for (int k = tid; k < S::HW; k += BG_T)
+    if (k != k_zero) sums[0] += T.W[k];
+  if (top >= 2)
+    for (int k = tid; k < S::H; k += BG_T) sums[1] += T.D2[k];
+  batch_block_sum<4>(sums, red);
+  const double dk0 = T.delta_k[0];
+  const int pool_n = 0;  // arrivals in the overflow pool are folded into the slots before this kernel runs
+  for (int g = 0; g < n; ++g) {
+    const Header& h = hs[g];
+    const double q = h.q;
+    Tables uu;
+    alloc_tables(phases + size_t(g) * per, T, uu);
+    double v[4] = {0, 0, 0, 0};  // phi and its gradient, window
+    for (int k = tid; k < S::HW; k += BG_T) {
       if (k == k_zero) continue;
-      const double2 u = phase_at(uu.root, k, dw);
-      const double2 g = T.out_root[k];
-      const double bx = g.x - q * u.x, by = g.y - q * u.y;
+      const double2 u = phase_at(uu.root, k, S::DW);
+      const double2 gk = T.out_root[k];
+      const double bx = gk.x - q * u.x, by = gk.y - q * u.y;
       const double w = T.W[k];
-      sums[0] += w;
       v[0] += (u.x * bx + u.y * by) * w;
       const double im = (u.y * bx - u.x * by) * w;  // Im(u conj(b))
-      const int ix = k % dw, iy = (k / dw) % dw, iz = k / (dw * dw);
-      gw[0] += dk0 * (ix - nw) * im;
-      gw[1] += dk0 * (iy - nw) * im;
-      gw[2] += dk0 * (iz - nw) * im;
+      const int ix = k % S::DW, iy = (k / S::DW) % S::DW, iz = k / (S::DW * S::DW);
+      v[1] += dk0 * (ix - NW) * im;
+      v[2] += dk0 * (iy - NW) * im;
+      v[3] += dk0 * (iz - NW) * im;
     }
-  }
-  {
-    const int base = T.pw_base, d = T.dd, n = T.n_diff;
-    for (int k = threadIdx.x; k < T.H; k += blockDim.x) {
-      const int ix = k % d, iy = (k / d) % d, iz = k / (d * d);
-      const double dd2 = T.D2[k];
-      sums[1] += dd2;
-      for (int l = 2; l <= lo_max; ++l) {
-        const double2 u = cmul(uu.lev[l][2][iz], cmul(uu.lev[l][1][iy], uu.lev[l][0][ix]));
-        const double2 cc = T.inc[size_t(h.path_o[l] - base) * T.H + k];
-        const double f = c_level[l] * dd2;
-        v[1] += (u.x * cc.x - u.y * cc.y - q * (u.x * u.x + u.y * u.y)) * f;
-        const double im = (u.x * cc.y + u.y * cc.x) * f;  // Im(u cc)
-        const double dkl = level_dk(T, l);
-        gd[0] += dkl * (ix - n) * im;
-        gd[1] += dkl * (iy - n) * im;
-        gd[2] += dkl * (iz - n) * im;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) v[a] *= c_window;
+    const double b = level_box(T, h.depth_o - 1);
+    batch_near<GRP>(T, srcs, g, h.xo, b, pool_n, [&](double qj, double dx, double dy, double dz, double r2) {
+      const double r = sqrt(r2);
+      v[0] += qj * poly(r, b);
+      const double gr = qj * poly.deriv(r, b) / r;
+      v[1] += gr * dx;
+      v[2] += gr * dy;
+      v[3] += gr * dz;
+    });
+    batch_block_sum<4>(v, red);
+    if (tid == 0) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+        for (int w = 0; w < BG_W; ++w) v[a] += dsum[g][a][w];
+      double cself = 0.5 * c_window * sums[0] - self_w;
+      for (int l = 2; l <= h.depth_o - 2; ++l) {
+        v[0] -= c_level[l] * q * sums[1];
+        cself += 0.5 * c_level[l] * sums[1] - Sl[l];
       }
+      int c = 0;
+#pragma unroll
+      for (int k = 0; k < GRP; ++k)
+        if (k == g) c = cand[k];
+      phi_out[c] = v[0] + 2.0 * q * cself;
+      if (field_out)
+        for (int a = 0; a < 3; ++a) field_out[3 * size_t(c) + a] = -v[1 + a];
     }
-  }
-  // near field: the source lists of the particle's leaf, the particle itself excluded
-  double gr[3] = {0, 0, 0};
-  {
-    const int lv = h.depth_o - 1;
-    const int leaf = h.path_o[lv];
-    const double b = level_box(T, lv);
-    const double eps = 2.220446049250313e-16;
-    __shared__ int m_beg[36], m_pre[37];
-    __shared__ double m_off[36][3];
-    if (threadIdx.x < 36) {
-      const int src = threadIdx.x;
-      int j = -1;
-      if (src == 0) j = leaf;
-      else if (src <= 27) j = (src - 1 == 13) ? -1 : T.col27[size_t(leaf) * 27 + (src - 1)];
-      else j = T.coarse8[size_t(leaf) * 8 + (src - 28)];
-      int beg = 0, cnt = 0;
-      double off[3] = {0, 0, 0};
-      if (j >= 0) {
-        const int lj = T.node_level[j];
-        const unsigned long long pj = T.node_prefix[j];
-        beg = T.node_begin[j];
-        cnt = (T.node_child0[j] < 0 ? beg + T.leaf_count[j] : T.node_end[j]) - beg;
-        const double bj = level_box(T, lj);
-        const int Xj[3] = {int(compact3(pj)), int(compact3(pj >> 1)), int(compact3(pj >> 2))};
-        for (int a = 0; a < 3; ++a)
-          off[a] = -periodic_shift_d(center_of(T.L, lv, h.Xo[lv][a]), center_of(T.L, lj, Xj[a]), T.L, b, bj) * T.L;
-      }
-      m_beg[src] = beg;
-      m_pre[src] = cnt;
-      for (int a = 0; a < 3; ++a) m_off[src][a] = off[a];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int acc = 0;
-      for (int src = 0; src < 36; ++src) {
-        const int nn = m_pre[src];
-        m_pre[src] = acc;
-        acc += nn;
-      }
-      m_pre[36] = acc;
-    }
-    __syncthreads();
-    const int total = m_pre[36];
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
-      int lo = 0, hi = 36;
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (m_pre[mid] <= e) lo = mid;
-        else hi = mid;
-      }
-      const int s = m_beg[lo] + (e - m_pre[lo]);
-      const double dx = h.xo[0] - (T.sx[s] + m_off[lo][0]), dy = h.xo[1] - (T.sy[s] + m_off[lo][1]),
-                   dz = h.xo[2] - (T.sz[s] + m_off[lo][2]);
-      const double r2 = dx * dx + dy * dy + dz * dz;
-      if (r2 > eps && r2 < b * b) {
-        const double r = sqrt(r2), qj = T.sq[s];
-        v[2] += qj * poly(r, b);
-        const double g = qj * poly.deriv(r, b) / r;
-        gr[0] += g * dx;
-        gr[1] += g * dy;
-        gr[2] += g * dz;
-      }
-    }
-    // arrivals parked in the overflow pool that belong to a source's subtree
-    // are folded into the slots by the host before this kernel runs
-  }
-  double v4[4] = {v[0], v[1], v[2], 0.0};
-  block_sum4(v4, red);
-  double w4[4] = {gw[0], gw[1], gw[2], 0.0};
-  block_sum4(w4, red);
-  double d4[4] = {gd[0], gd[1], gd[2], 0.0};
-  block_sum4(d4, red);
-  double r4[4] = {gr[0], gr[1], gr[2], 0.0};
-  block_sum4(r4, red);
-  block_sum4(sums, red);
-  if (threadIdx.x == 0) {
-    double cself = 0.5 * c_window * sums[0] - self_w;
-    for (int l = 2; l <= lo_max; ++l) cself += 0.5 * c_level[l] * sums[1] - Sl[l];
-    phi_out[c] = v4[0] * c_window + v4[1] + v4[2] + 2.0 * q * cself;
-    if (field_out)
-      for (int a = 0; a < 3; ++a) field_out[3 * size_t(c) + a] = -(w4[a] * c_window + d4[a] + r4[a]);
   }
 }
 
-using PotentialKernel = void (*)(DevTree, const int*, double, double, const double*, double*, double*);
-PotentialKernel potential_kernel(int np) {
+using PotentialKernel = void (*)(DevTree, const int*, const int*, int, double, double, const double*, double*, double*);
+PotentialKernel potential_kernel(int np, int grp) {
   switch (np) {
-    case 7: return k_potential_batch<7>;
-    case 13: return k_potential_batch<13>;
-    case 19: return k_potential_batch<19>;
-    case 25: return k_potential_batch<25>;
+    case 7: return grp > 1 ? k_potential_batch<7, BG_GROUP> : k_potential_batch<7, 1>;
+    case 13: return grp > 1 ? k_potential_batch<13, BG_GROUP> : k_potential_batch<13, 1>;
+    case 19: return grp > 1 ? k_potential_batch<19, BG_GROUP> : k_potential_batch<19, 1>;
+    case 25: return grp > 1 ? k_potential_batch<25, BG_GROUP> : k_potential_batch<25, 1>;
     default: throw std::invalid_argument("unsupported residual polynomial");
   }
 }
@@ -3209,20 +3625,49 @@ void DmkTree::mc_run_device(int n_moves, const int* d_idx, const double* d_disp,
   mark_moved();
 }
 
-// All candidates in one launch of k_shift_batch (one block per candidate).
-void DmkTree::shift_batch_device(int m, const int* d_idx, const double* d_disp, double* d_dE) {
+// The batch kernels' groups: BG_GROUP particles a block in Morton order when
+// there are enough of them (order: room for m indices, or null), else one.
+int DmkTree::batch_groups(int m, const int* d_idx, int* order) {
+  const int grp = order && m >= kGroupMin ? BG_GROUP : 1;
+  if (grp > 1) {
+    k_order_particles<<<1, 1024, 0, st_>>>(dev_, d_idx, m, order);
+    PDMK_LAUNCH_CHECK();
+  }
+  return grp;
+}
+
+// The tree's own index array for the order; null while a capture that would
+// have to allocate it is under way.
+int* DmkTree::batch_order(int m) {
+  if (m < kGroupMin) return nullptr;
+  if (m > order_cap_) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    PDMK_CUDA(cudaStreamIsCapturing(st_, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return nullptr;
+    order_cap_ = std::max(m, 2 * order_cap_);
+    d_order_ = static_cast<int*>(alloc(sizeof(int) * size_t(order_cap_)));
+  }
+  return d_order_;
+}
+
+void DmkTree::launch_shift_batch(int m, const int* d_idx, const double* d_disp, int* order, double* d_dE) {
   DevTree& D = dev_;
-  if (m <= 0) return;
-  const size_t smem = tables_smem(D, D.max_depth, 2);
-  const ShiftBatchKernel kern = shift_batch_kernel(D.n_poly);
+  const int grp = batch_groups(m, d_idx, order);
+  const size_t smem = batch_smem(D.n_poly, D.max_depth, 2 * grp);
+  const ShiftBatchKernel kern = shift_batch_kernel(D.n_poly, grp);
   raise_smem_limit(reinterpret_cast<const void*>(kern), smem);
   const double pi = 3.14159265358979323846;
   const double c_window = std::pow(D.delta_k[0], 3) / std::pow(2 * pi, 3);
-  kern<<<unsigned(m), SB_T, smem, st_>>>(D, d_idx, d_disp, c_window, d_dE);
+  kern<<<unsigned((m + grp - 1) / grp), BG_T, smem, st_>>>(D, d_idx, d_disp, grp > 1 ? order : nullptr, m, c_window, d_dE);
   PDMK_LAUNCH_CHECK();
-  last_valid_ = false;
 }
 
+// All candidates in one launch of k_shift_batch.
+void DmkTree::shift_batch_device(int m, const int* d_idx, const double* d_disp, double* d_dE) {
+  if (m <= 0) return;
+  launch_shift_batch(m, d_idx, d_disp, batch_order(m), d_dE);
+  last_valid_ = false;
+}
 
 // ---------------------------------------------------------------------------
 // Candidate batch through a fixed static device buffer. For callers that may
@@ -3230,8 +3675,8 @@ void DmkTree::shift_batch_device(int m, const int* d_idx, const double* d_disp, 
 // device memory up front, a host thread that must not enter the allocator
 // between steps): the candidates' indices and displacements are staged into
 // g_static_scratch and their energy shifts come back through it, and the
-// batch is the same single launch of k_shift_batch as the allocating batch
-// (one block per candidate; its phase tables live in shared memory). The
+// batch is the same launch of k_shift_batch as the allocating batch (its phase
+// tables live in shared memory; the order of a large batch in the array). The
 // array's device address is looked up once per device, with that device
 // current. Nothing in the buffer has to start at zero: every call writes the
 // inputs it reads, and the kernel writes every output before it is read.
@@ -3242,7 +3687,8 @@ constexpr int kStaticMaxMoves = 4096;  // candidates per call
 constexpr size_t kOffIdx = 0;
 constexpr size_t kOffDisp = kOffIdx + sizeof(int) * kStaticMaxMoves;
 constexpr size_t kOffDE = kOffDisp + sizeof(double) * 3 * kStaticMaxMoves;
-constexpr size_t kStaticBytes = kOffDE + sizeof(double) * kStaticMaxMoves;  // 144 KB
+constexpr size_t kOffOrder = kOffDE + sizeof(double) * kStaticMaxMoves;
+constexpr size_t kStaticBytes = kOffOrder + sizeof(int) * kStaticMaxMoves;  // 160 KB
 
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticBytes];
 
@@ -3283,13 +3729,14 @@ void DmkTree::shift_batch_static(int m, const long* h_idx, const double* h_disp,
     PDMK_CUDA(cudaMemcpyAsync(s_idx + c0, chunk, sizeof(int) * nc, cudaMemcpyHostToDevice, st_));
   }
   PDMK_CUDA(cudaMemcpyAsync(s_disp, h_disp, sizeof(double) * 3 * m, cudaMemcpyHostToDevice, st_));
-  const size_t smem = tables_smem(D, D.max_depth, 2);
-  const ShiftBatchKernel kern = shift_batch_kernel(D.n_poly);
-  raise_smem_limit(reinterpret_cast<const void*>(kern), smem);
-  const double pi = 3.14159265358979323846;
-  const double c_window = std::pow(D.delta_k[0], 3) / std::pow(2 * pi, 3);
-  kern<<<unsigned(m), SB_T, smem, st_>>>(D, s_idx, s_disp, c_window, s_dE);
-  PDMK_LAUNCH_CHECK();
+  // both forms of the kernel are loaded by the first call, so that no later
+  // one enters the driver's allocator
+  for (int grp : {1, BG_GROUP})
+    raise_smem_limit(reinterpret_cast<const void*>(shift_batch_kernel(D.n_poly, grp)),
+                     batch_smem(D.n_poly, D.max_depth, 2 * grp));
+  cudaFuncAttributes fa;
+  PDMK_CUDA(cudaFuncGetAttributes(&fa, k_order_particles));
+  launch_shift_batch(m, s_idx, s_disp, reinterpret_cast<int*>(base + kOffOrder), s_dE);
   PDMK_CUDA(cudaMemcpyAsync(h_dE, s_dE, sizeof(double) * m, cudaMemcpyDeviceToHost, st_));
   PDMK_CUDA(cudaStreamSynchronize(st_));
 }
@@ -3379,13 +3826,16 @@ void DmkTree::potential_batch(int m, const int* d_idx, double* d_phi, double* d_
   if (m <= 0) return;
   ensure_packed();  // the near-field source lists read the slots only
   prepare_box_lists();  // the per-level self terms S_l
-  const size_t smem = tables_smem(D, D.max_depth, 1);
-  const PotentialKernel kern = potential_kernel(D.n_poly);
+  int* order = batch_order(m);
+  const int grp = batch_groups(m, d_idx, order);
+  const size_t smem = batch_smem(D.n_poly, D.max_depth, grp);
+  const PotentialKernel kern = potential_kernel(D.n_poly, grp);
   raise_smem_limit(reinterpret_cast<const void*>(kern), smem);
   const double pi = 3.14159265358979323846;
   const double c_window = std::pow(D.delta_k[0], 3) / std::pow(2 * pi, 3);
   const double self_w = ps_.psi0_0 / (2 * D.boxsize[2] * ps_.C0);
-  kern<<<unsigned(m), SB_T, smem, st_>>>(D, d_idx, c_window, self_w, d_Sl_, d_phi, d_field);
+  kern<<<unsigned((m + grp - 1) / grp), BG_T, smem, st_>>>(D, d_idx, grp > 1 ? order : nullptr, m, c_window, self_w,
+                                                           d_Sl_, d_phi, d_field);
   PDMK_LAUNCH_CHECK();
 }
 

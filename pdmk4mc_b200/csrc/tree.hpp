@@ -352,6 +352,12 @@ class DmkTree {
   int mc_grid_ = 0;
   double* mc_partials_ = nullptr;
   unsigned int* mc_sync_ = nullptr;
+  // batches of candidates or points: their Morton order
+  int* d_order_ = nullptr;
+  int order_cap_ = 0;
+  int* batch_order(int m);
+  int batch_groups(int m, const int* d_idx, int* order);
+  void launch_shift_batch(int m, const int* d_idx, const double* d_disp, int* order, double* d_dE);
   // deferred expansion updates of Metropolis sequences (shift.cu)
   static constexpr int kPendPerBlock = 16;  // listed moves one block of the persistent kernel keeps
   bool inc_formed_ = false;  // the incoming rows follow from the outgoing ones (a deferred update recomputes them)
