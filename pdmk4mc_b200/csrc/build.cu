@@ -935,6 +935,7 @@ namespace {
 struct KernelTables {
   const double* W = nullptr;
   const double* D2 = nullptr;
+  double sum_w = 0, sum_d2 = 0;  // over the half grid; W(0) is zero
 };
 
 struct ModeTransforms {
@@ -1003,6 +1004,8 @@ KernelTables kernel_tables(const ProlateSetup& s, double L, std::vector<double>&
         }
   }
   KernelTables t{W, D2};
+  for (size_t i = 0; i < hw; ++i) t.sum_w += W[i];
+  for (size_t i = 0; i < hd; ++i) t.sum_d2 += D2[i];
   if (cached) cache.emplace(key, t);
   return t;
 }
@@ -1031,6 +1034,8 @@ void DmkTree::build_setup() {
   // window and difference tables, shared by every tree of this (digits, L)
   std::vector<double> own;
   const KernelTables kt = kernel_tables(s, L_, own);
+  sum_w_ = kt.sum_w;
+  sum_d2_ = kt.sum_d2;
   D.W = static_cast<double*>(alloc(sizeof(double) * D.Hw));
   D.D2 = static_cast<double*>(alloc(sizeof(double) * D.H));
   PDMK_CUDA(cudaMemcpyAsync(D.W, kt.W, sizeof(double) * D.Hw, cudaMemcpyHostToDevice, st_));

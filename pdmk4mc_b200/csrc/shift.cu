@@ -2622,6 +2622,7 @@ template <int NP>
 __device__ void load_octant(const DevTree& T, double* tab) {
   using S = BatchShape<NP>;
   if constexpr (S::TAB)
+#pragma unroll 8
     for (int i = threadIdx.x; i < S::TAB_DOUBLES; i += BG_T) {
       const int mx = i % S::DS, r = i / S::DS, mz = r / S::N1, my = r % S::N1;
       tab[i] = mx < S::N1 ? T.D2[((S::N1 - 1 - mz) * S::D + S::N1 - 1 + my) * S::D + S::N1 - 1 + mx] : 0.0;
@@ -2787,9 +2788,10 @@ __device__ void batch_block_sum(double (&v)[N], double (*sm)[BG_W]) {
   }
 }
 
-// GRP = 4 groups along the Morton order where there are enough particles to
-// fill the SMs with groups, else one particle a block.
-constexpr int BG_GROUP = 4;
+// GRP = 2: pairs along the Morton order where there are enough particles to
+// fill the SMs, else one particle a block. (Groups of 4 read a third less, but their
+// columns leave room for one block per SM: 1.43 against 1.12 ms for 4096 candidates.)
+constexpr int BG_GROUP = 2;
 constexpr int kGroupMin = 4 * 148 * 2;  // two groups per SM
 
 // order[]: the particles idx[0 .. m) by the level-4 cell of their positions (one
@@ -2839,9 +2841,9 @@ __global__ void __launch_bounds__(1024) k_order_particles(DevTree T, const int* 
 }
 
 template <int NP, int GRP>
-__global__ void __launch_bounds__(BG_T) k_shift_batch(DevTree T, const int* __restrict__ idx,
+__global__ void __launch_bounds__(BG_T, 2) k_shift_batch(DevTree T, const int* __restrict__ idx,
                                                       const double* __restrict__ disp, const int* __restrict__ order, int m,
-                                                      double c_window, double* __restrict__ dE_out) {
+                                                      double c_window, double sum_d2, double* __restrict__ dE_out) {
   using S = BatchShape<NP>;
   constexpr int PTS = 2 * GRP, NT = (PTS + 3) / 4;  // point 2 g: target of candidate g, 2 g + 1: its origin
   extern __shared__ double sm_b[];
@@ -2895,8 +2897,8 @@ __global__ void __launch_bounds__(BG_T) k_shift_batch(DevTree T, const int* __re
     leaf = (p & 1) ? h.path_o[l] : h.path_t[l];
     Xl = (p & 1) ? h.Xo[l] : h.Xt[l];
   });
-  // window (src/energy_shift.cpp:72-90) and the sum of D over the half grid (|o|^2 = q^2)
-  double v[GRP], sum_d[1] = {0.0};
+  // window (src/energy_shift.cpp:72-90)
+  double v[GRP];
 #pragma unroll
   for (int g = 0; g < GRP; ++g) v[g] = 0.0;
   for (int k = tid; k < S::HW; k += BG_T) {
@@ -2915,8 +2917,6 @@ __global__ void __launch_bounds__(BG_T) k_shift_batch(DevTree T, const int* __re
   }
 #pragma unroll
   for (int g = 0; g < GRP; ++g) v[g] *= c_window;
-  if (top >= 2)
-    for (int k = tid; k < S::H; k += BG_T) sum_d[0] += T.D2[k];
   // near field (src/energy_shift.cpp:233-302)
   const int pool_n = *T.pool_n;
 #pragma unroll
@@ -2935,7 +2935,6 @@ __global__ void __launch_bounds__(BG_T) k_shift_batch(DevTree T, const int* __re
   }
   // difference (src/energy_shift.cpp:92-140), row by row; a warp's sums of a
   // point add up over the levels in its own words
-  double* mine = &red[0][0];  // [point][warp]
   if (lane < PTS) red[lane][warp] = 0.0;
   __syncwarp();
   for (int l = 2; l <= top; ++l)
@@ -2974,14 +2973,12 @@ __global__ void __launch_bounds__(BG_T) k_shift_batch(DevTree T, const int* __re
       if (NT > 1 && np > 4) run(std::integral_constant<int, NT>{});
       else run(std::integral_constant<int, 1>{});
     }
-  (void)mine;
   // totals: one thread per candidate adds its points' words of all warps
   __syncthreads();
   double diff = 0.0;
   if (tid < n)
     for (int p = 0; p < 2; ++p)
       for (int w = 0; w < BG_W; ++w) diff += red[2 * tid + p][w];
-  batch_block_sum<1>(sum_d, red);
   batch_block_sum<GRP>(v, red);
   if (tid < n) {
     const Header& h = hs[tid];
@@ -2989,7 +2986,7 @@ __global__ void __launch_bounds__(BG_T) k_shift_batch(DevTree T, const int* __re
 #pragma unroll
     for (int g = 0; g < GRP; ++g)
       if (g == tid) tot = v[g];
-    for (int l = 2; l <= h.depth_o - 2; ++l) diff += c_level[l] * h.q * h.q * sum_d[0];
+    for (int l = 2; l <= h.depth_o - 2; ++l) diff += c_level[l] * h.q * h.q * sum_d2;  // |o|^2 = q^2 at every mode
     double self = 0;
     if (h.dr != 0) self = poly(h.dr, level_box(T, 2)) * h.q * h.q;
     int c = 0;
@@ -3000,7 +2997,7 @@ __global__ void __launch_bounds__(BG_T) k_shift_batch(DevTree T, const int* __re
   }
 }
 
-using ShiftBatchKernel = void (*)(DevTree, const int*, const double*, const int*, int, double, double*);
+using ShiftBatchKernel = void (*)(DevTree, const int*, const double*, const int*, int, double, double, double*);
 ShiftBatchKernel shift_batch_kernel(int np, int grp) {
   switch (np) {
     case 7: return grp > 1 ? k_shift_batch<7, BG_GROUP> : k_shift_batch<7, 1>;
@@ -3034,9 +3031,10 @@ size_t batch_smem(int np, int max_depth, int points) {
 // -i k u: the row products carry two more columns per point, kx ex, and the y
 // and z derivatives take their factors at the lines.
 template <int NP, int GRP>
-__global__ void __launch_bounds__(BG_T) k_potential_batch(DevTree T, const int* __restrict__ idx,
+__global__ void __launch_bounds__(BG_T, 2) k_potential_batch(DevTree T, const int* __restrict__ idx,
                                                           const int* __restrict__ order, int m, double c_window,
-                                                          double self_w, const double* __restrict__ Sl,
+                                                          double self_w, double sum_w, double sum_d2,
+                                                          const double* __restrict__ Sl,
                                                           double* __restrict__ phi_out, double* __restrict__ field_out) {
   using S = BatchShape<NP>;
   constexpr int ND = S::N1 - 1, NW = (S::DW - 1) / 2, NT = (GRP + 1) / 2;
@@ -3143,16 +3141,10 @@ __global__ void __launch_bounds__(BG_T) k_potential_batch(DevTree T, const int* 
       if (NT > 1 && np > 2) run(std::integral_constant<int, NT>{});
       else run(std::integral_constant<int, 1>{});
     }
-  double sums[4] = {0, 0, 0, 0};  // sum_{k != 0} W, sum D_2
   // the k = 0 mode is left out, as in Ewald summation: a neutral system has
   // g(0) = 0, but all particles but one carry the net charge -q, whose
   // k = 0 term is the uniform neutralising background's business
   const int k_zero = (NW * S::DW + NW) * S::DW + NW;
-  for (int k = tid; k < S::HW; k += BG_T)
-    if (k != k_zero) sums[0] += T.W[k];
-  if (top >= 2)
-    for (int k = tid; k < S::H; k += BG_T) sums[1] += T.D2[k];
-  batch_block_sum<4>(sums, red);
   const double dk0 = T.delta_k[0];
   const int pool_n = 0;  // arrivals in the overflow pool are folded into the slots before this kernel runs
   for (int g = 0; g < n; ++g) {
@@ -3190,10 +3182,10 @@ __global__ void __launch_bounds__(BG_T) k_potential_batch(DevTree T, const int* 
 #pragma unroll
       for (int a = 0; a < 4; ++a)
         for (int w = 0; w < BG_W; ++w) v[a] += dsum[g][a][w];
-      double cself = 0.5 * c_window * sums[0] - self_w;
+      double cself = 0.5 * c_window * sum_w - self_w;
       for (int l = 2; l <= h.depth_o - 2; ++l) {
-        v[0] -= c_level[l] * q * sums[1];
-        cself += 0.5 * c_level[l] * sums[1] - Sl[l];
+        v[0] -= c_level[l] * q * sum_d2;
+        cself += 0.5 * c_level[l] * sum_d2 - Sl[l];
       }
       int c = 0;
 #pragma unroll
@@ -3206,7 +3198,8 @@ __global__ void __launch_bounds__(BG_T) k_potential_batch(DevTree T, const int* 
   }
 }
 
-using PotentialKernel = void (*)(DevTree, const int*, const int*, int, double, double, const double*, double*, double*);
+using PotentialKernel = void (*)(DevTree, const int*, const int*, int, double, double, double, double, const double*,
+                                 double*, double*);
 PotentialKernel potential_kernel(int np, int grp) {
   switch (np) {
     case 7: return grp > 1 ? k_potential_batch<7, BG_GROUP> : k_potential_batch<7, 1>;
@@ -3658,7 +3651,8 @@ void DmkTree::launch_shift_batch(int m, const int* d_idx, const double* d_disp, 
   raise_smem_limit(reinterpret_cast<const void*>(kern), smem);
   const double pi = 3.14159265358979323846;
   const double c_window = std::pow(D.delta_k[0], 3) / std::pow(2 * pi, 3);
-  kern<<<unsigned((m + grp - 1) / grp), BG_T, smem, st_>>>(D, d_idx, d_disp, grp > 1 ? order : nullptr, m, c_window, d_dE);
+  kern<<<unsigned((m + grp - 1) / grp), BG_T, smem, st_>>>(D, d_idx, d_disp, grp > 1 ? order : nullptr, m, c_window, sum_d2_,
+                                                           d_dE);
   PDMK_LAUNCH_CHECK();
 }
 
@@ -3835,7 +3829,7 @@ void DmkTree::potential_batch(int m, const int* d_idx, double* d_phi, double* d_
   const double c_window = std::pow(D.delta_k[0], 3) / std::pow(2 * pi, 3);
   const double self_w = ps_.psi0_0 / (2 * D.boxsize[2] * ps_.C0);
   kern<<<unsigned((m + grp - 1) / grp), BG_T, smem, st_>>>(D, d_idx, grp > 1 ? order : nullptr, m, c_window, self_w,
-                                                           d_Sl_, d_phi, d_field);
+                                                           sum_w_, sum_d2_, d_Sl_, d_phi, d_field);
   PDMK_LAUNCH_CHECK();
 }
 

@@ -352,6 +352,7 @@ class DmkTree {
   int mc_grid_ = 0;
   double* mc_partials_ = nullptr;
   unsigned int* mc_sync_ = nullptr;
+  double sum_w_ = 0, sum_d2_ = 0;  // the window and level-2 difference tables summed over the half grid
   // batches of candidates or points: their Morton order
   int* d_order_ = nullptr;
   int order_cap_ = 0;
