@@ -615,32 +615,43 @@ constexpr int RES_SCH = 256;  // sources staged in shared memory per round
 // listed coarse level first, so the big items start first. The up to 35
 // source boxes (self, colleagues, coarse-grain) are flattened into one index
 // range, staged in rounds of RES_SCH with their periodic offsets applied.
-// Each thread keeps one target in registers and walks a share of the staged
-// sources (a warp reads the same source: a shared-memory broadcast).
+//
+// About one pair in six lies inside the cut-off. Testing all of them in FP64
+// took most of the kernel's instructions, so the pairs are sieved first: a
+// warp holds 32 targets, which are neighbours in Morton order (as a tile of 32
+// sources is), and skips the tiles whose bounding box is out of reach; the
+// pairs left are tested in FP32 with a margin above its rounding, and the ones
+// that may be inside go to the warp's queue as (target, source) indices, a
+// tile's at once: a lane keeps its target's 32 answers as a bit mask (nine
+// instructions a pair, where asking the warp for every pair took 28). The
+// queue is evaluated 32 pairs at a time in FP64, distance and polynomial, so
+// the sum is the one over all pairs (a pair beyond the cut-off adds zero there).
 template <int NP>
 __global__ void __launch_bounds__(RES_T) k_residual(DevTree T, const int* __restrict__ leaves, int ny,
                                                     double* part) {
   __shared__ double ux[RES_SCH], uy[RES_SCH], uz[RES_SCH], uq[RES_SCH];
-  __shared__ int uslot[RES_SCH];
+  __shared__ float4 uf[RES_SCH];                  // relative to the leaf's centre
+  __shared__ float t_lo[RES_SCH / 32][3], t_hi[RES_SCH / 32][3];  // bounding boxes of the source tiles
+  __shared__ double gx[RES_TCH], gy[RES_TCH], gz[RES_TCH], gq[RES_TCH];
   __shared__ int m_beg[36], m_pre[37];
   __shared__ double m_off[36][3], m_w[36];
   __shared__ double sm[32];
-  // per warp, the pairs inside the cut-off waiting for a polynomial: r^2 and
-  // q_target q_source (at most 31 waiting plus 32 added in one step)
-  __shared__ double q_r2[RES_T / 32][64], q_w[RES_T / 32][64];
+  __shared__ unsigned short q_pair[RES_T / 32][1056];  // per warp: at most 31 pairs waiting and a tile's 1024
   const ResidualPoly<NP> poly(T);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int qn = 0;  // pairs waiting in this warp's queue (warp-uniform)
   const int node = leaves[blockIdx.x / ny], chunk = blockIdx.x % ny;
   const int l = T.node_level[node];
   const int cnt = T.leaf_count[node];
   double e = 0;
-  double inv_b_all = 0;
   if (l >= 2 && cnt > chunk * RES_TCH) {
     const double b = level_box(T, l), inv_b = 1.0 / b;
-    inv_b_all = inv_b;
-    const double b2 = b * b * (1.0 + 1e-14);  // square roots only near or inside the cut-off
+    // FP32 coordinates reach 2 b from the centre: each is off by 2^-23 b at
+    // most, a squared distance near b^2 by less than 2e-6 b^2
+    const float cut = float(b * b * (1.0 + 8e-6));
+    const float far = 1e18f;  // where a lane without a target, or a tile's empty place, is put
     const int tb = T.node_begin[node];
+    double ci[3];
+    node_center(T, node, ci);
     if (threadIdx.x < 36) {
       const int src = threadIdx.x;
       int j = -1;
@@ -657,8 +668,7 @@ __global__ void __launch_bounds__(RES_T) k_residual(DevTree T, const int* __rest
       int beg = 0, n = 0;
       double off[3] = {0, 0, 0};
       if (j >= 0 && !skip && T.node_count[j] > 0) {
-        double ci[3], cj[3];
-        node_center(T, node, ci);
+        double cj[3];
         node_center(T, j, cj);
         const double bj = level_box(T, T.node_level[j]);
         for (int dd = 0; dd < 3; ++dd) off[dd] = -periodic_shift_d(ci[dd], cj[dd], T.L, b, bj) * T.L;
@@ -684,78 +694,121 @@ __global__ void __launch_bounds__(RES_T) k_residual(DevTree T, const int* __rest
     const int total = m_pre[36];
     for (int t0 = chunk * RES_TCH; t0 < cnt; t0 += ny * RES_TCH) {
       const int nt = min(RES_TCH, cnt - t0);
-      const int npad = nt <= 32 ? 32 : 64;
-      const int nparts = RES_T / npad;
-      const int it = threadIdx.x % npad, sp = threadIdx.x / npad;
-      const bool act = it < nt;
-      int tslot = -2;
-      double tx = 0, ty = 0, tz = 0, tq = 0;
-      if (act) {
-        tslot = tb + t0 + it;
-        tx = T.sx[tslot];
-        ty = T.sy[tslot];
-        tz = T.sz[tslot];
-        tq = T.sq[tslot];
+      // groups of 32 targets, the warps of one group sharing the source tiles
+      const int ngrp = nt <= 32 ? 1 : 2, nparts = RES_T / 32 / ngrp;
+      const int grp = wid % ngrp, sp = wid / ngrp;
+      const int it = grp * 32 + lane;
+      if (threadIdx.x < nt) {
+        const int s = tb + t0 + threadIdx.x;
+        gx[threadIdx.x] = T.sx[s];
+        gy[threadIdx.x] = T.sy[s];
+        gz[threadIdx.x] = T.sz[s];
+        gq[threadIdx.x] = T.sq[s];
       }
+      __syncthreads();
+      const bool act = it < nt;
+      const float fx = act ? float(gx[it] - ci[0]) : far, fy = act ? float(gy[it] - ci[1]) : far,
+                  fz = act ? float(gz[it] - ci[2]) : far;
+      float lo[3] = {fx, fy, fz}, hi[3] = {act ? fx : -far, act ? fy : -far, act ? fz : -far};
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+        for (int o = 16; o > 0; o >>= 1) {
+          lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
+          hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
+        }
       for (int u0 = 0; u0 < total; u0 += RES_SCH) {
         const int ns = min(RES_SCH, total - u0);
         __syncthreads();
-        for (int t = threadIdx.x; t < ns; t += blockDim.x) {
-          const int ei = u0 + t;
-          int lo = 0, hi = 36;  // largest src with m_pre[src] <= ei
-          while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (m_pre[mid] <= ei) lo = mid;
-            else hi = mid;
+        for (int t = threadIdx.x; t < (ns + 31) / 32 * 32; t += blockDim.x) {  // whole warps
+          float4 f = make_float4(-far, -far, -far, 0.0f);  // far from everything, from an absent target too
+          float flo[3] = {far, far, far}, fhi[3] = {-far, -far, -far};
+          if (t < ns) {
+            const int ei = u0 + t;
+            int a = 0, z = 36;  // largest src with m_pre[src] <= ei
+            while (z - a > 1) {
+              const int mid = (a + z) >> 1;
+              if (m_pre[mid] <= ei) a = mid;
+              else z = mid;
+            }
+            const int s = m_beg[a] + (ei - m_pre[a]);
+            const double x = T.sx[s] + m_off[a][0], y = T.sy[s] + m_off[a][1], zz = T.sz[s] + m_off[a][2];
+            ux[t] = x;
+            uy[t] = y;
+            uz[t] = zz;
+            uq[t] = T.sq[s] * m_w[a];
+            f = make_float4(float(x - ci[0]), float(y - ci[1]), float(zz - ci[2]), 0.0f);
+            flo[0] = fhi[0] = f.x;
+            flo[1] = fhi[1] = f.y;
+            flo[2] = fhi[2] = f.z;
           }
-          const int s = m_beg[lo] + (ei - m_pre[lo]);
-          ux[t] = T.sx[s] + m_off[lo][0];
-          uy[t] = T.sy[s] + m_off[lo][1];
-          uz[t] = T.sz[s] + m_off[lo][2];
-          uq[t] = T.sq[s] * m_w[lo];
-          uslot[t] = lo == 0 ? s : -1;
+          uf[t] = f;
+#pragma unroll
+          for (int a = 0; a < 3; ++a)
+            for (int o = 16; o > 0; o >>= 1) {
+              flo[a] = fminf(flo[a], __shfl_xor_sync(0xffffffffu, flo[a], o));
+              fhi[a] = fmaxf(fhi[a], __shfl_xor_sync(0xffffffffu, fhi[a], o));
+            }
+          if (lane < 3) {
+            t_lo[t >> 5][lane] = lane == 0 ? flo[0] : lane == 1 ? flo[1] : flo[2];
+            t_hi[t >> 5][lane] = lane == 0 ? fhi[0] : lane == 1 ? fhi[1] : fhi[2];
+          }
         }
         __syncthreads();
-        // About one pair in six lies inside the cut-off, and a warp would run
-        // the Horner chain whenever any lane needs it: the lanes push their
-        // in-range pairs into the warp's queue instead, and the warp
-        // evaluates the polynomial 32 queued pairs at a time. The loop is
-        // warp-uniform (every lane of a warp has the same source partition).
-        for (int js = sp; js < ns; js += nparts) {
-          const double dx = tx - ux[js], dy = ty - uy[js], dz = tz - uz[js];
-          const double r2 = dx * dx + dy * dy + dz * dz;
-          const bool in = act && r2 <= b2 && uslot[js] != tslot;
-          const unsigned m = __ballot_sync(0xffffffffu, in);
-          if (in) {
-            const int pos = qn + __popc(m & ((1u << lane) - 1u));
-            q_r2[wid][pos] = r2;
-            q_w[wid][pos] = tq * uq[js];
+        int qn = 0;  // pairs waiting in this warp's queue (warp-uniform)
+        auto evaluate = [&](int at, int n) {  // n queued pairs from place `at`
+          if (lane < n) {
+            const int p = q_pair[wid][at + lane];
+            const int js = p & 255, i = p >> 8;
+            const double dx = gx[i] - ux[js], dy = gy[i] - uy[js], dz = gz[i] - uz[js];
+            const double r2 = dx * dx + dy * dy + dz * dz;
+            e += gq[i] * uq[js] * poly.from_r2(r2, inv_b);  // zero at r = 0 (the target itself) and beyond the cut-off
           }
-          qn += __popc(m);
-          if (qn >= 32) {
-            __syncwarp();
-            e += q_w[wid][lane] * poly.from_r2(q_r2[wid][lane], inv_b);  // from_r2 is zero beyond the cut-off
-            const int rem = qn - 32;
-            double r2m = 0, wm = 0;
-            if (lane < rem) {
-              r2m = q_r2[wid][32 + lane];
-              wm = q_w[wid][32 + lane];
-            }
-            __syncwarp();
-            if (lane < rem) {
-              q_r2[wid][lane] = r2m;
-              q_w[wid][lane] = wm;
-            }
-            __syncwarp();
-            qn = rem;
+        };
+        for (int tile = sp; tile * 32 < ns; tile += nparts) {
+          float d2 = 0.0f;
+#pragma unroll
+          for (int a = 0; a < 3; ++a) {
+            const float d = fmaxf(0.0f, fmaxf(lo[a] - t_hi[tile][a], t_lo[tile][a] - hi[a]));
+            d2 = fmaf(d, d, d2);
           }
+          if (d2 > cut) continue;
+          const float4* tp = uf + tile * 32;
+          unsigned mask = 0;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const float4 s = tp[j];
+            const float dx = fx - s.x, dy = fy - s.y, dz = fz - s.z;
+            if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= cut) mask |= 1u << j;
+          }
+          // this lane's places in the queue: after the pairs waiting and the lanes below
+          const int mine = __popc(mask);
+          int at = mine;
+          for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= o) at += y;
+          }
+          const int all = __shfl_sync(0xffffffffu, at, 31);
+          at += qn - mine;
+          while (mask) {
+            q_pair[wid][at++] = static_cast<unsigned short>((it << 8) | (tile * 32 + __ffs(mask) - 1));
+            mask &= mask - 1;
+          }
+          qn += all;
+          __syncwarp();
+          int done = 0;
+          for (; qn - done >= 32; done += 32) evaluate(done, 32);
+          qn -= done;
+          unsigned short left = 0;  // the rest moves to the front
+          if (lane < qn) left = q_pair[wid][done + lane];
+          __syncwarp();
+          if (lane < qn) q_pair[wid][lane] = left;
         }
+        __syncwarp();
+        evaluate(0, qn);  // the queue names places of this round's sources
       }
+      __syncthreads();  // the targets are replaced
     }
   }
-  // the pairs still queued
-  __syncwarp();
-  if (lane < qn) e += q_w[wid][lane] * poly.from_r2(q_r2[wid][lane], inv_b_all);
   double s = block_sum(0.5 * e, sm);
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
