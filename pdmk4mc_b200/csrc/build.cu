@@ -49,6 +49,12 @@ void put_small(void* dst, const void* src, size_t bytes, cudaStream_t st) {
   PDMK_LAUNCH_CHECK();
 }
 
+__global__ void k_root(uint64_t* list, int* n_refined, uint32_t* bitmap) {
+  *list = 0;
+  *n_refined = 1;
+  *bitmap = 1u;
+}
+
 // ---------------------------------------------------------------------------
 __global__ void k_keys(const double* r, long n, double L, uint64_t* key, int* val) {
   long i = long(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -157,6 +163,45 @@ __global__ void k_balance_level(Bitmaps B, int level, int fan) {
   }
 }
 
+// Word prefixes and refined-cell counts of the shallow levels 0 .. kEager, one
+// block per level (a level deeper than those takes a scan of its own)
+constexpr int kEager = 6;
+
+__global__ void __launch_bounds__(1024) k_rank_levels(Bitmaps B, int* total) {
+  __shared__ int wsum[32];
+  __shared__ int s_carry;
+  const int l = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nwords = l < 2 ? 1 : 1 << (3 * l - 5);
+  if (threadIdx.x == 0) s_carry = 0;
+  __syncthreads();
+  for (int w0 = 0; w0 < nwords; w0 += 1024) {
+    const int w = w0 + threadIdx.x;
+    const int c = w < nwords ? __popc(B.bm[l][w]) : 0;
+    int x = c;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+      int v = wsum[lane];
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += y;
+      }
+      wsum[lane] = v;
+    }
+    __syncthreads();
+    const int carry = s_carry;
+    if (w < nwords) B.wprefix[l][w] = carry + (warp > 0 ? wsum[warp - 1] : 0) + x - c;
+    __syncthreads();
+    if (threadIdx.x == 0) s_carry = carry + wsum[31];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) total[l] = s_carry;
+}
+
 __global__ void k_word_popc(const uint32_t* bm, long nwords, int* out) {
   long w = long(blockIdx.x) * blockDim.x + threadIdx.x;
   if (w < nwords) out[w] = __popc(bm[w]);
@@ -172,6 +217,35 @@ struct NodeArrays {
   int* parent;
   int* child0;
 };
+
+// The nodes of the shallow levels 0 .. last (cells of all of them, one thread
+// each, in one launch: a thread per bitmap word walked up to 256 nodes alone,
+// 40 us a level at N = 1e6)
+struct LevelStarts {
+  int v[MAX_LEVELS + 2];
+};
+
+__global__ void k_enum_shallow(Bitmaps B, int last, int maxref, LevelStarts ls, NodeArrays na) {
+  long t = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  int l = 0;
+  while (l <= last && t >= (1L << (3 * l))) {
+    t -= 1L << (3 * l);
+    ++l;
+  }
+  if (l > last) return;
+  const uint64_t cell = uint64_t(t);
+  int id = 0, parent = -1;
+  if (l > 0) {
+    const uint64_t pc = cell >> 3;
+    if (!bit_get(B.bm[l - 1], pc)) return;
+    id = ls.v[l] + 8 * cell_rank(B, l - 1, pc) + int(cell & 7);
+    parent = l == 1 ? 0 : ls.v[l - 1] + 8 * cell_rank(B, l - 2, pc >> 3) + int(pc & 7);
+  }
+  na.prefix[id] = cell;
+  na.level[id] = l;
+  na.parent[id] = parent;
+  na.child0[id] = l <= maxref && bit_get(B.bm[l], cell) ? ls.v[l + 1] + 8 * cell_rank(B, l, cell) : -1;
+}
 
 __global__ void k_enum_nodes(Bitmaps B, int level, int maxref, const int* level_start, NodeArrays na) {
   // nodes at `level` are the children of refined cells at level-1
@@ -554,7 +628,7 @@ void DmkTree::build(const double* r_in, const double* q_in, bool on_device) {
   PDMK_CUDA(cudaMallocAsync(&sort_scr, radix_sort_scratch_bytes(std::max<long>(n, 64)), st_));
   k_keys<<<grid_for(n), TPB, 0, st_>>>(r, n, L_, keys, ord);
   PDMK_LAUNCH_CHECK();
-  radix_sort_pairs(keys, ord, n, 8, sort_scr, st_);
+  radix_sort_pairs(keys, ord, n, 0, sort_scr, st_);
   // the sorted particles, kept for the outgoing pass: four rows x, y, z, q
   // (read as one 2-D tensor by the mixed pass, so the stride is even)
   dense_stride_ = (n + 31) & ~31L;
@@ -575,17 +649,22 @@ void DmkTree::build(const double* r_in, const double* q_in, bool on_device) {
   long list_cap = std::max<long>(1024, 8 * (n / std::max(1, n_per_leaf_) + 64) + 4096);
   PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&lists[0]), size_t(list_cap) * 8, st_));
   PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&lists[1]), size_t(list_cap) * 8, st_));
-  uint64_t zero = 0;
-  put_small(lists[0], &zero, 8, st_);
   int maxref = 0;  // deepest level holding a refined cell
   {
-    const int one = 1;
-    put_small(d_lvl, &one, 4, st_);
-    // root: refined (all nodes above level 2 are refined)
-    B.bm[0] = static_cast<uint32_t*>(alloc(4));
-    put_small(B.bm[0], &one, 4, st_);
+    // bitmaps of the shallow levels in one block, cleared together
+    long shallow = 0;
+    for (int l = 0; l <= kEager; ++l) shallow += nwords[l];
+    uint32_t* words = static_cast<uint32_t*>(alloc(size_t(shallow) * 4));
+    PDMK_CUDA(cudaMemsetAsync(words, 0, size_t(shallow) * 4, st_));
+    for (int l = 0; l <= kEager; ++l) {
+      B.bm[l] = words;
+      words += nwords[l];
+    }
+    // root: refined (all nodes above level 2 are refined), the first list's only cell
+    k_root<<<1, 1, 0, st_>>>(lists[0], d_lvl, B.bm[0]);
+    PDMK_LAUNCH_CHECK();
     auto refine = [&](int l, unsigned grid) {
-      if (l < MAX_LEVEL) {
+      if (l > kEager && l < MAX_LEVEL) {
         B.bm[l] = static_cast<uint32_t*>(alloc(size_t(nwords[l]) * 4));
         PDMK_CUDA(cudaMemsetAsync(B.bm[l], 0, size_t(nwords[l]) * 4, st_));
       }
@@ -595,8 +674,7 @@ void DmkTree::build(const double* r_in, const double* q_in, bool on_device) {
     };
     // the shallow levels (bitmaps of at most 32 KB) go back to back with one
     // read-back; deeper trees continue level by level
-    constexpr int kEager = 6;
-    for (int l = 1; l <= kEager; ++l) refine(l, grid_for(list_cap));
+    for (int l = 1; l <= kEager; ++l) refine(l, grid_for(std::min(list_cap, 1L << (3 * l))));
     int cnt[kBadWord + 1] = {0};
     PDMK_CUDA(cudaMemcpyAsync(cnt, d_lvl, sizeof(cnt), cudaMemcpyDeviceToHost, st_));
     PDMK_CUDA(cudaStreamSynchronize(st_));
@@ -632,8 +710,18 @@ void DmkTree::build(const double* r_in, const double* q_in, bool on_device) {
   }
   // ranks of refined cells
   std::vector<int> refined(maxref + 1, 0);
-  for (int l = 0; l <= maxref; ++l) {
-    B.wprefix[l] = static_cast<int*>(alloc(size_t(nwords[l]) * 4));
+  {
+    long words = 0;
+    for (int l = 0; l <= maxref; ++l) words += nwords[l];
+    int* pre = static_cast<int*>(alloc(size_t(words) * 4));
+    for (int l = 0; l <= maxref; ++l) {
+      B.wprefix[l] = pre;
+      pre += nwords[l];
+    }
+  }
+  k_rank_levels<<<unsigned(std::min(maxref, kEager) + 1), 1024, 0, st_>>>(B, d_cnt);
+  PDMK_LAUNCH_CHECK();
+  for (int l = kEager + 1; l <= maxref; ++l) {
     k_word_popc<<<grid_for(nwords[l]), TPB, 0, st_>>>(B.bm[l], nwords[l], B.wprefix[l]);
     PDMK_LAUNCH_CHECK();
     void* scr;
@@ -655,12 +743,34 @@ void DmkTree::build(const double* r_in, const double* q_in, bool on_device) {
   const int n_nodes = h_level_start_[nlev];
   D.n_nodes = n_nodes;
   for (int l = 0; l <= nlev && l < MAX_LEVELS + 2; ++l) D.level_start[l] = h_level_start_[l];
-  int* d_level_start = static_cast<int*>(alloc(sizeof(int) * (nlev + 1)));
-  put_small(d_level_start, h_level_start_.data(), sizeof(int) * (nlev + 1), st_);
   D.boxsize[0] = L_;
   for (int l = 1; l < MAX_LEVELS + 2; ++l) D.boxsize[l] = 0.5 * D.boxsize[l - 1];
-  double* d_boxsize = static_cast<double*>(alloc(sizeof(double) * (MAX_LEVELS + 2)));
-  put_small(d_boxsize, D.boxsize, sizeof(double) * (MAX_LEVELS + 2), st_);
+  for (int l = 0; l < MAX_LEVELS; ++l) {
+    D.bm[l] = l <= maxref ? B.bm[l] : nullptr;
+    D.wprefix[l] = l <= maxref ? B.wprefix[l] : nullptr;
+  }
+  D.maxref = maxref;
+  // the per-level tables, in one block and one launch
+  struct LevelTables {
+    const void* ptrs[2 * MAX_LEVELS];
+    double boxsize[MAX_LEVELS + 2];
+    int start[MAX_LEVELS + 3];
+    int pad;
+  } lt{};
+  static_assert(sizeof(LevelTables) % 4 == 0, "words");
+  for (int l = 0; l < MAX_LEVELS; ++l) {
+    lt.ptrs[l] = D.bm[l];
+    lt.ptrs[MAX_LEVELS + l] = D.wprefix[l];
+  }
+  for (int l = 0; l < MAX_LEVELS + 2; ++l) lt.boxsize[l] = D.boxsize[l];
+  for (int l = 0; l <= nlev; ++l) lt.start[l] = h_level_start_[l];
+  LevelTables* d_lt = static_cast<LevelTables*>(alloc(sizeof(LevelTables)));
+  put_small(d_lt, &lt, sizeof(lt), st_);
+  D.bm_d = reinterpret_cast<const uint32_t* const*>(d_lt->ptrs);
+  D.wprefix_d = reinterpret_cast<const int* const*>(d_lt->ptrs + MAX_LEVELS);
+  const double* d_boxsize = d_lt->boxsize;
+  const int* d_level_start = d_lt->start;
+  D.level_start_d = d_level_start;
 
   NodeArrays na;
   na.prefix = static_cast<uint64_t*>(alloc(sizeof(uint64_t) * n_nodes));
@@ -668,33 +778,17 @@ void DmkTree::build(const double* r_in, const double* q_in, bool on_device) {
   na.parent = static_cast<int*>(alloc(sizeof(int) * n_nodes));
   na.child0 = static_cast<int*>(alloc(sizeof(int) * n_nodes));
   {
-    uint64_t p0 = 0;
-    int l0 = 0, par0 = -1, c0 = 1;
-    put_small(na.prefix, &p0, 8, st_);
-    put_small(na.level, &l0, 4, st_);
-    put_small(na.parent, &par0, 4, st_);
-    put_small(na.child0, &c0, 4, st_);
-  }
-  for (int l = 1; l < nlev; ++l) {
-    k_enum_nodes<<<grid_for(nwords[l - 1]), TPB, 0, st_>>>(B, l, maxref, d_level_start, na);
+    const int last = std::min(nlev - 1, kEager);
+    LevelStarts ls{};
+    for (int l = 0; l <= nlev; ++l) ls.v[l] = h_level_start_[l];
+    long cells = 0;
+    for (int l = 0; l <= last; ++l) cells += 1L << (3 * l);
+    k_enum_shallow<<<grid_for(cells), TPB, 0, st_>>>(B, last, maxref, ls, na);
     PDMK_LAUNCH_CHECK();
   }
-  for (int l = 0; l < MAX_LEVELS; ++l) {
-    D.bm[l] = l <= maxref ? B.bm[l] : nullptr;
-    D.wprefix[l] = l <= maxref ? B.wprefix[l] : nullptr;
-  }
-  D.maxref = maxref;
-  D.level_start_d = d_level_start;
-  {
-    const void* ptrs[2 * MAX_LEVELS];
-    for (int l = 0; l < MAX_LEVELS; ++l) {
-      ptrs[l] = D.bm[l];
-      ptrs[MAX_LEVELS + l] = D.wprefix[l];
-    }
-    void** d_ptrs = static_cast<void**>(alloc(sizeof(ptrs)));
-    put_small(d_ptrs, ptrs, sizeof(ptrs), st_);
-    D.bm_d = reinterpret_cast<const uint32_t* const*>(d_ptrs);
-    D.wprefix_d = reinterpret_cast<const int* const*>(d_ptrs + MAX_LEVELS);
+  for (int l = kEager + 1; l < nlev; ++l) {
+    k_enum_nodes<<<grid_for(nwords[l - 1]), TPB, 0, st_>>>(B, l, maxref, d_level_start, na);
+    PDMK_LAUNCH_CHECK();
   }
   D.node_prefix = na.prefix;
   D.node_level = na.level;
@@ -734,7 +828,9 @@ void DmkTree::build(const double* r_in, const double* q_in, bool on_device) {
   {
     void* scr;
     PDMK_CUDA(cudaMallocAsync(&scr, radix_sort_scratch_bytes(std::max(nl, 64)), st_));
-    radix_sort_pairs(lkey, lid, nl, 8, scr, st_);
+    // leaves of level <= nlev - 1: the key bits below it are zero (an even
+    // number of byte passes leaves the result in place)
+    radix_sort_pairs(lkey, lid, nl, (3 * (KEY_BITS - (nlev - 1)) / 8) & ~1, scr, st_);
     PDMK_CUDA(cudaFreeAsync(scr, st_));
   }
   int* cnt = static_cast<int*>(alloc(sizeof(int) * nl));

@@ -13,8 +13,9 @@ size_t scan_scratch_bytes(long n);
 void exclusive_scan(const int* in, int* out, long n, void* scratch, cudaStream_t st);
 // same for 64-bit element sums of int inputs
 size_t radix_sort_scratch_bytes(long n);
-// stable sort by key over key bits [0, 8*passes); keys/vals are sorted in
-// place (an equal-sized alternate buffer lives in scratch)
-void radix_sort_pairs(uint64_t* keys, int* vals, long n, int passes, void* scratch, cudaStream_t st);
+// sort by key, stable for values that come in ascending order (and for any
+// with distinct keys); keys/vals are sorted in place (an equal-sized alternate
+// buffer lives in scratch). The low `first` bytes of every key are zero.
+void radix_sort_pairs(uint64_t* keys, int* vals, long n, int first, void* scratch, cudaStream_t st);
 
 }  // namespace pdmk
