@@ -1153,6 +1153,16 @@ void DmkTree::build_setup() {
   D.prop = static_cast<Proposal*>(alloc(sizeof(Proposal)));
   PDMK_CUDA(cudaMemsetAsync(D.prop, 0, sizeof(Proposal), st_));
   D.recv = static_cast<Receiver*>(alloc(sizeof(Receiver) * MAX_RECV));
+  // per-level constants of eval_energy_diff (src/energy.cpp:50-57)
+  double coef[2][MAX_LEVELS + 2] = {};
+  for (int l = 2; l < MAX_LEVELS + 1; ++l) {
+    coef[0][l] = 1 / (2 * std::pow(2 * pi, 3)) * std::pow(D.delta_k[l], 3);
+    coef[1][l] = s.psi0_0 * (1 / (2 * D.boxsize[l + 1] * s.C0) - 1 / (2 * D.boxsize[l] * s.C0));
+  }
+  d_Cl_ = static_cast<double*>(alloc(sizeof(coef)));
+  d_Sl_ = d_Cl_ + (MAX_LEVELS + 2);
+  put_small(d_Cl_, coef, sizeof(coef), st_);
+  d_scalars_ = static_cast<double*>(alloc(sizeof(double) * 8));
   d_one_idx_ = static_cast<int*>(alloc(64));
   d_one_disp_ = static_cast<double*>(alloc(64));
   d_one_u_ = static_cast<double*>(alloc(64));

@@ -25,6 +25,7 @@
 
 #include "common.cuh"
 #include "mixed.hpp"
+#include "plan.hpp"
 #include "tree.hpp"
 
 namespace pdmk {
@@ -47,18 +48,6 @@ __device__ inline double block_sum(double v, double* sm) {
 }
 
 // ---------------------------------------------------------------------------
-// NUDFT work item: one box (or one split-K chunk of it) over a range of the
-// particles in leaf order, pos = rows x, y, z, q (without the leaves' free
-// slots, which were 26 % of the slots at N = 1e6)
-struct NudftWork {
-  double cx, cy, cz;  // box centre
-  double dk;
-  int X, Y, Z;        // integer box coordinates at its level
-  int M;              // decentring multiplier: 1 for levels >= 2, 3 for the root
-  int s_begin, s_end;
-  double2* out;       // H complex outputs of this box (or of this split-K chunk)
-};
-
 // T as an FP64 tensor-core product (mma m8n8k4): rows (a, b), columns c,
 // summed over particles. Rows come in tiles of eight b for one a, the two a
 // (cosine, sine) of one kz together: a warp holds CPW such (kz, b tile) pairs
@@ -94,7 +83,7 @@ struct NudftShape {
 // spends about 3 % of its time here; a separate pass wrote and read 1.6 KB
 // per particle and level, 2.8 ms at N = 1e6.)
 template <int NK>
-__device__ __forceinline__ void nudft_factors(const NudftWork& w, int base, double* buf, const double* __restrict__ pos,
+__device__ __forceinline__ void nudft_factors(const PwItem& w, int base, double* buf, const double* __restrict__ pos,
                                               long stride) {
   using S = NudftShape<NK>;
   for (int t = threadIdx.x; t < S::KC * 3; t += S::THREADS) {
@@ -130,11 +119,11 @@ __device__ __forceinline__ void nudft_factors(const NudftWork& w, int base, doub
 
 template <int NK>
 __global__ void __launch_bounds__(NudftShape<NK>::THREADS, 2)
-    k_nudft(const NudftWork* __restrict__ work, const double* __restrict__ pos, long stride) {
+    k_nudft(const PwItem* __restrict__ work, const double* __restrict__ pos, long stride) {
   using S = NudftShape<NK>;
   constexpr int NT = S::NT, CPW = S::CPW, STR = S::STR, N1 = S::N1, D = S::D;
   extern __shared__ double smem_d[];
-  const NudftWork w = work[blockIdx.x / S::TILES];
+  const PwItem w = work[blockIdx.x / S::TILES];
   const int tile = blockIdx.x % S::TILES;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int q4 = lane & 3, q8 = lane >> 2;
@@ -239,7 +228,7 @@ __global__ void __launch_bounds__(NudftShape<NK>::THREADS, 2)
 }
 
 template <int NK>
-void launch_nudft(const NudftWork* d_work, int nwork, const double* pos, long stride, cudaStream_t st) {
+void launch_nudft(const PwItem* d_work, int nwork, const double* pos, long stride, cudaStream_t st) {
   using S = NudftShape<NK>;
   if (nwork == 0) return;
   // per device and thread-safe: replica energies call this from several host threads
@@ -265,7 +254,7 @@ int nudft_tiles(int nk) {
   }
 }
 
-void dispatch_nudft(int nk, const NudftWork* d_work, int nwork, const double* pos, long stride, cudaStream_t st) {
+void dispatch_nudft(int nk, const PwItem* d_work, int nwork, const double* pos, long stride, cudaStream_t st) {
   switch (nk) {
     case 4: launch_nudft<4>(d_work, nwork, pos, stride, st); break;
     case 6: launch_nudft<6>(d_work, nwork, pos, stride, st); break;
@@ -282,15 +271,14 @@ void dispatch_nudft(int nk, const NudftWork* d_work, int nwork, const double* po
 }
 
 // sum split-K chunk partials of box b into its output, in chunk order
-__global__ void k_reduce_chunks(const double2* part, const int* chunk_first, const int* chunk_n, double2* const* outs,
-                                int H) {
-  int b = blockIdx.y;
+__global__ void k_reduce_chunks(const double2* part, const PwSplit* __restrict__ split, int H) {
+  const PwSplit b = split[blockIdx.y];
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= H) return;
-  const double2* p = part + size_t(chunk_first[b]) * H + k;
+  const double2* p = part + size_t(b.first) * H + k;
   double2 s = make_double2(0, 0);
-  for (int c = 0; c < chunk_n[b]; ++c) s = cadd(s, p[size_t(c) * H]);
-  outs[b][k] = s;
+  for (int c = 0; c < b.n; ++c) s = cadd(s, p[size_t(c) * H]);
+  b.out[k] = s;
 }
 
 // ---------------------------------------------------------------------------
@@ -1040,51 +1028,6 @@ void DmkTree::form_outgoing_pw() {
   ensure_dense();
   DevTree& D = dev_;
   const int n_all = int(N_);
-  // split-K bookkeeping: chunks go to a partial buffer, then reduce
-  struct Chunked {
-    int first, n;
-    double2* out;
-  };
-  // one box (or box chunk) over the slots [sb, se)
-  auto make_work = [&](std::vector<NudftWork>& wl, int l, uint64_t p, double2* out, int sb, int se) {
-    NudftWork w{};
-    double scale = std::ldexp(1.0, -l);
-    int X = int(compact3(p)), Y = int(compact3(p >> 1)), Z = int(compact3(p >> 2));
-    w.cx = L_ * (double(X) * scale + 0.5 * scale);
-    w.cy = L_ * (double(Y) * scale + 0.5 * scale);
-    w.cz = L_ * (double(Z) * scale + 0.5 * scale);
-    w.dk = D.delta_k[l];
-    w.X = X;
-    w.Y = Y;
-    w.Z = Z;
-    w.M = l == 0 ? 3 : 1;
-    w.s_begin = sb;
-    w.s_end = se;
-    w.out = out;
-    wl.push_back(w);
-  };
-  // the mixed pass: one item per (box or box chunk, pair of 128-row M tiles)
-  auto make_mix = [&](std::vector<MixItem>& wl, int nk, int l, uint64_t p, double2* out, int sb, int se) {
-    MixItem w{};
-    double scale = std::ldexp(1.0, -l);
-    int X = int(compact3(p)), Y = int(compact3(p >> 1)), Z = int(compact3(p >> 2));
-    w.cx = L_ * (double(X) * scale + 0.5 * scale);
-    w.cy = L_ * (double(Y) * scale + 0.5 * scale);
-    w.cz = L_ * (double(Z) * scale + 0.5 * scale);
-    w.dk = D.delta_k[l];
-    w.X = X;
-    w.Y = Y;
-    w.Z = Z;
-    w.M = l == 0 ? 3 : 1;
-    w.s_begin = sb;
-    w.s_end = se;
-    w.out = out;
-    const int pairs = mixed_pairs(nk);
-    for (int t = 0; t < pairs; ++t) {
-      w.pair = t;
-      wl.push_back(w);
-    }
-  };
   const bool mixed = opt_.precision == 1;
   CUtensorMap tmap_root{}, tmap_box{};
   if (mixed) {
@@ -1100,67 +1043,40 @@ void DmkTree::form_outgoing_pw() {
     make_coord_map(&tmap_box, dense_, int(dense_stride_), mixed_chunk(D.n_diff));
   }
   int* d_mix_err = mixed ? reinterpret_cast<int*>(d_mix_ + 1) : nullptr;
-  auto align16 = [](size_t b) { return (b + 15) & ~size_t(15); };
-  // one upload per pass: the work items, their table chunk lists, then per
-  // split-K group its first chunk, chunk count and output
-  auto upload = [&](const auto& wl, const std::vector<int2>& ch, const std::vector<Chunked>& sp, size_t* off_ch,
-                    size_t* off_meta, size_t* off_out) {
-    using Item = typename std::decay_t<decltype(wl)>::value_type;
-    *off_ch = align16(sizeof(Item) * wl.size());
-    *off_meta = align16(*off_ch + sizeof(int2) * ch.size());
-    *off_out = align16(*off_meta + sizeof(int) * 2 * sp.size());
-    const size_t bytes = align16(*off_out + sizeof(double2*) * sp.size()) + 16;
-    std::vector<unsigned char> blob(bytes, 0);
-    std::memcpy(blob.data(), wl.data(), sizeof(Item) * wl.size());
-    std::memcpy(blob.data() + *off_ch, ch.data(), sizeof(int2) * ch.size());
-    int* meta = reinterpret_cast<int*>(blob.data() + *off_meta);
-    double2** outs = reinterpret_cast<double2**>(blob.data() + *off_out);
-    for (size_t i = 0; i < sp.size(); ++i) {
-      meta[i] = sp[i].first;
-      meta[sp.size() + i] = sp[i].n;
-      outs[i] = sp[i].out;
-    }
-    unsigned char* d_blob;
-    PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d_blob), bytes, st_));
-    PDMK_CUDA(cudaMemcpyAsync(d_blob, blob.data(), bytes, cudaMemcpyHostToDevice, st_));
-    return d_blob;
+  auto get = [&](size_t bytes) {
+    void* p = nullptr;
+    PDMK_CUDA(cudaMallocAsync(&p, bytes + 16, st_));
+    return static_cast<unsigned char*>(p);
   };
-  auto reduce = [&](const std::vector<Chunked>& sp, const double2* pbase, int H, const unsigned char* d_blob,
-                    size_t off_meta, size_t off_out, cudaStream_t st) {
-    if (sp.empty()) return;
-    const int nbx = int(sp.size());
-    const int* d_meta = reinterpret_cast<const int*>(d_blob + off_meta);
-    double2* const* d_outs = reinterpret_cast<double2* const*>(d_blob + off_out);
-    dim3 grid(grid_for(H), unsigned(nbx));
-    k_reduce_chunks<<<grid, TPB, 0, st>>>(pbase, d_meta, d_meta + nbx, d_outs, H);
+  // a pass's items, split entries and chunk list in one block
+  struct Lists {
+    unsigned char* block;
+    PwItem* items;
+    PwSplit* split;
+    int2* chunks;
+  };
+  auto get_lists = [&](int n_items, int n_split, int n_chunks) {
+    Lists l;
+    l.block = get(sizeof(PwItem) * size_t(n_items) + sizeof(PwSplit) * size_t(n_split) + sizeof(int2) * size_t(n_chunks));
+    l.items = reinterpret_cast<PwItem*>(l.block);
+    l.split = reinterpret_cast<PwSplit*>(l.items + n_items);
+    l.chunks = reinterpret_cast<int2*>(l.split + n_split);
+    return l;
+  };
+  auto contract = [&](int nk, const CUtensorMap& tmap, const Lists& l, int n_items, int n_chunks, cudaStream_t st) {
+    if (mixed) dispatch_mixed(nk, tmap, l.items, n_items, l.chunks, n_chunks, d_mix_, d_mix_err, st);
+    else dispatch_nudft(nk, l.items, n_items, dense_, dense_stride_, st);
+  };
+  auto reduce = [&](const Lists& l, int n_split, const double2* part, int H, cudaStream_t st) {
+    if (n_split == 0) return;
+    k_reduce_chunks<<<dim3(grid_for(H), unsigned(n_split)), TPB, 0, st>>>(part, l.split, H);
     PDMK_LAUNCH_CHECK();
-  };
-  // the mixed pass's chunk tables: one block of mixed_table_bytes per chunk
-  // of each slot range, shared by the range's consecutive tile items; the
-  // chunk list names each chunk's range by its first tile item
-  auto plan_mix_tables = [&](int nk, std::vector<MixItem>& wl, unsigned char** tab, std::vector<int2>& ch) {
-    const int kcp = mixed_chunk(nk), tiles = mixed_pairs(nk);
-    const size_t tb = size_t(mixed_table_bytes(nk));
-    size_t total = 0;
-    for (size_t i = 0; i < wl.size(); i += tiles) total += size_t((wl[i].s_end - wl[i].s_begin + kcp - 1) / kcp);
-    PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(tab), total * tb + 16, st_));
-    size_t cur = 0;
-    for (size_t i = 0; i < wl.size(); i += tiles) {
-      const int n = (wl[i].s_end - wl[i].s_begin + kcp - 1) / kcp;
-      for (int t = 0; t < tiles; ++t) wl[i + t].tab = *tab + cur * tb;
-      for (int c = 0; c < n; ++c) ch.push_back(make_int2(int(i), c));
-      cur += size_t(n);
-    }
   };
   if (!aux_) {
     PDMK_CUDA(cudaStreamCreateWithFlags(&aux_, cudaStreamNonBlocking));
     PDMK_CUDA(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
     PDMK_CUDA(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
   }
-
-  // Root pass first, on the second stream: the root (node 0, all slots) needs
-  // no host view of the tree, so it runs while the host lays out the boxes.
-  // Its allocations are made on the tree's stream before the fork event.
   // A small system would leave most SMs idle behind a few blocks that each
   // walk all particles: its items are cut until about two waves of blocks are
   // there (not below 64 particles, where the partials' sum costs more).
@@ -1168,186 +1084,89 @@ void DmkTree::form_outgoing_pw() {
     const long want = (2L * resident + tiles - 1) / tiles;  // items for two waves
     return int(std::min<long>(split, std::max<long>(64, (particles + want - 1) / std::max<long>(want, 1))));
   };
-  const int KSPLIT_ROOT = mixed ? tune_.ksplit_root : fill_split(tune_.ksplit_root, n_all, nudft_tiles(D.n_window), 296);
+  auto shape = [&](int nk, int ksplit) {
+    return PlanShape{ksplit, mixed ? mixed_chunk(nk) : 1, mixed ? long(mixed_table_bytes(nk)) : 0L};
+  };
   const long pw_levels = std::max(0, D.pw_hi - D.pw_lo + 1);
-  const int KSPLIT = mixed ? tune_.ksplit
-                           : fill_split(tune_.ksplit, pw_levels * n_all, nudft_tiles(D.n_diff), 296);
-  const int nch_root = std::max(1, (n_all + KSPLIT_ROOT - 1) / KSPLIT_ROOT);
-  std::vector<Chunked> root_split{{0, nch_root, D.out_root}};
-  double2* part_r = nullptr;
-  PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&part_r), sizeof(double2) * (size_t(nch_root) * D.Hw + 1), st_));
-  std::vector<NudftWork> wroot;
-  std::vector<MixItem> mroot;
-  for (int c = 0; c < nch_root; ++c) {
-    int sb = c * KSPLIT_ROOT, se = std::min(n_all, sb + KSPLIT_ROOT);
-    if (mixed) make_mix(mroot, D.n_window, 0, 0, part_r + size_t(c) * D.Hw, sb, se);
-    else make_work(wroot, 0, 0, part_r + size_t(c) * D.Hw, sb, se);
-  }
-  unsigned char* mtab_root = nullptr;
-  std::vector<int2> ch_root;
-  size_t rch, rmeta, rout;
-  unsigned char* d_root = nullptr;
-  if (mixed) {
-    plan_mix_tables(D.n_window, mroot, &mtab_root, ch_root);
-    d_root = upload(mroot, ch_root, root_split, &rch, &rmeta, &rout);
-  } else {
-    d_root = upload(wroot, ch_root, root_split, &rch, &rmeta, &rout);
-  }
+  const PlanShape root_shape = shape(
+      D.n_window, mixed ? tune_.ksplit_root : fill_split(tune_.ksplit_root, n_all, nudft_tiles(D.n_window), 296));
+  const PlanShape box_shape = shape(
+      D.n_diff, mixed ? tune_.ksplit : fill_split(tune_.ksplit, pw_levels * n_all, nudft_tiles(D.n_diff), 296));
+
+  // the boxes' totals, counted before the root pass takes the device
+  const bool lists = !box_lists_ready_;
+  const size_t state_bytes = (sizeof(PlanState) + 15) & ~size_t(15);
+  unsigned char* d_plan = get(state_bytes + sizeof(int) * 3 * size_t(plan_blocks(D.n_nodes)));
+  PlanState* d_state = reinterpret_cast<PlanState*>(d_plan);
+  int* d_blk = reinterpret_cast<int*>(d_plan + state_bytes);
+  PDMK_CUDA(cudaMemsetAsync(d_state, 0, sizeof(PlanState), st_));
+  launch_plan_count(D, box_shape, lists, d_state, d_blk, st_);
+
+  // Root pass on the second stream: the root (node 0, all particles) needs no
+  // totals, so it runs while they travel. Its allocations are made on the
+  // tree's stream before the fork event.
+  const int n_root = std::max(1, (n_all + root_shape.ksplit - 1) / root_shape.ksplit);
+  const int root_full = (root_shape.ksplit + root_shape.kcp - 1) / root_shape.kcp;
+  const int n_root_chunks = !mixed ? 0
+                                   : (n_root - 1) * root_full +
+                                         (n_all - (n_root - 1) * root_shape.ksplit + root_shape.kcp - 1) / root_shape.kcp;
+  double2* part_r = reinterpret_cast<double2*>(get(sizeof(double2) * size_t(n_root) * D.Hw));
+  unsigned char* tab_r = mixed ? get(size_t(n_root_chunks) * root_shape.tab_bytes) : nullptr;
+  const Lists root = get_lists(n_root, 1, n_root_chunks);
+  launch_plan_root(D, root_shape, n_all, n_root, n_root_chunks, part_r, tab_r, root.items, root.chunks, root.split, st_);
   PDMK_CUDA(cudaEventRecord(ev_fork_, st_));
   PDMK_CUDA(cudaStreamWaitEvent(aux_, ev_fork_, 0));
-  if (mixed)
-    dispatch_mixed(D.n_window, tmap_root, reinterpret_cast<const MixItem*>(d_root), int(mroot.size()),
-                   reinterpret_cast<const int2*>(d_root + rch), int(ch_root.size()), d_mix_, d_mix_err, aux_);
-  else
-    dispatch_nudft(D.n_window, reinterpret_cast<const NudftWork*>(d_root), int(wroot.size()), dense_, dense_stride_, aux_);
-  reduce(root_split, part_r, D.Hw, d_root, rmeta, rout, aux_);
+  contract(D.n_window, tmap_root, root, n_root, n_root_chunks, aux_);
+  reduce(root, 1, part_r, D.Hw, aux_);
   PDMK_CUDA(cudaEventRecord(ev_join_, aux_));
 
-  // host view of the nodes' particle ranges and coordinates for the box work list
-  // (and, on a new tree, of the children for the box lists: one round trip)
-  const int nn = D.n_nodes;
-  std::vector<int> nb(nn), ne(nn), lv(nn), c0;
-  std::vector<uint64_t> pf(nn);
-  PDMK_CUDA(cudaMemcpyAsync(nb.data(), node_dense_, 4 * nn, cudaMemcpyDeviceToHost, st_));
-  PDMK_CUDA(cudaMemcpyAsync(ne.data(), D.node_count, 4 * nn, cudaMemcpyDeviceToHost, st_));
-  PDMK_CUDA(cudaMemcpyAsync(lv.data(), D.node_level, 4 * nn, cudaMemcpyDeviceToHost, st_));
-  PDMK_CUDA(cudaMemcpyAsync(pf.data(), D.node_prefix, 8 * nn, cudaMemcpyDeviceToHost, st_));
-  if (!box_lists_ready_) {
-    c0.resize(nn);
-    PDMK_CUDA(cudaMemcpyAsync(c0.data(), D.node_child0, 4 * nn, cudaMemcpyDeviceToHost, st_));
-  }
+  PlanTotals t;
+  PDMK_CUDA(cudaMemcpyAsync(&t, &d_state->t, sizeof(t), cudaMemcpyDeviceToHost, st_));
   PDMK_CUDA(cudaStreamSynchronize(st_));
-  if (!box_lists_ready_) build_box_lists(c0);
-  struct Box {
-    int node, sb, se, level;
-    double2* out;
-  };
-  std::vector<Box> boxes;
-  const int base = D.level_start[D.pw_lo];
-  if (D.pw_hi >= D.pw_lo)
-    for (int id = base; id < D.level_start[D.pw_hi + 1]; ++id)
-      boxes.push_back({id, nb[id], nb[id] + ne[id], lv[id], D.out + size_t(id - base) * D.H});
-  // boxes: largest first (longest-processing-time order), split when large
-  std::vector<int> order(boxes.size());
-  for (size_t i = 0; i < order.size(); ++i) order[i] = int(i);
-  std::stable_sort(order.begin(), order.end(),
-                   [&](int a, int b) { return boxes[a].se - boxes[a].sb > boxes[b].se - boxes[b].sb; });
-  std::vector<Chunked> box_split;
-  long chunk_cursor = 0;
-  for (int oi : order) {
-    const Box& bx = boxes[oi];
-    int cntp = bx.se - bx.sb;
-    if (cntp > KSPLIT) {
-      int nch = (cntp + KSPLIT - 1) / KSPLIT;
-      box_split.push_back({int(chunk_cursor), nch, bx.out});
-      chunk_cursor += nch;
-    }
-  }
-  double2* part_b = nullptr;
-  PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&part_b), sizeof(double2) * (size_t(chunk_cursor) * D.H + 1), st_));
-  std::vector<NudftWork> wbox;
-  std::vector<MixItem> mbox;
-  {
-    size_t si = 0;
-    long cur = 0;
-    auto add = [&](int l, uint64_t p, double2* out, int sb, int se) {
-      if (mixed) make_mix(mbox, D.n_diff, l, p, out, sb, se);
-      else make_work(wbox, l, p, out, sb, se);
-    };
-    for (int oi : order) {
-      const Box& bx = boxes[oi];
-      int cntp = bx.se - bx.sb;
-      if (cntp > KSPLIT) {
-        int nch = box_split[si].n;
-        for (int c = 0; c < nch; ++c) {
-          int sb = bx.sb + c * KSPLIT, se = std::min(bx.se, sb + KSPLIT);
-          add(bx.level, pf[bx.node], part_b + size_t(cur + c) * D.H, sb, se);
-        }
-        cur += nch;
-        ++si;
-      } else {
-        add(bx.level, pf[bx.node], bx.out, bx.sb, bx.se);
-      }
-    }
-  }
-  unsigned char* mtab_box = nullptr;
-  std::vector<int2> ch_box;
-  size_t bch, bmeta, bout;
-  unsigned char* d_box = nullptr;
-  if (mixed) {
-    plan_mix_tables(D.n_diff, mbox, &mtab_box, ch_box);
-    d_box = upload(mbox, ch_box, box_split, &bch, &bmeta, &bout);
-  } else {
-    d_box = upload(wbox, ch_box, box_split, &bch, &bmeta, &bout);
-  }
+  double2* part_b = reinterpret_cast<double2*>(get(sizeof(double2) * size_t(t.n_split_items) * D.H));
+  unsigned char* tab_b = mixed ? get(size_t(t.n_chunks) * box_shape.tab_bytes) : nullptr;
+  const Lists box = get_lists(t.n_items, t.n_split, t.n_chunks);
+  launch_plan_items(D, box_shape, node_dense_, d_state, part_b, tab_b, box.items, box.chunks, box.split, st_);
   time_begin(3);
-  if (mixed)
-    dispatch_mixed(D.n_diff, tmap_box, reinterpret_cast<const MixItem*>(d_box), int(mbox.size()),
-                   reinterpret_cast<const int2*>(d_box + bch), int(ch_box.size()), d_mix_, d_mix_err, st_);
-  else
-    dispatch_nudft(D.n_diff, reinterpret_cast<const NudftWork*>(d_box), int(wbox.size()), dense_, dense_stride_, st_);
+  contract(D.n_diff, tmap_box, box, t.n_items, t.n_chunks, st_);
   time_end(3);
-  reduce(box_split, part_b, D.H, d_box, bmeta, bout, st_);
+  reduce(box, t.n_split, part_b, D.H, st_);
+  if (lists) fill_box_lists(t, d_blk);
   // the root pass's buffers are released after it joins the tree's stream
   PDMK_CUDA(cudaStreamWaitEvent(st_, ev_join_, 0));
-  for (void* p : {static_cast<void*>(d_root), static_cast<void*>(mtab_root), static_cast<void*>(part_r),
-                  static_cast<void*>(d_box), static_cast<void*>(mtab_box), static_cast<void*>(part_b)})
+  for (void* p : {static_cast<void*>(root.block), static_cast<void*>(tab_r), static_cast<void*>(part_r),
+                  static_cast<void*>(box.block), static_cast<void*>(tab_b), static_cast<void*>(part_b),
+                  static_cast<void*>(d_plan)})
     if (p) PDMK_CUDA(cudaFreeAsync(p, st_));
   diff_cached_ = false;
 }
 
 void DmkTree::prepare_box_lists() {
   if (box_lists_ready_) return;
-  std::vector<int> c0(dev_.n_nodes);
-  PDMK_CUDA(cudaMemcpyAsync(c0.data(), dev_.node_child0, 4 * dev_.n_nodes, cudaMemcpyDeviceToHost, st_));
+  void* d_plan = nullptr;
+  const size_t state_bytes = (sizeof(PlanState) + 15) & ~size_t(15);
+  PDMK_CUDA(cudaMallocAsync(&d_plan, state_bytes + sizeof(int) * 3 * size_t(plan_blocks(dev_.n_nodes)), st_));
+  PlanState* state = static_cast<PlanState*>(d_plan);
+  int* blk = reinterpret_cast<int*>(static_cast<unsigned char*>(d_plan) + state_bytes);
+  PDMK_CUDA(cudaMemsetAsync(state, 0, sizeof(PlanState), st_));
+  launch_plan_count(dev_, PlanShape{1 << 30, 1, 0}, true, state, blk, st_);
+  PlanTotals t;
+  PDMK_CUDA(cudaMemcpyAsync(&t, &state->t, sizeof(t), cudaMemcpyDeviceToHost, st_));
   PDMK_CUDA(cudaStreamSynchronize(st_));
-  build_box_lists(c0);
+  fill_box_lists(t, blk);
+  PDMK_CUDA(cudaFreeAsync(d_plan, st_));
 }
 
-void DmkTree::build_box_lists(const std::vector<int>& c0) {
+// the lists behind counted totals (blk: the per-block counts)
+void DmkTree::fill_box_lists(const PlanTotals& t, const int* blk) {
   DevTree& D = dev_;
-  std::vector<int> nonleaf;
-  if (D.pw_hi >= D.pw_lo)
-    for (int id = D.level_start[D.pw_lo]; id < D.level_start[D.pw_hi + 1]; ++id)
-      if (c0[id] >= 0) nonleaf.push_back(id);
-  std::vector<int> leaves;
-  for (int id = D.level_start[2]; id < D.n_nodes; ++id)
-    if (c0[id] < 0) leaves.push_back(id);
-  // boxes two levels above the expansion levels with a non-leaf grandchild:
-  // each names the 4 x 4 x 4 receiving boxes of one incoming block
-  std::vector<int> cubes;
-  if (D.pw_hi >= D.pw_lo)
-    for (int id = D.level_start[D.pw_lo - 2]; id < D.level_start[D.pw_hi - 1]; ++id) {
-      if (c0[id] < 0) continue;
-      bool any = false;
-      for (int a = 0; a < 8 && !any; ++a) {
-        const int ch = c0[id] + a;
-        if (c0[ch] < 0) continue;
-        for (int b = 0; b < 8; ++b) any = any || c0[c0[ch] + b] >= 0;
-      }
-      if (any) cubes.push_back(id);
-    }
-  n_cubes_ = int(cubes.size());
-  d_cubes_ = static_cast<int*>(alloc(sizeof(int) * (n_cubes_ + 1)));
-  PDMK_CUDA(cudaMemcpyAsync(d_cubes_, cubes.data(), sizeof(int) * n_cubes_, cudaMemcpyHostToDevice, st_));
-  n_nonleaf_ = int(nonleaf.size());
-  n_leaves_ = int(leaves.size());
-  d_nonleaf_ = static_cast<int*>(alloc(sizeof(int) * (n_nonleaf_ + 1)));
-  d_leaves_ = static_cast<int*>(alloc(sizeof(int) * (n_leaves_ + 1)));
-  PDMK_CUDA(cudaMemcpyAsync(d_nonleaf_, nonleaf.data(), sizeof(int) * n_nonleaf_, cudaMemcpyHostToDevice, st_));
-  PDMK_CUDA(cudaMemcpyAsync(d_leaves_, leaves.data(), sizeof(int) * n_leaves_, cudaMemcpyHostToDevice, st_));
-  // per-level constants of eval_energy_diff (src/energy.cpp:50-57)
-  const double pi = 3.14159265358979323846;
-  std::vector<double> Cl(MAX_LEVELS + 2, 0.0), Sl(MAX_LEVELS + 2, 0.0);
-  for (int l = 2; l < MAX_LEVELS + 1; ++l) {
-    Cl[l] = 1 / (2 * std::pow(2 * pi, 3)) * std::pow(D.delta_k[l], 3);
-    Sl[l] = ps_.psi0_0 * (1 / (2 * D.boxsize[l + 1] * ps_.C0) - 1 / (2 * D.boxsize[l] * ps_.C0));
-  }
-  d_Cl_ = static_cast<double*>(alloc(sizeof(double) * 2 * (MAX_LEVELS + 2)));
-  d_Sl_ = d_Cl_ + (MAX_LEVELS + 2);
-  PDMK_CUDA(cudaMemcpyAsync(d_Cl_, Cl.data(), sizeof(double) * (MAX_LEVELS + 2), cudaMemcpyHostToDevice, st_));
-  PDMK_CUDA(cudaMemcpyAsync(d_Sl_, Sl.data(), sizeof(double) * (MAX_LEVELS + 2), cudaMemcpyHostToDevice, st_));
-  d_scalars_ = static_cast<double*>(alloc(sizeof(double) * 8));
+  n_nonleaf_ = t.n_nonleaf;
+  n_leaves_ = t.n_leaves;
+  n_cubes_ = t.n_cubes;
+  d_nonleaf_ = static_cast<int*>(alloc(sizeof(int) * size_t(n_nonleaf_ + n_leaves_ + n_cubes_ + 1)));
+  d_leaves_ = d_nonleaf_ + n_nonleaf_;
+  d_cubes_ = d_leaves_ + n_leaves_;
+  launch_plan_lists(D, blk, d_nonleaf_, d_leaves_, d_cubes_, st_);
   // sum(q^2) for the window self term: 64 block partials, then a fixed-order sum
   k_sum_q2<<<64, 256, 0, st_>>>(D.sq, D.n_slots, D.partials);
   PDMK_LAUNCH_CHECK();
@@ -1511,9 +1330,9 @@ double DmkTree::ewald_energy(double* parts) {
   const int n_all = int(N_);
   const int kspl = std::max(4096, (n_all + 295) / 296);
   const int nch = std::max(1, (n_all + kspl - 1) / kspl);
-  std::vector<NudftWork> wl;
+  std::vector<PwItem> wl;
   for (int c = 0; c < nch; ++c) {
-    NudftWork w{};
+    PwItem w{};
     w.cx = w.cy = w.cz = 0.5 * L_;
     w.dk = dk;
     w.M = 3;  // exp(-i k L/2) = (-1)^m: the root's decentring
@@ -1523,28 +1342,24 @@ double DmkTree::ewald_energy(double* parts) {
   }
   double2* part = nullptr;
   double2* S = nullptr;
-  NudftWork* d_work = nullptr;
+  PwItem* d_work = nullptr;
   const int nblk_real = nbox * ny, nblk_rec = 1024;
   double* sums = nullptr;
   PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&part), sizeof(double2) * size_t(Hs) * nch, st_));
   PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&S), sizeof(double2) * size_t(Hs), st_));
   PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&sums), sizeof(double) * (nblk_real + nblk_rec + 8), st_));
   for (size_t i = 0; i < wl.size(); ++i) wl[i].out = part + i * size_t(Hs);
-  PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d_work), sizeof(NudftWork) * wl.size(), st_));
-  PDMK_CUDA(cudaMemcpyAsync(d_work, wl.data(), sizeof(NudftWork) * wl.size(), cudaMemcpyHostToDevice, st_));
+  PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d_work), sizeof(PwItem) * wl.size(), st_));
+  PDMK_CUDA(cudaMemcpyAsync(d_work, wl.data(), sizeof(PwItem) * wl.size(), cudaMemcpyHostToDevice, st_));
   dispatch_nudft(nk, d_work, int(wl.size()), dense_, dense_stride_, st_);
   {
-    int* d_meta;
-    double2** d_outs;
-    const int meta[2] = {0, nch};
-    PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d_meta), sizeof(int) * 2, st_));
-    PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d_outs), sizeof(double2*), st_));
-    PDMK_CUDA(cudaMemcpyAsync(d_meta, meta, sizeof(meta), cudaMemcpyHostToDevice, st_));
-    PDMK_CUDA(cudaMemcpyAsync(d_outs, &S, sizeof(double2*), cudaMemcpyHostToDevice, st_));
-    k_reduce_chunks<<<dim3(grid_for(Hs), 1u), TPB, 0, st_>>>(part, d_meta, d_meta + 1, d_outs, Hs);
+    PwSplit* d_split;
+    const PwSplit all{0, nch, S};
+    PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d_split), sizeof(PwSplit), st_));
+    PDMK_CUDA(cudaMemcpyAsync(d_split, &all, sizeof(PwSplit), cudaMemcpyHostToDevice, st_));
+    k_reduce_chunks<<<dim3(grid_for(Hs), 1u), TPB, 0, st_>>>(part, d_split, Hs);
     PDMK_LAUNCH_CHECK();
-    PDMK_CUDA(cudaFreeAsync(d_meta, st_));
-    PDMK_CUDA(cudaFreeAsync(d_outs, st_));
+    PDMK_CUDA(cudaFreeAsync(d_split, st_));
   }
   k_ewald_recip<<<unsigned(nblk_rec), TPB, 0, st_>>>(S, nk, dk, alpha, sums + nblk_real);
   PDMK_LAUNCH_CHECK();

@@ -301,7 +301,7 @@ __device__ void axis_factors_d(double xr, double dk, int M, int X, int m0, int c
 // consecutive lanes on consecutive particles.
 template <int NK>
 __global__ void __launch_bounds__(MixShape<NK>::TTHREADS)
-    k_pw_tables(const __grid_constant__ CUtensorMap coords, const MixItem* __restrict__ items,
+    k_pw_tables(const __grid_constant__ CUtensorMap coords, const PwItem* __restrict__ items,
                 const int2* __restrict__ chunks, int nchunks, const double* __restrict__ qmax_p,
                 int* __restrict__ err) {
   using S = MixShape<NK>;
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(MixShape<NK>::TTHREADS)
   for (int q = blockIdx.x; q < nchunks; q += gridDim.x, ++i) {
     const int b = i & 1;
     const int2 ch = chunks[q];
-    const MixItem it = items[ch.x];
+    const PwItem it = items[ch.x];
     const int sb = it.s_begin + ch.y * KCP;
     const int nk = min(KCP, it.s_end - sb);
     const int off = sb - (sb & ~1);
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(MixShape<NK>::TTHREADS)
     tc::fence_async_smem();
     __syncthreads();
     if (tid == 0) {
-      tc::bulk_store(const_cast<unsigned char*>(it.tab) + size_t(ch.y) * S::T_BYTES, blk, S::T_BYTES);
+      tc::bulk_store(it.tab + size_t(ch.y) * S::T_BYTES, blk, S::T_BYTES);
       tc::bulk_commit();
     }
   }
@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(MixShape<NK>::TTHREADS)
 // chunks' table blocks.
 template <int NK>
 __global__ void __launch_bounds__(MixShape<NK>::THREADS, 1)
-    k_pw_mixed(const MixItem* __restrict__ items, const double* __restrict__ qmax_p, int* __restrict__ err) {
+    k_pw_mixed(const PwItem* __restrict__ items, const double* __restrict__ qmax_p, int* __restrict__ err) {
   using S = MixShape<NK>;
   constexpr int D = S::D, NPAD = S::NPAD, HALF = S::HALF, KCP = S::KCP, KB = S::KB;
   extern __shared__ unsigned char smem_raw[];
@@ -429,8 +429,8 @@ __global__ void __launch_bounds__(MixShape<NK>::THREADS, 1)
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const bool control = tid >= S::CTHREADS;
-  const MixItem it = items[blockIdx.x];
-  const int row0 = it.pair * RPC;                 // first computed row of this CTA
+  const PwItem it = items[blockIdx.x / S::TILES];
+  const int row0 = int(blockIdx.x % S::TILES) * RPC;                 // first computed row of this CTA
   const int nrows = min(RPC, S::ROWS_C - row0);  // valid rows of this CTA
   const int nch = (it.s_end - it.s_begin + KCP - 1) / KCP;
   const double qmax = *qmax_p;
@@ -643,7 +643,7 @@ __global__ void k_absmax(const double* __restrict__ q, int n, double* out) {
 }
 
 template <int NK>
-void launch_mixed(const CUtensorMap& tmap, const MixItem* d_items, int nitems, const int2* d_chunks, int nchunks,
+void launch_mixed(const CUtensorMap& tmap, const PwItem* d_items, int nitems, const int2* d_chunks, int nchunks,
                   const double* d_qmax, int* d_err, cudaStream_t st) {
   using S = MixShape<NK>;
   if (nitems == 0) return;
@@ -661,7 +661,7 @@ void launch_mixed(const CUtensorMap& tmap, const MixItem* d_items, int nitems, c
     PDMK_LAUNCH_CHECK();
   }
   raise_smem_limit(reinterpret_cast<const void*>(k_pw_mixed<NK>), S::SMEM);
-  k_pw_mixed<NK><<<unsigned(nitems), S::THREADS, S::SMEM, st>>>(d_items, d_qmax, d_err);
+  k_pw_mixed<NK><<<unsigned(nitems) * S::TILES, S::THREADS, S::SMEM, st>>>(d_items, d_qmax, d_err);
   PDMK_LAUNCH_CHECK();
 }
 
@@ -740,7 +740,7 @@ void launch_absmax(const double* sq, int n, double* out, cudaStream_t st) {
   PDMK_LAUNCH_CHECK();
 }
 
-void dispatch_mixed(int nk, const CUtensorMap& tmap, const MixItem* d_items, int nitems, const int2* d_chunks,
+void dispatch_mixed(int nk, const CUtensorMap& tmap, const PwItem* d_items, int nitems, const int2* d_chunks,
                     int nchunks, const double* d_qmax, int* d_err, cudaStream_t st) {
 #define PDMK_MIX_CASE(n) \
   case n: launch_mixed<n>(tmap, d_items, nitems, d_chunks, nchunks, d_qmax, d_err, st); break;

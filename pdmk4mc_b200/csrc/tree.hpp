@@ -20,6 +20,8 @@ namespace pdmk {
 constexpr int MAX_POLY = 25;
 constexpr int PATH_LEN_MAX = MAX_LEVELS;
 
+struct PlanTotals;  // totals of the work and box lists (plan.hpp)
+
 // One proposed single-particle move and what the shift kernel found for it.
 struct Proposal {
   int i_orig;
@@ -276,7 +278,7 @@ class DmkTree {
   void launch_update();  // accept-and-update and membership commit, one launch
   void ensure_packed();
   void prepare_box_lists();
-  void build_box_lists(const std::vector<int>& child0);  // from a host copy of node_child0
+  void fill_box_lists(const PlanTotals& t, const int* blk);
   void launch_window_energy();  // enqueue the window energy into d_scalars_[0]
   void launch_res_energy();     // enqueue the near-field energy into d_scalars_[2]
   void run_incoming(bool write_inc);
