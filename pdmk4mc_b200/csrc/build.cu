@@ -526,6 +526,46 @@ __global__ void k_validate(const double* r, const double* q, long n, double L, i
 
 
 // ---------------------------------------------------------------------------
+namespace {
+constexpr int kIdleStreams = 16;  // per device
+struct IdleStreams {
+  std::mutex mu;
+  int n = 0;
+  cudaStream_t s[kIdleStreams];
+};
+IdleStreams g_idle_streams[64];
+}  // namespace
+
+cudaStream_t take_stream(int* device) {
+  int dev = 0;
+  PDMK_CUDA(cudaGetDevice(&dev));
+  if (device) *device = dev;
+  if (dev >= 0 && dev < 64) {
+    IdleStreams& I = g_idle_streams[dev];
+    std::lock_guard<std::mutex> g(I.mu);
+    if (I.n > 0) return I.s[--I.n];
+  }
+  cudaStream_t s = nullptr;
+  PDMK_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  return s;
+}
+
+void return_stream(int device, cudaStream_t s) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  const bool idle = cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone &&
+                    cudaStreamSynchronize(s) == cudaSuccess;
+  if (idle && device >= 0 && device < 64) {
+    IdleStreams& I = g_idle_streams[device];
+    std::lock_guard<std::mutex> g(I.mu);
+    if (I.n < kIdleStreams) {
+      I.s[I.n++] = s;
+      return;
+    }
+  }
+  cudaStreamDestroy(s);
+}
+
+// ---------------------------------------------------------------------------
 // Tree-lifetime allocations come from the device's stream-ordered pool, kept
 // cached across trees (the release threshold is raised once per device), so
 // building a fresh tree per full-energy evaluation costs no driver
@@ -541,11 +581,23 @@ void* DmkTree::alloc(size_t bytes) {
     PDMK_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr));
     pool_ready[dev] = true;
   }
-  void* p = nullptr;
   if (bytes == 0) bytes = 16;
-  cudaError_t e = cudaMallocAsync(&p, bytes, st_);
-  if (e != cudaSuccess) throw CudaError(std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
-  allocs_.push_back(p);
+  auto get = [&](size_t n) {
+    void* p = nullptr;
+    cudaError_t e = cudaMallocAsync(&p, n, st_);
+    if (e != cudaSuccess) throw CudaError(std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
+    allocs_.push_back(p);
+    return p;
+  };
+  if (bytes > kArenaSmall) return get(bytes);
+  bytes = (bytes + 255) & ~size_t(255);
+  if (bytes > arena_left_) {
+    arena_ = static_cast<unsigned char*>(get(kArenaBlock));
+    arena_left_ = kArenaBlock;
+  }
+  void* p = arena_;
+  arena_ += bytes;
+  arena_left_ -= bytes;
   return p;
 }
 
@@ -570,7 +622,7 @@ DmkTree::~DmkTree() {
   cudaStreamSynchronize(st_);
   if (aux_) {
     cudaStreamSynchronize(aux_);
-    cudaStreamDestroy(aux_);
+    return_stream(aux_device_, aux_);
     cudaEventDestroy(ev_fork_);
     cudaEventDestroy(ev_join_);
   }
@@ -1143,8 +1195,6 @@ void DmkTree::build_setup() {
   if (D.pw_hi >= D.pw_lo) n_pw = long(D.level_start[D.pw_hi + 1]) - D.level_start[D.pw_lo];
   D.out = static_cast<double2*>(alloc(sizeof(double2) * size_t(std::max<long>(n_pw, 1)) * D.H));
   D.inc = static_cast<double2*>(alloc(sizeof(double2) * size_t(std::max<long>(n_pw, 1)) * D.H));
-  PDMK_CUDA(cudaMemsetAsync(D.out, 0, sizeof(double2) * size_t(std::max<long>(n_pw, 1)) * D.H, st_));
-  PDMK_CUDA(cudaMemsetAsync(D.inc, 0, sizeof(double2) * size_t(std::max<long>(n_pw, 1)) * D.H, st_));
   // scratch for partial sums and the proposal record
   partials_cap_ = partials_needed();
   D.partials = static_cast<double*>(alloc(sizeof(double) * partials_cap_));
@@ -1312,7 +1362,7 @@ void DmkTree::export_positions(double* r) const {
   }
 }
 
-void DmkTree::export_pw(long node, int which, double* out) const {
+void DmkTree::export_pw(long node, int which, double* out) {
   if (node == 0) {
     if (which != 0) throw std::invalid_argument("the root has no incoming expansion");
     PDMK_CUDA(cudaMemcpyAsync(out, dev_.out_root, sizeof(double2) * dev_.Hw, cudaMemcpyDeviceToHost, st_));
@@ -1320,6 +1370,16 @@ void DmkTree::export_pw(long node, int which, double* out) const {
     long lo = dev_.level_start[dev_.pw_lo];
     long hi = dev_.pw_hi >= dev_.pw_lo ? dev_.level_start[dev_.pw_hi + 1] : lo;
     if (node < lo || node >= hi) throw std::invalid_argument("node carries no expansion");
+    ensure_rows(which == 0, which != 0);
+    if (which != 0) {
+      int child = -1;
+      PDMK_CUDA(cudaMemcpyAsync(&child, dev_.node_child0 + node, sizeof(int), cudaMemcpyDeviceToHost, st_));
+      PDMK_CUDA(cudaStreamSynchronize(st_));
+      if (child < 0) {  // leaves receive nothing: their rows are never written
+        std::fill(out, out + 2 * size_t(dev_.H), 0.0);
+        return;
+      }
+    }
     const double2* src = (which == 0 ? dev_.out : dev_.inc) + size_t(node - lo) * dev_.H;
     PDMK_CUDA(cudaMemcpyAsync(out, src, sizeof(double2) * dev_.H, cudaMemcpyDeviceToHost, st_));
   }

@@ -518,7 +518,10 @@ __global__ void k_diff_finish_cube(DevTree T, const int* __restrict__ cubes, int
   }
   for (int b = threadIdx.x; b < nboxes; b += blockDim.x) e -= q2[b] * Sl[T.node_level[boxes[b]]];
   double s = block_sum(e, sm);
-  if (threadIdx.x == 0) *out = s;
+  if (threadIdx.x == 0) {
+    *out = s;
+    T.counter[15] = 1;  // the incoming rows are written
+  }
 }
 
 // Re sum out_B inc_B D_2 per (box, k tile) on the stored incoming expansions
@@ -925,6 +928,17 @@ __global__ void k_ewald_recip(const double2* __restrict__ S, int nk, double dk, 
   if (threadIdx.x == 0) part[blockIdx.x] = sum;
 }
 
+// rows 0 .. n unless a pass or an earlier call defined them
+__global__ void k_zero_undefined(double2* rows, size_t n, const unsigned int* defined) {
+  if (*defined) return;
+  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
+    rows[i] = make_double2(0.0, 0.0);
+}
+__global__ void k_set_defined(unsigned int* counter, bool out, bool inc) {
+  if (out) counter[14] = 1;
+  if (inc) counter[15] = 1;
+}
+
 __global__ void k_sum(const double* part, int n, double* out) {
   __shared__ double sm[32];
   double e = 0;
@@ -1023,6 +1037,29 @@ void DmkTree::ensure_packed() {
   moved_ = false;
 }
 
+// A tree's rows are zero until a pass forms them. Clearing them in the build
+// wrote every row twice (4.5 GB, 0.7 ms at N = 1e6 and 9 digits), so it waits
+// for a call that reads a row no pass has formed. The device's own flags
+// decide, so that a captured call does not clear formed rows when it is
+// replayed.
+void DmkTree::ensure_rows(bool out, bool inc) {
+  out = out && !out_defined_;
+  inc = inc && !inc_defined_;
+  if (!out && !inc) return;
+  const DevTree& D = dev_;
+  const long n_pw = D.pw_hi >= D.pw_lo ? long(D.level_start[D.pw_hi + 1]) - D.level_start[D.pw_lo] : 0;
+  const size_t n = size_t(std::max<long>(n_pw, 1)) * D.H;
+  if (out) k_zero_undefined<<<1184, 256, 0, st_>>>(D.out, n, D.counter + 14);
+  if (inc) k_zero_undefined<<<1184, 256, 0, st_>>>(D.inc, n, D.counter + 15);
+  k_set_defined<<<1, 1, 0, st_>>>(D.counter, out, inc);
+  PDMK_LAUNCH_CHECK();
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  PDMK_CUDA(cudaStreamIsCapturing(st_, &cs));
+  if (cs != cudaStreamCaptureStatusNone) return;  // nothing ran yet
+  out_defined_ |= out;
+  inc_defined_ |= inc;
+}
+
 void DmkTree::form_outgoing_pw() {
   ensure_packed();
   ensure_dense();
@@ -1073,7 +1110,7 @@ void DmkTree::form_outgoing_pw() {
     PDMK_LAUNCH_CHECK();
   };
   if (!aux_) {
-    PDMK_CUDA(cudaStreamCreateWithFlags(&aux_, cudaStreamNonBlocking));
+    aux_ = take_stream(&aux_device_);
     PDMK_CUDA(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
     PDMK_CUDA(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
   }
@@ -1131,6 +1168,7 @@ void DmkTree::form_outgoing_pw() {
   contract(D.n_diff, tmap_box, box, t.n_items, t.n_chunks, st_);
   time_end(3);
   reduce(box, t.n_split, part_b, D.H, st_);
+  out_defined_ = true;
   if (lists) fill_box_lists(t, d_blk);
   // the root pass's buffers are released after it joins the tree's stream
   PDMK_CUDA(cudaStreamWaitEvent(st_, ev_join_, 0));
@@ -1179,6 +1217,7 @@ void DmkTree::run_incoming(bool write_inc) {
   ensure_packed();
   prepare_box_lists();
   DevTree& D = dev_;
+  ensure_rows(true, !write_inc);
   if (n_nonleaf_ == 0) {
     PDMK_CUDA(cudaMemsetAsync(d_scalars_ + 1, 0, sizeof(double), st_));
     return;
@@ -1193,6 +1232,7 @@ void DmkTree::run_incoming(bool write_inc) {
     // about inc_waves resident waves of blocks (two per SM), each walking a
     // strided set of tiles
     const int slots = inc_slots();
+    inc_defined_ = true;  // the non-leaf boxes' rows; a leaf's row is read by nothing
     if (n_cubes_ > 0) launch_incoming(D, d_cubes_, n_cubes_, slots, part, nullptr, st_);
     k_diff_finish_cube<<<1, 1024, 0, st_>>>(D, d_cubes_, n_cubes_, slots, part, d_nonleaf_, n_nonleaf_, q2, d_Cl_,
                                             d_Sl_, d_scalars_ + 1);

@@ -92,7 +92,10 @@ __global__ void k_plan_root(DevTree T, PlanShape s, int n, int n_items, int n_ch
     items[i] = w;
   }
   if (i < n_chunks) chunks[i] = make_int2(i / full, i % full);
-  if (i == 0) *split = PwSplit{0, n_items, T.out_root};
+  if (i == 0) {
+    *split = PwSplit{0, n_items, T.out_root};
+    T.counter[14] = 1;  // every outgoing row is about to be written
+  }
 }
 
 __global__ void k_plan_count(DevTree T, PlanShape s, bool lists, PlanState* state, int* blk) {

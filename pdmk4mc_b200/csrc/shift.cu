@@ -3275,6 +3275,7 @@ void DmkTree::ensure_move_resources() {
     d_cursor_ = static_cast<MoveCursor*>(alloc(sizeof(MoveCursor)));
   }
   ensure_shift_config();
+  ensure_rows(true, true);
 }
 
 // Grid size and dynamic shared memory limit of the shift kernel (no allocation).
@@ -3645,6 +3646,7 @@ int* DmkTree::batch_order(int m) {
 
 void DmkTree::launch_shift_batch(int m, const int* d_idx, const double* d_disp, int* order, double* d_dE) {
   DevTree& D = dev_;
+  ensure_rows(true, true);
   const int grp = batch_groups(m, d_idx, order);
   const size_t smem = batch_smem(D.n_poly, D.max_depth, 2 * grp);
   const ShiftBatchKernel kern = shift_batch_kernel(D.n_poly, grp);
@@ -3745,6 +3747,7 @@ void DmkTree::replicas_mc_run(const std::vector<DmkTree*>& ts, int m, const int*
   for (DmkTree* t : ts) {
     if (t->dev_.n_poly != np) throw std::invalid_argument("replicas must share the digits setting");
     t->ensure_packed();
+    t->ensure_rows(true, true);
     smem = std::max(smem, tables_smem(t->dev_, t->dev_.max_depth, 2));
   }
   cudaStream_t st = ts[0]->st_;
@@ -3819,7 +3822,7 @@ void DmkTree::potential_batch(int m, const int* d_idx, double* d_phi, double* d_
   DevTree& D = dev_;
   if (m <= 0) return;
   ensure_packed();  // the near-field source lists read the slots only
-  prepare_box_lists();  // the per-level self terms S_l
+  ensure_rows(true, true);
   int* order = batch_order(m);
   const int grp = batch_groups(m, d_idx, order);
   const size_t smem = batch_smem(D.n_poly, D.max_depth, grp);

@@ -20,6 +20,14 @@ namespace pdmk {
 constexpr int MAX_POLY = 25;
 constexpr int PATH_LEN_MAX = MAX_LEVELS;
 
+// A stream of the current device for a tree's work, and its return. Creating
+// a stream takes 51-60 us and destroying it 65-79 us, two of each per tree,
+// which was a third of the energy of a new small system; up to 16 idle streams
+// of a device wait for the next tree instead (any thread's). A stream is kept
+// once its work is done; one that is capturing or has failed is destroyed.
+cudaStream_t take_stream(int* device = nullptr);  // device: the current one
+void return_stream(int device, cudaStream_t s);
+
 struct PlanTotals;  // totals of the work and box lists (plan.hpp)
 
 // One proposed single-particle move and what the shift kernel found for it.
@@ -119,7 +127,7 @@ struct DevTree {
   double* D2;  // [H], the level-2 difference kernel
   // scratch
   double* partials;
-  unsigned int* counter;
+  unsigned int* counter;  // [0] blocks done; [14], [15]: the outgoing, incoming rows are defined
   Proposal* prop;
   Receiver* recv;  // [MAX_RECV]
   int* err;  // device error word (nonzero: pool overflow etc.)
@@ -258,7 +266,7 @@ class DmkTree {
   int digits() const { return digits_; }
   const TreeOptions& options() const { return opt_; }
   double box() const { return L_; }
-  void export_pw(long node, int which, double* out) const;
+  void export_pw(long node, int which, double* out);
   void export_W(double* out) const;
   void export_D(int level, double* out) const;
   void synchronize() const;
@@ -277,6 +285,8 @@ class DmkTree {
                     double* d_dE, int* d_acc);
   void launch_update();  // accept-and-update and membership commit, one launch
   void ensure_packed();
+  bool out_defined_ = false, inc_defined_ = false;
+  void ensure_rows(bool out, bool inc);  // rows read before a pass formed them are zero
   void prepare_box_lists();
   void fill_box_lists(const PlanTotals& t, const int* blk);
   void launch_window_energy();  // enqueue the window energy into d_scalars_[0]
@@ -296,6 +306,10 @@ class DmkTree {
   std::vector<int> h_level_start_;
   std::vector<void*> allocs_;
   void* alloc(size_t bytes);
+  // small buffers come from blocks of the pool's memory
+  static constexpr size_t kArenaBlock = size_t(256) << 10, kArenaSmall = size_t(32) << 10;
+  unsigned char* arena_ = nullptr;
+  size_t arena_left_ = 0;
   // leaves in depth-first order and their slot bookkeeping (device)
   struct LeafArrays {
     int n = 0;
@@ -391,6 +405,7 @@ class DmkTree {
   void ensure_shift_config();
   void build_mc_graph(int timed);
   void launch_shift_cursor(int move);
+  int aux_device_ = -1;
   cudaStream_t aux_ = nullptr;  // second stream for the root plane-wave pass
   // mixed precision: [0] max |q| (fixed-point scale), [1] error word (as int) of the tensor-core pass
   double* d_mix_ = nullptr;
