@@ -526,6 +526,46 @@ __global__ void k_validate(const double* r, const double* q, long n, double L, i
 
 
 // ---------------------------------------------------------------------------
+namespace {
+constexpr int kIdleStreams = 16;  // per device
+struct IdleStreams {
+  std::mutex mu;
+  int n = 0;
+  cudaStream_t s[kIdleStreams];
+};
+IdleStreams g_idle_streams[64];
+}  // namespace
+
+cudaStream_t take_stream(int* device) {
+  int dev = 0;
+  PDMK_CUDA(cudaGetDevice(&dev));
+  if (device) *device = dev;
+  if (dev >= 0 && dev < 64) {
+    IdleStreams& I = g_idle_streams[dev];
+    std::lock_guard<std::mutex> g(I.mu);
+    if (I.n > 0) return I.s[--I.n];
+  }
+  cudaStream_t s = nullptr;
+  PDMK_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  return s;
+}
+
+void return_stream(int device, cudaStream_t s) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  const bool idle = cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone &&
+                    cudaStreamSynchronize(s) == cudaSuccess;
+  if (idle && device >= 0 && device < 64) {
+    IdleStreams& I = g_idle_streams[device];
+    std::lock_guard<std::mutex> g(I.mu);
+    if (I.n < kIdleStreams) {
+      I.s[I.n++] = s;
+      return;
+    }
+  }
+  cudaStreamDestroy(s);
+}
+
+// ---------------------------------------------------------------------------
 // Tree-lifetime allocations come from the device's stream-ordered pool, kept
 // cached across trees (the release threshold is raised once per device), so
 // building a fresh tree per full-energy evaluation costs no driver
@@ -541,11 +581,23 @@ void* DmkTree::alloc(size_t bytes) {
     PDMK_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr));
     pool_ready[dev] = true;
   }
-  void* p = nullptr;
   if (bytes == 0) bytes = 16;
-  cudaError_t e = cudaMallocAsync(&p, bytes, st_);
-  if (e != cudaSuccess) throw CudaError(std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
-  allocs_.push_back(p);
+  auto get = [&](size_t n) {
+    void* p = nullptr;
+    cudaError_t e = cudaMallocAsync(&p, n, st_);
+    if (e != cudaSuccess) throw CudaError(std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
+    allocs_.push_back(p);
+    return p;
+  };
+  if (bytes > kArenaSmall) return get(bytes);
+  bytes = (bytes + 255) & ~size_t(255);
+  if (bytes > arena_left_) {
+    arena_ = static_cast<unsigned char*>(get(kArenaBlock));
+    arena_left_ = kArenaBlock;
+  }
+  void* p = arena_;
+  arena_ += bytes;
+  arena_left_ -= bytes;
   return p;
 }
 
@@ -570,7 +622,7 @@ DmkTree::~DmkTree() {
   cudaStreamSynchronize(st_);
   if (aux_) {
     cudaStreamSynchronize(aux_);
-    cudaStreamDestroy(aux_);
+    return_stream(aux_device_, aux_);
     cudaEventDestroy(ev_fork_);
     cudaEventDestroy(ev_join_);
   }

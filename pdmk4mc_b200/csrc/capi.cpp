@@ -55,7 +55,7 @@ struct Handle {
     if (d_u) cudaFree(d_u);
     if (d_dE) cudaFree(d_dE);
     if (d_acc) cudaFree(d_acc);
-    if (stream && own_stream) cudaStreamDestroy(stream);
+    if (stream && own_stream) pdmk::return_stream(device, stream);
   }
   void ensure(int m) {
     if (m <= cap) return;
@@ -229,7 +229,7 @@ hpdmk_tree init_impl(HPDMKParams params, const HPDMKExtParams* ext, int n, const
       hh->stream = static_cast<cudaStream_t>(ext->stream);
       hh->own_stream = false;
     } else {
-      PDMK_CUDA(cudaStreamCreateWithFlags(&hh->stream, cudaStreamNonBlocking));
+      hh->stream = pdmk::take_stream();
     }
     hh->n = n;
     hh->L = params.L;

@@ -1110,7 +1110,7 @@ void DmkTree::form_outgoing_pw() {
     PDMK_LAUNCH_CHECK();
   };
   if (!aux_) {
-    PDMK_CUDA(cudaStreamCreateWithFlags(&aux_, cudaStreamNonBlocking));
+    aux_ = take_stream(&aux_device_);
     PDMK_CUDA(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
     PDMK_CUDA(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
   }

@@ -20,6 +20,14 @@ namespace pdmk {
 constexpr int MAX_POLY = 25;
 constexpr int PATH_LEN_MAX = MAX_LEVELS;
 
+// A stream of the current device for a tree's work, and its return. Creating
+// a stream takes 51-60 us and destroying it 65-79 us, two of each per tree,
+// which was a third of the energy of a new small system; up to 16 idle streams
+// of a device wait for the next tree instead (any thread's). A stream is kept
+// once its work is done; one that is capturing or has failed is destroyed.
+cudaStream_t take_stream(int* device = nullptr);  // device: the current one
+void return_stream(int device, cudaStream_t s);
+
 struct PlanTotals;  // totals of the work and box lists (plan.hpp)
 
 // One proposed single-particle move and what the shift kernel found for it.
@@ -298,6 +306,10 @@ class DmkTree {
   std::vector<int> h_level_start_;
   std::vector<void*> allocs_;
   void* alloc(size_t bytes);
+  // small buffers come from blocks of the pool's memory
+  static constexpr size_t kArenaBlock = size_t(256) << 10, kArenaSmall = size_t(32) << 10;
+  unsigned char* arena_ = nullptr;
+  size_t arena_left_ = 0;
   // leaves in depth-first order and their slot bookkeeping (device)
   struct LeafArrays {
     int n = 0;
@@ -393,6 +405,7 @@ class DmkTree {
   void ensure_shift_config();
   void build_mc_graph(int timed);
   void launch_shift_cursor(int move);
+  int aux_device_ = -1;
   cudaStream_t aux_ = nullptr;  // second stream for the root plane-wave pass
   // mixed precision: [0] max |q| (fixed-point scale), [1] error word (as int) of the tensor-core pass
   double* d_mix_ = nullptr;
