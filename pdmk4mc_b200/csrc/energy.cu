@@ -1091,17 +1091,19 @@ void DmkTree::form_outgoing_pw() {
     PwItem* items;
     PwSplit* split;
     int2* chunks;
+    int* next;  // the mixed pass's tile counter
   };
   auto get_lists = [&](int n_items, int n_split, int n_chunks) {
     Lists l;
-    l.block = get(sizeof(PwItem) * size_t(n_items) + sizeof(PwSplit) * size_t(n_split) + sizeof(int2) * size_t(n_chunks));
+    l.block = get(sizeof(PwItem) * size_t(n_items) + sizeof(PwSplit) * size_t(n_split) + sizeof(int2) * size_t(n_chunks + 1));
     l.items = reinterpret_cast<PwItem*>(l.block);
     l.split = reinterpret_cast<PwSplit*>(l.items + n_items);
     l.chunks = reinterpret_cast<int2*>(l.split + n_split);
+    l.next = reinterpret_cast<int*>(l.chunks + n_chunks);
     return l;
   };
   auto contract = [&](int nk, const CUtensorMap& tmap, const Lists& l, int n_items, int n_chunks, cudaStream_t st) {
-    if (mixed) dispatch_mixed(nk, tmap, l.items, n_items, l.chunks, n_chunks, d_mix_, d_mix_err, st);
+    if (mixed) dispatch_mixed(nk, tmap, l.items, n_items, l.chunks, n_chunks, l.next, d_mix_, d_mix_err, st);
     else dispatch_nudft(nk, l.items, n_items, dense_, dense_stride_, st);
   };
   auto reduce = [&](const Lists& l, int n_split, const double2* part, int H, cudaStream_t st) {
@@ -1150,7 +1152,7 @@ void DmkTree::form_outgoing_pw() {
   double2* part_r = reinterpret_cast<double2*>(get(sizeof(double2) * size_t(n_root) * D.Hw));
   unsigned char* tab_r = mixed ? get(size_t(n_root_chunks) * root_shape.tab_bytes) : nullptr;
   const Lists root = get_lists(n_root, 1, n_root_chunks);
-  launch_plan_root(D, root_shape, n_all, n_root, n_root_chunks, part_r, tab_r, root.items, root.chunks, root.split, st_);
+  launch_plan_root(D, root_shape, n_all, n_root, n_root_chunks, part_r, tab_r, root.items, root.chunks, root.split, root.next, st_);
   PDMK_CUDA(cudaEventRecord(ev_fork_, st_));
   PDMK_CUDA(cudaStreamWaitEvent(aux_, ev_fork_, 0));
   contract(D.n_window, tmap_root, root, n_root, n_root_chunks, aux_);
@@ -1163,7 +1165,7 @@ void DmkTree::form_outgoing_pw() {
   double2* part_b = reinterpret_cast<double2*>(get(sizeof(double2) * size_t(t.n_split_items) * D.H));
   unsigned char* tab_b = mixed ? get(size_t(t.n_chunks) * box_shape.tab_bytes) : nullptr;
   const Lists box = get_lists(t.n_items, t.n_split, t.n_chunks);
-  launch_plan_items(D, box_shape, node_dense_, d_state, part_b, tab_b, box.items, box.chunks, box.split, st_);
+  launch_plan_items(D, box_shape, node_dense_, d_state, part_b, tab_b, box.items, box.chunks, box.split, box.next, st_);
   time_begin(3);
   contract(D.n_diff, tmap_box, box, t.n_items, t.n_chunks, st_);
   time_end(3);

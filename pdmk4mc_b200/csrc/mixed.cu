@@ -79,18 +79,37 @@ constexpr int NACC = 4;            // accumulators: slice-product orders s + t =
 constexpr int SMEM_MAX = 227 * 1024;
 
 __host__ __device__ constexpr int npad_of(int nk) { return (2 * (2 * nk + 1) + 15) / 16 * 16; }
-__host__ __device__ constexpr int ezs_of(int nk) { return (nk + 1) | 1; }
-// bytes of one chunk's table block: B slices, then the ey and ez factors
-__host__ __device__ constexpr int table_bytes(int nk, int kcp) {
-  return 4 * npad_of(nk) * 2 * kcp + kcp * ((2 * nk + 1) + ezs_of(nk)) * 16;
+// computed rows (below), and the planes kz a tile of them reads: first, last
+__host__ __device__ constexpr int rows_of(int nk) { return nk * (2 * nk + 1) + nk + 1; }
+__host__ __device__ constexpr int plane_of(int nk, int rho) {
+  return (rho < nk * (2 * nk + 1) ? rho : rho + nk) / (2 * nk + 1);
 }
-__host__ __device__ constexpr int table_stride(int nk, int kcp) { return (table_bytes(nk, kcp) + 127) / 128 * 128; }
+__host__ __device__ constexpr int plane_lo(int nk, int tile) { return plane_of(nk, tile * RPC); }
+__host__ __device__ constexpr int plane_hi(int nk, int tile) {
+  return plane_of(nk, tile * RPC + RPC < rows_of(nk) ? tile * RPC + RPC - 1 : rows_of(nk) - 1);
+}
+__host__ __device__ constexpr int max_planes(int nk) {
+  int m = 0;
+  for (int t = 0; t * RPC < rows_of(nk); ++t) {
+    const int n = plane_hi(nk, t) - plane_lo(nk, t) + 1;
+    m = n > m ? n : m;
+  }
+  return m;
+}
+// bytes of a chunk's B slices and ey factors, and of its stage in the
+// contraction: these and the ez planes of one tile
+__host__ __device__ constexpr int front_bytes(int nk, int kcp) {
+  return 4 * npad_of(nk) * 2 * kcp + kcp * (2 * nk + 1) * 16;
+}
+__host__ __device__ constexpr int stage_stride(int nk, int kcp) {
+  return (front_bytes(nk, kcp) + max_planes(nk) * kcp * 16 + 127) / 128 * 128;
+}
 // TMEM columns: the four accumulators, then two A stages of 2 kcp columns
 // (four slices of 2 kcp bytes per row, four bytes to a column)
 __host__ __device__ constexpr int tmem_cols(int nk, int kcp) { return NACC * npad_of(nk) + 2 * 2 * kcp; }
 // chunks of 32 particles when three table stages and the TMEM columns fit
 __host__ __device__ constexpr bool chunk32_fits(int nk) {
-  return 3 * table_stride(nk, 32) + 1024 <= SMEM_MAX && tmem_cols(nk, 32) <= 512;
+  return 3 * stage_stride(nk, 32) + 1024 <= SMEM_MAX && tmem_cols(nk, 32) <= 512;
 }
 
 template <int NK>
@@ -102,56 +121,63 @@ struct MixShape {
   // out(-k) = conj(out(k))). Computed row rho maps to r = rho below NK D and
   // to r = rho + NK above.
   static constexpr int ROWS_C = NK * D + NK + 1;
-  static_assert(ROWS_C <= ROWS, "computed rows");
+  static_assert(ROWS_C <= ROWS && ROWS_C == rows_of(NK), "computed rows");
   static constexpr int NPAD = npad_of(NK);  // MMA N: Re columns [0, D), Im columns [HALF, HALF + D)
   static constexpr int HALF = NPAD / 2;
-  static constexpr int EZS = ezs_of(NK);    // odd row strides keep 16-byte stores on distinct bank groups
   static constexpr int TILES = (ROWS_C + RPC - 1) / RPC;  // CTAs per box
   static constexpr int KCP = chunk32_fits(NK) ? 32 : 16;  // particles per chunk
   static constexpr int KB = 2 * KCP;        // K bytes per chunk (real and imaginary part per particle)
   static constexpr int KSTEPS = KB / 32;    // MMA K steps (32 bytes each) per chunk
-  static constexpr int CPR = KB / 16;            // consumer threads per row: one per 16-byte K group (8 particles)
-  static constexpr int CTHREADS = RPC * CPR;
-  static constexpr int THREADS = CTHREADS + 32;  // consumers + the control warp
+  // consumers: two groups of eight warps, each forming every other chunk's A;
+  // then the MMA warp and the load warp
+  static constexpr int GWARPS = 8, CTHREADS = 512;
+  static constexpr int KGT = KB / 16 / 2;  // 16-byte K groups (8 particles) of a chunk per consumer thread
+  static constexpr int THREADS = CTHREADS + 64;
   static constexpr int TTHREADS = 6 * KCP;       // table kernel: one thread per (particle, axis, half)
   static constexpr int COORD_BOX = KCP + 2;      // TMA box along the slots: even start, one spare each side
   static constexpr int COORD_BYTES = 4 * COORD_BOX * 8;
   // TMEM: accumulators at columns [0, NACC NPAD), A stage s slice t at
   // columns A_COL0 + s KB + t KB / 4 (lane = row)
   static constexpr int A_COL0 = NACC * NPAD;
-  static constexpr int TCOLS_USED = tmem_cols(NK, KCP);
-  static constexpr int TCOLS = TCOLS_USED <= 32 ? 32 : TCOLS_USED <= 64 ? 64 : TCOLS_USED <= 128 ? 128
-                               : TCOLS_USED <= 256 ? 256 : 512;
+  static constexpr int TCOLS_MIN = tmem_cols(NK, KCP);
+  static constexpr int TCOLS = TCOLS_MIN <= 32 ? 32 : TCOLS_MIN <= 64 ? 64 : TCOLS_MIN <= 128 ? 128
+                               : TCOLS_MIN <= 256 ? 256 : 512;
+  // A stages: two at least, as many as the allocated columns hold
+  static constexpr int ASTAGES = (TCOLS - A_COL0) / KB < 4 ? (TCOLS - A_COL0) / KB : 4;
+  static_assert(ASTAGES >= 2 && A_COL0 + ASTAGES * KB <= 512, "accumulators and A stages exceed TMEM");
   // one chunk's table block
   // B: the four slices side by side along N ([16-byte K group][slice][column]
   // [16 bytes]), so that one MMA can take up to BGROUP consecutive slices
   static constexpr int B_KGROUP = 4 * NPAD * 16;  // bytes per 16-byte K group
   static constexpr int B_BYTES = (KB / 16) * B_KGROUP;
   static constexpr int BGROUP = 3 * NPAD <= 256 ? 3 : 2;  // slices per MMA (N <= 256)
-  // then the FP64 factors (double2): ey [particle][ky], ez [particle][kz]
+  // then the FP64 factors (double2): ey [particle][ky], ez [kz][particle] (a
+  // tile reads a few planes of it)
   static constexpr int EY_OFF = B_BYTES;
   static constexpr int EZ_OFF = EY_OFF + KCP * D * 16;
-  static constexpr int T_BYTES = EZ_OFF + KCP * EZS * 16;
-  static constexpr int T_STRIDE = table_stride(NK, KCP);
-  // contraction kernel shared memory: the table stages (four when they fit)
-  static constexpr int TSTAGES = 4 * T_STRIDE + 1024 <= SMEM_MAX ? 4 : 3;
-  static constexpr int PIPE_BYTES = TSTAGES * T_STRIDE;
-  static constexpr int STAGE_OUT = RPC * D * 16;  // epilogue staging, reuses the table stages
-  static constexpr int SMEM = (PIPE_BYTES > STAGE_OUT ? PIPE_BYTES : STAGE_OUT) + 1024;  // + alignment slack
+  static_assert(EZ_OFF == front_bytes(NK, KCP), "stage layout");
+  static constexpr int T_BYTES = EZ_OFF + KCP * (NK + 1) * 16;
+  static constexpr int T_STRIDE = stage_stride(NK, KCP);
+  // contraction kernel shared memory: the consumer warps' output staging (32
+  // rows x 4 modes, padded), then the table stages: four where the columns
+  // let two CTAs share an SM, as many as fit where they do not
+  static constexpr int OUT_COLS = 4, OUT_STRIDE = OUT_COLS + 1;
+  static constexpr int OUT_WARP = 32 * OUT_STRIDE * 16;
+  static constexpr int OUT_BYTES = (CTHREADS / 32) * OUT_WARP;
+  static constexpr int TS_FIT = (SMEM_MAX - 1024 - 512 - OUT_BYTES) / T_STRIDE;
+  static constexpr int TSTAGES = TCOLS < 512 ? (TS_FIT < 4 ? TS_FIT : 4) : (TS_FIT < 6 ? TS_FIT : 6);
+  static_assert(TSTAGES >= ASTAGES, "table stages");
+  static constexpr int SMEM = TSTAGES * T_STRIDE + OUT_BYTES + 1024;  // + alignment slack
   // table kernel shared memory: coordinates, ex scratch, the block
   static constexpr int TK_COORD_STRIDE = (COORD_BYTES + 127) / 128 * 128;  // two coordinate buffers
   static constexpr int TK_OFF_EX = 2 * TK_COORD_STRIDE;
   static constexpr int TK_OFF_T = (TK_OFF_EX + KCP * D * 16 + 127) / 128 * 128;
-  static constexpr int TK_SMEM = TK_OFF_T + T_STRIDE + 1024;
-  static_assert(TCOLS_USED <= 512, "accumulators and A stages exceed TMEM");
+  static constexpr int TK_SMEM = TK_OFF_T + T_BYTES + 1024;
   static_assert(HALF >= D, "imaginary columns overlap the real ones");
   static_assert(SMEM <= SMEM_MAX && TK_SMEM <= SMEM_MAX, "shared memory");
   static_assert(KB % 32 == 0, "chunks are whole MMA K steps");
   static_assert(T_BYTES % 16 == 0, "bulk copies move multiples of 16 bytes");
 };
-
-// named barrier ids: A stage s ready (consumers -> control), consumers only
-constexpr int BAR_AREADY0 = 1, BAR_CONS = 5;
 
 constexpr double SL_SCALE = 127.0;  // operands are scaled to |t| <= 127
 
@@ -249,11 +275,12 @@ __device__ __forceinline__ void sincos_taylor(double th, double& s, double& c) {
 }
 
 // FP64 phase factors exp(-i m dk (x - c)) w6^{-M (2X+1) m} for m = m0 .. m0 + cnt - 1,
-// times `scale`, into dst[0 .. cnt): the step exp(-i th), the start
+// times `scale`, into dst[0], dst[ds], ...: the step exp(-i th), the start
 // exp(-i m0 th) by binary powering of the step (|m0| <= 26: at most five
 // squarings), then six interleaved recurrence chains, each with its own
 // exact root of unity, as in the FP64 path
-__device__ void axis_factors_d(double xr, double dk, int M, int X, int m0, int cnt, double scale, double2* dst) {
+__device__ void axis_factors_d(double xr, double dk, int M, int X, int m0, int cnt, double scale, double2* dst,
+                               int ds) {
   const double th = dk * xr;
   double s, c;
   sincos_taylor(-th, s, c);
@@ -281,7 +308,7 @@ __device__ void axis_factors_d(double xr, double dk, int M, int X, int m0, int c
 #pragma unroll
     for (int r = 0; r < 6; ++r) {
       if (t + r < cnt) {
-        dst[t + r] = v[r];
+        dst[(t + r) * ds] = v[r];
         v[r] = cmul_d(v[r], st6);
       }
     }
@@ -357,7 +384,9 @@ __global__ void __launch_bounds__(MixShape<NK>::TTHREADS)
       const int len = a == 2 ? NK + 1 : D;
       const int h0 = (len + 1) / 2;
       const int m0 = half ? -NK + h0 : -NK, cnt = half ? len - h0 : h0;
-      double2* dst = (a == 0 ? ex + j * D : (a == 1 ? ey + j * D : ez + j * S::EZS)) + (m0 + NK);
+      // ez by planes: consecutive lanes store consecutive particles
+      double2* dst = a == 2 ? ez + (m0 + NK) * KCP + j : (a == 0 ? ex : ey) + j * D + (m0 + NK);
+      const int ds = a == 2 ? KCP : 1;
       if (j < nk) {
         const double xa = P[a * S::COORD_BOX + off + j];
         const double ca = a == 0 ? it.cx : (a == 1 ? it.cy : it.cz);
@@ -366,9 +395,9 @@ __global__ void __launch_bounds__(MixShape<NK>::TTHREADS)
         // fixed point is formed by fix24_dot without a further scaling
         const double scale =
             a == 0 ? SL_SCALE : (a == 1 ? 1.0 : SL_SCALE * 16777216.0 * P[3 * S::COORD_BOX + off + j] * inv_qmax);
-        axis_factors_d(xa - ca, it.dk, it.M, Xa, m0, cnt, scale, dst);
+        axis_factors_d(xa - ca, it.dk, it.M, Xa, m0, cnt, scale, dst, ds);
       } else {
-        for (int m = 0; m < cnt; ++m) dst[m] = make_double2(0.0, 0.0);
+        for (int m = 0; m < cnt; ++m) dst[m * ds] = make_double2(0.0, 0.0);
       }
     }
     __syncthreads();
@@ -410,35 +439,50 @@ __global__ void __launch_bounds__(MixShape<NK>::TTHREADS)
   if (tid == 0) tc::bulk_wait_all();
 }
 
-// Contraction: one 128-row M tile of one box (or split-K chunk) over its
-// chunks' table blocks.
+// Contraction: 128-row M tiles of boxes (or split-K chunks) over their chunks'
+// table blocks. Persistent: a CTA takes (item, tile) pairs from a counter until
+// none is left. Started per tile instead, a CTA spent 11 us outside its chunks
+// (launch, TMEM allocation, first tables, epilogue, its stores' completion)
+// beside 6 us in the eight chunks of an average deepest box; here the load
+// warp runs ahead over the tile's end, and a consumer group forms its first A
+// of the next tile before it takes this one's sums out of TMEM.
+//   load warp     takes the tiles and fetches table blocks into TSTAGES stages
+//   consumers     two groups of eight warps: group c % 2 forms chunk c's A
+//   MMA warp      issues a chunk's products once its A is in TMEM
+// Every wait is bounded; when one runs out the error word is set and all roles
+// leave their loops.
 template <int NK>
 __global__ void __launch_bounds__(MixShape<NK>::THREADS, 1)
-    k_pw_mixed(const PwItem* __restrict__ items, const double* __restrict__ qmax_p, int* __restrict__ err) {
+    k_pw_mixed(const PwItem* __restrict__ items, int n_tiles, int* __restrict__ next_tile,
+               const double* __restrict__ qmax_p, int* __restrict__ err) {
   using S = MixShape<NK>;
   constexpr int D = S::D, NPAD = S::NPAD, HALF = S::HALF, KCP = S::KCP, KB = S::KB;
+  constexpr int AST = S::ASTAGES, TST = S::TSTAGES, QUEUE = 4;
   extern __shared__ unsigned char smem_raw[];
   // the 1024-aligned base as an offset from the shared array, so that the
   // compiler keeps shared-memory (not generic) loads and stores
   unsigned char* sm = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
-  __shared__ __align__(8) uint64_t mma_bar[2];
-  __shared__ __align__(8) uint64_t tma_bar[4];
+  __shared__ __align__(8) uint64_t t_full[TST], t_free[TST];  // table stages
+  __shared__ __align__(8) uint64_t a_full[AST], a_free[AST];  // A stages
+  __shared__ __align__(8) uint64_t q_full[QUEUE], q_free[QUEUE];
+  __shared__ __align__(8) uint64_t acc_full, acc_free;        // a tile's sums
+  struct Tile {
+    double2* out;  // of the item
+    int tile, nch;  // which M tile (-1: no more), its chunks
+  };
+  __shared__ Tile s_queue[QUEUE];  // the tiles taken
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
 
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31;
   const int warp = tid >> 5;
-  const bool control = tid >= S::CTHREADS;
-  const PwItem it = items[blockIdx.x / S::TILES];
-  const int row0 = int(blockIdx.x % S::TILES) * RPC;                 // first computed row of this CTA
-  const int nrows = min(RPC, S::ROWS_C - row0);  // valid rows of this CTA
-  const int nch = (it.s_end - it.s_begin + KCP - 1) / KCP;
-  const double qmax = *qmax_p;
-
+  constexpr int CWARPS = S::CTHREADS / 32;
   if (tid == 0) {
-    tc::mbar_init(&mma_bar[0], 1);
-    tc::mbar_init(&mma_bar[1], 1);
-    for (int i = 0; i < S::TSTAGES; ++i) tc::mbar_init(&tma_bar[i], 1);
+    for (int i = 0; i < TST; ++i) tc::mbar_init(&t_full[i], 1), tc::mbar_init(&t_free[i], 1);
+    for (int i = 0; i < AST; ++i) tc::mbar_init(&a_full[i], S::GWARPS), tc::mbar_init(&a_free[i], 1);
+    for (int i = 0; i < QUEUE; ++i) tc::mbar_init(&q_full[i], 1), tc::mbar_init(&q_free[i], CWARPS + 1);
+    tc::mbar_init(&acc_full, 1);
+    tc::mbar_init(&acc_free, CWARPS);
     tc::mbar_fence_init();
     s_abort = 0;
   }
@@ -448,176 +492,237 @@ __global__ void __launch_bounds__(MixShape<NK>::THREADS, 1)
   tc::tc_fence_after();
   const uint32_t tmem = s_tmem;
 
+  // false: a wait gave up, here or elsewhere
   auto wait_bar = [&](uint64_t* bar, uint32_t parity) {
-    if (*(volatile int*)&s_abort) return;
+    if (*(volatile int*)&s_abort) return false;
     if (!tc::mbar_wait(bar, parity)) {
       atomicOr(err, 4);
-      s_abort = 1;
+      *(volatile int*)&s_abort = 1;
+      return false;
     }
+    return true;
   };
-  auto fetch = [&](int c) {  // chunk c's table block into table stage c % TSTAGES
-    const int t = c % S::TSTAGES;
-    tc::mbar_arrive_expect_tx(&tma_bar[t], S::T_BYTES);
-    tc::bulk_load(sm + t * S::T_STRIDE, it.tab + size_t(c) * S::T_BYTES, S::T_BYTES, &tma_bar[t]);
+  // the k-th tile of this CTA, for the warps that read the queue
+  auto take = [&](int k) {
+    const bool ok = wait_bar(&q_full[k % QUEUE], uint32_t(k / QUEUE) & 1);
+    Tile t = s_queue[k % QUEUE];
+    if (!__all_sync(0xffffffffu, ok)) t.tile = -1;
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(&q_free[k % QUEUE]);
+    return t;
   };
-  int last_fetch = -1;   // the last chunk requested (control lane 0)
-  int last_commit = -1;  // the last chunk whose MMAs were committed (control lane 0)
 
-  if (control) {
-    // ------------------------------------------------------------ control warp
-    const bool lead = (tid & 31) == 0;
-    if (lead)
-      for (int c = 0; c < min(S::TSTAGES, nch); ++c) {
-        fetch(c);
-        last_fetch = c;
+  if (warp == CWARPS + 1) {
+    // --------------------------------------------------------------- load warp
+    if (lane == 0) {
+      int g = 0;  // chunks fetched
+      for (int k = 0;; ++k) {
+        bool ok = k < QUEUE || wait_bar(&q_free[k % QUEUE], uint32_t(k / QUEUE - 1) & 1);
+        const int w = ok ? atomicAdd(next_tile, 1) : n_tiles;
+        PwItem it{};
+        if (w < n_tiles) it = items[w / S::TILES];
+        const int tile = w < n_tiles ? w % S::TILES : -1;
+        const int nch = (it.s_end - it.s_begin + KCP - 1) / KCP;
+        s_queue[k % QUEUE] = Tile{it.out, tile, nch};
+        tc::mbar_arrive(&q_full[k % QUEUE]);
+        if (tile < 0) break;
+        const int kz_lo = plane_lo(NK, tile), n_planes = plane_hi(NK, tile) - kz_lo + 1;
+        for (int c = 0; c < nch && ok; ++c, ++g) {
+          const int t = g % TST;
+          ok = g < TST || wait_bar(&t_free[t], uint32_t(g / TST - 1) & 1);
+          if (!ok) break;
+          const unsigned char* src = it.tab + size_t(c) * S::T_BYTES;
+          unsigned char* dst = sm + t * S::T_STRIDE;
+          tc::mbar_arrive_expect_tx(&t_full[t], S::EZ_OFF + n_planes * KCP * 16);
+          tc::bulk_load(dst, src, S::EZ_OFF, &t_full[t]);
+          tc::bulk_load(dst + S::EZ_OFF, src + S::EZ_OFF + kz_lo * KCP * 16, n_planes * KCP * 16, &t_full[t]);
+        }
       }
-    for (int c = 0; c < nch; ++c) {
-      const int s2 = c & 1, t = c % S::TSTAGES;
-      tc::bar_sync(BAR_AREADY0 + s2, S::THREADS);  // A of chunk c is in TMEM (and its tables landed)
-      if (lead && !s_abort) {
-        tc::tc_fence_after();
-        const uint32_t abase = tmem + uint32_t(S::A_COL0 + s2 * KB);
-        // descriptor of the stage's B; the others differ by constant address offsets
-        const uint64_t bdesc = tc::smem_desc(tc::smem_u32(sm + t * S::T_STRIDE), S::B_KGROUP, 128);
-        const uint32_t acc0 = c > 0 ? 1u : 0u;
+      // every load has landed before the CTA ends
+      for (int c = max(0, g - TST); c < g; ++c) tc::mbar_wait(&t_full[c % TST], uint32_t(c / TST) & 1);
+    }
+  } else if (warp == CWARPS) {
+    // ---------------------------------------------------------------- MMA warp
+    int g = 0, tiles = 0;  // chunks issued, tiles with any
+    for (int k = 0;; ++k) {
+      const Tile tl = take(k);
+      if (tl.tile < 0) break;
+      const int nch = tl.nch;
+      if (nch == 0) continue;
+      if (lane == 0) {
+        // the previous tile's sums are out of the accumulators
+        bool ok = tiles == 0 || wait_bar(&acc_free, uint32_t(tiles - 1) & 1);
+        for (int c = 0; c < nch && ok; ++c, ++g) {
+          const int st = g % AST, t = g % TST;
+          ok = wait_bar(&a_full[st], uint32_t(g / AST) & 1);  // A is in TMEM (and the chunk's tables landed)
+          if (!ok) break;
+          tc::tc_fence_after();
+          const uint32_t abase = tmem + uint32_t(S::A_COL0 + st * KB);
+          // descriptor of the stage's B; the others differ by constant address offsets
+          const uint64_t bdesc = tc::smem_desc(tc::smem_u32(sm + t * S::T_STRIDE), S::B_KGROUP, 128);
+          const uint32_t acc0 = c > 0 ? 1u : 0u;
 #pragma unroll
-        for (int ks = 0; ks < S::KSTEPS; ++ks) {
-          // slice products (a slice sa, b slices sb) of order sa + sb <= 3 into
-          // accumulators sa + sb: one MMA per run of up to BGROUP b slices,
-          // whose accumulators are adjacent in TMEM as the slices are in B
+          for (int ks = 0; ks < S::KSTEPS; ++ks) {
+            // slice products (a slice sa, b slices sb) of order sa + sb <= 3 into
+            // accumulators sa + sb: one MMA per run of up to BGROUP b slices,
+            // whose accumulators are adjacent in TMEM as the slices are in B
 #pragma unroll
-          for (int sa = 0; sa < 4; ++sa) {
+            for (int sa = 0; sa < 4; ++sa) {
 #pragma unroll
-            for (int sb = 0; sb < 4 - sa; sb += S::BGROUP) {
-              const int nb = min(S::BGROUP, 4 - sa - sb);
-              const uint32_t acc = (ks == 0 && sa == 0) ? acc0 : 1u;
-              const uint64_t bd = bdesc + uint64_t((ks * 2 * S::B_KGROUP + sb * NPAD * 16) >> 4);
-              tc::mma_i8_ts(tmem + uint32_t((sa + sb) * NPAD), abase + uint32_t(sa * (KB / 4) + ks * 8), bd,
-                            tc::idesc_i8(RPC, nb * NPAD), acc);
+              for (int sb = 0; sb < 4 - sa; sb += S::BGROUP) {
+                const int nb = min(S::BGROUP, 4 - sa - sb);
+                const uint32_t acc = (ks == 0 && sa == 0) ? acc0 : 1u;
+                const uint64_t bd = bdesc + uint64_t((ks * 2 * S::B_KGROUP + sb * NPAD * 16) >> 4);
+                tc::mma_i8_ts(tmem + uint32_t((sa + sb) * NPAD), abase + uint32_t(sa * (KB / 4) + ks * 8), bd,
+                              tc::idesc_i8(RPC, nb * NPAD), acc);
+              }
             }
           }
+          tc::mma_commit(&a_free[st]);
+          tc::mma_commit(&t_free[t]);
+          if (c + 1 == nch) tc::mma_commit(&acc_full);
         }
-        tc::mma_commit(&mma_bar[s2]);
-        last_commit = c;
-        // the table stage of chunk c is free once these MMAs have read its B
-        // (the consumers are past its factors: they signalled above)
-        if (c + S::TSTAGES < nch) {
-          wait_bar(&mma_bar[s2], uint32_t(c >> 1) & 1);
-          if (!s_abort) {
-            fetch(c + S::TSTAGES);
-            last_fetch = c + S::TSTAGES;
+      }
+      ++tiles;
+      __syncwarp();
+    }
+    // every MMA and its arrivals have ended before the CTA does
+    if (lane == 0) {
+      for (int c = max(0, g - AST); c < g; ++c) tc::mbar_wait(&a_free[c % AST], uint32_t(c / AST) & 1);
+      for (int c = max(0, g - TST); c < g; ++c) tc::mbar_wait(&t_free[c % TST], uint32_t(c / TST) & 1);
+    }
+  } else {
+    // --------------------------------------------------------------- consumers
+    const int quarter = warp & 3;                    // TMEM lanes 32 quarter + lane
+    const int grp = warp >> 3, kh = (warp >> 2) & 1;  // 16-byte K groups kh, kh + 2 of the group's chunks
+    const int lr = 32 * quarter + lane;              // row of the tile
+    const double scale = *qmax_p / (SL_SCALE * SL_SCALE);
+    const uint32_t lanes = tmem + (uint32_t(32 * quarter) << 16);
+    double2* stage = reinterpret_cast<double2*>(sm + TST * S::T_STRIDE + warp * S::OUT_WARP);
+    int filled = 0;  // tiles with chunks whose sums were taken
+
+    // a tile's sums out of TMEM: the accumulators combined in FP64, four modes
+    // of the warp's 32 rows at a time through the warp's staging
+    auto finish = [&](const Tile& tl) {
+      double2* out = tl.out;
+      const int row0 = tl.tile * RPC, nch = tl.nch;
+      bool ok = true;
+      if (nch > 0) {
+        ok = wait_bar(&acc_full, uint32_t(filled) & 1);
+        ++filled;
+        tc::tc_fence_after();
+      }
+      ok = __all_sync(0xffffffffu, ok);
+      constexpr int BLOCKS = (D + 3) / 4;
+      // the warp's last read of the accumulators: the next tile's MMAs may start
+      auto release = [&]() {
+        tc::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&acc_free);
+      };
+      if (nch > 0 && (warp >> 2) >= BLOCKS) release();
+      for (int b = warp >> 2; b < BLOCKS; b += 4) {
+        double v[2][4];
+        if (nch > 0 && ok) {
+#pragma unroll
+          for (int im = 0; im < 2; ++im) {
+            uint32_t a[4][4];
+            const uint32_t ta = lanes + uint32_t(im * HALF + b * 4);
+#pragma unroll
+            for (int o = 0; o < 4; ++o) tc::tmem_ld4(ta + o * NPAD, a[o]);
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              v[im][i] = scale * fma(i2d(a[3][i]), 1.0 / 16777216.0,
+                                     fma(i2d(a[2][i]), 1.0 / 65536.0, fma(i2d(a[1][i]), 1.0 / 256.0, i2d(a[0][i]))));
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) v[0][i] = v[1][i] = 0.0;
+        }
+        if (nch > 0 && b + 4 >= BLOCKS) release();
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) stage[lane * S::OUT_STRIDE + i] = make_double2(v[0][i], v[1][i]);
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          // eight rows x four modes (64 contiguous bytes a row)
+          const int rl = h * 8 + (lane >> 2), kx = b * 4 + (lane & 3);
+          const int rho = row0 + 32 * quarter + rl;
+          if (kx < D && rho < S::ROWS_C) {
+            const double2 u = stage[rl * S::OUT_STRIDE + (lane & 3)];
+            const int m = rho - NK * D;  // kz = 0: ky = NK + m
+            out[size_t(m < 0 ? rho : rho + NK) * D + kx] = u;
+            // out[NK][2 NK - ky][2 NK - kx] = conj(out[NK][ky][kx])
+            if (m > 0) out[size_t(NK * D + NK - m) * D + 2 * NK - kx] = make_double2(u.x, -u.y);
           }
         }
       }
-      __syncwarp();
-    }
-  } else {
-    // ------------------------------------------------------------ consumers
-    const int lr = tid & (RPC - 1);  // local row = TMEM lane
-    const int kh = tid / RPC;        // this thread's 16-byte K group (8 particles) of each chunk
-    const int rho = row0 + lr;
-    const bool active = lr < nrows;
-    const int r = rho < NK * D ? rho : rho + NK;  // the expansion row
-    const int kz = active ? r / D : 0, ky = active ? r % D : 0;
-    // this thread's four A columns of slice 0 of stage 0 (its warp's lane quarter)
-    const uint32_t arow = tmem + (uint32_t(32 * (warp & 3)) << 16) + uint32_t(S::A_COL0 + kh * 4);
-    for (int c = 0; c < nch; ++c) {
-      const int s2 = c & 1, t = c % S::TSTAGES;
-      wait_bar(&tma_bar[t], uint32_t(c / S::TSTAGES) & 1);    // this chunk's tables have landed
-      if (c >= 2) {
-        wait_bar(&mma_bar[s2], uint32_t((c >> 1) - 1) & 1);  // A stage s2 is free
+    };
+
+    int g = 0;               // chunks of the earlier tiles
+    Tile last{nullptr, -1, 0};  // the tile whose sums are still to be taken
+    for (int k = 0;; ++k) {
+      const Tile tl = take(k);
+      if (tl.tile < 0) break;
+      const int row0 = tl.tile * RPC, nch = tl.nch;
+      const int rho = row0 + lr;
+      const bool active = rho < S::ROWS_C;
+      const int r = rho < NK * D ? rho : rho + NK;  // the expansion row
+      const int ky = active ? r % D : 0;
+      const int kzo = active ? (r / D - plane_lo(NK, tl.tile)) * KCP : 0;
+      for (int c = (g + grp) & 1; c < nch; c += 2) {
+        const int gc = g + c, st = gc % AST, t = gc % TST;
+        bool ok = gc < AST || wait_bar(&a_free[st], uint32_t(gc / AST - 1) & 1);  // the A stage is free
+        ok = ok && wait_bar(&t_full[t], uint32_t(gc / TST) & 1);                  // the chunk's tables have landed
+        if (!__all_sync(0xffffffffu, ok)) break;
         tc::tc_fence_after();
-      }
-      uint32_t w[4][4] = {};
-      if (active) {
         const unsigned char* tb = sm + t * S::T_STRIDE;
-        const double2* ey = reinterpret_cast<const double2*>(tb + S::EY_OFF);
-        const double2* ez = reinterpret_cast<const double2*>(tb + S::EZ_OFF);
+        const double2* ey = reinterpret_cast<const double2*>(tb + S::EY_OFF) + ky;
+        const double2* ez = reinterpret_cast<const double2*>(tb + S::EZ_OFF) + kzo;
 #pragma unroll
-        for (int p = 0; p < 4; ++p) {
-          const int j0 = kh * 8 + 2 * p;
-          // A = ez ey with ez carrying 2^24: each component in fixed point
-          // from two FMAs
-          const double2 z0 = ez[j0 * S::EZS + kz], y0 = ey[j0 * D + ky];
-          const double2 z1 = ez[(j0 + 1) * S::EZS + kz], y1 = ey[(j0 + 1) * D + ky];
-          uint32_t by[4];
-          transpose4(fix24_dot(z0.x, y0.x, -z0.y, y0.y), fix24_dot(z0.x, y0.y, z0.y, y0.x),
-                     fix24_dot(z1.x, y1.x, -z1.y, y1.y), fix24_dot(z1.x, y1.y, z1.y, y1.x), by);
+        for (int kg = 0; kg < S::KGT; ++kg) {
+          const int k4 = kh + 2 * kg;
+          uint32_t a[4][4] = {};
+          if (active) {
 #pragma unroll
-          for (int sl = 0; sl < 4; ++sl) w[sl][p] = by[3 - sl];
+            for (int p = 0; p < 4; ++p) {
+              const int j0 = k4 * 8 + 2 * p;
+              // A = ez ey with ez carrying 2^24: each component in fixed point
+              // from two FMAs
+              const double2 z0 = ez[j0], y0 = ey[j0 * D];
+              const double2 z1 = ez[j0 + 1], y1 = ey[(j0 + 1) * D];
+              uint32_t by[4];
+              transpose4(fix24_dot(z0.x, y0.x, -z0.y, y0.y), fix24_dot(z0.x, y0.y, z0.y, y0.x),
+                         fix24_dot(z1.x, y1.x, -z1.y, y1.y), fix24_dot(z1.x, y1.y, z1.y, y1.x), by);
+#pragma unroll
+              for (int sl = 0; sl < 4; ++sl) a[sl][p] = by[3 - sl];
+            }
+          }
+          // every lane stores (rows past the end store zeros, never read back)
+          __syncwarp();
+#pragma unroll
+          for (int sl = 0; sl < 4; ++sl)
+            tc::tmem_st4(lanes + uint32_t(S::A_COL0 + st * KB + sl * (KB / 4) + k4 * 4), a[sl][0], a[sl][1], a[sl][2],
+                         a[sl][3]);
+        }
+        tc::tmem_st_wait();
+        tc::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&a_full[st]);
+        if (last.tile >= 0) {
+          finish(last);
+          last.tile = -1;
         }
       }
-      // every lane stores (rows past the tile's end store zeros, never read back)
-#pragma unroll
-      for (int sl = 0; sl < 4; ++sl)
-        tc::tmem_st4(arow + uint32_t(s2 * KB + sl * (KB / 4)), w[sl][0], w[sl][1], w[sl][2], w[sl][3]);
-      tc::tmem_st_wait();
-      tc::tc_fence_before();
-      tc::bar_arrive(BAR_AREADY0 + s2, S::THREADS);
+      if (last.tile >= 0) finish(last);
+      last = tl;
+      g += nch;
     }
-    // ------------------------------------------------------------ epilogue
-    if (nch > 0) {
-      const int cl = nch - 1;
-      wait_bar(&mma_bar[cl & 1], uint32_t(cl >> 1) & 1);
-    }
-    tc::tc_fence_after();
-    tc::bar_sync(BAR_CONS, S::CTHREADS);  // every consumer is past its last read of the pipeline buffers
-    const int q = warp & 3;            // TMEM lane quarter (warps 4k .. 4k + 3 read lanes 0 .. 127)
-    double2* stage = reinterpret_cast<double2*>(sm) + size_t(lr) * D;
-    const double scale = qmax / (SL_SCALE * SL_SCALE);
-    if (nch > 0 && !s_abort) {
-#pragma unroll 1
-      for (int cb = kh; cb < NPAD / 16; cb += S::CPR) {
-        uint32_t a0[16], a1[16], a2[16], a3[16];
-        const uint32_t ta = tmem + (uint32_t(32 * q) << 16) + uint32_t(cb * 16);
-        tc::tmem_ld16(ta, a0);
-        tc::tmem_ld16(ta + NPAD, a1);
-        tc::tmem_ld16(ta + 2 * NPAD, a2);
-        tc::tmem_ld16(ta + 3 * NPAD, a3);
-        tc::tmem_ld_wait();
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-          const int n = cb * 16 + k;
-          const double v = scale * fma(i2d(a3[k]), 1.0 / 16777216.0,
-                                       fma(i2d(a2[k]), 1.0 / 65536.0, fma(i2d(a1[k]), 1.0 / 256.0, i2d(a0[k]))));
-          if (n < D) stage[n].x = v;
-          else if (n >= HALF && n < HALF + D) reinterpret_cast<double*>(stage + (n - HALF))[1] = v;
-        }
-      }
-    } else {
-      for (int n = kh; n < D; n += S::CPR) stage[n] = make_double2(0.0, 0.0);
-    }
-    tc::fence_async_smem();
-    tc::bar_sync(BAR_CONS, S::CTHREADS);
-    // computed rows below NK D are the expansion rows themselves; those above
-    // lie NK rows further on (the kz = 0, ky >= 0 rows)
-    const int n_lo = max(0, min(nrows, NK * D - row0));
-    if (tid == 0) {
-      if (n_lo > 0) tc::bulk_store(it.out + size_t(row0) * D, sm, uint32_t(n_lo) * D * 16u);
-      if (nrows > n_lo)
-        tc::bulk_store(it.out + size_t(row0 + n_lo + NK) * D, sm + size_t(n_lo) * D * 16, uint32_t(nrows - n_lo) * D * 16u);
-      tc::bulk_commit();
-    }
-    // the kz = 0, ky < 0 rows: out[NK][ky][kx] = conj(out[NK][2 NK - ky][2 NK - kx])
-    // from the staged rows ky = 2 NK - ky > NK of this CTA
-    {
-      const double2* st0 = reinterpret_cast<const double2*>(sm);
-      const int m_lo = max(row0, NK * D + 1), m_hi = row0 + nrows;  // computed rows with ky > NK
-      for (int idx = tid; idx < (m_hi - m_lo) * D; idx += S::CTHREADS) {
-        const int src = m_lo + idx / D, kx = idx % D;
-        const int ky = NK + (src - NK * D);          // > NK
-        const double2 v = st0[size_t(src - row0) * D + (2 * NK - kx)];
-        it.out[size_t(NK * D + 2 * NK - ky) * D + kx] = make_double2(v.x, -v.y);
-      }
-    }
-    if (tid == 0) tc::bulk_wait_all();
+    if (last.tile >= 0) finish(last);
   }
-  // copies and MMAs this CTA started have ended (bounded waits; they only
-  // matter when a pipeline wait gave up) before its TMEM is released
-  if (control && (tid & 31) == 0) {
-    if (last_fetch >= 0) tc::mbar_wait(&tma_bar[last_fetch % S::TSTAGES], uint32_t(last_fetch / S::TSTAGES) & 1);
-    if (last_commit >= 0) tc::mbar_wait(&mma_bar[last_commit & 1], uint32_t(last_commit >> 1) & 1);
-  }
+  __syncwarp();
   tc::tc_fence_before();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem, S::TCOLS);
@@ -644,16 +749,17 @@ __global__ void k_absmax(const double* __restrict__ q, int n, double* out) {
 
 template <int NK>
 void launch_mixed(const CUtensorMap& tmap, const PwItem* d_items, int nitems, const int2* d_chunks, int nchunks,
-                  const double* d_qmax, int* d_err, cudaStream_t st) {
+                  int* d_next, const double* d_qmax, int* d_err, cudaStream_t st) {
   using S = MixShape<NK>;
   if (nitems == 0) return;
+  int dev = 0, sms = 0;
+  PDMK_CUDA(cudaGetDevice(&dev));
+  PDMK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   if (nchunks > 0) {
     raise_smem_limit(reinterpret_cast<const void*>(k_pw_tables<NK>), S::TK_SMEM);
     // persistent: as many CTAs as are resident at once, each walking a
     // strided share of the chunks
-    int dev = 0, sms = 0, per_sm = 0;
-    PDMK_CUDA(cudaGetDevice(&dev));
-    PDMK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int per_sm = 0;
     PDMK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pw_tables<NK>, S::TTHREADS, S::TK_SMEM));
     const int grid = std::max(1, std::min(nchunks, std::max(1, per_sm) * sms));
     k_pw_tables<NK><<<unsigned(grid), S::TTHREADS, S::TK_SMEM, st>>>(tmap, d_items, d_chunks, nchunks, d_qmax,
@@ -661,7 +767,11 @@ void launch_mixed(const CUtensorMap& tmap, const PwItem* d_items, int nitems, co
     PDMK_LAUNCH_CHECK();
   }
   raise_smem_limit(reinterpret_cast<const void*>(k_pw_mixed<NK>), S::SMEM);
-  k_pw_mixed<NK><<<unsigned(nitems) * S::TILES, S::THREADS, S::SMEM, st>>>(d_items, d_qmax, d_err);
+  // persistent: as many CTAs as the SMs' columns and shared memory hold
+  int per_sm = 0;
+  PDMK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pw_mixed<NK>, S::THREADS, S::SMEM));
+  const int grid = std::min(nitems * S::TILES, std::max(1, std::min(per_sm, 512 / S::TCOLS)) * sms);
+  k_pw_mixed<NK><<<unsigned(grid), S::THREADS, S::SMEM, st>>>(d_items, nitems * S::TILES, d_next, d_qmax, d_err);
   PDMK_LAUNCH_CHECK();
 }
 
@@ -741,9 +851,9 @@ void launch_absmax(const double* sq, int n, double* out, cudaStream_t st) {
 }
 
 void dispatch_mixed(int nk, const CUtensorMap& tmap, const PwItem* d_items, int nitems, const int2* d_chunks,
-                    int nchunks, const double* d_qmax, int* d_err, cudaStream_t st) {
+                    int nchunks, int* d_next, const double* d_qmax, int* d_err, cudaStream_t st) {
 #define PDMK_MIX_CASE(n) \
-  case n: launch_mixed<n>(tmap, d_items, nitems, d_chunks, nchunks, d_qmax, d_err, st); break;
+  case n: launch_mixed<n>(tmap, d_items, nitems, d_chunks, nchunks, d_next, d_qmax, d_err, st); break;
   switch (nk) {
     PDMK_MIX_CASE(4)
     PDMK_MIX_CASE(6)

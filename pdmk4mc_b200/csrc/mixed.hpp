@@ -8,7 +8,7 @@
 
 namespace pdmk {
 
-// CTAs per box for n modes per axis half
+// M tiles per box for n modes per axis half
 int mixed_pairs(int nk);
 // particles per pipeline chunk of the mixed pass for n modes per axis half
 int mixed_chunk(int nk);
@@ -21,9 +21,10 @@ void make_coord_map(CUtensorMap* map, const double* sx, int slot_capacity, int k
 void launch_absmax(const double* sq, int n, double* out, cudaStream_t st);
 // the mixed pass over device-resident lists: the table pass over nchunks
 // (item, chunk) pairs into the items' chunk table blocks, then the
-// contraction: mixed_pairs(nk) CTAs per item, one per 128-row M tile, which
-// share the item's blocks (ceil((s_end - s_begin) / chunk) of them)
+// contraction: mixed_pairs(nk) 128-row M tiles per item, which share the
+// item's blocks (ceil((s_end - s_begin) / chunk) of them); d_next: the counter
+// the tiles are taken from, at zero
 void dispatch_mixed(int nk, const CUtensorMap& tmap, const PwItem* d_items, int nitems, const int2* d_chunks,
-                    int nchunks, const double* d_qmax, int* d_err, cudaStream_t st);
+                    int nchunks, int* d_next, const double* d_qmax, int* d_err, cudaStream_t st);
 
 }  // namespace pdmk

@@ -82,7 +82,7 @@ __device__ __forceinline__ PwItem box_item(const DevTree& T, int l, uint64_t p, 
 }
 
 __global__ void k_plan_root(DevTree T, PlanShape s, int n, int n_items, int n_chunks, double dk, double2* part,
-                            unsigned char* tab, PwItem* items, int2* chunks, PwSplit* split) {
+                            unsigned char* tab, PwItem* items, int2* chunks, PwSplit* split, int* next) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int full = s.tab_bytes ? (s.ksplit + s.kcp - 1) / s.kcp : 1;
   if (i < n_items) {
@@ -94,6 +94,7 @@ __global__ void k_plan_root(DevTree T, PlanShape s, int n, int n_items, int n_ch
   if (i < n_chunks) chunks[i] = make_int2(i / full, i % full);
   if (i == 0) {
     *split = PwSplit{0, n_items, T.out_root};
+    *next = 0;
     T.counter[14] = 1;  // every outgoing row is about to be written
   }
 }
@@ -164,11 +165,12 @@ __global__ void __launch_bounds__(PLAN_T) k_plan_lists(DevTree T, const int* __r
 
 __global__ void __launch_bounds__(PLAN_T)
     k_plan_items(DevTree T, PlanShape s, const int* __restrict__ node_first, PlanState* state, double2* part,
-                 unsigned char* tab, PwItem* items, int2* chunks, PwSplit* split) {
+                 unsigned char* tab, PwItem* items, int2* chunks, PwSplit* split, int* next) {
   __shared__ int start[kPlanBuckets], cnt[kPlanBuckets];
   __shared__ int n_ch, ch0;
   for (int i = threadIdx.x; i < kPlanBuckets; i += PLAN_T) cnt[i] = 0;
   if (threadIdx.x == 0) n_ch = 0;
+  if (threadIdx.x == 0 && blockIdx.x == 0) *next = 0;
   // exclusive sums of the buckets: four per lane of the first warp
   if (threadIdx.x < 32) {
     int h[4], v = 0;
@@ -233,10 +235,11 @@ __global__ void __launch_bounds__(PLAN_T)
 int plan_blocks(int n_nodes) { return (n_nodes + PLAN_T - 1) / PLAN_T; }
 
 void launch_plan_root(const DevTree& T, const PlanShape& s, int n, int n_items, int n_chunks, double2* part,
-                      unsigned char* tab, PwItem* items, int2* chunks, PwSplit* split, cudaStream_t st) {
+                      unsigned char* tab, PwItem* items, int2* chunks, PwSplit* split, int* next,
+                       cudaStream_t st) {
   const int m = std::max(n_items, n_chunks);
   k_plan_root<<<unsigned((m + 127) / 128), 128, 0, st>>>(T, s, n, n_items, n_chunks, T.delta_k[0], part, tab, items,
-                                                         chunks, split);
+                                                         chunks, split, next);
   PDMK_LAUNCH_CHECK();
 }
 
@@ -251,12 +254,13 @@ void launch_plan_lists(const DevTree& T, const int* blk, int* nonleaf, int* leav
 }
 
 void launch_plan_items(const DevTree& T, const PlanShape& s, const int* node_first, PlanState* state, double2* part,
-                       unsigned char* tab, PwItem* items, int2* chunks, PwSplit* split, cudaStream_t st) {
+                       unsigned char* tab, PwItem* items, int2* chunks, PwSplit* split, int* next,
+                       cudaStream_t st) {
   if (T.pw_hi < T.pw_lo) return;
   const int n_pw = T.level_start[T.pw_hi + 1] - T.level_start[T.pw_lo];
   if (n_pw == 0) return;
   k_plan_items<<<unsigned(plan_blocks(n_pw)), PLAN_T, 0, st>>>(T, s, node_first, state, part, tab, items, chunks,
-                                                              split);
+                                                              split, next);
   PDMK_LAUNCH_CHECK();
 }
 

@@ -48,16 +48,17 @@ struct PlanShape {
 };
 
 int plan_blocks(int n_nodes);
-// the root's items, chunk list and split entry (grid-sized by the host)
+// the root's items, chunk list and split entry (grid-sized by the host); *next = 0
 void launch_plan_root(const DevTree& T, const PlanShape& s, int n, int n_items, int n_chunks, double2* part,
-                      unsigned char* tab, PwItem* items, int2* chunks, PwSplit* split, cudaStream_t st);
+                      unsigned char* tab, PwItem* items, int2* chunks, PwSplit* split, int* next, cudaStream_t st);
 // totals over the nodes into *state (zeroed by the caller); `lists`: the box
 // lists' as well, with per-block counts in blk[3 plan_blocks]
 void launch_plan_count(const DevTree& T, const PlanShape& s, bool lists, PlanState* state, int* blk, cudaStream_t st);
 // the box lists in node order
 void launch_plan_lists(const DevTree& T, const int* blk, int* nonleaf, int* leaves, int* cubes, cudaStream_t st);
-// the items in order of falling size, their chunk list and the split boxes
+// the items in order of falling size, their chunk list and the split boxes;
+// *next = 0
 void launch_plan_items(const DevTree& T, const PlanShape& s, const int* node_first, PlanState* state, double2* part,
-                       unsigned char* tab, PwItem* items, int2* chunks, PwSplit* split, cudaStream_t st);
+                       unsigned char* tab, PwItem* items, int2* chunks, PwSplit* split, int* next, cudaStream_t st);
 
 }  // namespace pdmk
