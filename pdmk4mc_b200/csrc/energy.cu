@@ -510,11 +510,11 @@ __global__ void k_diff_finish_cube(DevTree T, const int* __restrict__ cubes, int
                                    const double* Cl, const double* Sl, double* out) {
   __shared__ double sm[32];
   double e = 0;
-  for (int c = threadIdx.x; c < ncubes; c += blockDim.x) {
-    const int l = T.node_level[cubes[c]] + 2;
-    double t = 0;
-    for (int sl = 0; sl < slots; ++sl) t += part[size_t(sl) * ncubes + c];
-    e += Cl[l] * level_dscale(l) * t;
+  // all (slot, cube) terms over the threads: a small tree has one cube of 500
+  // slots, which one thread summed in 28 us
+  for (int i = threadIdx.x; i < slots * ncubes; i += blockDim.x) {
+    const int l = T.node_level[cubes[i % ncubes]] + 2;
+    e += Cl[l] * level_dscale(l) * part[i];
   }
   for (int b = threadIdx.x; b < nboxes; b += blockDim.x) e -= q2[b] * Sl[T.node_level[boxes[b]]];
   double s = block_sum(e, sm);
@@ -941,9 +941,16 @@ __global__ void k_set_defined(unsigned int* counter, bool out, bool inc) {
 
 __global__ void k_sum(const double* part, int n, double* out) {
   __shared__ double sm[32];
-  double e = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) e += part[i];
-  double s = block_sum(e, sm);
+  // eight loads in flight a thread: one at a time, the 2.6e5 near-field
+  // partials of N = 1e6 took 31 us
+  double e[8] = {};
+  const int st = blockDim.x;
+  for (int i = threadIdx.x; i < n; i += 8 * st) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (i + u * st < n) e[u] += part[i + u * st];
+  }
+  double s = block_sum(((e[0] + e[1]) + (e[2] + e[3])) + ((e[4] + e[5]) + (e[6] + e[7])), sm);
   if (threadIdx.x == 0) *out = s;
 }
 
