@@ -600,6 +600,33 @@ constexpr int RES_T = 128;
 constexpr int RES_TCH = 64;   // targets of one work item
 constexpr int RES_SCH = 256;  // sources staged in shared memory per round
 
+// the smallest and largest of a full warp's values (one instruction on sm_100)
+__device__ __forceinline__ float warp_min(float a) {
+  float d;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(d) : "f"(a));
+  return d;
+}
+__device__ __forceinline__ float warp_max(float a) {
+  float d;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(d) : "f"(a));
+  return d;
+}
+// two FP32 values in one 64-bit register (sm_100's packed arithmetic)
+__device__ __forceinline__ unsigned long long both_f32x2(float a) {
+  const unsigned long long w = __float_as_uint(a);
+  return w << 32 | w;
+}
+__device__ __forceinline__ unsigned long long add_f32x2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long fma_f32x2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
 // leaf near field: 1/2 sum_{i in B} q_i sum_{j in N(B), j != i} q_j res(r_ij; bs_B)
 // (eval_energy_res, src/energy.cpp:82-173). One block per (leaf, chunk of
 // RES_TCH targets), so a large leaf is spread over several blocks; leaves are
@@ -617,11 +644,17 @@ constexpr int RES_SCH = 256;  // sources staged in shared memory per round
 // instructions a pair, where asking the warp for every pair took 28). The
 // queue is evaluated 32 pairs at a time in FP64, distance and polynomial, so
 // the sum is the one over all pairs (a pair beyond the cut-off adds zero there).
-template <int NP>
-__global__ void __launch_bounds__(RES_T) k_residual(DevTree T, const int* __restrict__ leaves, int ny,
+//
+// MINB, resident blocks: filled tiles want registers (N = 1e5, 55 particles a
+// leaf: 0.46 ms at 7 blocks, 0.49 at 8, 0.54 at 9), small leaves want blocks to
+// hide the staging behind (N = 1e6, 30 a leaf: 1.04 ms at 7, 1.00 at 8, 0.92 at
+// 9).
+template <int NP, int MINB>
+__global__ void __launch_bounds__(RES_T, MINB) k_residual(DevTree T, const int* __restrict__ leaves, int ny,
                                                     double* part) {
   __shared__ double ux[RES_SCH], uy[RES_SCH], uz[RES_SCH], uq[RES_SCH];
-  __shared__ float4 uf[RES_SCH];                  // relative to the leaf's centre
+  // negated coordinates relative to the leaf's centre
+  __shared__ __align__(16) float ufx[RES_SCH], ufy[RES_SCH], ufz[RES_SCH];
   __shared__ float t_lo[RES_SCH / 32][3], t_hi[RES_SCH / 32][3];  // bounding boxes of the source tiles
   __shared__ double gx[RES_TCH], gy[RES_TCH], gz[RES_TCH], gq[RES_TCH];
   __shared__ int m_beg[36], m_pre[37];
@@ -700,18 +733,16 @@ __global__ void __launch_bounds__(RES_T) k_residual(DevTree T, const int* __rest
       const bool act = it < nt;
       const float fx = act ? float(gx[it] - ci[0]) : far, fy = act ? float(gy[it] - ci[1]) : far,
                   fz = act ? float(gz[it] - ci[2]) : far;
+      const unsigned long long fx2 = both_f32x2(fx), fy2 = both_f32x2(fy), fz2 = both_f32x2(fz);
+      const unsigned long long ncut2 = both_f32x2(-cut);
       float lo[3] = {fx, fy, fz}, hi[3] = {act ? fx : -far, act ? fy : -far, act ? fz : -far};
 #pragma unroll
-      for (int a = 0; a < 3; ++a)
-        for (int o = 16; o > 0; o >>= 1) {
-          lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-          hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
-        }
+      for (int a = 0; a < 3; ++a) lo[a] = warp_min(lo[a]), hi[a] = warp_max(hi[a]);
       for (int u0 = 0; u0 < total; u0 += RES_SCH) {
         const int ns = min(RES_SCH, total - u0);
         __syncthreads();
         for (int t = threadIdx.x; t < (ns + 31) / 32 * 32; t += blockDim.x) {  // whole warps
-          float4 f = make_float4(-far, -far, -far, 0.0f);  // far from everything, from an absent target too
+          float f[3] = {-far, -far, -far};  // far from everything, from an absent target too
           float flo[3] = {far, far, far}, fhi[3] = {-far, -far, -far};
           if (t < ns) {
             const int ei = u0 + t;
@@ -727,18 +758,15 @@ __global__ void __launch_bounds__(RES_T) k_residual(DevTree T, const int* __rest
             uy[t] = y;
             uz[t] = zz;
             uq[t] = T.sq[s] * m_w[a];
-            f = make_float4(float(x - ci[0]), float(y - ci[1]), float(zz - ci[2]), 0.0f);
-            flo[0] = fhi[0] = f.x;
-            flo[1] = fhi[1] = f.y;
-            flo[2] = fhi[2] = f.z;
-          }
-          uf[t] = f;
+            f[0] = float(x - ci[0]), f[1] = float(y - ci[1]), f[2] = float(zz - ci[2]);
 #pragma unroll
-          for (int a = 0; a < 3; ++a)
-            for (int o = 16; o > 0; o >>= 1) {
-              flo[a] = fminf(flo[a], __shfl_xor_sync(0xffffffffu, flo[a], o));
-              fhi[a] = fmaxf(fhi[a], __shfl_xor_sync(0xffffffffu, fhi[a], o));
-            }
+            for (int a2 = 0; a2 < 3; ++a2) flo[a2] = fhi[a2] = f[a2];
+          }
+          ufx[t] = -f[0];
+          ufy[t] = -f[1];
+          ufz[t] = -f[2];
+#pragma unroll
+          for (int a = 0; a < 3; ++a) flo[a] = warp_min(flo[a]), fhi[a] = warp_max(fhi[a]);
           if (lane < 3) {
             t_lo[t >> 5][lane] = lane == 0 ? flo[0] : lane == 1 ? flo[1] : flo[2];
             t_hi[t >> 5][lane] = lane == 0 ? fhi[0] : lane == 1 ? fhi[1] : fhi[2];
@@ -763,13 +791,22 @@ __global__ void __launch_bounds__(RES_T) k_residual(DevTree T, const int* __rest
             d2 = fmaf(d, d, d2);
           }
           if (d2 > cut) continue;
-          const float4* tp = uf + tile * 32;
+          // r^2 - cut for two sources at a time (packed FP32), its sign the
+          // answer: source j ends up at bit 31 - j
           unsigned mask = 0;
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float4 s = tp[j];
-            const float dx = fx - s.x, dy = fy - s.y, dz = fz - s.z;
-            if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= cut) mask |= 1u << j;
+          for (int j = 0; j < 32; j += 4) {
+            const ulonglong2 sx = *reinterpret_cast<const ulonglong2*>(ufx + tile * 32 + j);
+            const ulonglong2 sy = *reinterpret_cast<const ulonglong2*>(ufy + tile * 32 + j);
+            const ulonglong2 sz = *reinterpret_cast<const ulonglong2*>(ufz + tile * 32 + j);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const unsigned long long dx = add_f32x2(fx2, h ? sx.y : sx.x), dy = add_f32x2(fy2, h ? sy.y : sy.x),
+                                       dz = add_f32x2(fz2, h ? sz.y : sz.x);
+              const unsigned long long r = fma_f32x2(dz, dz, fma_f32x2(dy, dy, fma_f32x2(dx, dx, ncut2)));
+              mask = __funnelshift_l(unsigned(r), mask, 1);
+              mask = __funnelshift_l(unsigned(r >> 32), mask, 1);
+            }
           }
           // this lane's places in the queue: after the pairs waiting and the lanes below
           const int mine = __popc(mask);
@@ -781,8 +818,9 @@ __global__ void __launch_bounds__(RES_T) k_residual(DevTree T, const int* __rest
           const int all = __shfl_sync(0xffffffffu, at, 31);
           at += qn - mine;
           while (mask) {
-            q_pair[wid][at++] = static_cast<unsigned short>((it << 8) | (tile * 32 + __ffs(mask) - 1));
-            mask &= mask - 1;
+            const int j = __clz(mask);
+            q_pair[wid][at++] = static_cast<unsigned short>((it << 8) | (tile * 32 + j));
+            mask &= ~(0x80000000u >> j);
           }
           qn += all;
           __syncwarp();
@@ -1302,8 +1340,13 @@ void DmkTree::launch_res_energy() {
   prepare_box_lists();
   DevTree& D = dev_;
   if (n_leaves_ > 0) {
-    auto kern = D.n_poly == 7 ? k_residual<7> : D.n_poly == 13 ? k_residual<13> : D.n_poly == 19 ? k_residual<19>
-                                                                                                 : k_residual<25>;
+    auto pick = [&](auto minb) {
+      constexpr int B = decltype(minb)::value;
+      return D.n_poly == 7 ? k_residual<7, B> : D.n_poly == 13 ? k_residual<13, B> : D.n_poly == 19 ? k_residual<19, B>
+                                                                                                    : k_residual<25, B>;
+    };
+    // between the two measured fillings
+    auto kern = N_ >= 40 * long(n_leaves_) ? pick(std::integral_constant<int, 7>{}) : pick(std::integral_constant<int, 9>{});
     const int ny = res_chunks();
     kern<<<unsigned(n_leaves_ * ny), RES_T, 0, st_>>>(D, d_leaves_, ny, D.partials);
     PDMK_LAUNCH_CHECK();
