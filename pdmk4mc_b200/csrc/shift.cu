@@ -3539,7 +3539,12 @@ bool DmkTree::mc_run_long(int n_moves, const int* d_idx, const double* d_disp, c
     mcl_grid_ = sms;
   }
   prepare_box_lists();
-  const int chunk = std::min(n_pw >= 1024 ? 2048 : 1024, kPendPerBlock * mcl_grid_);
+  // A longer list makes each move's pair sums longer (5 ns per listed move at
+  // N = 1e5, 7.4 ns at 1e6), a shorter one updates the rows more often (0.38 and
+  // 2.1 ms). 2000 moves at N = 1e5 / 4000 at 1e6 (9 digits, positions
+  // read at the end): 20.8 / 75.1 ms at 384 moves a list, 20.7 / 71.3 at 512, 20.9 /
+  // 69.8 at 768, 21.3 / 68.1 at 1024, 23.6 / 69.9 at 2048.
+  const int chunk = std::min(n_pw >= 1024 ? 1024 : 512, kPendPerBlock * mcl_grid_);
   ensure_pending(std::min(chunk, n_moves));
   const double pi = 3.14159265358979323846;
   for (int m0 = 0; m0 < n_moves; m0 += chunk) {
