@@ -565,6 +565,49 @@ void return_stream(int device, cudaStream_t s) {
   cudaStreamDestroy(s);
 }
 
+namespace {
+struct HostSlots {
+  std::mutex mu;
+  unsigned char* page = nullptr;  // one 4 KB page for the process
+  bool failed = false;
+  uint64_t used = 0;
+};
+HostSlots g_host_slots;
+}  // namespace
+
+double* take_host_slot(double** device_address) {
+  HostSlots& S = g_host_slots;
+  std::lock_guard<std::mutex> g(S.mu);
+  if (!S.page && !S.failed) {
+    // another thread's capture must not see the allocation as its own
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void* p = nullptr;
+    S.failed = cudaHostAlloc(&p, 4096, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess;
+    if (S.failed) cudaGetLastError();
+    else S.page = static_cast<unsigned char*>(p);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  }
+  if (!S.page || S.used == ~uint64_t(0)) return nullptr;
+  int k = 0;
+  while (S.used >> k & 1) ++k;
+  double* slot = reinterpret_cast<double*>(S.page + 64 * k);
+  void* d = nullptr;
+  if (cudaHostGetDevicePointer(&d, slot, 0) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  S.used |= uint64_t(1) << k;
+  *device_address = static_cast<double*>(d);
+  return slot;
+}
+
+void return_host_slot(double* slot) {
+  HostSlots& S = g_host_slots;
+  std::lock_guard<std::mutex> g(S.mu);
+  S.used &= ~(uint64_t(1) << ((reinterpret_cast<unsigned char*>(slot) - S.page) / 64));
+}
+
 // ---------------------------------------------------------------------------
 // Tree-lifetime allocations come from the device's stream-ordered pool, kept
 // cached across trees (the release threshold is raised once per device), so
@@ -620,6 +663,7 @@ DmkTree::DmkTree(double L, int n_per_leaf, int digits, long n, const double* r, 
 
 DmkTree::~DmkTree() {
   cudaStreamSynchronize(st_);
+  if (slot_) return_host_slot(slot_);
   if (aux_) {
     cudaStreamSynchronize(aux_);
     return_stream(aux_device_, aux_);
@@ -1213,9 +1257,6 @@ void DmkTree::build_setup() {
   d_Sl_ = d_Cl_ + (MAX_LEVELS + 2);
   put_small(d_Cl_, coef, sizeof(coef), st_);
   d_scalars_ = static_cast<double*>(alloc(sizeof(double) * 8));
-  d_one_idx_ = static_cast<int*>(alloc(64));
-  d_one_disp_ = static_cast<double*>(alloc(64));
-  d_one_u_ = static_cast<double*>(alloc(64));
 }
 
 int DmkTree::check_device_error() const {

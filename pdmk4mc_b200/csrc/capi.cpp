@@ -356,8 +356,7 @@ int hpdmk_update_shift(hpdmk_tree t, long i, double dx, double dy, double dz) {
   if (check_move(H(t), i, dx, dy, dz) != HPDMK_OK) return g_last_error;
   return guarded([&]() {
     DeviceGuard dg(H(t)->device);
-    H(t)->tree->update_shift(i, dx, dy, dz);
-    if (int e = H(t)->tree->check_device_error()) return device_fail(e);
+    if (int e = H(t)->tree->update_shift(i, dx, dy, dz)) return device_fail(e);
     return ok();
   });
 }

@@ -835,12 +835,21 @@ struct ShiftArgs {
   double2* ptab;          // phase tables published for k_update
   long ptab_per;          // complex entries per path
   const MoveCursor* cur;  // non-null: proposals come from the cursor (captured graphs)
+  double* host_out;       // dE and its five parts for the host (mapped memory; may be null)
 };
 
-// Grid: blocks [0, G-2) do the plane-wave sums; block G-2 the target
-// residual, block G-1 the origin residual. The last block to finish reduces.
+// a proposal passed with the launch (ShiftArgs::idx null)
+struct OneMove {
+  int i;
+  double d[3];
+};
+
+// Grid: blocks [0, G-3) do the plane-wave sums; block G-3 the target
+// residual, block G-2 the origin residual, block G-1 lists the receivers of an
+// update (beside the sums: behind them it lengthened the launch by 2 us). The
+// last block to finish reduces.
 template <int NP>
-__global__ void __launch_bounds__(SH_T) k_shift(DevTree T, ShiftArgs a) {
+__global__ void __launch_bounds__(SH_T) k_shift(DevTree T, ShiftArgs a, const __grid_constant__ OneMove one) {
   extern __shared__ double2 sm2[];
   __shared__ Header h;
   __shared__ double red[4][32];
@@ -864,9 +873,9 @@ __global__ void __launch_bounds__(SH_T) k_shift(DevTree T, ShiftArgs a) {
     a.move += c.off;
   }
   const int move = a.move;
-  resolve(T, a.idx[move], a.disp + 3 * move, h);
+  resolve(T, a.idx ? a.idx[move] : one.i, a.idx ? a.disp + 3 * move : one.d, h);
   const int G = gridDim.x;
-  const int Gpw = G - 2;
+  const int Gpw = G - 3;
   double acc[4] = {0, 0, 0, 0};  // window, difference, residual target, residual origin
   if (blockIdx.x < Gpw) {
     // dE needs the non-leaf path levels 2 .. depth-2; an accept-and-update
@@ -924,9 +933,12 @@ __global__ void __launch_bounds__(SH_T) k_shift(DevTree T, ShiftArgs a) {
   } else if (blockIdx.x == Gpw) {
     const int lt = h.depth_t - 1;
     acc[2] = residual_sum(T, poly, h.path_t[lt], lt, h.Xt[lt], h.xt) * h.q;
-  } else {
+  } else if (blockIdx.x == Gpw + 1) {
     const int lo = h.depth_o - 1;
     acc[3] = residual_sum(T, poly, h.path_o[lo], lo, h.Xo[lo], h.xo) * h.q;
+  } else {
+    const int n = build_receivers(T, h, T.recv);
+    if (threadIdx.x == 0) a.prop->n_recv = n;
   }
   block_sum4(acc, red);
   if (threadIdx.x == 0) {
@@ -944,7 +956,6 @@ __global__ void __launch_bounds__(SH_T) k_shift(DevTree T, ShiftArgs a) {
   for (int b = threadIdx.x; b < G; b += blockDim.x)
     for (int c = 0; c < 4; ++c) tot[c] += __ldcg(a.partials + 4 * size_t(b) + c);
   block_sum4(tot, red);
-  const int nrecv = build_receivers(T, h, T.recv);
   if (threadIdx.x == 0) {
     const double dEw = tot[0] * a.c_window;  // 2 * sum * dk0^3 / (2 (2 pi)^3)
     const double d = tot[1], rt = tot[2], ro = tot[3];
@@ -971,6 +982,10 @@ __global__ void __launch_bounds__(SH_T) k_shift(DevTree T, ShiftArgs a) {
     P->parts[2] = rt;
     P->parts[3] = ro;
     P->parts[4] = self;
+    if (a.host_out) {
+      a.host_out[0] = dE;
+      for (int c = 0; c < 5; ++c) a.host_out[1 + c] = P->parts[c];
+    }
     int accd = 0;
     if (a.mode == 1) {
       const double u = a.u[move];
@@ -980,7 +995,6 @@ __global__ void __launch_bounds__(SH_T) k_shift(DevTree T, ShiftArgs a) {
     if (a.dE_out) a.dE_out[move] = dE;
     P->accepted = accd;
     P->valid = 1;
-    P->n_recv = nrecv;
     *a.counter = 0u;
   }
 }
@@ -996,11 +1010,12 @@ constexpr int UPD_UNROLL = 8;
 
 __device__ void commit_move(const DevTree& T, const Proposal& P);
 
-__global__ void __launch_bounds__(UPD_T) k_update(DevTree T, const double2* __restrict__ ptab, long ptab_per) {
+__global__ void __launch_bounds__(UPD_T) k_update(DevTree T, const double2* __restrict__ ptab, long ptab_per,
+                                                  bool force, int* host_err) {
   __shared__ Receiver rs[MAX_RECV];
   __shared__ int s_acc, s_nr;
   if (threadIdx.x == 0) {
-    s_acc = T.prop->accepted;
+    s_acc = force || T.prop->accepted;
     s_nr = T.prop->n_recv;
   }
   __syncthreads();
@@ -1011,7 +1026,9 @@ __global__ void __launch_bounds__(UPD_T) k_update(DevTree T, const double2* __re
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
     atomicAdd(&T.work[0], 1ull);
     atomicAdd(&T.work[1], 32ull * ((unsigned long long)T.Hw + (unsigned long long)nr * T.H));
+    if (force) T.prop->accepted = 1;
     commit_move(T, *T.prop);
+    if (host_err) *host_err = *T.err;
   }
   __syncthreads();
   Tables tt, to;
@@ -3211,7 +3228,7 @@ PotentialKernel potential_kernel(int np, int grp) {
 }
 
 // the shift kernel for a residual polynomial of np coefficients (3, 6, 9, 12 digits)
-using ShiftKernel = void (*)(DevTree, ShiftArgs);
+using ShiftKernel = void (*)(DevTree, ShiftArgs, const OneMove);
 ShiftKernel shift_kernel(int np) {
   switch (np) {
     case 7: return k_shift<7>;
@@ -3231,9 +3248,11 @@ size_t tables_smem(const DevTree& T, int lmax, int copies) {
 
 // ---------------------------------------------------------------------------
 void DmkTree::launch_shift(const int* d_idx, const double* d_disp, const double* d_u, double beta, int move, int mode,
-                           double* d_dE, int* d_acc) {
+                           double* d_dE, int* d_acc, long one_i, const double* one_d) {
   DevTree& D = dev_;
   const double pi = 3.14159265358979323846;
+  OneMove one{int(one_i), {0, 0, 0}};
+  if (one_d) std::copy(one_d, one_d + 3, one.d);
   ShiftArgs a{};
   a.idx = d_idx;
   a.disp = d_disp;
@@ -3251,9 +3270,10 @@ void DmkTree::launch_shift(const int* d_idx, const double* d_disp, const double*
   a.cur = use_cursor_ ? d_cursor_ : nullptr;
   a.ptab = ptab_;
   a.ptab_per = ptab_per_;
+  a.host_out = one_d ? slot_dev_ : nullptr;
   size_t smem = tables_smem(D, D.max_depth, 2);
   time_begin(0);
-  shift_kernel(D.n_poly)<<<unsigned(shift_grid_), SH_T, smem, st_>>>(D, a);
+  shift_kernel(D.n_poly)<<<unsigned(shift_grid_), SH_T, smem, st_>>>(D, a, one);
   PDMK_LAUNCH_CHECK();
   time_end(0);
 }
@@ -3285,7 +3305,7 @@ void DmkTree::ensure_shift_config() {
     int dev = 0, sms = 148;
     PDMK_CUDA(cudaGetDevice(&dev));
     PDMK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    shift_grid_ = 2 + sms;
+    shift_grid_ = 3 + sms;
     const size_t smem = tables_smem(D, D.max_depth, 2);
     raise_smem_limit(reinterpret_cast<const void*>(shift_kernel(D.n_poly)), smem);
   }
@@ -3323,17 +3343,18 @@ void DmkTree::build_mc_graph(int timed) {
   PDMK_CUDA(cudaGraphDestroy(g));
 }
 
-void DmkTree::launch_update() {
+void DmkTree::launch_update(bool force) {
   DevTree& D = dev_;
   const int levels = std::max(D.pw_hi - 1, 0);
   // rows: root, up to 2 x 28 receivers per expansion level, commit
   // x: one mode per thread; y: receiver ranges, enough for ~16 warps per SM
   const int gx = (std::max(D.H, D.Hw) + UPD_T - 1) / UPD_T;
-  const int gy = std::max(1, std::min(8, (16 * (shift_grid_ - 2) * 32 / UPD_T + gx - 1) / std::max(gx, 1)));
+  const int gy = std::max(1, std::min(8, (16 * (shift_grid_ - 3) * 32 / UPD_T + gx - 1) / std::max(gx, 1)));
   (void)levels;
   const dim3 grid{unsigned(gx), unsigned(gy), 1u};
   time_begin(1);
-  k_update<<<grid, UPD_T, 0, st_>>>(D, ptab_, ptab_per_);
+  k_update<<<grid, UPD_T, 0, st_>>>(D, ptab_, ptab_per_, force,
+                                      force && slot_ ? reinterpret_cast<int*>(slot_dev_ + 6) : nullptr);
   PDMK_LAUNCH_CHECK();
   time_end(1);
 }
@@ -3396,35 +3417,45 @@ void DmkTree::reset_work() { PDMK_CUDA(cudaMemsetAsync(dev_.work, 0, 3 * sizeof(
 
 double DmkTree::eval_shift_energy(long i, double dx, double dy, double dz, double* parts) {
   double disp[3] = {dx, dy, dz};
-  int ii = int(i);
-  PDMK_CUDA(cudaMemcpyAsync(d_one_idx_, &ii, sizeof(int), cudaMemcpyHostToDevice, st_));
-  PDMK_CUDA(cudaMemcpyAsync(d_one_disp_, disp, sizeof(disp), cudaMemcpyHostToDevice, st_));
-  launch_shift(d_one_idx_, d_one_disp_, nullptr, 0.0, 0, 0, nullptr, nullptr);
-  Proposal P;
-  PDMK_CUDA(cudaMemcpyAsync(&P, dev_.prop, sizeof(Proposal), cudaMemcpyDeviceToHost, st_));
-  PDMK_CUDA(cudaStreamSynchronize(st_));
-  if (parts)
-    for (int c = 0; c < 5; ++c) parts[c] = P.parts[c];
+  // the proposal goes with the launch and the result comes through mapped
+  // memory: the copies took 3 and 5 us of a trial's 46
+  if (!slot_tried_) {
+    slot_ = take_host_slot(&slot_dev_);
+    slot_tried_ = true;
+  }
+  launch_shift(nullptr, nullptr, nullptr, 0.0, 0, 0, nullptr, nullptr, i, disp);
+  double got[6];
+  if (slot_) {
+    PDMK_CUDA(cudaStreamSynchronize(st_));
+    std::copy(slot_, slot_ + 6, got);
+  } else {
+    Proposal P;
+    PDMK_CUDA(cudaMemcpyAsync(&P, dev_.prop, sizeof(Proposal), cudaMemcpyDeviceToHost, st_));
+    PDMK_CUDA(cudaStreamSynchronize(st_));
+    got[0] = P.dE;
+    std::copy(P.parts, P.parts + 5, got + 1);
+  }
+  if (parts) std::copy(got + 1, got + 6, parts);
   last_i_ = i;
   last_d_[0] = dx;
   last_d_[1] = dy;
   last_d_[2] = dz;
   last_valid_ = true;
-  return P.dE;
+  return got[0];
 }
 
-void DmkTree::update_shift(long i, double dx, double dy, double dz) {
+int DmkTree::update_shift(long i, double dx, double dy, double dz) {
   // the reference requires the same arguments as the preceding
   // eval_shift_energy (src/tree.cpp:471-489); recompute when they differ
   if (!(last_valid_ && last_i_ == i && last_d_[0] == dx && last_d_[1] == dy && last_d_[2] == dz))
     eval_shift_energy(i, dx, dy, dz, nullptr);
-  int one = 1;
-  PDMK_CUDA(cudaMemcpyAsync(&dev_.prop->accepted, &one, sizeof(int), cudaMemcpyHostToDevice, st_));
-  launch_update();
-  PDMK_CUDA(cudaStreamSynchronize(st_));
+  launch_update(true);
   last_valid_ = false;
   diff_cached_ = false;
   mark_moved();
+  if (!slot_) return check_device_error();
+  PDMK_CUDA(cudaStreamSynchronize(st_));
+  return *reinterpret_cast<const volatile int*>(slot_ + 6);
 }
 
 // The deferred-update list of a tree, its marks and the folded difference

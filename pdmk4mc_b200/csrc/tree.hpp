@@ -28,6 +28,12 @@ constexpr int PATH_LEN_MAX = MAX_LEVELS;
 cudaStream_t take_stream(int* device = nullptr);  // device: the current one
 void return_stream(int device, cudaStream_t s);
 
+// 64 bytes of mapped host memory that kernels write a single move's result to
+// (null when the process's 64 slots are taken: the caller copies instead), and
+// their return.
+double* take_host_slot(double** device_address);
+void return_host_slot(double* slot);
+
 struct PlanTotals;  // totals of the work and box lists (plan.hpp)
 
 // One proposed single-particle move and what the shift kernel found for it.
@@ -226,7 +232,7 @@ class DmkTree {
   double ewald_energy(double* parts = nullptr);
   // single move through the drop-in API: host scalars in, host scalar out
   double eval_shift_energy(long i, double dx, double dy, double dz, double* parts = nullptr);
-  void update_shift(long i, double dx, double dy, double dz);
+  int update_shift(long i, double dx, double dy, double dz);  // the device error word
   // sequential Metropolis over device-resident proposals; no host sync
   void mc_run_device(int n_moves, const int* d_idx, const double* d_disp, const double* d_u, double beta,
                      double* d_dE, int* d_acc);
@@ -282,8 +288,9 @@ class DmkTree {
   size_t partials_needed() const;
   int res_chunks() const;
   void launch_shift(const int* d_idx, const double* d_disp, const double* d_u, double beta, int move, int mode,
-                    double* d_dE, int* d_acc);
-  void launch_update();  // accept-and-update and membership commit, one launch
+                    double* d_dE, int* d_acc, long one_i = 0, const double* one_d = nullptr);  // d_idx null: one_i, one_d
+  // accept-and-update and membership commit, one launch; force: whatever the proposal's decision
+  void launch_update(bool force = false);
   void ensure_packed();
   bool out_defined_ = false, inc_defined_ = false;
   void ensure_rows(bool out, bool inc);  // rows read before a pass formed them are zero
@@ -427,14 +434,13 @@ class DmkTree {
   cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
   double2* ptab_ = nullptr;  // phase tables of the last proposal, both paths
   long ptab_per_ = 0;
+  double* slot_ = nullptr;  // mapped host memory for the results of single moves, and its device address
+  double* slot_dev_ = nullptr;
+  bool slot_tried_ = false;
   // host-side copy of the last proposal arguments (for update_shift)
   long last_i_ = -1;
   double last_d_[3] = {0, 0, 0};
   bool last_valid_ = false;
-  // arguments of the single-move API in device memory
-  int* d_one_idx_ = nullptr;
-  double* d_one_disp_ = nullptr;
-  double* d_one_u_ = nullptr;
 };
 
 }  // namespace pdmk
