@@ -1,6 +1,7 @@
 // Exclusive scan (one launch up to 4096 items, else reduce-then-scan in three
-// launches) and stable LSD radix sort with 8-bit digits (tile histogram ->
-// digit-major scan -> stable warp-multisplit scatter). Used to bin particles
+// launches) and stable LSD radix sort with 8-bit digits (one histogram launch
+// for all digits, then one launch a digit: stable warp-multisplit ranks, each
+// tile's place from its predecessors' published counts). Used to bin particles
 // by Morton key.
 #include <algorithm>
 
@@ -113,27 +114,50 @@ constexpr int RS_ITEMS = 8;     // items per thread
 constexpr int RS_TILE = RS_T * RS_ITEMS;
 constexpr int RS_WARPS = RS_T / 32;
 
-__global__ void k_radix_hist(const uint64_t* keys, long n, int shift, int ntiles, int* hist) {
-  __shared__ int h[256];
-  for (int i = threadIdx.x; i < 256; i += RS_T) h[i] = 0;
+// counts of every digit of the passes first .. 7 into total[pass][256]
+__global__ void __launch_bounds__(RS_T) k_radix_totals(const uint64_t* __restrict__ keys, long n, int first, int* total) {
+  __shared__ int h[8][256];
+  for (int i = threadIdx.x; i < 8 * 256; i += RS_T) (&h[0][0])[i] = 0;
   __syncthreads();
-  long base = long(blockIdx.x) * RS_TILE;
-  for (int k = 0; k < RS_ITEMS; ++k) {
-    long i = base + k * RS_T + threadIdx.x;
-    if (i < n) atomicAdd(&h[int((keys[i] >> shift) & 0xff)], 1);
+  for (long i = long(blockIdx.x) * RS_T + threadIdx.x; i < n; i += long(gridDim.x) * RS_T) {
+    const uint64_t k = keys[i];
+    for (int p = first; p < 8; ++p) atomicAdd(&h[p][int((k >> (8 * p)) & 0xff)], 1);
   }
   __syncthreads();
-  for (int d = threadIdx.x; d < 256; d += RS_T) hist[long(d) * ntiles + blockIdx.x] = h[d];
+  for (int i = threadIdx.x; i < 8 * 256; i += RS_T) {
+    const int v = (&h[0][0])[i];
+    if (v) atomicAdd(total + i, v);
+  }
 }
 
-__global__ void k_radix_scatter(const uint64_t* kin, const int* vin, uint64_t* kout, int* vout, long n, int shift,
-                                int ntiles, const int* offs) {
+// One digit in one launch. A tile publishes its digit counts, then adds up its
+// predecessors': from the next one back, eight loads at a time, to the first
+// that has published its sum with all before it. Tiles are numbered by a
+// ticket, so a tile only waits for blocks that already run and that wait for
+// earlier ones alone; the wait is bounded all the same, and a tile that gives
+// up counts the keys before it itself. What bounds a pass is the scattered
+// write; the histogram and three scan launches of a pass that this replaces
+// took as long again (N = 1e5: 15 of 27 us).
+constexpr unsigned RS_SUM = 1u << 30, RS_ALL = 2u << 30, RS_MASK = RS_SUM - 1;
+constexpr int RS_LOOK = 8;
+constexpr int RS_SPIN = 1 << 20;
+
+__global__ void __launch_bounds__(RS_T)
+    k_radix_pass(const uint64_t* kin, const int* vin, uint64_t* kout, int* vout, long n, int shift, const int* total,
+                 unsigned* state, int* ticket) {
   __shared__ int wh[RS_WARPS][256];
+  __shared__ int base[256];
+  __shared__ int s_tile, s_fail, wsum[RS_WARPS];
+  if (threadIdx.x == 0) {
+    s_tile = atomicAdd(ticket, 1);
+    s_fail = 0;
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int i = threadIdx.x; i < RS_WARPS * 256; i += RS_T) (&wh[0][0])[i] = 0;
   __syncthreads();
   // warp w owns tile elements [w*256, w*256+256), visited in rounds of 32
-  const long wbase = long(blockIdx.x) * RS_TILE + long(warp) * 32 * RS_ITEMS;
+  const int tile = s_tile;
+  const long wbase = long(tile) * RS_TILE + long(warp) * 32 * RS_ITEMS;
   uint64_t key[RS_ITEMS];
   int val[RS_ITEMS], dig[RS_ITEMS], pos[RS_ITEMS];
   const unsigned lt = (1u << lane) - 1u;
@@ -154,21 +178,65 @@ __global__ void k_radix_scatter(const uint64_t* kin, const int* vin, uint64_t* k
     __syncwarp();
   }
   __syncthreads();
-  // per digit, exclusive prefix over warps (warp order = element order)
-  for (int d = threadIdx.x; d < 256; d += RS_T) {
-    int s = 0;
-    for (int w = 0; w < RS_WARPS; ++w) {
-      int c = wh[w][d];
-      wh[w][d] = s;
-      s += c;
-    }
+  static_assert(RS_T == 256, "a thread per digit");
+  const int d = threadIdx.x;
+  // exclusive prefix over warps (warp order = element order), the tile's count
+  int cnt = 0;
+  for (int w = 0; w < RS_WARPS; ++w) {
+    const int c = wh[w][d];
+    wh[w][d] = cnt;
+    cnt += c;
   }
+  volatile unsigned* st = state;
+  st[long(tile) * 256 + d] = (tile == 0 ? RS_ALL : RS_SUM) | unsigned(cnt);
+  // keys of smaller digits: exclusive sum of the totals
+  int x = total[d];
+  const int mine = x;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) wsum[warp] = x;
+  __syncthreads();
+  int below = x - mine;
+  for (int w = 0; w < warp; ++w) below += wsum[w];
+  int before = 0;
+  if (tile > 0) {
+    int t = tile - 1, spins = 0;
+    bool found = false;
+    while (!found && spins < RS_SPIN) {
+      unsigned v[RS_LOOK];
+#pragma unroll
+      for (int k = 0; k < RS_LOOK; ++k) v[k] = t - k >= 0 ? unsigned(st[long(t - k) * 256 + d]) : unsigned(RS_ALL);
+      int used = 0;
+#pragma unroll
+      for (int k = 0; k < RS_LOOK; ++k)
+        if (!found && used == k && (v[k] & ~RS_MASK)) {
+          before += int(v[k] & RS_MASK);
+          found = (v[k] & RS_ALL) != 0;
+          ++used;
+        }
+      t -= used;
+      spins = used ? 0 : spins + 1;
+    }
+    if (!found) s_fail = 1;
+  }
+  __syncthreads();
+  if (s_fail) {
+    base[d] = 0;
+    __syncthreads();
+    for (long i = threadIdx.x; i < long(tile) * RS_TILE; i += RS_T) atomicAdd(&base[int((kin[i] >> shift) & 0xff)], 1);
+    __syncthreads();
+    before = base[d];
+  }
+  if (tile > 0) st[long(tile) * 256 + d] = RS_ALL | unsigned(before + cnt);
+  base[d] = below + before;
   __syncthreads();
   for (int k = 0; k < RS_ITEMS; ++k) {
     long i = wbase + k * 32 + lane;
     if (i < n) {
-      int d = dig[k];
-      long dst = long(offs[long(d) * ntiles + blockIdx.x]) + wh[warp][d] + pos[k];
+      const int dst = base[dig[k]] + wh[warp][dig[k]] + pos[k];
       kout[dst] = key[k];
       vout[dst] = val[k];
     }
@@ -236,13 +304,14 @@ void exclusive_scan(const int* in, int* out, long n, void* scratch, cudaStream_t
   PDMK_LAUNCH_CHECK();
 }
 
+// the totals and tickets of the passes, then every tile's published counts
+static size_t radix_state_bytes(long n) {
+  const long ntiles = (n + RS_TILE - 1) / RS_TILE;
+  return sizeof(int) * (8 * 256 + 64) + size_t(8 * ntiles) * 256 * sizeof(unsigned);
+}
+
 size_t radix_sort_scratch_bytes(long n) {
-  long ntiles = (n + RS_TILE - 1) / RS_TILE;
-  long hist = 256 * ntiles;
-  size_t b = size_t(n) * (sizeof(uint64_t) + sizeof(int)) + 256;
-  b += size_t(hist) * sizeof(int) + 256;
-  b += scan_scratch_bytes(hist);
-  return b;
+  return size_t(n) * (sizeof(uint64_t) + sizeof(int)) + 768 + radix_state_bytes(n);
 }
 
 void radix_sort_pairs(uint64_t* keys, int* vals, long n, int first, void* scratch, cudaStream_t st) {
@@ -260,17 +329,17 @@ void radix_sort_pairs(uint64_t* keys, int* vals, long n, int first, void* scratc
   p += ((size_t(n) * sizeof(uint64_t) + 255) / 256) * 256;
   int* v2 = reinterpret_cast<int*>(p);
   p += ((size_t(n) * sizeof(int) + 255) / 256) * 256;
-  int* hist = reinterpret_cast<int*>(p);
-  p += ((size_t(256 * ntiles) * sizeof(int) + 255) / 256) * 256;
-  void* sscr = p;
+  int* total = reinterpret_cast<int*>(p);
+  int* tickets = total + 8 * 256;
+  unsigned* state = reinterpret_cast<unsigned*>(tickets + 64);
+  PDMK_CUDA(cudaMemsetAsync(p, 0, radix_state_bytes(n), st));
+  k_radix_totals<<<unsigned(std::min<long>(ntiles, 592)), RS_T, 0, st>>>(keys, n, first, total);
+  PDMK_LAUNCH_CHECK();
   uint64_t *ka = keys, *kb = k2;
   int *va = vals, *vb = v2;
   for (int pass = first; pass < 8; ++pass) {
-    int shift = 8 * pass;
-    k_radix_hist<<<unsigned(ntiles), RS_T, 0, st>>>(ka, n, shift, int(ntiles), hist);
-    PDMK_LAUNCH_CHECK();
-    exclusive_scan(hist, hist, 256 * ntiles, sscr, st);
-    k_radix_scatter<<<unsigned(ntiles), RS_T, 0, st>>>(ka, va, kb, vb, n, shift, int(ntiles), hist);
+    k_radix_pass<<<unsigned(ntiles), RS_T, 0, st>>>(ka, va, kb, vb, n, 8 * pass, total + 256 * pass,
+                                                    state + size_t(pass) * ntiles * 256, tickets + pass);
     PDMK_LAUNCH_CHECK();
     std::swap(ka, kb);
     std::swap(va, vb);

@@ -39,3 +39,28 @@ def test_build_matches_the_oracle(n, npl, kind):
         np.testing.assert_array_equal(g.sorted_order(), o.sorted_order())
     finally:
         g.close()
+
+
+@pytest.mark.parametrize("n", [4097, 6144, 20481, 300001])
+@pytest.mark.parametrize("kind", ["uniform", "line", "equal"])
+def test_large_sorts_are_stable(n, kind):
+    # tiles of 2048 keys: whole, one over, many; one digit value for all keys of a pass
+    L = 5.0
+    rng = np.random.default_rng(n)
+    r = rng.uniform(0, L, (n, 3))
+    if kind == "line":
+        r[:, 1:] = 1.25
+    if kind == "equal":
+        r = r[rng.integers(0, 7, n)]
+    q = np.where(np.arange(n) % 2 == 0, 1.0, -1.0)
+    # leaf sizes that keep the trees shallow: the order is what is tested
+    g = P.HPDMKPtTree(P.HPDMKParams(n_per_leaf=n, digits=3, L=L, init=P.DIRECT), r.reshape(-1), q)
+    try:
+        cell = np.minimum(np.floor(r / L * 2.0 ** 21), 2 ** 21 - 1).astype(np.uint64)
+        key = np.zeros(n, np.uint64)
+        for b in range(21):
+            for a in range(3):
+                key |= ((cell[:, a] >> np.uint64(b)) & np.uint64(1)) << np.uint64(3 * b + a)
+        np.testing.assert_array_equal(g.sorted_order(), np.argsort(key, kind="stable"))
+    finally:
+        g.close()
