@@ -49,12 +49,6 @@ void put_small(void* dst, const void* src, size_t bytes, cudaStream_t st) {
   PDMK_LAUNCH_CHECK();
 }
 
-__global__ void k_root(uint64_t* list, int* n_refined, uint32_t* bitmap) {
-  *list = 0;
-  *n_refined = 1;
-  *bitmap = 1u;
-}
-
 // ---------------------------------------------------------------------------
 __global__ void k_keys(const double* r, long n, double L, uint64_t* key, int* val) {
   long i = long(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -110,6 +104,36 @@ struct Bitmaps {
 __device__ inline int cell_rank(const Bitmaps& B, int level, uint64_t cell) {
   uint32_t w = B.bm[level][cell >> 5];
   return B.wprefix[level][cell >> 5] + __popc(w & ((1u << (cell & 31)) - 1u));
+}
+
+// The refined cells of levels 0 .. deepest in one launch, from the sorted keys:
+// the particle i that is the first of its cell at level l finds the cell
+// refined when particle i + n_per_leaf still lies in it (a refined cell's
+// ancestors hold as many, so no level waits for the one above; levels 0 and 1
+// are refined throughout). Level by level, with a list of cells and two
+// searches a cell, the same took six launches and 34 us at N = 1e3, 91 us at
+// 1e6; now 5 and 9. The cells of the deepest level go to `list` for the levels
+// below it.
+__global__ void k_refine_shallow(const uint64_t* __restrict__ keys, long n, int n_per_leaf, Bitmaps B, int deepest,
+                                 uint64_t* list, int list_cap, int* out_n) {
+  const long i = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i == 0) {
+    B.bm[0][0] = 1u;
+    B.bm[1][0] = 0xffu;
+    out_n[0] = 1;
+    out_n[1] = 8;
+  }
+  if (i >= n || n - i <= n_per_leaf) return;
+  // levels down to which two keys share their cells
+  auto shared = [](uint64_t a, uint64_t b) { return a == b ? KEY_BITS : KEY_BITS - 1 - (63 - __clzll(a ^ b)) / 3; };
+  const uint64_t k = keys[i];
+  const int last = min(shared(k, keys[i + n_per_leaf]), deepest);
+  for (int l = max(2, i == 0 ? 0 : shared(k, keys[i - 1]) + 1); l <= last; ++l) {
+    const uint64_t cell = k >> (3 * (KEY_BITS - l));
+    bit_set(B.bm[l], cell);
+    const int at = atomicAdd(out_n + l, 1);
+    if (l == deepest && at < list_cap) list[at] = cell;
+  }
 }
 
 // candidates at `level` are the 8 children of each refined cell of the level above
@@ -756,11 +780,8 @@ void DmkTree::build(const double* r_in, const double* q_in, bool on_device) {
       B.bm[l] = words;
       words += nwords[l];
     }
-    // root: refined (all nodes above level 2 are refined), the first list's only cell
-    k_root<<<1, 1, 0, st_>>>(lists[0], d_lvl, B.bm[0]);
-    PDMK_LAUNCH_CHECK();
     auto refine = [&](int l, unsigned grid) {
-      if (l > kEager && l < MAX_LEVEL) {
+      if (l < MAX_LEVEL) {
         B.bm[l] = static_cast<uint32_t*>(alloc(size_t(nwords[l]) * 4));
         PDMK_CUDA(cudaMemsetAsync(B.bm[l], 0, size_t(nwords[l]) * 4, st_));
       }
@@ -768,9 +789,10 @@ void DmkTree::build(const double* r_in, const double* q_in, bool on_device) {
                                              l < MAX_LEVEL ? B.bm[l] : nullptr, lists[l & 1], d_lvl + l);
       PDMK_LAUNCH_CHECK();
     };
-    // the shallow levels (bitmaps of at most 32 KB) go back to back with one
+    // the shallow levels (bitmaps of at most 32 KB) in one launch with one
     // read-back; deeper trees continue level by level
-    for (int l = 1; l <= kEager; ++l) refine(l, grid_for(std::min(list_cap, 1L << (3 * l))));
+    k_refine_shallow<<<grid_for(n), TPB, 0, st_>>>(keys, n, n_per_leaf_, B, kEager, lists[kEager & 1], int(list_cap), d_lvl);
+    PDMK_LAUNCH_CHECK();
     int cnt[kBadWord + 1] = {0};
     PDMK_CUDA(cudaMemcpyAsync(cnt, d_lvl, sizeof(cnt), cudaMemcpyDeviceToHost, st_));
     PDMK_CUDA(cudaStreamSynchronize(st_));
