@@ -243,39 +243,80 @@ __global__ void __launch_bounds__(RS_T)
   }
 }
 
-// Up to SMALL_SORT pairs in one block: a bitonic sort by (key, value) in shared
-// memory, which is the stable order when the values come in ascending order
-// or the keys are distinct. What bounds it is one launch and about 80 barriers
-// (8 us at 4096 pairs), where the passes below take 24 launches of 4 to 9 us.
+// Up to SMALL_SORT pairs in one block: a bitonic sort by (key, value), which is
+// the stable order when the values come in ascending order or the keys are
+// distinct. A thread holds R pairs, block-strided: partners less than 32 apart
+// meet by shuffle, up to the block's width through shared memory (one barrier
+// a step, two buffers in turn), beyond it in the thread's registers. What
+// bounds it is the chain of 55 to 78 steps (all through shared memory it took
+// 13 us for 1024 pairs, 54 for 4096; now 8 and 27); the passes above would
+// take nine launches.
 constexpr int SMALL_SORT = 4096;
 
-__global__ void __launch_bounds__(1024) k_sort_small(uint64_t* keys, int* vals, int n, int pow2) {
-  __shared__ uint64_t sk[SMALL_SORT];
-  __shared__ int sv[SMALL_SORT];
-  for (int i = threadIdx.x; i < pow2; i += blockDim.x) {
-    sk[i] = i < n ? keys[i] : ~uint64_t(0);
-    sv[i] = i < n ? vals[i] : 0x7fffffff;
+template <int R>
+__global__ void __launch_bounds__(1024) k_sort_small(uint64_t* keys, int* vals, int n) {
+  extern __shared__ uint64_t sm_sort[];  // two buffers of blockDim keys, then of values
+  const int T = blockDim.x, t = threadIdx.x;
+  uint64_t* sk = sm_sort;
+  int* sv = reinterpret_cast<int*>(sm_sort + 2 * T);
+  uint64_t key[R];
+  int val[R];
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int e = t + i * T;
+    key[i] = e < n ? keys[e] : ~uint64_t(0);
+    val[i] = e < n ? vals[e] : 0x7fffffff;
   }
-  for (int k = 2; k <= pow2; k <<= 1)
+  // the smaller or the larger of a pair and its partner
+  auto meet = [](uint64_t& k, int& v, uint64_t pk, int pv, bool small) {
+    const bool above = k > pk || (k == pk && v > pv);
+    if (above == small) k = pk, v = pv;
+  };
+  int buf = 0;
+  for (int k = 2; k <= R * T; k <<= 1)
     for (int j = k >> 1; j > 0; j >>= 1) {
-      __syncthreads();
-      for (int t = threadIdx.x; t < pow2 / 2; t += blockDim.x) {
-        const int a = ((t & ~(j - 1)) << 1) | (t & (j - 1)), b = a | j;
-        const uint64_t ka = sk[a], kb = sk[b];
-        const int va = sv[a], vb = sv[b];
-        const bool above = ka > kb || (ka == kb && va > vb);
-        if (above == ((a & k) == 0)) {
-          sk[a] = kb;
-          sk[b] = ka;
-          sv[a] = vb;
-          sv[b] = va;
+      if (R > 1 && j >= T) {
+        const int x = j / T;
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+#pragma unroll
+          for (int h = 0; h < R; ++h)
+            if (h == (i ^ x) && i < h) {
+              const bool up = ((t + i * T) & k) == 0;
+              const uint64_t a = key[i];
+              const int av = val[i];
+              meet(key[i], val[i], key[h], val[h], up);
+              meet(key[h], val[h], a, av, !up);
+            }
+      } else {
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          const int e = t + i * T;
+          const bool small = ((e & j) == 0) == ((e & k) == 0);
+          uint64_t pk;
+          int pv;
+          if (j < 32) {
+            pk = __shfl_xor_sync(0xffffffffu, key[i], j);
+            pv = __shfl_xor_sync(0xffffffffu, val[i], j);
+          } else {
+            sk[buf * T + t] = key[i];
+            sv[buf * T + t] = val[i];
+            __syncthreads();
+            pk = sk[buf * T + (t ^ j)];
+            pv = sv[buf * T + (t ^ j)];
+            buf ^= 1;
+          }
+          meet(key[i], val[i], pk, pv, small);
         }
       }
     }
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    keys[i] = sk[i];
-    vals[i] = sv[i];
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int e = t + i * T;
+    if (e < n) {
+      keys[e] = key[i];
+      vals[e] = val[i];
+    }
   }
 }
 
@@ -317,9 +358,11 @@ size_t radix_sort_scratch_bytes(long n) {
 void radix_sort_pairs(uint64_t* keys, int* vals, long n, int first, void* scratch, cudaStream_t st) {
   if (n <= 1) return;
   if (n <= SMALL_SORT) {
-    int pow2 = 2;
+    int pow2 = 32;
     while (pow2 < n) pow2 <<= 1;
-    k_sort_small<<<1, unsigned(std::min(1024, std::max(32, pow2 / 2))), 0, st>>>(keys, vals, int(n), pow2);
+    const int T = std::min(1024, pow2);
+    auto kern = pow2 <= 1024 ? k_sort_small<1> : pow2 == 2048 ? k_sort_small<2> : k_sort_small<4>;
+    kern<<<1, unsigned(T), size_t(2 * T) * (sizeof(uint64_t) + sizeof(int)), st>>>(keys, vals, int(n));
     PDMK_LAUNCH_CHECK();
     return;
   }
