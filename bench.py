@@ -473,21 +473,21 @@ def run_b200(args, rank, ws):
     M = W["moves_per_step"]
     steps_time = sum(float(np.sum(a.t_moves) + np.sum(a.t_energy) + np.sum(a.t_cand)) for a in arms.values())
 
-    # roofline of the dominant kernel of the step: k_mc (persistent
-    # Metropolis) of the mixed arm, HBM bound; algorithmic bytes from the
-    # device work counters (dE reads + update read-modify-writes) over its
-    # CUDA-event duration on the tree's stream
+    # roofline of the move phase of the mixed arm (k_mc_long, then the row
+    # updates of its list: k_flush_outgoing and the touched k_incoming_cube);
+    # algorithmic bytes from the device work counters (dE reads + rows written)
+    # over the CUDA-event duration of each list's launches on the tree's stream
     hbm, peak_kind = peaks()
     mc_ms, mc_n = timing["mc"]
     bytes_per_launch = (mixed.work[1] + mixed.work[2]) / max(mc_n, 1)
     achieved = bytes_per_launch / (mc_ms / mc_n / 1e3) / 1e9 if mc_n else None
     traffic = None
-    # DRAM bytes per move from the ncu capture summarised in the k_mc profile
-    tpath = os.path.join(ROOT, "profiles", "k_mc_uniform_n1e5_d9.md")
+    # DRAM bytes per move from the ncu capture summarised in the k_mc_long profile
+    tpath = os.path.join(ROOT, "profiles", "k_mc_long_uniform_n1e5_d9.md")
     if os.path.exists(tpath):
         mt = re.search(r"^dram_bytes_per_move = (\d+)", open(tpath).read(), re.M)
         if mt:
-            traffic = int(mt.group(1)) * M
+            traffic = int(mt.group(1)) * M * args.steps / max(mc_n, 1)
 
     # end to end through the C-ABI with host buffers, mixed path: the moves
     # (hpdmk_mc_run: indices, displacements and uniforms in, shifts and
@@ -591,11 +591,10 @@ def run_b200(args, rank, ws):
             "replicas": replicas,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                          "frac": (achieved / hbm) if achieved else None, "traffic": traffic,
-                         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of a 256-move k_mc "
-                                           "launch on this workload, scaled by moves per launch "
-                                           "(profiles/k_mc_uniform_n1e5_d9.md)" if traffic else None,
-                         "kernel": f"k_mc (persistent Metropolis, mixed arm: dE reads + accept-and-update "
-                                   f"read-modify-writes, {M} moves per launch)",
+                         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per move, scaled by moves per "
+                                           "list (profiles/k_mc_long_uniform_n1e5_d9.md)" if traffic else None,
+                         "kernel": f"k_mc_long with its row updates (mixed arm: dE reads, then the touched rows once per "
+                                   f"list of moves; {M} moves per step)",
                          "timed_launches": int(mc_n), "peak_source": peak_kind},
             "cpu_baseline": cpu,
             "e2e": {"value": ws * M * args.steps / te2e, "unit": "moves/s", "h2d_bytes_per_step": M * (8 + 24 + 8),

@@ -146,14 +146,14 @@ int hpdmk_eval_shift_energy_batch(hpdmk_tree tree, int m, const long *i, const d
 
 /* As hpdmk_eval_shift_energy_batch with device-resident int32 indices d_i[m],
  * displacements d_d[3m] and output d_dE[m], enqueued on the tree's stream
- * without a host synchronisation (one launch, one thread block per candidate). */
+ * without a host synchronisation (a thread block per candidate; from 1184
+ * candidates on, a block per two that share boxes). */
 int hpdmk_eval_shift_energy_batch_device(hpdmk_tree tree, int m, const int *d_i, const double *d_d, double *d_dE);
 
-/* No reference counterpart. The same single launch as
- * hpdmk_eval_shift_energy_batch (one thread block per candidate, phase tables
- * in shared memory), so the same results bit for bit, but the call allocates
+/* No reference counterpart. The same launches as
+ * hpdmk_eval_shift_energy_batch (phase tables in shared memory), so the same results bit for bit, but the call allocates
  * no device memory: the candidates' indices and displacements and their
- * energy shifts are staged through one fixed static device array (144 KB per
+ * energy shifts are staged through one fixed static device array (160 KB per
  * device, its address looked up once per device). For callers that may not
  * allocate device memory once the tree exists: a process that budgets its
  * device memory up front, or one whose memory is handed out by another
@@ -207,7 +207,7 @@ int hpdmk_mc_run_device(hpdmk_tree tree, int n, const int *d_i, const double *d_
  * particles and of the periodic images of all particles including its own,
  * so that E = 1/2 sum_i q_i phi_i; field[3c..3c+2] = -grad phi there (may be
  * NULL; the force on the particle is its charge times the field). The same
- * expansions and near field as an energy shift; one launch for all m. */
+ * expansions and near field as an energy shift; one batch for all m. */
 int hpdmk_eval_potential(hpdmk_tree tree, int m, const long *i, double *phi, double *field);
 
 /* Tree maintenance (no counterpart in the reference, which keeps the tree

@@ -1177,18 +1177,23 @@ void DmkTree::form_outgoing_pw() {
     PDMK_CUDA(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
   }
   // A small system would leave most SMs idle behind a few blocks that each
-  // walk all particles: its items are cut until about two waves of blocks are
-  // there (not below 64 particles, where the partials' sum costs more).
-  auto fill_split = [&](int split, long particles, int tiles, int resident) {
-    const long want = (2L * resident + tiles - 1) / tiles;  // items for two waves
-    return int(std::min<long>(split, std::max<long>(64, (particles + want - 1) / std::max<long>(want, 1))));
+  // walk all particles: its items are cut until they give one wave of blocks
+  // (the root, which runs beside the boxes: half a wave), not below 64
+  // particles. Finer cuts cost more than they fill: a partial row's way to
+  // memory and back is worth 45 particles. Outgoing pass in us, uncut / half and
+  // one wave / two and two waves: N = 1e3 (6 digits) 172 / 63 / 61, 5e3 (9
+  // digits) 170 / 118 / 186, 2e4 223 / 217 / 321, 5e4 437 / 441 / 560, 128e3 (3
+  // digits) 218 / 172 / 160.
+  auto fill_split = [&](int split, long particles, int tiles, int blocks) {
+    const long want = std::max(1, (blocks + tiles - 1) / tiles);  // items
+    return int(std::min<long>(split, std::max<long>(64, (particles + want - 1) / want)));
   };
   auto shape = [&](int nk, int ksplit) {
     return PlanShape{ksplit, mixed ? mixed_chunk(nk) : 1, mixed ? long(mixed_table_bytes(nk)) : 0L};
   };
   const long pw_levels = std::max(0, D.pw_hi - D.pw_lo + 1);
   const PlanShape root_shape = shape(
-      D.n_window, mixed ? tune_.ksplit_root : fill_split(tune_.ksplit_root, n_all, nudft_tiles(D.n_window), 296));
+      D.n_window, mixed ? tune_.ksplit_root : fill_split(tune_.ksplit_root, n_all, nudft_tiles(D.n_window), 148));
   const PlanShape box_shape = shape(
       D.n_diff, mixed ? tune_.ksplit : fill_split(tune_.ksplit, pw_levels * n_all, nudft_tiles(D.n_diff), 296));
 
@@ -1291,7 +1296,7 @@ void DmkTree::run_incoming(bool write_inc) {
   k_box_q2<<<unsigned(n_nonleaf_), TPB, 0, st_>>>(D, d_nonleaf_, q2);
   PDMK_LAUNCH_CHECK();
   if (write_inc) {
-    // about inc_waves resident waves of blocks (two per SM), each walking a
+    // about inc_waves waves of blocks (counted at two per SM), each walking a
     // strided set of tiles
     const int slots = inc_slots();
     inc_defined_ = true;  // the non-leaf boxes' rows; a leaf's row is read by nothing

@@ -45,18 +45,16 @@
 //     into the tensor core's shared-memory layout, and the block (B slices,
 //     ey and ez factors) goes to HBM with one bulk copy. Every M tile of the
 //     box reads these once-formed tables.
-//   - k_pw_mixed, one CTA per 128-row M tile of a box (or split-K chunk): a
-//     control warp brings each chunk's table block into shared memory with a
-//     bulk copy (three or four chunks in flight) and issues the MMAs, A from
-//     tensor memory and B from shared memory; the consumer warps form
-//     A = ez ey in FP64, one thread per output row (kz, ky) and group of 8
-//     particles, slice it and store the slices into tensor memory
-//     (tcgen05.st), which keeps A's traffic off shared memory; the A stages
-//     are double-buffered, so the tensor core works on chunk c while the
-//     consumers build chunk c + 1; the
-//     epilogue reads the accumulators (tcgen05.ld), combines them in FP64,
-//     stages the rows in shared memory and writes them with one bulk copy
-//     into the box's expansion row range, which is contiguous in HBM.
+//   - k_pw_mixed, persistent, over the 128-row M tiles of the boxes (and
+//     split-K chunks): a load warp brings each chunk's table block into shared
+//     memory with bulk copies (B, ey and the ez planes of the tile's rows), an
+//     MMA warp issues the products, A from tensor memory and B from shared
+//     memory; two groups of consumer warps form every other chunk's A = ez ey
+//     in FP64, a thread per output row (kz, ky) and group of 8 particles,
+//     slice it and store the slices into tensor memory (tcgen05.st), which
+//     keeps A's traffic off shared memory; then they read the accumulators
+//     (tcgen05.ld), combine them in FP64 and store the rows, 64 contiguous
+//     bytes a row at a time.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -134,7 +132,7 @@ struct MixShape {
   static constexpr int KGT = KB / 16 / 2;  // 16-byte K groups (8 particles) of a chunk per consumer thread
   static constexpr int THREADS = CTHREADS + 64;
   static constexpr int TTHREADS = 6 * KCP;       // table kernel: one thread per (particle, axis, half)
-  static constexpr int COORD_BOX = KCP + 2;      // TMA box along the slots: even start, one spare each side
+  static constexpr int COORD_BOX = KCP + 2;      // TMA box along the particles: even start, one spare each side
   static constexpr int COORD_BYTES = 4 * COORD_BOX * 8;
   // TMEM: accumulators at columns [0, NACC NPAD), A stage s slice t at
   // columns A_COL0 + s KB + t KB / 4 (lane = row)
@@ -237,8 +235,7 @@ __device__ __forceinline__ double2 root6_d(int m) {
   }
 }
 
-// sin and cos of th, |th| <= pi (slots hold particles inside their box, or
-// the leaf centre when empty, so th = dk (x - c) stays in range: |th| <= pi / 3
+// sin and cos of th, |th| <= pi (particles lie inside their box, so th = dk (x - c) stays in range: |th| <= pi / 3
 // at the difference levels, <= pi at the root): the Taylor series of sin and
 // cos at h = th / 2 (|h| <= pi / 2; the first omitted terms are below 1e-19)
 // as two Horner chains in h^2, then the double-angle formulas
@@ -728,7 +725,7 @@ __global__ void __launch_bounds__(MixShape<NK>::THREADS, 1)
   if (warp == 0) tc::tmem_dealloc(tmem, S::TCOLS);
 }
 
-// max |q| over the slots (the fixed-point scale of A): a grid-strided block
+// max |q| over the particles (the fixed-point scale of A): a grid-strided block
 // maximum, then an atomic maximum on the bit patterns, whose integer order
 // is the numeric order for non-negative doubles (*out must start at zero;
 // the maximum does not depend on the order of the arrivals)

@@ -14,8 +14,8 @@ int mixed_pairs(int nk);
 int mixed_chunk(int nk);
 // bytes of one chunk's table block (a multiple of 16)
 int mixed_table_bytes(int nk);
-// 2-D tensor map over the slot arrays x, y, z, q (stride slot_capacity, which
-// must be even), in boxes of kcp + 2 slots
+// 2-D tensor map over the particle rows x, y, z, q (stride slot_capacity, which
+// must be even), in boxes of kcp + 2 particles
 void make_coord_map(CUtensorMap* map, const double* sx, int slot_capacity, int kcp);
 // max |q| over n charges into *out (one block)
 void launch_absmax(const double* sq, int n, double* out, cudaStream_t st);

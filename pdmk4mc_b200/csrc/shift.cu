@@ -6,9 +6,9 @@
 // (src/tree.cpp:204-236), form_outgoing_pw_single (src/planewave.cpp:157-181)
 // and update_shift (src/tree.cpp:447-597).
 //
-// One trial move runs as: k_shift (grid-wide partial sums; the last block
-// finishes dE and the Metropolis test, lists the expansion vectors an
-// accepted move changes and writes the Proposal record), then k_update (one
+// One trial move runs as: k_shift (grid-wide partial sums, and one block that
+// lists the expansion vectors an accepted move changes; the last block finishes
+// dE and the Metropolis test and writes the Proposal record), then k_update (one
 // read-modify-write per touched vector, target and origin contributions
 // merged; block 0 also commits the particle membership). Both kernels read
 // the Proposal record, so the sequence is stream-ordered and can be captured
@@ -2809,7 +2809,10 @@ __device__ void batch_block_sum(double (&v)[N], double (*sm)[BG_W]) {
 // fill the SMs, else one particle a block. (Groups of 4 read a third less, but their
 // columns leave room for one block per SM: 1.43 against 1.12 ms for 4096 candidates.)
 constexpr int BG_GROUP = 2;
-constexpr int kGroupMin = 4 * 148 * 2;  // two groups per SM
+// two groups of two per SM and residency; in pairs / one by one, us (N = 1e6, 9
+// digits, host arrays): candidates 438 / 394 for 888, 502 / 508 for 1184, 634 /
+// 679 for 1776; potentials 330 / 336, 353 / 414, 478 / 583
+constexpr int kGroupMin = 4 * 148 * 2;
 
 // order[]: the particles idx[0 .. m) by the level-4 cell of their positions (one
 // block; the order within a cell is free, no result depends on it)
@@ -3547,12 +3550,15 @@ void DmkTree::mc_run_persistent(int n_moves, const int* d_idx, const double* d_d
 
 // The same for a sequence long enough to defer its row updates (k_mc_long);
 // false when it is not. The passes that bring the rows up to date cost with the
-// number of rows, an update move by move with the number of moves.
+// number of rows, an update move by move with the number of moves. Deferred /
+// move by move, us a call (9 digits): 64 rows (N = 2e4) 221 / 256 for 8 moves,
+// 276 / 420 for 16; 576 rows (1e5) 498 / 433 for 16, 628 / 822 for 32; 4672
+// rows (1e6) 1524 / 1114 for 32, 2052 / 2152 for 64, 2903 / 4847 for 146.
 bool DmkTree::mc_run_long(int n_moves, const int* d_idx, const double* d_disp, const double* d_u, double beta, double* d_dE,
                           int* d_acc) {
   DevTree& D = dev_;
   const int n_pw = D.pw_hi >= D.pw_lo ? D.level_start[D.pw_hi + 1] - D.pw_base : 0;
-  if (!inc_formed_ || n_pw == 0 || n_moves < std::max(16, n_pw / 32)) return false;
+  if (!inc_formed_ || n_pw == 0 || n_moves < 12 + n_pw / 80) return false;
   const McLongKernel kern = mc_long_kernel(D.n_poly);
   const size_t smem = tables_smem(D, D.max_depth, 4) + mc_long_smem(D.n_poly, kPendPerBlock);
   if (mcl_grid_ == 0) {

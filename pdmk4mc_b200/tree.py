@@ -74,7 +74,7 @@ def launch_count() -> int:
 
 
 def replicas_mc_run(trees, idx, disp, u, beta):
-    """Metropolis sequences of many trees in one launch (one block per tree).
+    """Metropolis sequences of many trees at once, one block per tree.
     idx, u: [n_trees, m]; disp: [n_trees, m, 3]. Returns (dE, accepted), [n_trees, m]."""
     nt = len(trees)
     idx = np.ascontiguousarray(idx, dtype=np.int64).reshape(nt, -1)
