@@ -269,31 +269,45 @@ void dispatch_nudft(int nk, const PwItem* d_work, int nwork, const double* pos, 
   }
 }
 
-// sum split-K chunk partials of box b into its output: 32 modes x 8 chunk
-// lanes a block, four loads in flight a thread (a thread per mode alone took
-// 47 us over the 592 chunks of a small root, now 9)
+// sum split-K chunk partials of box b into its output: 256 / ROWS modes x ROWS
+// chunk lanes a block, four loads in flight a thread. Eight lanes where there are
+// many chunks (the 592 of a small root: 11 us, a lane per mode 47), one where
+// there are few (64 boxes of two chunks, N = 1e6: 15 us, eight lanes 57).
+template <int ROWS>
 __global__ void __launch_bounds__(256) k_reduce_chunks(const double2* __restrict__ part,
                                                        const PwSplit* __restrict__ split, int H) {
-  __shared__ double2 sm[8][32];
+  constexpr int MODES = 256 / ROWS;
+  __shared__ double2 sm[ROWS][MODES];
   const PwSplit b = split[blockIdx.y];
-  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
-  const int k = blockIdx.x * 32 + lane;
+  const int lane = threadIdx.x % MODES, row = threadIdx.x / MODES;
+  const int k = blockIdx.x * MODES + lane;
   const double2* p = part + size_t(b.first) * H + k;
   double2 s[4] = {};
   if (k < H)
-    for (int c = row; c < b.n; c += 32) {
+    for (int c = row; c < b.n; c += 4 * ROWS) {
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (c + 8 * u < b.n) s[u] = cadd(s[u], p[size_t(c + 8 * u) * H]);
+        if (c + ROWS * u < b.n) s[u] = cadd(s[u], p[size_t(c + ROWS * u) * H]);
     }
-  sm[row][lane] = cadd(cadd(s[0], s[1]), cadd(s[2], s[3]));
-  __syncthreads();
-  if (row == 0 && k < H) {
-    double2 t = sm[0][lane];
+  double2 t = cadd(cadd(s[0], s[1]), cadd(s[2], s[3]));
+  if (ROWS > 1) {
+    sm[row][lane] = t;
+    __syncthreads();
+    if (row > 0) return;
 #pragma unroll
-    for (int r = 1; r < 8; ++r) t = cadd(t, sm[r][lane]);
-    b.out[k] = t;
+    for (int r = 1; r < ROWS; ++r) t = cadd(t, sm[r][lane]);
   }
+  if (k < H) b.out[k] = t;
+}
+
+// n_split boxes with n_items partials in all
+void launch_reduce_chunks(const double2* part, const PwSplit* split, int n_split, long n_items, int H, cudaStream_t st) {
+  if (n_split == 0) return;
+  const bool many = n_items >= 16L * n_split;
+  auto kern = many ? k_reduce_chunks<8> : k_reduce_chunks<1>;
+  const int modes = many ? 32 : 256;
+  kern<<<dim3(unsigned((H + modes - 1) / modes), unsigned(n_split)), 256, 0, st>>>(part, split, H);
+  PDMK_LAUNCH_CHECK();
 }
 
 // ---------------------------------------------------------------------------
@@ -1166,11 +1180,6 @@ void DmkTree::form_outgoing_pw() {
     if (mixed) dispatch_mixed(nk, tmap, l.items, n_items, l.chunks, n_chunks, l.next, d_mix_, d_mix_err, st);
     else dispatch_nudft(nk, l.items, n_items, dense_, dense_stride_, st);
   };
-  auto reduce = [&](const Lists& l, int n_split, const double2* part, int H, cudaStream_t st) {
-    if (n_split == 0) return;
-    k_reduce_chunks<<<dim3(unsigned((H + 31) / 32), unsigned(n_split)), 256, 0, st>>>(part, l.split, H);
-    PDMK_LAUNCH_CHECK();
-  };
   if (!aux_) {
     aux_ = take_stream(&aux_device_);
     PDMK_CUDA(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
@@ -1221,7 +1230,7 @@ void DmkTree::form_outgoing_pw() {
   PDMK_CUDA(cudaEventRecord(ev_fork_, st_));
   PDMK_CUDA(cudaStreamWaitEvent(aux_, ev_fork_, 0));
   contract(D.n_window, tmap_root, root, n_root, n_root_chunks, aux_);
-  reduce(root, 1, part_r, D.Hw, aux_);
+  launch_reduce_chunks(part_r, root.split, 1, n_root, D.Hw, aux_);
   PDMK_CUDA(cudaEventRecord(ev_join_, aux_));
 
   PlanTotals t;
@@ -1234,7 +1243,7 @@ void DmkTree::form_outgoing_pw() {
   time_begin(3);
   contract(D.n_diff, tmap_box, box, t.n_items, t.n_chunks, st_);
   time_end(3);
-  reduce(box, t.n_split, part_b, D.H, st_);
+  launch_reduce_chunks(part_b, box.split, t.n_split, t.n_split_items, D.H, st_);
   out_defined_ = true;
   if (lists) fill_box_lists(t, d_blk);
   // the root pass's buffers are released after it joins the tree's stream
@@ -1272,10 +1281,11 @@ void DmkTree::fill_box_lists(const PlanTotals& t, const int* blk) {
   d_leaves_ = d_nonleaf_ + n_nonleaf_;
   d_cubes_ = d_leaves_ + n_leaves_;
   launch_plan_lists(D, blk, d_nonleaf_, d_leaves_, d_cubes_, st_);
-  // sum(q^2) for the window self term: 64 block partials, then a fixed-order sum
-  k_sum_q2<<<64, 256, 0, st_>>>(D.sq, D.n_slots, D.partials);
+  // sum(q^2) for the window self term: 592 block partials (64 took 38 us at
+  // N = 1e6), then a fixed-order sum
+  k_sum_q2<<<592, 256, 0, st_>>>(D.sq, D.n_slots, D.partials);
   PDMK_LAUNCH_CHECK();
-  k_sum<<<1, 1024, 0, st_>>>(D.partials, 64, d_scalars_ + 4);
+  k_sum<<<1, 1024, 0, st_>>>(D.partials, 592, d_scalars_ + 4);
   PDMK_LAUNCH_CHECK();
   box_lists_ready_ = true;
 }
@@ -1469,8 +1479,7 @@ double DmkTree::ewald_energy(double* parts) {
     const PwSplit all{0, nch, S};
     PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d_split), sizeof(PwSplit), st_));
     PDMK_CUDA(cudaMemcpyAsync(d_split, &all, sizeof(PwSplit), cudaMemcpyHostToDevice, st_));
-    k_reduce_chunks<<<dim3(unsigned((Hs + 31) / 32), 1u), 256, 0, st_>>>(part, d_split, Hs);
-    PDMK_LAUNCH_CHECK();
+    launch_reduce_chunks(part, d_split, 1, nch, Hs, st_);
     PDMK_CUDA(cudaFreeAsync(d_split, st_));
   }
   k_ewald_recip<<<unsigned(nblk_rec), TPB, 0, st_>>>(S, nk, dk, alpha, sums + nblk_real);
