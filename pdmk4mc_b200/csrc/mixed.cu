@@ -813,20 +813,6 @@ int mixed_table_bytes(int nk) {
   }
 }
 
-int mixed_pairs(int nk) {
-  switch (nk) {
-    case 4: return MixShape<4>::TILES;
-    case 6: return MixShape<6>::TILES;
-    case 8: return MixShape<8>::TILES;
-    case 12: return MixShape<12>::TILES;
-    case 13: return MixShape<13>::TILES;
-    case 17: return MixShape<17>::TILES;
-    case 19: return MixShape<19>::TILES;
-    case 26: return MixShape<26>::TILES;
-    default: throw std::invalid_argument("mixed precision: unsupported mode count");
-  }
-}
-
 void make_coord_map(CUtensorMap* map, const double* sx, int slot_capacity, int kcp) {
   if (slot_capacity % 2 != 0) throw std::logic_error("slot capacity must be even for the coordinate tensor map");
   // the four slot arrays x, y, z, q lie back to back with stride slot_capacity

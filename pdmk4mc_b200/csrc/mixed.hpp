@@ -8,8 +8,6 @@
 
 namespace pdmk {
 
-// M tiles per box for n modes per axis half
-int mixed_pairs(int nk);
 // particles per pipeline chunk of the mixed pass for n modes per axis half
 int mixed_chunk(int nk);
 // bytes of one chunk's table block (a multiple of 16)
@@ -21,7 +19,7 @@ void make_coord_map(CUtensorMap* map, const double* sx, int slot_capacity, int k
 void launch_absmax(const double* sq, int n, double* out, cudaStream_t st);
 // the mixed pass over device-resident lists: the table pass over nchunks
 // (item, chunk) pairs into the items' chunk table blocks, then the
-// contraction: mixed_pairs(nk) 128-row M tiles per item, which share the
+// contraction: the 128-row M tiles of each item, which share the
 // item's blocks (ceil((s_end - s_begin) / chunk) of them); d_next: the counter
 // the tiles are taken from, at zero
 void dispatch_mixed(int nk, const CUtensorMap& tmap, const PwItem* d_items, int nitems, const int2* d_chunks,

@@ -92,12 +92,6 @@ __device__ __forceinline__ void bulk_wait_read_all() {
 // generic-proxy shared-memory writes -> visible to the async proxy (tcgen05.mma, TMA)
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 
-// named barriers (ids 1..15; id 0 is __syncthreads)
-__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(n) : "memory"); }
-__device__ __forceinline__ void bar_arrive(int id, int n) {
-  asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(n) : "memory");
-}
-
 // ---------------------------------------------------------------------------
 // tcgen05 (one CTA, cta_group::1)
 
@@ -136,16 +130,6 @@ __host__ __device__ constexpr uint32_t idesc_i8(int M, int N) {
          | (1u << 10)                    // B: signed 8-bit
          | (uint32_t(N >> 3) << 17)      // N / 8
          | (uint32_t(M >> 4) << 24);     // M / 16
-}
-
-// D[tmem] (+)= A[smem] * B[smem]^T over K = 32 bytes; accumulate != 0 adds to D
-__device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                       uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
 }
 
 // D[tmem] (+)= A[tmem] * B[smem]^T over K = 32 bytes: A's row m in TMEM lane
