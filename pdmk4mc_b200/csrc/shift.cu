@@ -2096,10 +2096,14 @@ __global__ void __launch_bounds__(MCL_T, 1) k_mc_long(const __grid_constant__ De
           v += p == 0 ? r : -r;
         }
       }
-      // arrivals parked in the overflow pool that belong to a source's subtree
+      // arrivals parked in the overflow pool that belong to a source's subtree:
+      // every block takes its own range, since n_near is not the same in all of
+      // them (the one that commits has a warp less)
       const int pn = s_pn;
-      if (pn > 0)
-        for (int e2 = B * n_near + nt_; e2 < 2 * 36 * pn; e2 += G * n_near) {
+      if (pn > 0) {
+        const long n2 = 2L * 36 * pn;
+        const int p0 = int(n2 * B / G), p1 = int(n2 * (B + 1) / G);
+        for (int e2 = p0 + nt_; e2 < p1; e2 += n_near) {
           const int p = e2 / (36 * pn), sj = (e2 / pn) % 36, qi = e2 % pn;
           const SrcList& M = S[p];
           if (M.lvl[sj] < 0 || __ldcg(T.p_orig + qi) < 0) continue;
@@ -2116,6 +2120,7 @@ __global__ void __launch_bounds__(MCL_T, 1) k_mc_long(const __grid_constant__ De
             v += p == 0 ? r : -r;
           }
         }
+      }
       v *= h.q;
     } else if (warp == MCL_W - 1 && more) {
       // helper: resolve the next move from what it loaded a move ago, and load
