@@ -3511,6 +3511,7 @@ void DmkTree::flush_pending() {
 void DmkTree::mc_run_persistent(int n_moves, const int* d_idx, const double* d_disp, const double* d_u, double beta,
                                 double* d_dE, int* d_acc) {
   DevTree& D = dev_;
+  ensure_rows(true, true);
   if (mc_run_long(n_moves, d_idx, d_disp, d_u, beta, d_dE, d_acc)) return;
   const size_t smem = tables_smem(D, D.max_depth, 2);
   const McKernel kern = mc_kernel(D.n_poly);
