@@ -1245,6 +1245,8 @@ void DmkTree::form_outgoing_pw() {
   time_end(3);
   launch_reduce_chunks(part_b, box.split, t.n_split, t.n_split_items, D.H, st_);
   out_defined_ = true;
+  if (!out_formed_) inc_formed_ = false;  // incoming rows formed before are not of these
+  out_formed_ = true;
   if (lists) fill_box_lists(t, d_blk);
   // the root pass's buffers are released after it joins the tree's stream
   PDMK_CUDA(cudaStreamWaitEvent(st_, ev_join_, 0));

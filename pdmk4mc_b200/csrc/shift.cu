@@ -3792,11 +3792,13 @@ void DmkTree::replicas_mc_run(const std::vector<DmkTree*>& ts, int m, const int*
   if (ts.empty() || m <= 0) return;
   const int np = ts[0]->dev_.n_poly;
   size_t smem = 0;
+  bool deferred = true;
   for (DmkTree* t : ts) {
     if (t->dev_.n_poly != np) throw std::invalid_argument("replicas must share the digits setting");
     t->ensure_packed();
     t->ensure_rows(true, true);
     smem = std::max(smem, tables_smem(t->dev_, t->dev_.max_depth, 2));
+    deferred = deferred && (t->inc_formed_ || t->dev_.pw_hi < t->dev_.pw_lo);
   }
   cudaStream_t st = ts[0]->st_;
   // Each tree's list is filled by its block of the launch on the first tree's
@@ -3805,6 +3807,28 @@ void DmkTree::replicas_mc_run(const std::vector<DmkTree*>& ts, int m, const int*
   const size_t nt = ts.size();
   std::vector<cudaEvent_t> evs(nt);
   for (auto& e : evs) PDMK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  if (!deferred) {
+    // Deferred updates recompute incoming rows from the outgoing ones, which is
+    // what accepted moves do to them only where a pass formed them so. A set
+    // with a tree whose rows were not formed runs tree by tree, move by move.
+    PDMK_CUDA(cudaEventRecord(evs[0], st));
+    for (size_t i = 0; i < nt; ++i) {
+      DmkTree* t = ts[i];
+      if (i > 0) PDMK_CUDA(cudaStreamWaitEvent(t->st_, evs[0], 0));
+      const size_t c = i * size_t(m);
+      t->mc_run_persistent(m, d_idx + c, d_disp + 3 * c, d_u + c, beta, d_dE ? d_dE + c : nullptr,
+                           d_acc ? d_acc + c : nullptr);
+      if (i > 0) {
+        PDMK_CUDA(cudaEventRecord(evs[i], t->st_));
+        PDMK_CUDA(cudaStreamWaitEvent(st, evs[i], 0));
+      }
+      t->last_valid_ = false;
+      t->diff_cached_ = false;
+      t->mark_moved();
+    }
+    for (auto& e : evs) PDMK_CUDA(cudaEventDestroy(e));
+    return;
+  }
   const int chunk = std::min(m, REP_CHUNK);
   std::vector<unsigned char> blob(nt * (sizeof(DevTree) + 4 * sizeof(void*)));
   DevTree* h_trees = reinterpret_cast<DevTree*>(blob.data());

@@ -385,6 +385,7 @@ class DmkTree {
   // deferred expansion updates of Metropolis sequences (shift.cu)
   static constexpr int kPendPerBlock = 16;  // listed moves one block of the persistent kernel keeps
   bool inc_formed_ = false;  // the incoming rows follow from the outgoing ones (a deferred update recomputes them)
+  bool out_formed_ = false;  // the outgoing pass ran (again: the same rows, to rounding)
   int mcl_grid_ = 0;
   void* d_pos4_ = nullptr;   // position and charge by particle, for the particles of a sequence
   unsigned long long* d_packets_ = nullptr;

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 N, L = 4000, 16.0
 ABS_DE = 2e-10
-PASSES = {"nothing": "", "outgoing": "o", "incoming": "i"}
+PASSES = {"nothing": "", "outgoing": "o", "incoming": "i", "incoming_first": "io"}
 
 
 def system():
@@ -63,8 +63,37 @@ def test_sequence_on_unformed_rows(formed, moves, digits):
         t = open_tree(prm, PASSES[formed])
         try:
             t.set_mc_mode(mode)
-            got.append(t.mc_run(idx, disp, u, 1.0))
+            got.append([t.mc_run(idx, disp, u, 1.0) for _ in range(2)])  # again on the rows of the first
         finally:
             t.close()
-    np.testing.assert_array_equal(got[0][1], got[1][1])
-    assert close(got[0][0], got[1][0])
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a[1], b[1])
+        assert close(a[0], b[0])
+
+
+@pytest.mark.parametrize("sets", [["nothing"] * 2, ["outgoing", "formed"], ["incoming_first", "formed"], ["incoming"]])
+def test_replicas_with_unformed_rows(sets):
+    # more moves than a replica lists, then a second call on the rows of the first
+    m, prm = 150, params(6)
+    passes = dict(PASSES, formed="oi")
+    prop = [proposals(m, 7 + k) for k in range(len(sets))]
+    want = []
+    for name, p in zip(sets, prop):
+        dirty_pool(prm)
+        t = open_tree(prm, passes[name])
+        try:
+            t.set_mc_mode(P.MC_GRAPH)
+            want.append([t.mc_run(*p, 1.0) for _ in range(2)])
+        finally:
+            t.close()
+    dirty_pool(prm)
+    ts = [open_tree(prm, passes[name]) for name in sets]
+    try:
+        for call in range(2):
+            dE, acc = P.replicas_mc_run(ts, *(np.stack([p[k] for p in prop]) for k in range(3)), 1.0)
+            for k in range(len(sets)):
+                np.testing.assert_array_equal(acc[k], want[k][call][1])
+                assert close(dE[k], want[k][call][0])
+    finally:
+        for t in ts:
+            t.close()
