@@ -1105,7 +1105,7 @@ void DmkTree::repack(int leaf_slack) {
 // The particles without the free slots, for the outgoing pass: kept from the
 // build or the last pack, gathered again after moves.
 void DmkTree::ensure_dense() {
-  if (dense_ready_) return;
+  if (dense_ready_ && !captured_moves_) return;
   DevTree& D = dev_;
   const int nl = leaf_dev_.n;
   int* cnt;

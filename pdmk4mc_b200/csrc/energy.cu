@@ -1103,7 +1103,7 @@ size_t DmkTree::partials_needed() const {
 void DmkTree::ensure_packed() {
   // only accepted moves put particles into the overflow pool: a tree without
   // moves since its build or last pack needs no device round trip
-  if (!moved_) return;
+  if (!moved_ && !captured_moves_) return;
   int pn = 0;
   PDMK_CUDA(cudaMemcpyAsync(&pn, dev_.pool_n, 4, cudaMemcpyDeviceToHost, st_));
   PDMK_CUDA(cudaStreamSynchronize(st_));

@@ -3628,6 +3628,9 @@ bool DmkTree::mc_run_long(int n_moves, const int* d_idx, const double* d_disp, c
 void DmkTree::mc_run_device(int n_moves, const int* d_idx, const double* d_disp, const double* d_u, double beta,
                             double* d_dE, int* d_acc) {
   if (mc_mode_ == 0) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    PDMK_CUDA(cudaStreamIsCapturing(st_, &cs));
+    captured_moves_ = captured_moves_ || cs != cudaStreamCaptureStatusNone;
     if (n_moves > 0) mc_run_persistent(n_moves, d_idx, d_disp, d_u, beta, d_dE, d_acc);
     last_valid_ = false;
     diff_cached_ = false;

@@ -341,6 +341,9 @@ class DmkTree {
   bool diff_cached_ = false;
   void mark_moved() { moved_ = true, dense_ready_ = false; }
   bool moved_ = false;  // moves ran since the last pack: the overflow pool may hold particles
+  // a sequence was captured: its graph may move particles at any time, unseen by
+  // the host, so nothing that moves outdate is taken for current from then on
+  bool captured_moves_ = false;
   bool box_lists_ready_ = false;
   int n_nonleaf_ = 0, n_leaves_ = 0;
   int* d_nonleaf_ = nullptr;  // non-leaf nodes of the expansion levels
