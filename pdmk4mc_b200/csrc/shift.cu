@@ -3512,7 +3512,6 @@ void DmkTree::mc_run_persistent(int n_moves, const int* d_idx, const double* d_d
                                 double* d_dE, int* d_acc) {
   DevTree& D = dev_;
   ensure_rows(true, true);
-  if (mc_run_long(n_moves, d_idx, d_disp, d_u, beta, d_dE, d_acc)) return;
   const size_t smem = tables_smem(D, D.max_depth, 2);
   const McKernel kern = mc_kernel(D.n_poly);
   if (mc_grid_ == 0) {
@@ -3529,6 +3528,7 @@ void DmkTree::mc_run_persistent(int n_moves, const int* d_idx, const double* d_d
     mc_sync_ = static_cast<unsigned int*>(alloc(64));
     mc_grid_ = sms;
   }
+  if (mc_run_long(n_moves, d_idx, d_disp, d_u, beta, d_dE, d_acc)) return;
   const double pi = 3.14159265358979323846;
   for (int m0 = 0; m0 < n_moves; m0 += kMcChunk) {
     const int cnt = std::min(kMcChunk, n_moves - m0);
@@ -3565,6 +3565,20 @@ bool DmkTree::mc_run_long(int n_moves, const int* d_idx, const double* d_disp, c
   DevTree& D = dev_;
   const int n_pw = D.pw_hi >= D.pw_lo ? D.level_start[D.pw_hi + 1] - D.pw_base : 0;
   if (!inc_formed_ || n_pw == 0 || n_moves < 12 + n_pw / 80) return false;
+  // A longer list makes each move's pair sums longer (5 ns per listed move at
+  // N = 1e5, 7.4 ns at 1e6), a shorter one updates the rows more often (0.38 and
+  // 2.1 ms). 2000 moves at N = 1e5 / 4000 at 1e6 (9 digits, positions
+  // read at the end): 20.8 / 75.1 ms at 384 moves a list, 20.7 / 71.3 at 512, 20.9 /
+  // 69.8 at 768, 21.3 / 68.1 at 1024, 23.6 / 69.9 at 2048.
+  const int longest = n_pw >= 1024 ? 1024 : 512;
+  // What this form keeps is allocated and filled by its first call outside a
+  // capture: memory taken inside one belongs to the graph. Until then a captured
+  // sequence runs move by move.
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  PDMK_CUDA(cudaStreamIsCapturing(st_, &cs));
+  if (cs != cudaStreamCaptureStatusNone &&
+      !(mcl_grid_ > 0 && box_lists_ready_ && d_oct_ && pending_cap_ >= std::min(longest, kPendPerBlock * mcl_grid_)))
+    return false;
   const McLongKernel kern = mc_long_kernel(D.n_poly);
   const size_t smem = tables_smem(D, D.max_depth, 4) + mc_long_smem(D.n_poly, kPendPerBlock);
   if (mcl_grid_ == 0) {
@@ -3582,13 +3596,8 @@ bool DmkTree::mc_run_long(int n_moves, const int* d_idx, const double* d_disp, c
     mcl_grid_ = sms;
   }
   prepare_box_lists();
-  // A longer list makes each move's pair sums longer (5 ns per listed move at
-  // N = 1e5, 7.4 ns at 1e6), a shorter one updates the rows more often (0.38 and
-  // 2.1 ms). 2000 moves at N = 1e5 / 4000 at 1e6 (9 digits, positions
-  // read at the end): 20.8 / 75.1 ms at 384 moves a list, 20.7 / 71.3 at 512, 20.9 /
-  // 69.8 at 768, 21.3 / 68.1 at 1024, 23.6 / 69.9 at 2048.
-  const int chunk = std::min(n_pw >= 1024 ? 1024 : 512, kPendPerBlock * mcl_grid_);
-  ensure_pending(std::min(chunk, n_moves));
+  const int chunk = std::min(longest, kPendPerBlock * mcl_grid_);
+  ensure_pending(chunk);
   const double pi = 3.14159265358979323846;
   for (int m0 = 0; m0 < n_moves; m0 += chunk) {
     const int cnt = std::min(chunk, n_moves - m0);

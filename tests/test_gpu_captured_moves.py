@@ -85,3 +85,42 @@ def test_energy_after_replayed_moves(moves, slack, precision):
         del g
     finally:
         t.close()
+
+
+@pytest.mark.parametrize("warm,captured,after", [(8, 200, 600), (200, 8, 30), (20, 600, 600), (600, 600, 20)])
+def test_captured_and_direct_sequences_share_a_tree(warm, captured, after):
+    # neither leaves the other with memory that belongs to a graph. Shifts as in
+    # the move-by-move form: under 2e5 terms below 1e3, rounded to 1.2e-16 of that
+    r, q = system()
+    parts = [Sequence(m, 50 + k) for k, m in enumerate((warm, captured, after))]
+    order = (0, 1, 2, 1)
+    want = []
+    t = P.HPDMKPtTree(params(), r, q)
+    try:
+        energy(t)
+        t.set_mc_mode(P.MC_GRAPH)
+        for k in order:
+            parts[k].run(t)
+            t.synchronize()
+            want.append(parts[k].dE.cpu().numpy())
+    finally:
+        t.close()
+    t = P.HPDMKPtTree(params(), r, q)
+    try:
+        energy(t)
+        parts[0].run(t)
+        t.synchronize()
+        got = [parts[0].dE.cpu().numpy()]
+        g = capture(t, lambda: parts[1].run(t))
+        for k in order[1:]:
+            if k == 1:
+                replay(t, g)
+            else:
+                parts[k].run(t)
+                t.synchronize()
+            got.append(parts[k].dE.cpu().numpy())
+        del g
+    finally:
+        t.close()
+    for a, b in zip(got, want):
+        assert np.all(np.abs(a - b) <= 2e-10 * np.maximum(1.0, np.abs(b)))
