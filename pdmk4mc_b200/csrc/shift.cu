@@ -3690,14 +3690,16 @@ int DmkTree::batch_groups(int m, const int* d_idx, int* order) {
   return grp;
 }
 
-// The tree's own index array for the order; null while a capture that would
-// have to allocate it is under way.
+// The tree's own index array for the order; null under capture: a graph may be
+// replayed on a stream beside the tree's, where a direct call would share it (a
+// captured batch runs one candidate a block: 1.30 instead of 1.04 ms for 4096 at N
+// = 1e6, 9 digits).
 int* DmkTree::batch_order(int m) {
   if (m < kGroupMin) return nullptr;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  PDMK_CUDA(cudaStreamIsCapturing(st_, &cs));
+  if (cs != cudaStreamCaptureStatusNone) return nullptr;
   if (m > order_cap_) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    PDMK_CUDA(cudaStreamIsCapturing(st_, &cs));
-    if (cs != cudaStreamCaptureStatusNone) return nullptr;
     order_cap_ = std::max(m, 2 * order_cap_);
     d_order_ = static_cast<int*>(alloc(sizeof(int) * size_t(order_cap_)));
   }

@@ -124,3 +124,37 @@ def test_captured_and_direct_sequences_share_a_tree(warm, captured, after):
         t.close()
     for a, b in zip(got, want):
         assert np.all(np.abs(a - b) <= 2e-10 * np.maximum(1.0, np.abs(b)))
+
+
+def test_captured_batch_beside_direct_ones():
+    # the graph runs on another stream while the tree's own evaluates other batches
+    import torch
+    r, q = system()
+    t = P.HPDMKPtTree(params(), r, q)
+    try:
+        energy(t)
+        a, b = Sequence(3000, 1), Sequence(1500, 2)
+
+        def batch(s):
+            t.eval_shift_energy_batch_device(s.m, s.i.data_ptr(), s.d.data_ptr(), s.dE.data_ptr())
+
+        want = []
+        for s in (a, b):
+            batch(s)
+            t.synchronize()
+            want.append(s.dE.clone())
+        g = capture(t, lambda: batch(a))
+        other = torch.cuda.Stream()
+        for _ in range(20):
+            a.dE.zero_()
+            b.dE.zero_()
+            torch.cuda.synchronize()
+            with torch.cuda.stream(other):
+                g.replay()
+            batch(b)
+            torch.cuda.synchronize()
+            t.synchronize()
+            assert torch.equal(a.dE, want[0]) and torch.equal(b.dE, want[1])  # whatever the groups
+        del g
+    finally:
+        t.close()
