@@ -682,7 +682,7 @@ template <int NP, int MINB>
 __global__ void __launch_bounds__(RES_T, MINB) k_residual(DevTree T, const int* __restrict__ leaves, int ny,
                                                     double* part) {
   __shared__ double ux[RES_SCH], uy[RES_SCH], uz[RES_SCH], uq[RES_SCH];
-  // negated coordinates relative to the leaf's centre
+  // negated coordinates relative to the leaf's centre, in box sides
   __shared__ __align__(16) float ufx[RES_SCH], ufy[RES_SCH], ufz[RES_SCH];
   __shared__ float t_lo[RES_SCH / 32][3], t_hi[RES_SCH / 32][3];  // bounding boxes of the source tiles
   __shared__ double gx[RES_TCH], gy[RES_TCH], gz[RES_TCH], gq[RES_TCH];
@@ -698,9 +698,10 @@ __global__ void __launch_bounds__(RES_T, MINB) k_residual(DevTree T, const int* 
   double e = 0;
   if (l >= 2 && cnt > chunk * RES_TCH) {
     const double b = level_box(T, l), inv_b = 1.0 / b;
-    // FP32 coordinates reach 2 b from the centre: each is off by 2^-23 b at
-    // most, a squared distance near b^2 by less than 2e-6 b^2
-    const float cut = float(b * b * (1.0 + 8e-6));
+    // FP32 coordinates in units of b (any box size is in their range) reach 2.5
+    // from the centre: each is off by 2^-23 at most, a squared distance near 1 by
+    // less than 2e-6
+    const float cut = 1.0f + 8e-6f;
     const float far = 1e18f;  // where a lane without a target, or a tile's empty place, is put
     const int tb = T.node_begin[node];
     double ci[3];
@@ -760,8 +761,8 @@ __global__ void __launch_bounds__(RES_T, MINB) k_residual(DevTree T, const int* 
       }
       __syncthreads();
       const bool act = it < nt;
-      const float fx = act ? float(gx[it] - ci[0]) : far, fy = act ? float(gy[it] - ci[1]) : far,
-                  fz = act ? float(gz[it] - ci[2]) : far;
+      const float fx = act ? float((gx[it] - ci[0]) * inv_b) : far, fy = act ? float((gy[it] - ci[1]) * inv_b) : far,
+                  fz = act ? float((gz[it] - ci[2]) * inv_b) : far;
       const unsigned long long fx2 = both_f32x2(fx), fy2 = both_f32x2(fy), fz2 = both_f32x2(fz);
       const unsigned long long ncut2 = both_f32x2(-cut);
       float lo[3] = {fx, fy, fz}, hi[3] = {act ? fx : -far, act ? fy : -far, act ? fz : -far};
@@ -787,7 +788,7 @@ __global__ void __launch_bounds__(RES_T, MINB) k_residual(DevTree T, const int* 
             uy[t] = y;
             uz[t] = zz;
             uq[t] = T.sq[s] * m_w[a];
-            f[0] = float(x - ci[0]), f[1] = float(y - ci[1]), f[2] = float(zz - ci[2]);
+            f[0] = float((x - ci[0]) * inv_b), f[1] = float((y - ci[1]) * inv_b), f[2] = float((zz - ci[2]) * inv_b);
 #pragma unroll
             for (int a2 = 0; a2 < 3; ++a2) flo[a2] = fhi[a2] = f[a2];
           }
