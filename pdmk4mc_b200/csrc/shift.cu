@@ -1712,7 +1712,7 @@ __device__ inline void packet_store(unsigned long long* p, double v, unsigned ep
                "l"(lo), "l"(hi)
                : "memory");
 }
-__device__ inline void packet_load(const unsigned long long* p, double& v, unsigned& epoch, unsigned& extra) {
+__device__ inline void packet_load(const unsigned long long* p, double& v, unsigned& epoch) {
   unsigned long long lo, hi;
   asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}\n"
                : "=l"(lo), "=l"(hi)
@@ -1720,7 +1720,19 @@ __device__ inline void packet_load(const unsigned long long* p, double& v, unsig
                : "memory");
   v = __longlong_as_double((long long)lo);
   epoch = unsigned(hi);
-  extra = unsigned(hi >> 32);
+}
+
+// The pool fill of a packet that has arrived, by the same load as an acquire: what
+// was released before the packet is visible after it. (A fence behind the relaxed
+// loads would order as much, for 800 cycles of every move.)
+__device__ inline unsigned packet_acquire(const unsigned long long* p) {
+  unsigned long long hi;
+  asm volatile(
+      "{\n .reg .b128 t;\n .reg .b64 sum;\n ld.acquire.gpu.global.b128 t, [%1];\n mov.b128 {sum, %0}, t;\n}\n"
+      : "=l"(hi)
+      : "l"(p)
+      : "memory");
+  return unsigned(hi >> 32);
 }
 
 // positions and charges of the particles a launch will move
@@ -2191,7 +2203,6 @@ __global__ void __launch_bounds__(MCL_T, 1) k_mc_long(const __grid_constant__ De
       bool ok = true;
       for (int b0 = 0; b0 < G; b0 += 32 * MCL_POLL) {
         double pv[MCL_POLL];
-        unsigned px[MCL_POLL];
         for (long long it = 0;; ++it) {
           bool all = true;
 #pragma unroll
@@ -2199,7 +2210,7 @@ __global__ void __launch_bounds__(MCL_T, 1) k_mc_long(const __grid_constant__ De
             const int b = b0 + lane + 32 * j;
             unsigned pe = epoch;
             pv[j] = 0.0;
-            if (b < G) packet_load(pk + 2 * b, pv[j], pe, px[j]);
+            if (b < G) packet_load(pk + 2 * b, pv[j], pe);
             all = all && pe == epoch;
           }
           if (all) break;
@@ -2211,10 +2222,9 @@ __global__ void __launch_bounds__(MCL_T, 1) k_mc_long(const __grid_constant__ De
 #pragma unroll
         for (int j = 0; j < MCL_POLL; ++j) {
           tot += pv[j];
-          if (b0 + lane + 32 * j == G / 2) {
-            s_pn = int(px[j]);
-            ld_acquire(a.committed);  // the commits before that packet are visible from here on
-          }
+          // the committing block's packet follows its fence: its commits so far
+          // are visible from here on
+          if (b0 + lane + 32 * j == G / 2) s_pn = int(packet_acquire(pk + 2 * (G / 2)));
         }
       }
       if (!ok) atomicOr(T.err, 2);
