@@ -95,7 +95,6 @@ __global__ void k_plan_root(DevTree T, PlanShape s, int n, int n_items, int n_ch
   if (i == 0) {
     *split = PwSplit{0, n_items, T.out_root};
     *next = 0;
-    T.counter[14] = 1;  // every outgoing row is about to be written
   }
 }
 
@@ -170,7 +169,12 @@ __global__ void __launch_bounds__(PLAN_T)
   __shared__ int n_ch, ch0;
   for (int i = threadIdx.x; i < kPlanBuckets; i += PLAN_T) cnt[i] = 0;
   if (threadIdx.x == 0) n_ch = 0;
-  if (threadIdx.x == 0 && blockIdx.x == 0) *next = 0;
+  if (threadIdx.x == 0 && blockIdx.x == 0) {
+    *next = 0;
+    // every outgoing row is about to be written: the pass has all its memory (had
+    // it failed, a later call would find the rows undefined and clear them)
+    T.counter[14] = 1;
+  }
   // exclusive sums of the buckets: four per lane of the first warp
   if (threadIdx.x < 32) {
     int h[4], v = 0;
