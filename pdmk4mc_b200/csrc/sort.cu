@@ -138,7 +138,11 @@ __global__ void __launch_bounds__(RS_T) k_radix_totals(const uint64_t* __restric
 // up counts the keys before it itself. What bounds a pass is the scattered
 // write; the histogram and three scan launches of a pass that this replaces
 // took as long again (N = 1e5: 15 of 27 us).
-constexpr unsigned RS_SUM = 1u << 30, RS_ALL = 2u << 30, RS_MASK = RS_SUM - 1;
+//
+// A published word: 0 nothing yet, 1 + count for the tile's own count (at most
+// RS_TILE), RS_ALL + sum for its sum with all before it (any int fits).
+constexpr unsigned RS_ALL = RS_TILE + 2;
+static_assert(RS_ALL + 0x7fffffffu > RS_ALL, "a sum of any number of pairs fits a word");
 constexpr int RS_LOOK = 8;
 constexpr int RS_SPIN = 1 << 20;
 
@@ -188,7 +192,7 @@ __global__ void __launch_bounds__(RS_T)
     cnt += c;
   }
   volatile unsigned* st = state;
-  st[long(tile) * 256 + d] = (tile == 0 ? RS_ALL : RS_SUM) | unsigned(cnt);
+  st[long(tile) * 256 + d] = (tile == 0 ? RS_ALL : 1u) + unsigned(cnt);
   // keys of smaller digits: exclusive sum of the totals
   int x = total[d];
   const int mine = x;
@@ -212,9 +216,9 @@ __global__ void __launch_bounds__(RS_T)
       int used = 0;
 #pragma unroll
       for (int k = 0; k < RS_LOOK; ++k)
-        if (!found && used == k && (v[k] & ~RS_MASK)) {
-          before += int(v[k] & RS_MASK);
-          found = (v[k] & RS_ALL) != 0;
+        if (!found && used == k && v[k] != 0) {
+          found = v[k] >= RS_ALL;
+          before += int(v[k] - (found ? RS_ALL : 1u));
           ++used;
         }
       t -= used;
@@ -230,7 +234,7 @@ __global__ void __launch_bounds__(RS_T)
     __syncthreads();
     before = base[d];
   }
-  if (tile > 0) st[long(tile) * 256 + d] = RS_ALL | unsigned(before + cnt);
+  if (tile > 0) st[long(tile) * 256 + d] = RS_ALL + unsigned(before + cnt);
   base[d] = below + before;
   __syncthreads();
   for (int k = 0; k < RS_ITEMS; ++k) {
