@@ -3566,15 +3566,19 @@ void DmkTree::mc_run_persistent(int n_moves, const int* d_idx, const double* d_d
 
 // The same for a sequence long enough to defer its row updates (k_mc_long);
 // false when it is not. The passes that bring the rows up to date cost with the
-// number of rows, an update move by move with the number of moves. Deferred /
-// move by move, us a call (9 digits): 64 rows (N = 2e4) 221 / 256 for 8 moves,
-// 276 / 420 for 16; 576 rows (1e5) 498 / 433 for 16, 628 / 822 for 32; 4672
-// rows (1e6) 1524 / 1114 for 32, 2052 / 2152 for 64, 2903 / 4847 for 146.
+// rows' bytes, an update move by move with the number of moves. Both forms take
+// the same time at (moves of up to 0.3 spacings per axis at beta = 1; digits, rows,
+// MB of rows): fewer than 8 moves up to 31 MB and for 3 digits up to 146 MB;
+// 14 (6, 576, 75); 23 (9, 576, 280); 48 (6, 4672, 607); 38 (12, 576, 699); 74 (9,
+// 4672, 2274); 106 (9, 7776, 3785); above 128 (12, 7632, 9261). The line lies along
+// these. Deferred / move by move, us a call: 24 moves at 280 MB 498 / 505, 128 at
+// 280 MB 1406 / 2518, 32 at 699 MB 1041 / 964, 128 at 2274 MB 2583 / 3647.
 bool DmkTree::mc_run_long(int n_moves, const int* d_idx, const double* d_disp, const double* d_u, double beta, double* d_dE,
                           int* d_acc) {
   DevTree& D = dev_;
   const int n_pw = D.pw_hi >= D.pw_lo ? D.level_start[D.pw_hi + 1] - D.pw_base : 0;
-  if (!inc_formed_ || n_pw == 0 || n_moves < 12 + n_pw / 80) return false;
+  const long mb = 16L * n_pw * D.H / 1000000;
+  if (!inc_formed_ || n_pw == 0 || n_moves < 8 + std::min(mb, 650L) / 16 + std::max(mb - 650, 0L) / 52) return false;
   // A longer list makes each move's pair sums longer (5 ns per listed move at
   // N = 1e5, 7.4 ns at 1e6), a shorter one updates the rows more often (0.38 and
   // 2.1 ms). 2000 moves at N = 1e5 / 4000 at 1e6 (9 digits, positions
