@@ -146,8 +146,9 @@ int hpdmk_eval_shift_energy_batch(hpdmk_tree tree, int m, const long *i, const d
 
 /* As hpdmk_eval_shift_energy_batch with device-resident int32 indices d_i[m],
  * displacements d_d[3m] and output d_dE[m], enqueued on the tree's stream
- * without a host synchronisation (a thread block per candidate; from 1184
- * candidates on, a block per two that share boxes). */
+ * without a host synchronisation (a thread block per candidate; at 6 and more
+ * digits, from 1184 candidates on and outside stream capture, a block per two
+ * that share boxes). */
 int hpdmk_eval_shift_energy_batch_device(hpdmk_tree tree, int m, const int *d_i, const double *d_d, double *d_dE);
 
 /* No reference counterpart. The same launches as

@@ -2828,6 +2828,13 @@ constexpr int BG_GROUP = 2;
 // digits, host arrays): candidates 438 / 394 for 888, 502 / 508 for 1184, 634 /
 // 679 for 1776; potentials 330 / 336, 353 / 414, 478 / 583
 constexpr int kGroupMin = 4 * 148 * 2;
+// At 3 digits (7 coefficients) a row is 19 KB and the work between two barriers so
+// small that more resident blocks are worth more than shared rows: four a SM, one
+// point each. 4096 candidates / potentials, us: N = 1e6 196 / 244 (in pairs at two
+// blocks a SM 292 / 315, a thread per mode 238 / 311), N = 128e3 157 / 208 (214 /
+// 253, 175 / 255).
+__host__ __device__ constexpr int batch_blocks(int np) { return np == 7 ? 4 : 2; }
+constexpr bool in_pairs(int np, int m) { return np > 7 && m >= kGroupMin; }
 
 // order[]: the particles idx[0 .. m) by the level-4 cell of their positions (one
 // block; the order within a cell is free, no result depends on it)
@@ -2876,7 +2883,7 @@ __global__ void __launch_bounds__(1024) k_order_particles(DevTree T, const int* 
 }
 
 template <int NP, int GRP>
-__global__ void __launch_bounds__(BG_T, 2) k_shift_batch(DevTree T, const int* __restrict__ idx,
+__global__ void __launch_bounds__(BG_T, batch_blocks(NP)) k_shift_batch(DevTree T, const int* __restrict__ idx,
                                                       const double* __restrict__ disp, const int* __restrict__ order, int m,
                                                       double c_window, double sum_d2, double* __restrict__ dE_out) {
   using S = BatchShape<NP>;
@@ -3035,7 +3042,7 @@ __global__ void __launch_bounds__(BG_T, 2) k_shift_batch(DevTree T, const int* _
 using ShiftBatchKernel = void (*)(DevTree, const int*, const double*, const int*, int, double, double, double*);
 ShiftBatchKernel shift_batch_kernel(int np, int grp) {
   switch (np) {
-    case 7: return grp > 1 ? k_shift_batch<7, BG_GROUP> : k_shift_batch<7, 1>;
+    case 7: return k_shift_batch<7, 1>;
     case 13: return grp > 1 ? k_shift_batch<13, BG_GROUP> : k_shift_batch<13, 1>;
     case 19: return grp > 1 ? k_shift_batch<19, BG_GROUP> : k_shift_batch<19, 1>;
     case 25: return grp > 1 ? k_shift_batch<25, BG_GROUP> : k_shift_batch<25, 1>;
@@ -3066,7 +3073,7 @@ size_t batch_smem(int np, int max_depth, int points) {
 // -i k u: the row products carry two more columns per point, kx ex, and the y
 // and z derivatives take their factors at the lines.
 template <int NP, int GRP>
-__global__ void __launch_bounds__(BG_T, 2) k_potential_batch(DevTree T, const int* __restrict__ idx,
+__global__ void __launch_bounds__(BG_T, batch_blocks(NP)) k_potential_batch(DevTree T, const int* __restrict__ idx,
                                                           const int* __restrict__ order, int m, double c_window,
                                                           double self_w, double sum_w, double sum_d2,
                                                           const double* __restrict__ Sl,
@@ -3237,7 +3244,7 @@ using PotentialKernel = void (*)(DevTree, const int*, const int*, int, double, d
                                  double*, double*);
 PotentialKernel potential_kernel(int np, int grp) {
   switch (np) {
-    case 7: return grp > 1 ? k_potential_batch<7, BG_GROUP> : k_potential_batch<7, 1>;
+    case 7: return k_potential_batch<7, 1>;
     case 13: return grp > 1 ? k_potential_batch<13, BG_GROUP> : k_potential_batch<13, 1>;
     case 19: return grp > 1 ? k_potential_batch<19, BG_GROUP> : k_potential_batch<19, 1>;
     case 25: return grp > 1 ? k_potential_batch<25, BG_GROUP> : k_potential_batch<25, 1>;
@@ -3693,10 +3700,10 @@ void DmkTree::mc_run_device(int n_moves, const int* d_idx, const double* d_disp,
   mark_moved();
 }
 
-// The batch kernels' groups: BG_GROUP particles a block in Morton order when
-// there are enough of them (order: room for m indices, or null), else one.
+// The batch kernels' groups: BG_GROUP particles a block in Morton order where that
+// pays (in_pairs; order: room for m indices, or null), else one.
 int DmkTree::batch_groups(int m, const int* d_idx, int* order) {
-  const int grp = order && m >= kGroupMin ? BG_GROUP : 1;
+  const int grp = order && in_pairs(dev_.n_poly, m) ? BG_GROUP : 1;
   if (grp > 1) {
     k_order_particles<<<1, 1024, 0, st_>>>(dev_, d_idx, m, order);
     PDMK_LAUNCH_CHECK();
@@ -3709,7 +3716,7 @@ int DmkTree::batch_groups(int m, const int* d_idx, int* order) {
 // captured batch runs one candidate a block: 1.30 instead of 1.04 ms for 4096 at N
 // = 1e6, 9 digits).
 int* DmkTree::batch_order(int m) {
-  if (m < kGroupMin) return nullptr;
+  if (!in_pairs(dev_.n_poly, m)) return nullptr;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   PDMK_CUDA(cudaStreamIsCapturing(st_, &cs));
   if (cs != cudaStreamCaptureStatusNone) return nullptr;
