@@ -546,24 +546,27 @@ int hpdmk_replicas_mc_run(int n_trees, const hpdmk_tree* trees, int m, const lon
     const size_t tot = size_t(n_trees) * m;
     std::vector<int> ii(i, i + tot);
     char* buf = nullptr;
-    const size_t bytes = tot * (4 + 24 + 8 + 8 + 4) + 64;
+    const size_t bytes = tot * (4 + 24 + 8 + 8 + 4) + 4 * size_t(n_trees) + 64;
     PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&buf), bytes, h0->stream));
     double* d_d = reinterpret_cast<double*>(buf);
     double* d_u = d_d + 3 * tot;
     double* d_dE = d_u + tot;
     int* d_i = reinterpret_cast<int*>(d_dE + tot);
     int* d_acc = d_i + tot;
+    int* d_err = d_acc + tot;
+    std::vector<int> errs(n_trees);
     PDMK_CUDA(cudaMemcpyAsync(d_i, ii.data(), sizeof(int) * tot, cudaMemcpyHostToDevice, h0->stream));
     PDMK_CUDA(cudaMemcpyAsync(d_d, d, sizeof(double) * 3 * tot, cudaMemcpyHostToDevice, h0->stream));
     PDMK_CUDA(cudaMemcpyAsync(d_u, u, sizeof(double) * tot, cudaMemcpyHostToDevice, h0->stream));
     for (auto* t : ts) t->reset_work();
-    pdmk::DmkTree::replicas_mc_run(ts, m, d_i, d_d, d_u, beta, d_dE, d_acc);
+    pdmk::DmkTree::replicas_mc_run(ts, m, d_i, d_d, d_u, beta, d_dE, d_acc, d_err);
     if (dE) PDMK_CUDA(cudaMemcpyAsync(dE, d_dE, sizeof(double) * tot, cudaMemcpyDeviceToHost, h0->stream));
     if (accepted) PDMK_CUDA(cudaMemcpyAsync(accepted, d_acc, sizeof(int) * tot, cudaMemcpyDeviceToHost, h0->stream));
+    PDMK_CUDA(cudaMemcpyAsync(errs.data(), d_err, sizeof(int) * n_trees, cudaMemcpyDeviceToHost, h0->stream));
     PDMK_CUDA(cudaFreeAsync(buf, h0->stream));
     PDMK_CUDA(cudaStreamSynchronize(h0->stream));
-    for (int t = 0; t < n_trees; ++t)
-      if (int e = ts[t]->check_device_error()) return device_fail(e);
+    for (int e : errs)
+      if (e) return device_fail(e);
     return ok();
   });
 }

@@ -337,10 +337,6 @@ __device__ inline int refined_rank(const DevTree& T, int level, uint64_t cell) {
   return T.wprefix_d[level][cell >> 5] + __popc(w & ((1u << (cell & 31)) - 1u));
 }
 
-// Grid: ncubes x slots blocks; block (slot, c) handles the tiles slot,
-// slot + slots, ... of cube c, so its set-up (the cube's cell lookup) is
-// paid once, and the cubes sharing a slot walk the same tiles together (the
-// cells two neighbouring cubes share meet in L2).
 // v exp(-2 pi i e / 3)
 __device__ __forceinline__ double2 rot3(double2 v, int e) {
   if (e == 0) return v;
@@ -348,10 +344,14 @@ __device__ __forceinline__ double2 rot3(double2 v, int e) {
   return make_double2(-0.5 * v.x - h * v.y, -0.5 * v.y + h * v.x);
 }
 
+// Block (slot, c) of slots x ncubes handles the tiles slot, slot + slots, ... of
+// cube c, so its set-up (the cube's cell lookup) is paid once, and the cubes
+// sharing a slot walk the same tiles together (the cells two neighbouring cubes
+// share meet in L2). part: the blocks' energy partials, or null; touched: only
+// cubes with a marked cell, or null.
 template <int NK>
-__global__ void __launch_bounds__(INC_T, 3) k_incoming_cube(DevTree T, const int* __restrict__ cubes, int ncubes,
-                                                             int slots, double* part,
-                                                             const int* __restrict__ touched) {
+__device__ __forceinline__ void incoming_cube(const DevTree& T, const int* __restrict__ cubes, int ncubes, int slots,
+                                              double* part, const int* __restrict__ touched) {
   constexpr int D = 2 * NK + 1, H = (NK + 1) * D * D;
   extern __shared__ double2 zs[];            // z sums [z][cy][cx][INC_KT]
   double2* own = zs + 4 * 36 * INC_KT;       // the receivers' own rows [receiver][INC_KT]
@@ -505,8 +505,27 @@ __global__ void __launch_bounds__(INC_T, 3) k_incoming_cube(DevTree T, const int
     }
     __syncthreads();
   }
+  if (!part) return;
   double s = block_sum(e, sm);
   if (tid == 0) part[blockIdx.x] = s;
+}
+
+template <int NK>
+__global__ void __launch_bounds__(INC_T, 3) k_incoming_cube(DevTree T, const int* __restrict__ cubes, int ncubes,
+                                                             int slots, double* part,
+                                                             const int* __restrict__ touched) {
+  incoming_cube<NK>(T, cubes, ncubes, slots, part, touched);
+}
+
+// the touched cubes of a set of trees
+template <int NK>
+__global__ void __launch_bounds__(INC_T, 3) k_incoming_cubes(const DevTree* __restrict__ trees,
+                                                              const SequenceRows* __restrict__ rows, int n) {
+  const int t = set_tree();
+  if (t >= n) return;
+  const SequenceRows r = rows[t];
+  if (int(blockIdx.x) >= r.slots * r.n_cubes || *r.n_list == 0) return;
+  incoming_cube<NK>(trees[t], r.cubes, r.n_cubes, r.slots, nullptr, r.touched);
 }
 
 template <int NK>
@@ -530,6 +549,13 @@ void launch_incoming(const DevTree& D, const int* cubes, int ncubes, int slots, 
     case 26: launch_incoming_nk<26>(D, cubes, ncubes, slots, part, touched, st); break;
     default: throw std::invalid_argument("incoming pass: unsupported mode count");
   }
+}
+
+template <int NK>
+void launch_incoming_set_nk(const DevTree* trees, const SequenceRows* rows, int n_trees, int blocks, cudaStream_t st) {
+  raise_smem_limit(reinterpret_cast<const void*>(k_incoming_cubes<NK>), INC_SMEM);
+  k_incoming_cubes<NK><<<set_grid(blocks, n_trees), INC_T, INC_SMEM, st>>>(trees, rows, n_trees);
+  PDMK_LAUNCH_CHECK();
 }
 
 // E_diff from the cube-tiled partials: sum over cubes C_l dscale_l
@@ -1329,6 +1355,18 @@ int DmkTree::inc_slots() const {
   const int kt = (dev_.H + INC_KT - 1) / INC_KT;
   const int nc = std::max(n_cubes_, 1);
   return std::max(1, std::min(kt, (tune_.inc_waves * 2 * 148 + nc - 1) / nc));
+}
+
+void launch_incoming_set(int n_diff, const DevTree* trees, const SequenceRows* rows, int n_trees, int blocks,
+                         cudaStream_t st) {
+  if (blocks == 0) return;
+  switch (n_diff) {
+    case 6: launch_incoming_set_nk<6>(trees, rows, n_trees, blocks, st); break;
+    case 12: launch_incoming_set_nk<12>(trees, rows, n_trees, blocks, st); break;
+    case 19: launch_incoming_set_nk<19>(trees, rows, n_trees, blocks, st); break;
+    case 26: launch_incoming_set_nk<26>(trees, rows, n_trees, blocks, st); break;
+    default: throw std::invalid_argument("incoming pass: unsupported mode count");
+  }
 }
 
 // The incoming rows next to outgoing rows that changed (touched[expansion

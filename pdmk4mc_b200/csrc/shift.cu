@@ -519,6 +519,8 @@ struct ModesOf {  // modes per half axis of the digits setting whose residual po
   static constexpr int CT = 3 * 4 * KS * 4;         // cosines of one unit
 };
 
+}  // namespace
+
 // an accepted move: point 0 its target (+), point 1 its origin (-); X the box
 // coordinates at level u, the deepest expansion level on the point's path
 struct Pending {
@@ -527,6 +529,8 @@ struct Pending {
   int X[2][3];
   int u[2];
 };
+
+namespace {
 
 __device__ inline void fill_pending(const DevTree& T, const Header& h, Pending& e) {
   const int ut = min(h.depth_t - 1, T.pw_hi), uo = min(h.depth_o - 1, T.pw_hi);
@@ -730,25 +734,24 @@ __device__ double diff_sum(const DevTree& tr, const Header& h, const Tables& oo,
 // phase tables go to shared memory (one sincos per entry, as build_tables),
 // then each thread adds them to its modes. FP64-bound: 10 operations per point
 // and mode.
-constexpr int FO_T = 256, FO_PTS = 8;
+constexpr int FO_T = 256, FO_PTS = 8, FO_PARTS = 8;
 
 template <int ND>
-__global__ void __launch_bounds__(FO_T) k_flush_outgoing(DevTree T, const Pending* __restrict__ list,
-                                                         const int* __restrict__ n_list, const int* __restrict__ touched,
-                                                         int parts2) {
+__device__ __forceinline__ void flush_row(const DevTree& T, const Pending* __restrict__ list,
+                                          const int* __restrict__ n_list, const int* __restrict__ touched) {
   constexpr int D = 2 * ND + 1, H = (ND + 1) * D * D, TAB = 3 * D;
   __shared__ double2 tab[FO_PTS][TAB];
   __shared__ int sel[FO_PTS];
   __shared__ int s_n, s_next;
-  // level-2 nodes in parts2 parts, the others whole
+  // level-2 nodes in FO_PARTS parts, the others whole
   const int n2 = T.level_start[3] - T.level_start[2];
   int node = T.pw_base, part = 0, parts = 1;
-  if (int(blockIdx.x) < n2 * parts2) {
-    node += blockIdx.x / parts2;
-    part = blockIdx.x % parts2;
-    parts = parts2;
+  if (int(blockIdx.x) < n2 * FO_PARTS) {
+    node += blockIdx.x / FO_PARTS;
+    part = blockIdx.x % FO_PARTS;
+    parts = FO_PARTS;
   } else {
-    node += n2 + int(blockIdx.x) - n2 * parts2;
+    node += n2 + int(blockIdx.x) - n2 * FO_PARTS;
   }
   if (touched[node - T.pw_base] == 0) return;
   const int l = T.node_level[node];
@@ -817,6 +820,46 @@ __global__ void __launch_bounds__(FO_T) k_flush_outgoing(DevTree T, const Pendin
       }
     __syncthreads();
   }
+}
+
+// blocks of a tree
+inline int flush_blocks(const DevTree& D) {
+  const int n_pw = D.pw_hi >= D.pw_lo ? D.level_start[D.pw_hi + 1] - D.pw_base : 0;
+  return n_pw > 0 ? n_pw + (FO_PARTS - 1) * (D.level_start[3] - D.level_start[2]) : 0;
+}
+
+template <int ND>
+__global__ void __launch_bounds__(FO_T) k_flush_outgoing(DevTree T, const Pending* __restrict__ list,
+                                                         const int* __restrict__ n_list,
+                                                         const int* __restrict__ touched) {
+  flush_row<ND>(T, list, n_list, touched);
+}
+
+// the rows of a set of trees
+template <int ND>
+__global__ void __launch_bounds__(FO_T) k_flush_set(const DevTree* __restrict__ trees, const SequenceRows* __restrict__ rows,
+                                                    int n) {
+  const int t = set_tree();
+  if (t >= n) return;
+  const SequenceRows r = rows[t];
+  const DevTree& T = trees[t];
+  if (r.n_pw == 0 || *r.n_list == 0 || int(blockIdx.x) >= r.n_pw + (FO_PARTS - 1) * (T.level_start[3] - T.level_start[2]))
+    return;
+  flush_row<ND>(T, r.list, r.n_list, r.touched);
+}
+
+// empties the lists of a set of trees
+__global__ void k_clear_set(const SequenceRows* __restrict__ rows, int n) {
+  const int t = set_tree();
+  if (t >= n) return;
+  const SequenceRows r = rows[t];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= r.n_pw; i += gridDim.x * blockDim.x) r.touched[i] = 0;
+}
+
+// the error words of a set of trees
+__global__ void k_errors_of_set(const DevTree* __restrict__ trees, int n, int* __restrict__ err) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) err[i] = *trees[i].err;
 }
 
 struct ShiftArgs {
@@ -2380,10 +2423,7 @@ struct RepArgs {
   double beta;
   double* dE_out;
   int* acc_out;
-  Pending* const* list; // per tree
-  int* const* n_list;
-  int* const* touched;
-  const double* const* oct;
+  const SequenceRows* rows;
 };
 
 template <int NP>
@@ -2413,9 +2453,10 @@ __global__ void __launch_bounds__(REP_T, 2) k_mc_rep(RepArgs a) {
   }
   const double dk0 = T.delta_k[0];
   const double c_window = dk0 * dk0 * dk0 / (8.0 * pi * pi * pi);
-  Pending* list = a.list[blockIdx.x];
-  int* touched = a.touched[blockIdx.x];
-  const double* oct = a.oct[blockIdx.x];
+  const SequenceRows rows = a.rows[blockIdx.x];
+  Pending* list = rows.list;
+  int* touched = rows.touched;
+  const double* oct = rows.oct;
   double* dyn = reinterpret_cast<double*>(sm2 + 2 * (3 * DW + max(T.max_depth - 1, 0) * 3 * D));
   if (MO::ND <= 19) {
     for (int i = threadIdx.x; i < MO::OCT; i += blockDim.x) dyn[i] = oct[i];
@@ -2516,7 +2557,7 @@ __global__ void __launch_bounds__(REP_T, 2) k_mc_rep(RepArgs a) {
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) *a.n_list[blockIdx.x] = n_acc;
+  if (threadIdx.x == 0) *rows.n_list = n_acc;
 }
 
 using McRepKernel = void (*)(RepArgs);
@@ -2572,14 +2613,26 @@ size_t rep_lazy_smem(int np) {
 
 // outgoing rows of the nodes the listed moves touched
 void launch_flush_outgoing(const DevTree& D, const Pending* list, const int* n_list, const int* touched, cudaStream_t st) {
-  const int n_pw = D.level_start[D.pw_hi + 1] - D.pw_base;
-  const int n2 = D.level_start[3] - D.level_start[2], parts2 = 8;
-  const unsigned grid = unsigned(n2 * parts2 + n_pw - n2);
+  const unsigned grid = unsigned(flush_blocks(D));
   switch (D.n_diff) {
-    case 6: k_flush_outgoing<6><<<grid, FO_T, 0, st>>>(D, list, n_list, touched, parts2); break;
-    case 12: k_flush_outgoing<12><<<grid, FO_T, 0, st>>>(D, list, n_list, touched, parts2); break;
-    case 19: k_flush_outgoing<19><<<grid, FO_T, 0, st>>>(D, list, n_list, touched, parts2); break;
-    case 26: k_flush_outgoing<26><<<grid, FO_T, 0, st>>>(D, list, n_list, touched, parts2); break;
+    case 6: k_flush_outgoing<6><<<grid, FO_T, 0, st>>>(D, list, n_list, touched); break;
+    case 12: k_flush_outgoing<12><<<grid, FO_T, 0, st>>>(D, list, n_list, touched); break;
+    case 19: k_flush_outgoing<19><<<grid, FO_T, 0, st>>>(D, list, n_list, touched); break;
+    case 26: k_flush_outgoing<26><<<grid, FO_T, 0, st>>>(D, list, n_list, touched); break;
+    default: throw std::invalid_argument("unsupported mode count");
+  }
+  PDMK_LAUNCH_CHECK();
+}
+
+// the same for a set of trees; blocks: the largest flush_blocks of one
+void launch_flush_set(int n_diff, const DevTree* trees, const SequenceRows* rows, int n_trees, int blocks, cudaStream_t st) {
+  if (blocks == 0) return;
+  const dim3 grid = set_grid(blocks, n_trees);
+  switch (n_diff) {
+    case 6: k_flush_set<6><<<grid, FO_T, 0, st>>>(trees, rows, n_trees); break;
+    case 12: k_flush_set<12><<<grid, FO_T, 0, st>>>(trees, rows, n_trees); break;
+    case 19: k_flush_set<19><<<grid, FO_T, 0, st>>>(trees, rows, n_trees); break;
+    case 26: k_flush_set<26><<<grid, FO_T, 0, st>>>(trees, rows, n_trees); break;
     default: throw std::invalid_argument("unsupported mode count");
   }
   PDMK_LAUNCH_CHECK();
@@ -3820,14 +3873,20 @@ void DmkTree::shift_batch_static(int m, const long* h_idx, const double* h_disp,
   PDMK_CUDA(cudaStreamSynchronize(st_));
 }
 
-// Metropolis sequences of many trees in one launch (k_mc_rep), ordered after
-// all their streams' earlier work on the first tree's stream.
+// Metropolis sequences of many trees (k_mc_rep), ordered after all their streams'
+// earlier work on the first tree's stream; d_err[i]: the trees' error words after
+// it, for the host to read with the results. Four launches per REP_CHUNK moves
+// serve the whole set (a clear, the moves, the outgoing and the incoming rows):
+// with a clear and two row launches for each tree, and its error word read by
+// itself, sets of many small trees paid more for these than for a short
+// sequence's moves.
 void DmkTree::replicas_mc_run(const std::vector<DmkTree*>& ts, int m, const int* d_idx, const double* d_disp,
-                              const double* d_u, double beta, double* d_dE, int* d_acc) {
+                              const double* d_u, double beta, double* d_dE, int* d_acc, int* d_err) {
   if (ts.empty() || m <= 0) return;
+  const size_t nt = ts.size();
   const int np = ts[0]->dev_.n_poly;
   size_t smem = 0;
-  bool deferred = true;
+  bool deferred = nt > 1;  // one tree has every SM to itself
   for (DmkTree* t : ts) {
     if (t->dev_.n_poly != np) throw std::invalid_argument("replicas must share the digits setting");
     t->ensure_packed();
@@ -3835,17 +3894,82 @@ void DmkTree::replicas_mc_run(const std::vector<DmkTree*>& ts, int m, const int*
     smem = std::max(smem, tables_smem(t->dev_, t->dev_.max_depth, 2));
     deferred = deferred && (t->inc_formed_ || t->dev_.pw_hi < t->dev_.pw_lo);
   }
+  const int chunk = std::min(m, REP_CHUNK);
+  std::vector<DevTree> trees(nt);
+  std::vector<SequenceRows> rows(nt);
+  int flush = 0, cubes = 0, inc = 0, n_pw_max = 0;
+  if (deferred) {
+    for (DmkTree* t : ts) {
+      t->ensure_pending(chunk);
+      if (t->dev_.pw_hi >= t->dev_.pw_lo) t->prepare_box_lists();
+      cubes += t->n_cubes_;
+    }
+    for (size_t i = 0; i < nt; ++i) {
+      DmkTree* t = ts[i];
+      const DevTree& D = t->dev_;
+      SequenceRows& r = rows[i];
+      r.list = static_cast<Pending*>(t->d_pending_);
+      r.n_list = t->d_n_list_;
+      r.touched = t->d_touched_;
+      r.oct = t->d_oct_;
+      r.n_pw = D.pw_hi >= D.pw_lo ? D.level_start[D.pw_hi + 1] - D.pw_base : 0;
+      r.cubes = t->d_cubes_;
+      r.n_cubes = r.n_pw > 0 ? t->n_cubes_ : 0;
+      // about 2^15 blocks for the set: more would pay their set-up for a few tiles
+      r.slots = std::min(t->inc_slots(), std::max(1, (1 << 15) / std::max(cubes, 1)));
+      flush = std::max(flush, flush_blocks(D));
+      inc = std::max(inc, r.slots * r.n_cubes);
+      n_pw_max = std::max(n_pw_max, r.n_pw);
+      trees[i] = D;
+    }
+  }
   cudaStream_t st = ts[0]->st_;
-  // Each tree's list is filled by its block of the launch on the first tree's
-  // stream and its rows are updated on its own stream; the trees' streams and
-  // the first one meet at events around each launch.
-  const size_t nt = ts.size();
   std::vector<cudaEvent_t> evs(nt);
   for (auto& e : evs) PDMK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  if (!deferred) {
+  if (deferred) {
+    for (size_t i = 1; i < nt; ++i) {
+      PDMK_CUDA(cudaEventRecord(evs[i], ts[i]->st_));
+      PDMK_CUDA(cudaStreamWaitEvent(st, evs[i], 0));
+    }
+    unsigned char* d_set = nullptr;
+    const size_t rows_at = (nt * sizeof(DevTree) + 15) & ~size_t(15);
+    PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d_set), rows_at + nt * sizeof(SequenceRows), st));
+    const DevTree* d_trees = reinterpret_cast<const DevTree*>(d_set);
+    const SequenceRows* d_rows = reinterpret_cast<const SequenceRows*>(d_set + rows_at);
+    PDMK_CUDA(cudaMemcpyAsync(d_set, trees.data(), nt * sizeof(DevTree), cudaMemcpyHostToDevice, st));
+    PDMK_CUDA(cudaMemcpyAsync(d_set + rows_at, rows.data(), nt * sizeof(SequenceRows), cudaMemcpyHostToDevice, st));
+    const McRepKernel kern = mc_rep_kernel(np);
+    smem += rep_lazy_smem(np);
+    raise_smem_limit(reinterpret_cast<const void*>(kern), smem);
+    RepArgs a{};
+    a.trees = d_trees;
+    a.m = m;
+    a.idx = d_idx;
+    a.disp = d_disp;
+    a.u = d_u;
+    a.beta = beta;
+    a.dE_out = d_dE;
+    a.acc_out = d_acc;
+    a.rows = d_rows;
+    const int n_diff = ts[0]->dev_.n_diff;
+    for (a.m0 = 0; a.m0 < m; a.m0 += chunk) {
+      a.cnt = std::min(chunk, m - a.m0);
+      k_clear_set<<<set_grid(std::min(n_pw_max / 1024 + 1, 64), int(nt)), 256, 0, st>>>(d_rows, int(nt));
+      PDMK_LAUNCH_CHECK();
+      kern<<<unsigned(nt), REP_T, smem, st>>>(a);
+      PDMK_LAUNCH_CHECK();
+      launch_flush_set(n_diff, d_trees, d_rows, int(nt), flush, st);
+      launch_incoming_set(n_diff, d_trees, d_rows, int(nt), inc, st);
+    }
+    k_errors_of_set<<<unsigned((nt + 127) / 128), 128, 0, st>>>(d_trees, int(nt), d_err);
+    PDMK_LAUNCH_CHECK();
+    PDMK_CUDA(cudaFreeAsync(d_set, st));
+    PDMK_CUDA(cudaEventRecord(evs[0], st));
+    for (size_t i = 1; i < nt; ++i) PDMK_CUDA(cudaStreamWaitEvent(ts[i]->st_, evs[0], 0));
+  } else {
     // Deferred updates recompute incoming rows from the outgoing ones, which is
     // what accepted moves do to them only where a pass formed them so. A set
-    // with a tree whose rows were not formed runs tree by tree, move by move.
+    // with a tree whose rows were not formed runs tree by tree.
     PDMK_CUDA(cudaEventRecord(evs[0], st));
     for (size_t i = 0; i < nt; ++i) {
       DmkTree* t = ts[i];
@@ -3853,69 +3977,13 @@ void DmkTree::replicas_mc_run(const std::vector<DmkTree*>& ts, int m, const int*
       const size_t c = i * size_t(m);
       t->mc_run_persistent(m, d_idx + c, d_disp + 3 * c, d_u + c, beta, d_dE ? d_dE + c : nullptr,
                            d_acc ? d_acc + c : nullptr);
+      PDMK_CUDA(cudaMemcpyAsync(d_err + i, t->dev_.err, sizeof(int), cudaMemcpyDeviceToDevice, t->st_));
       if (i > 0) {
         PDMK_CUDA(cudaEventRecord(evs[i], t->st_));
         PDMK_CUDA(cudaStreamWaitEvent(st, evs[i], 0));
       }
-      t->last_valid_ = false;
-      t->diff_cached_ = false;
-      t->mark_moved();
-    }
-    for (auto& e : evs) PDMK_CUDA(cudaEventDestroy(e));
-    return;
-  }
-  const int chunk = std::min(m, REP_CHUNK);
-  std::vector<unsigned char> blob(nt * (sizeof(DevTree) + 4 * sizeof(void*)));
-  DevTree* h_trees = reinterpret_cast<DevTree*>(blob.data());
-  void** h_ptr = reinterpret_cast<void**>(blob.data() + nt * sizeof(DevTree));
-  for (size_t i = 0; i < nt; ++i) {
-    DmkTree* t = ts[i];
-    const bool has_rows = t->dev_.pw_hi >= t->dev_.pw_lo;
-    t->ensure_pending(chunk);
-    if (has_rows) t->prepare_box_lists();
-    h_trees[i] = t->dev_;
-    h_ptr[i] = t->d_pending_;
-    h_ptr[nt + i] = t->d_n_list_;
-    h_ptr[2 * nt + i] = t->d_touched_;
-    h_ptr[3 * nt + i] = t->d_oct_;
-  }
-  unsigned char* d_blob = nullptr;
-  PDMK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d_blob), blob.size(), st));
-  PDMK_CUDA(cudaMemcpyAsync(d_blob, blob.data(), blob.size(), cudaMemcpyHostToDevice, st));
-  void** d_ptr = reinterpret_cast<void**>(d_blob + nt * sizeof(DevTree));
-  const McRepKernel kern = mc_rep_kernel(np);
-  smem += rep_lazy_smem(np);
-  raise_smem_limit(reinterpret_cast<const void*>(kern), smem);
-  RepArgs a{};
-  a.trees = reinterpret_cast<const DevTree*>(d_blob);
-  a.m = m;
-  a.idx = d_idx;
-  a.disp = d_disp;
-  a.u = d_u;
-  a.beta = beta;
-  a.dE_out = d_dE;
-  a.acc_out = d_acc;
-  a.list = reinterpret_cast<Pending* const*>(d_ptr);
-  a.n_list = reinterpret_cast<int* const*>(d_ptr + nt);
-  a.touched = reinterpret_cast<int* const*>(d_ptr + 2 * nt);
-  a.oct = reinterpret_cast<const double* const*>(d_ptr + 3 * nt);
-  for (a.m0 = 0; a.m0 < m; a.m0 += chunk) {
-    a.cnt = std::min(chunk, m - a.m0);
-    for (size_t i = 0; i < nt; ++i) {
-      ts[i]->clear_pending();
-      if (i == 0) continue;
-      PDMK_CUDA(cudaEventRecord(evs[i], ts[i]->st_));
-      PDMK_CUDA(cudaStreamWaitEvent(st, evs[i], 0));
-    }
-    kern<<<unsigned(nt), REP_T, smem, st>>>(a);
-    PDMK_LAUNCH_CHECK();
-    PDMK_CUDA(cudaEventRecord(evs[0], st));
-    for (size_t i = 0; i < nt; ++i) {
-      if (i > 0) PDMK_CUDA(cudaStreamWaitEvent(ts[i]->st_, evs[0], 0));
-      if (ts[i]->dev_.pw_hi >= ts[i]->dev_.pw_lo) ts[i]->flush_pending();
     }
   }
-  PDMK_CUDA(cudaFreeAsync(d_blob, st));
   for (auto& e : evs) PDMK_CUDA(cudaEventDestroy(e));  // released once the waits resolve
   for (DmkTree* t : ts) {
     t->last_valid_ = false;

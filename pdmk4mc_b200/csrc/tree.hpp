@@ -36,6 +36,31 @@ void return_host_slot(double* slot);
 
 struct PlanTotals;  // totals of the work and box lists (plan.hpp)
 
+struct Pending;  // an accepted move whose row updates are deferred (shift.cu)
+// A tree's deferred moves and what their row updates touch, in device memory for
+// the launches that serve a set of trees.
+struct SequenceRows {
+  Pending* list;
+  int* n_list;         // = touched + n_pw
+  int* touched;        // per expansion row
+  const double* oct;   // the folded difference table
+  const int* cubes;
+  int n_cubes, slots;  // the incoming pass's blocks: slots per cube
+  int n_pw, pad;
+};
+// a launch over a set: `blocks` for each tree, the trees along y and z
+inline dim3 set_grid(int blocks, int n_trees) {
+  const unsigned y = n_trees < 32768 ? unsigned(n_trees) : 32768u;
+  return dim3(unsigned(blocks), y, (unsigned(n_trees) + y - 1) / y);
+}
+__device__ inline int set_tree() { return int(blockIdx.y + gridDim.y * blockIdx.z); }
+
+struct DevTree;
+// the incoming rows of `n_trees` trees next to touched outgoing ones; blocks: the
+// largest slots x n_cubes of a tree (energy.cu)
+void launch_incoming_set(int n_diff, const DevTree* trees, const SequenceRows* rows, int n_trees, int blocks,
+                         cudaStream_t st);
+
 // One proposed single-particle move and what the shift kernel found for it.
 struct Proposal {
   int i_orig;
@@ -246,7 +271,7 @@ class DmkTree {
   // original particles d_idx[0..m) into d_phi[m] and d_field[3m] (may be null)
   void potential_batch(int m, const int* d_idx, double* d_phi, double* d_field);
   static void replicas_mc_run(const std::vector<DmkTree*>& trees, int m, const int* d_idx, const double* d_disp,
-                              const double* d_u, double beta, double* d_dE, int* d_acc);
+                              const double* d_u, double beta, double* d_dE, int* d_acc, int* d_err);
   int mc_mode() const { return mc_mode_; }
   // batched energy shifts of many candidates against the current state
   void shift_batch_device(int m, const int* d_idx, const double* d_disp, double* d_dE);
