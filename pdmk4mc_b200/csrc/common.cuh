@@ -131,6 +131,4 @@ __host__ __device__ inline double2 root6(int m) {
   }
 }
 
-__host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
-
 }  // namespace pdmk

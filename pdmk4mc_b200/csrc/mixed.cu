@@ -813,14 +813,14 @@ int mixed_table_bytes(int nk) {
   }
 }
 
-void make_coord_map(CUtensorMap* map, const double* sx, int slot_capacity, int kcp) {
-  if (slot_capacity % 2 != 0) throw std::logic_error("slot capacity must be even for the coordinate tensor map");
-  // the four slot arrays x, y, z, q lie back to back with stride slot_capacity
-  const cuuint64_t dims[2] = {cuuint64_t(slot_capacity), 4};
-  const cuuint64_t strides[1] = {cuuint64_t(slot_capacity) * sizeof(double)};
+void make_coord_map(CUtensorMap* map, const double* rows, int stride, int kcp) {
+  if (stride % 2 != 0) throw std::logic_error("row stride must be even for the coordinate tensor map");
+  // the four particle rows x, y, z, q lie back to back
+  const cuuint64_t dims[2] = {cuuint64_t(stride), 4};
+  const cuuint64_t strides[1] = {cuuint64_t(stride) * sizeof(double)};
   const cuuint32_t box[2] = {cuuint32_t(kcp + 2), 4};
   const cuuint32_t estr[2] = {1, 1};
-  CUresult r = encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<double*>(sx), dims, strides, box, estr,
+  CUresult r = encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<double*>(rows), dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw CudaError("cuTensorMapEncodeTiled failed: " + std::to_string(int(r)));

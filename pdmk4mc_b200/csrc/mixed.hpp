@@ -12,9 +12,9 @@ namespace pdmk {
 int mixed_chunk(int nk);
 // bytes of one chunk's table block (a multiple of 16)
 int mixed_table_bytes(int nk);
-// 2-D tensor map over the particle rows x, y, z, q (stride slot_capacity, which
-// must be even), in boxes of kcp + 2 particles
-void make_coord_map(CUtensorMap* map, const double* sx, int slot_capacity, int kcp);
+// 2-D tensor map over the particle rows x, y, z, q (back to back, of an even
+// stride), in boxes of kcp + 2 particles
+void make_coord_map(CUtensorMap* map, const double* rows, int stride, int kcp);
 // max |q| over n charges into *out (one block)
 void launch_absmax(const double* sq, int n, double* out, cudaStream_t st);
 // the mixed pass over device-resident lists: the table pass over nchunks

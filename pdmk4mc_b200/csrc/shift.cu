@@ -1755,7 +1755,7 @@ __device__ inline void packet_store(unsigned long long* p, double v, unsigned ep
                "l"(lo), "l"(hi)
                : "memory");
 }
-__device__ inline void packet_load(const unsigned long long* p, double& v, unsigned& epoch) {
+__device__ inline void packet_load(const unsigned long long* p, double& v, unsigned& epoch, unsigned& extra) {
   unsigned long long lo, hi;
   asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}\n"
                : "=l"(lo), "=l"(hi)
@@ -1763,19 +1763,16 @@ __device__ inline void packet_load(const unsigned long long* p, double& v, unsig
                : "memory");
   v = __longlong_as_double((long long)lo);
   epoch = unsigned(hi);
+  extra = unsigned(hi >> 32);
 }
 
-// The pool fill of a packet that has arrived, by the same load as an acquire: what
-// was released before the packet is visible after it. (A fence behind the relaxed
-// loads would order as much, for 800 cycles of every move.)
-__device__ inline unsigned packet_acquire(const unsigned long long* p) {
-  unsigned long long hi;
-  asm volatile(
-      "{\n .reg .b128 t;\n .reg .b64 sum;\n ld.acquire.gpu.global.b128 t, [%1];\n mov.b128 {sum, %0}, t;\n}\n"
-      : "=l"(hi)
-      : "l"(p)
-      : "memory");
-  return unsigned(hi >> 32);
+// The same load once more as an acquire, for a packet that has arrived (it reads the
+// same packet: the next one in its place waits for this block's own): what was
+// released before the packet is visible after it. A fence behind the relaxed loads
+// would order as much, for 800 cycles of every move; waiting for this load's value
+// would take 0.3 us of the 8 of a move at N = 1e5.
+__device__ inline void packet_acquire(const unsigned long long* p) {
+  asm volatile("{\n .reg .b128 t;\n ld.acquire.gpu.global.b128 t, [%0];\n}\n" ::"l"(p) : "memory");
 }
 
 // positions and charges of the particles a launch will move
@@ -2246,6 +2243,7 @@ __global__ void __launch_bounds__(MCL_T, 1) k_mc_long(const __grid_constant__ De
       bool ok = true;
       for (int b0 = 0; b0 < G; b0 += 32 * MCL_POLL) {
         double pv[MCL_POLL];
+        unsigned px[MCL_POLL];
         for (long long it = 0;; ++it) {
           bool all = true;
 #pragma unroll
@@ -2253,7 +2251,7 @@ __global__ void __launch_bounds__(MCL_T, 1) k_mc_long(const __grid_constant__ De
             const int b = b0 + lane + 32 * j;
             unsigned pe = epoch;
             pv[j] = 0.0;
-            if (b < G) packet_load(pk + 2 * b, pv[j], pe);
+            if (b < G) packet_load(pk + 2 * b, pv[j], pe, px[j]);
             all = all && pe == epoch;
           }
           if (all) break;
@@ -2267,7 +2265,10 @@ __global__ void __launch_bounds__(MCL_T, 1) k_mc_long(const __grid_constant__ De
           tot += pv[j];
           // the committing block's packet follows its fence: its commits so far
           // are visible from here on
-          if (b0 + lane + 32 * j == G / 2) s_pn = int(packet_acquire(pk + 2 * (G / 2)));
+          if (b0 + lane + 32 * j == G / 2) {
+            s_pn = int(px[j]);
+            packet_acquire(pk + 2 * (G / 2));
+          }
         }
       }
       if (!ok) atomicOr(T.err, 2);
@@ -2394,7 +2395,7 @@ __global__ void __launch_bounds__(MCL_T, 1) k_mc_long(const __grid_constant__ De
 }
 
 // ---------------------------------------------------------------------------
-// Replica sets: the Metropolis sequences of many independent trees in one
+// Replica sets: up to REP_CHUNK moves of many independent trees in one
 // launch, one thread block per tree (the block resolves, sums, decides,
 // updates and commits its tree's moves with block barriers only). Small
 // replicas do not need a whole GPU per move, so running them side by side
@@ -3423,12 +3424,10 @@ void DmkTree::build_mc_graph(int timed) {
 
 void DmkTree::launch_update(bool force) {
   DevTree& D = dev_;
-  const int levels = std::max(D.pw_hi - 1, 0);
   // rows: root, up to 2 x 28 receivers per expansion level, commit
   // x: one mode per thread; y: receiver ranges, enough for ~16 warps per SM
   const int gx = (std::max(D.H, D.Hw) + UPD_T - 1) / UPD_T;
   const int gy = std::max(1, std::min(8, (16 * (shift_grid_ - 3) * 32 / UPD_T + gx - 1) / std::max(gx, 1)));
-  (void)levels;
   const dim3 grid{unsigned(gx), unsigned(gy), 1u};
   time_begin(1);
   k_update<<<grid, UPD_T, 0, st_>>>(D, ptab_, ptab_per_, force,

@@ -62,10 +62,6 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const void* tmap, int x, 
       : "memory");
 }
 
-__device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
-  asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
-}
-
 // bulk copy global -> shared (16-byte aligned addresses, size a multiple of
 // 16); completion is signalled on the mbarrier as transaction bytes. No
 // multicast: the source may be any memory this GPU can address.

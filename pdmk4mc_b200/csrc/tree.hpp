@@ -261,15 +261,15 @@ class DmkTree {
   // sequential Metropolis over device-resident proposals; no host sync
   void mc_run_device(int n_moves, const int* d_idx, const double* d_disp, const double* d_u, double beta,
                      double* d_dE, int* d_acc);
-  // Metropolis sequence mode: 0 one persistent cooperative launch (default),
-  // 1 CUDA graphs of kGraphMoves (shift, update) launch pairs
+  // Metropolis sequence mode: 0 persistent cooperative launches (default), 1
+  // CUDA graphs of kGraphMoves (shift, update) launch pairs
   void set_mc_mode(int mode) { mc_mode_ = mode; }
-  // Metropolis sequences of m moves for each of many trees (same digits, same
-  // device) in one launch, one block per tree; arrays hold tree t's moves at
-  // [t m, (t + 1) m)
   // potential phi_i = sum_{j != i, images} q_j / r_ij and field -grad phi at
   // original particles d_idx[0..m) into d_phi[m] and d_field[3m] (may be null)
   void potential_batch(int m, const int* d_idx, double* d_phi, double* d_field);
+  // Metropolis sequences of m moves for each of many trees (same digits, same
+  // device), one block per tree; arrays hold tree t's moves at [t m, (t + 1) m);
+  // d_err: the trees' error words afterwards
   static void replicas_mc_run(const std::vector<DmkTree*>& trees, int m, const int* d_idx, const double* d_disp,
                               const double* d_u, double beta, double* d_dE, int* d_acc, int* d_err);
   int mc_mode() const { return mc_mode_; }

@@ -435,7 +435,7 @@ class HPDMKPtTree:
         return e.value, parts
 
     def set_mc_mode(self, mode):
-        """MC_PERSISTENT (one cooperative launch, default) or MC_GRAPH (graphs of launch pairs)."""
+        """MC_PERSISTENT (cooperative launches, default) or MC_GRAPH (graphs of launch pairs)."""
         _check(load_library().hpdmk_set_mc_mode(self._h, int(mode)))
 
     def get_timing(self, reset=False):
