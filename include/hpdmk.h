@@ -176,8 +176,9 @@ int hpdmk_mc_run(hpdmk_tree tree, int n, const long *i, const double *d, const d
                  int *accepted);
 
 /* Replica sets (no reference counterpart): the Metropolis sequences of
- * n_trees independent trees (same digits setting, same device) in one
- * launch, one thread block per tree. Tree t runs moves c = 0 .. m-1 taken
+ * n_trees independent trees (same digits setting, same device) at once,
+ * one thread block per tree and launch of up to 128 moves, after which the
+ * accepted moves' expansion rows are updated together. Tree t runs moves c = 0 .. m-1 taken
  * from i[t m + c], d[3 (t m + c) ..], u[t m + c]; outputs dE and accepted
  * (either may be NULL) in the same layout. Same results as hpdmk_mc_run on
  * each tree, to rounding. Host arrays. */
@@ -190,8 +191,10 @@ int hpdmk_replicas_mc_run(int n_trees, const hpdmk_tree *trees, int m, const lon
 int hpdmk_replicas_energy(int n_trees, const hpdmk_tree *trees, double *energy);
 
 /* How hpdmk_mc_run / hpdmk_mc_run_device execute the sequence (no reference
- * counterpart): HPDMK_MC_PERSISTENT (default) runs it as one cooperative
- * launch on every SM with grid barriers between the phases of a move;
+ * counterpart): HPDMK_MC_PERSISTENT (default) runs it as cooperative
+ * launches on every SM: long sequences 512 or 1024 moves at a time, whose
+ * accepted moves' expansion rows are updated together after each launch,
+ * short ones with the rows updated move by move between grid barriers;
  * HPDMK_MC_GRAPH runs CUDA graphs of 128 (shift, update) launch pairs.
  * Both give the same results to rounding. */
 #define HPDMK_MC_PERSISTENT 0

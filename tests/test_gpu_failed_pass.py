@@ -1,5 +1,7 @@
 """An outgoing pass that cannot get its memory raises and leaves box rows that read
 as zero, not as the memory's last contents; a later pass works."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -8,8 +10,19 @@ import pdmk4mc_b200 as P
 pytestmark = pytest.mark.gpu
 
 
+def empty_pool():
+    # what earlier trees left in the device's pool would serve the pass
+    import torch
+    torch.cuda.synchronize()
+    rt = ctypes.CDLL("libcudart.so.12")  # the one torch has loaded
+    pool = ctypes.c_void_p()
+    assert rt.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+    assert rt.cudaMemPoolTrimTo(pool, ctypes.c_size_t(0)) == 0
+
+
 def test_rows_stay_zero_when_a_pass_fails():
     import torch
+    empty_pool()
     n = 400000
     L = n ** (1 / 3)
     rng = np.random.default_rng(5)
