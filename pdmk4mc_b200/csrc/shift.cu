@@ -1051,7 +1051,7 @@ __global__ void __launch_bounds__(SH_T) k_shift(DevTree T, ShiftArgs a, const __
 constexpr int UPD_T = 128;
 constexpr int UPD_UNROLL = 8;
 
-__device__ void commit_move(const DevTree& T, const Proposal& P);
+__device__ bool commit_move(const DevTree& T, const Proposal& P);
 
 __global__ void __launch_bounds__(UPD_T) k_update(DevTree T, const double2* __restrict__ ptab, long ptab_per,
                                                   bool force, int* host_err) {
@@ -1071,7 +1071,7 @@ __global__ void __launch_bounds__(UPD_T) k_update(DevTree T, const double2* __re
     atomicAdd(&T.work[1], 32ull * ((unsigned long long)T.Hw + (unsigned long long)nr * T.H));
     if (force) T.prop->accepted = 1;
     commit_move(T, *T.prop);
-    if (host_err) *host_err = *T.err;
+    if (host_err) *host_err = ldm<true>(T.err);
   }
   __syncthreads();
   Tables tt, to;
@@ -1134,15 +1134,30 @@ __global__ void __launch_bounds__(UPD_T) k_update(DevTree T, const double2* __re
 // particle membership and position (exact on every level); one thread. The
 // independent loads are issued together and the per-level counts change by
 // atomic adds that need no reply, so the thread waits on few round trips.
-__device__ void commit_move(const DevTree& T, const Proposal& P) {
-  if (!P.accepted) return;
+//
+// False when the particle stays where it is: its arrival finds both the target
+// leaf and the overflow pool full, or (after such a move, by which the caller's
+// idea of its place may be wrong) its slot is not one of the leaf it is said to
+// leave. The error word then says so; slots, pool and counts stay as they were, so
+// whatever runs before the host reads it finds every particle in one place.
+__device__ bool commit_move(const DevTree& T, const Proposal& P) {
+  if (!P.accepted) return true;
   const int leafA = P.path_o[P.depth_o - 1];
   const int leafB = P.path_t[P.depth_t - 1];
   const int i = P.i_orig;
   const int s = P.slot;
   const double xt0 = P.xt[0], xt1 = P.xt[1], xt2 = P.xt[2], q = P.q;
+  const bool pooled = s >= T.n_slots;
+  const int cA = T.leaf_count[leafA], begA = T.node_begin[leafA];
+  const int cB = T.leaf_count[leafB], begB = T.node_begin[leafB], endB = T.node_end[leafB];
+  const int pn = *T.pool_n;
+  const bool there = pooled ? T.p_leaf[s - T.n_slots] == leafA && T.p_orig[s - T.n_slots] == i : s >= begA && s < begA + cA;
+  if (!there || (leafA != leafB && begB + cB >= endB && pn >= T.pool_cap)) {
+    atomicOr(T.err, 1);
+    return false;
+  }
   if (leafA == leafB) {
-    if (s < T.n_slots) {
+    if (!pooled) {
       T.sx[s] = xt0;
       T.sy[s] = xt1;
       T.sz[s] = xt2;
@@ -1152,13 +1167,10 @@ __device__ void commit_move(const DevTree& T, const Proposal& P) {
       T.py[p] = xt1;
       T.pz[p] = xt2;
     }
-    return;
+    return true;
   }
-  const int cA = T.leaf_count[leafA], begA = T.node_begin[leafA];
-  const int cB = T.leaf_count[leafB], begB = T.node_begin[leafB], endB = T.node_end[leafB];
-  const int pn = *T.pool_n;
   // remove from the origin leaf (swap with its last particle) or the pool
-  if (s < T.n_slots) {
+  if (!pooled) {
     const int last = begA + cA - 1;
     const int ol = T.s_orig[last];
     const double lx = T.sx[last], ly = T.sy[last], lz = T.sz[last], lq = T.sq[last];
@@ -1194,7 +1206,7 @@ __device__ void commit_move(const DevTree& T, const Proposal& P) {
     T.s_orig[slot] = i;
     T.orig_slot[i] = slot;
     T.leaf_count[leafB] = cB + 1;
-  } else if (pn < T.pool_cap) {
+  } else {
     T.px[pn] = xt0;
     T.py[pn] = xt1;
     T.pz[pn] = xt2;
@@ -1203,11 +1215,10 @@ __device__ void commit_move(const DevTree& T, const Proposal& P) {
     T.p_leaf[pn] = leafB;
     T.orig_slot[i] = T.n_slots + pn;
     *T.pool_n = pn + 1;
-  } else {
-    *T.err = 1;  // pool exhausted: the host repacks and reports
   }
   for (int l = 0; l < P.depth_o; ++l) atomicAdd(T.node_count + P.path_o[l], -1);
   for (int l = 0; l < P.depth_t; ++l) atomicAdd(T.node_count + P.path_t[l], 1);
+  return true;
 }
 
 
@@ -2379,11 +2390,10 @@ __global__ void __launch_bounds__(MCL_T, 1) k_mc_long(const __grid_constant__ De
     __syncthreads();
     // the commit runs beside the next move's sums
     if (accd && commits && warp == MCL_W - 2 && lane == 0) {
-      a.pos4[P.i_orig] = make_double4(P.xt[0], P.xt[1], P.xt[2], P.q);
       P.slot = __ldcg(T.orig_slot + P.i_orig);
       atomicAdd(&T.work[0], 1ull);
       atomicAdd(&T.work[1], 32ull * (unsigned long long)HW);
-      commit_move(T, P);
+      if (commit_move(T, P)) a.pos4[P.i_orig] = make_double4(P.xt[0], P.xt[1], P.xt[2], P.q);
       s_pool = int(*(volatile int*)T.pool_n);
       asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(a.committed), "r"(epoch) : "memory");
     }
