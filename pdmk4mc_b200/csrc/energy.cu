@@ -1272,7 +1272,6 @@ void DmkTree::form_outgoing_pw() {
   time_end(3);
   launch_reduce_chunks(part_b, box.split, t.n_split, t.n_split_items, D.H, st_);
   out_defined_ = true;
-  if (!out_formed_) inc_formed_ = false;  // incoming rows formed before are not of these
   out_formed_ = true;
   if (lists) fill_box_lists(t, d_blk);
   // the root pass's buffers are released after it joins the tree's stream
@@ -1378,7 +1377,9 @@ void DmkTree::launch_incoming_touched(const int* touched) {
 void DmkTree::form_incoming_pw() {
   run_incoming(true);
   diff_cached_ = true;
-  inc_formed_ = true;
+  // outgoing rows that no pass formed hold the accepted moves alone, and emptied
+  // boxes among them are not zero, as the recomputation takes them to be
+  inc_formed_ = out_formed_;
 }
 
 void DmkTree::launch_window_energy() {

@@ -71,6 +71,29 @@ def test_sequence_on_unformed_rows(formed, moves, digits):
         assert close(a[0], b[0])
 
 
+@pytest.mark.parametrize("digits", [3, 9])
+@pytest.mark.parametrize("formed", sorted(PASSES))
+def test_sequence_that_empties_boxes(formed, digits):
+    # a few particles on many boxes: a box left by its last particle keeps a row
+    n, l = 64, 4.0
+    rng = np.random.default_rng(5)
+    r, q = rng.uniform(0, l, 3 * n), np.where(np.arange(n) % 2 == 0, 1.0, -1.0)
+    prm = P.HPDMKParams(n_per_leaf=1, digits=digits, L=l, init=P.DIRECT)
+    idx, disp = rng.integers(0, n, 150), rng.uniform(-2.0, 2.0, (150, 3))
+    got = []
+    for mode in (P.MC_PERSISTENT, P.MC_GRAPH):
+        t = P.HPDMKPtTree(prm, r, q)
+        try:
+            for p in PASSES[formed]:
+                t.form_outgoing_pw() if p == "o" else t.form_incoming_pw()
+            t.set_mc_mode(mode)
+            got.append([t.mc_run(idx, disp, np.full(150, -1.0), 1.0)[0] for _ in range(3)] + [t.eval_energy_parts()])
+        finally:
+            t.close()
+    for a, b in zip(*got):
+        assert close(a, b)
+
+
 @pytest.mark.parametrize("sets", [["nothing"] * 2, ["outgoing", "formed"], ["incoming_first", "formed"], ["incoming"]])
 def test_replicas_with_unformed_rows(sets):
     # more moves than a replica lists, then a second call on the rows of the first
