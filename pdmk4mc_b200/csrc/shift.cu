@@ -2155,7 +2155,7 @@ __global__ void __launch_bounds__(MCL_T, 1) k_mc_long(const __grid_constant__ De
         const double dx = x[0] - (w.x + M.off[lo][0]), dy = x[1] - (w.y + M.off[lo][1]), dz = x[2] - (w.z + M.off[lo][2]);
         const double r2 = dx * dx + dy * dy + dz * dz;
         if (r2 > eps && r2 < b * b) {
-          const double r = w.w * poly.from_r2(r2, s_ibox[lv]);
+          const double r = w.w * poly.from_r2_as_above(r2, b, s_ibox[lv]);
           v += p == 0 ? r : -r;
         }
       }
@@ -2249,7 +2249,7 @@ __global__ void __launch_bounds__(MCL_T, 1) k_mc_long(const __grid_constant__ De
         dr2 = fmin(dr2, ax * ax + ay * ay + az * az);
       }
       for (int o = 16; o > 0; o >>= 1) dr2 = fmin(dr2, __shfl_xor_sync(0xffffffffu, dr2, o));
-      const double self = poly.from_r2(dr2, s_ibox[2]) * h.q * h.q;
+      const double self = dr2 > 0.0 ? poly.from_r2_as_above(dr2, s_box[2], s_ibox[2]) * h.q * h.q : 0.0;
       double tot = 0.0;
       bool ok = true;
       for (int b0 = 0; b0 < G; b0 += 32 * MCL_POLL) {

@@ -203,6 +203,12 @@ struct ResidualPoly {
     for (int i = 0; i < NP; ++i) v = fma(v, xs, c[i]);
     return v * ri;
   }
+  // from_r2 with the cut-off decided by the same roundings as above, so that pairs
+  // at the cut-off itself (lattices), where the kernel ends at the size of the
+  // method's error, count alike in every form of a move
+  __device__ double from_r2_as_above(double r2, double b, double inv_b) const {
+    return r2 > b * b * (1.0 - 1e-14) ? (*this)(sqrt(r2), b) : from_r2(r2, inv_b);
+  }
   // d/dr of the residual kernel, P'(x) (2 / b) / r - P(x) / r^2 with x = 2 r / b - 1
   __device__ double deriv(double r, double b) const {
     const double xs = (r / b - 0.5) * 2.0;
